@@ -336,6 +336,16 @@ typedef struct jpt_attn_params {
  * exp(logit - m); an empty row gives o = 0, m = -inf, l = 0.
  */
 int jpt_flash_decode(const jpt_attn_params* p, void* stream);
+/*
+ * The same for queries that are not contiguous, e.g. the [B,Hq,Tq,D] view of a
+ * [B,Tq,Hq,D] projection: q[b*q_b + h*q_h + t*q_t + d].  Only for the shapes of
+ * the prefill kernel (bf16 q / K / V, head_dim 128, an additive mask or none,
+ * more query rows per KV head than the decode kernels take); ..._ok says
+ * whether a call is one of them (1) or needs contiguous queries (0).  `o` is
+ * contiguous; the workspace is the one jpt_flash_decode_workspace_bytes asks for.
+ */
+int jpt_flash_attend_strided_q(const jpt_attn_params* p, int64_t q_b, int64_t q_h, int64_t q_t, void* stream);
+int jpt_flash_attend_strided_q_ok(const jpt_attn_params* p, int64_t q_b, int64_t q_h, int64_t q_t);
 size_t jpt_flash_decode_workspace_bytes(const jpt_attn_params* p);
 /*
  * Zero-fills a workspace (stream-ordered memset).  Call it once after

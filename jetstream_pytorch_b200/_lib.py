@@ -109,6 +109,8 @@ _SIGNATURES = {
     "jpt_silu_mul": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_size_t, c_void_p]),
     "jpt_quantize_tokens": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p]),
     "jpt_flash_decode": (c_int, [ctypes.POINTER(AttnParams), c_void_p]),
+    "jpt_flash_attend_strided_q": (c_int, [ctypes.POINTER(AttnParams), c_i64, c_i64, c_i64, c_void_p]),
+    "jpt_flash_attend_strided_q_ok": (c_int, [ctypes.POINTER(AttnParams), c_i64, c_i64, c_i64]),
     "jpt_flash_decode_static": (c_int, [ctypes.POINTER(AttnParams), c_void_p]),
     "jpt_decode_update_attend": (c_int, [ctypes.POINTER(AttnParams), ctypes.POINTER(NewTokenStruct), c_void_p]),
     "jpt_flash_decode_workspace_bytes": (c_size_t, [ctypes.POINTER(AttnParams)]),

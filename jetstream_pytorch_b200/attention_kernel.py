@@ -102,7 +102,10 @@ def _flash_decode(q, k, v, *, paged=False, page_table=None, page_size=0, k_scale
   workspace tensor is created or passed, the kernels use the scratch array
   built into the library (for callers that must not allocate at this point;
   shapes needing more than its 16 MiB raise ValueError)."""
-  q = q.contiguous()
+  # (a transposed view of a prompt's projection stays as it is where the prefill kernel takes its strides: see below)
+  strided = q.shape[2] > 1 and q.shape[3] == 128 and not q.is_contiguous() and q.stride(3) == 1
+  if not strided:
+    q = q.contiguous()
   b, hq, tq, d = q.shape
   dev = q.device
   if dev.index is not None and dev.index != torch.cuda.current_device():
@@ -162,7 +165,7 @@ def _flash_decode(q, k, v, *, paged=False, page_table=None, page_size=0, k_scale
                             or not t.is_contiguous()):
         raise ValueError("out[1], out[2] must be contiguous float32 tensors of B*Hq*Tq elements")
   else:
-    o = torch.empty_like(q)
+    o = torch.empty((b, hq, tq, d), dtype=q.dtype, device=dev)
     if want_ml:
       m = torch.empty((b, hq, tq), dtype=torch.float32, device=dev)
       l = torch.empty((b, hq, tq), dtype=torch.float32, device=dev)
@@ -172,6 +175,11 @@ def _flash_decode(q, k, v, *, paged=False, page_table=None, page_size=0, k_scale
   p.num_splits, p.force_generic = num_splits, int(force_generic)
   p.logit_rounding = int(logit_rounding)
   lib = _lib.lib()
+  if strided and (static_scratch or new_token is not None
+                  or not lib.jpt_flash_attend_strided_q_ok(ctypes.byref(p), q.stride(0), q.stride(1), q.stride(2))):
+    q, strided = q.contiguous(), False
+    p.q = _lib.ptr(q)
+    keep.append(q)
   if static_scratch:
     if new_token is not None:
       raise ValueError("the fused update needs a workspace that keeps its contents between calls")
@@ -181,7 +189,9 @@ def _flash_decode(q, k, v, *, paged=False, page_table=None, page_size=0, k_scale
     if need:
       ws = _workspace(dev, need)
       p.workspace, p.workspace_bytes = _lib.ptr(ws), ws.numel()
-    if new_token is not None:
+    if strided:
+      _lib.check(lib.jpt_flash_attend_strided_q(ctypes.byref(p), q.stride(0), q.stride(1), q.stride(2), _lib.stream()))
+    elif new_token is not None:
       _lib.check(lib.jpt_decode_update_attend(ctypes.byref(p), ctypes.byref(new_token), _lib.stream()))
     else:
       _lib.check(lib.jpt_flash_decode(ctypes.byref(p), _lib.stream()))

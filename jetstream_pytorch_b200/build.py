@@ -18,6 +18,7 @@ SOURCES = [
     "attention_generic.cu",
     "attention_mma.cu",
     "attention_umma.cu",
+    "attention_prefill.cu",
     "w8a16_linear.cu",
 ]
 

@@ -137,6 +137,10 @@ int launch_attention_mma(const jpt_attn_params& p, const AttnArgs& a, cudaStream
 // fits in attention_mma_workspace_bytes().
 bool attention_umma_eligible(const jpt_attn_params& p);
 int launch_attention_umma(const jpt_attn_params& p, const AttnArgs& a, cudaStream_t st, const NewTokenArgs* nt = nullptr);
+// Many query rows, bf16, head_dim 128, additive mask or none: the tcgen05 prefill kernel.  q strides in elements.
+bool attention_prefill_eligible(const jpt_attn_params& p, int64_t q_b, int64_t q_h, int64_t q_t);
+size_t attention_prefill_workspace_bytes(const jpt_attn_params& p);
+int launch_attention_prefill(const jpt_attn_params& p, const AttnArgs& a, int64_t q_b, int64_t q_h, int64_t q_t, cudaStream_t st);
 int launch_splitk_merge(const jpt_attn_params& p, const AttnArgs& a, cudaStream_t st);
 
 }  // namespace jpt

@@ -248,6 +248,12 @@ static int resolve_splits(const jpt_attn_params& p, int R) {
   return auto_splits_generic(p, R);
 }
 
+// The prefill kernel on contiguous queries (its strided form has an entry point of its own).
+static bool prefill_eligible(const jpt_attn_params& p) {
+  const int64_t q_h = (int64_t)p.Tq * p.D;
+  return p.force_generic == 0 && attention_prefill_eligible(p, q_h * p.Hq, q_h, p.D);
+}
+
 static int validate(const jpt_attn_params& p) {
   JPT_REQUIRE(p.q && p.k && p.v && p.o, JPT_EINVAL, "flash_decode: null tensor");
   JPT_REQUIRE(p.q_dtype == JPT_BF16 || p.q_dtype == JPT_F32, JPT_EINVAL, "flash_decode: q dtype must be bf16 or f32");
@@ -275,6 +281,7 @@ extern "C" size_t jpt_flash_decode_workspace_bytes(const jpt_attn_params* p) {
   if (!p || validate(*p) != 0) return 0;
   const int R = (p->Hq / p->Hkv) * p->Tq;
   if (p->force_generic != 1 && attention_mma_eligible(*p)) return attention_mma_workspace_bytes(*p);
+  if (prefill_eligible(*p)) return attention_prefill_workspace_bytes(*p);
   const int ns = resolve_splits(*p, R);
   if (ns <= 1) return 0;
   const size_t rows = (size_t)p->B * p->Hkv * R;
@@ -356,6 +363,11 @@ extern "C" int jpt_flash_decode(const jpt_attn_params* pp, void* stream) {
     if (p.force_generic != 2 && attention_umma_eligible(p)) return launch_attention_umma(p, a, st);
     return launch_attention_mma(p, a, st);
   }
+  if (prefill_eligible(p)) {
+    a.nsplit = 1;
+    const int64_t q_h = (int64_t)p.Tq * p.D;
+    return launch_attention_prefill(p, a, q_h * p.Hq, q_h, p.D, st);
+  }
   a.nsplit = resolve_splits(p, R);
   if (a.nsplit > 1) {
     const size_t rows = (size_t)p.B * p.Hkv * R;
@@ -371,6 +383,21 @@ extern "C" int jpt_flash_decode(const jpt_attn_params* pp, void* stream) {
   if (int rc = launch_attention_generic(p, a, st)) return rc;
   if (a.nsplit > 1) return launch_splitk_merge(p, a, st);
   return 0;
+}
+
+extern "C" int jpt_flash_attend_strided_q_ok(const jpt_attn_params* p, int64_t q_b, int64_t q_h, int64_t q_t) {
+  return p && validate(*p) == 0 && p->force_generic == 0 && !attention_mma_eligible(*p) && attention_prefill_eligible(*p, q_b, q_h, q_t);
+}
+
+extern "C" int jpt_flash_attend_strided_q(const jpt_attn_params* pp, int64_t q_b, int64_t q_h, int64_t q_t, void* stream) {
+  JPT_REQUIRE(pp, JPT_EINVAL, "flash_attend_strided_q: null params");
+  const jpt_attn_params& p = *pp;
+  if (int rc = validate(p)) return rc;
+  JPT_REQUIRE(jpt_flash_attend_strided_q_ok(pp, q_b, q_h, q_t), JPT_EINVAL,
+              "flash_attend_strided_q: this shape or these strides need contiguous queries (jpt_flash_decode)");
+  AttnArgs a = attn_args_of(p);
+  a.nsplit = 1;
+  return launch_attention_prefill(p, a, q_b, q_h, q_t, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int jpt_flash_decode_workspace_init(void* workspace, size_t bytes, void* stream) {

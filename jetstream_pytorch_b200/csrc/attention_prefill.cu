@@ -1,0 +1,755 @@
+// Prefill attention (many query rows per KV head, head_dim 128, bf16 q / K / V, an additive mask or none): tcgen05
+// with both contractions out of tensor memory and TMA.  Covers dense_attention and flash_attention
+// (jetstream_pt/attention_kernel.py:605-710) on the shapes of a prompt.
+//
+// Bound: compute (4 Hq D per score; the exponentials of the softmax cost about as much as the MMAs).
+//
+// Work item of a CTA: two tiles of 128 query rows of one KV head ("a" and "b": two grouped query heads at the same
+// token block where the model groups heads, two consecutive token blocks otherwise), so that a K/V tile read from L2
+// serves 256 rows and the tensor core works on one tile while the other one's 128 threads do their softmax.  Tiles are
+// made per query head through a tensor map with the caller's strides: a transposed view of the projection needs no copy.
+// Items with the most K/V tiles under a causal mask start first.
+//
+//   warps 0-3, 4-7  softmax of tile a / b: thread = query row = TMEM lane
+//   warp 8          thread 0 requests Q once and K, V tiles through two rings of two 32 KB slots
+//   warp 9          thread 0 issues the MMAs: S_t = Q_t K^T (shared x shared), O_t += P_t V (TMEM x shared)
+//
+// P lies over S in tensor memory (S: 128 fp32 columns; P: 64 columns of bf16 pairs for the leading part and 64 for
+// the rest p - bf16(p), so that the probabilities keep 16 bits; two MMAs per step).  S of the next K tile is issued
+// behind the PV product that reads P: the tensor core takes them in order.
+// The row maximum is raised lazily (when a tile's maximum is more than 2^8 above the reference in exp2 units): O
+// is rescaled in tensor memory only then, and m, l that go out are those of the true maximum.
+//
+// An additive mask is classified beforehand, one byte per [128 x 128] tile: all zero (no mask work), all -inf (tile
+// skipped), mixed (added value by value).  With up to kSmallK tiles per row every tile counts as mixed and that launch
+// (2 us and more) is saved.  Every wait is bounded; a CTA that gives up raises the workspace's status word.
+#include <cuda.h>
+#include <string.h>
+
+#include <atomic>
+#include <cmath>
+
+#include "attention_tiles.cuh"
+
+namespace jpt {
+namespace {
+
+constexpr int kDp = 128, kRowsP = 128, kKeysP = 128;
+constexpr int kThreadsP = 320;
+constexpr int kMaxKTiles = 512;  // K/V tiles of a row (65 536 tokens)
+constexpr int kSmallK = 3;
+constexpr uint32_t kTileBytes = 128 * 128 * 2;  // one bf16 tile: two halves of 64 dims, [128 x 128 B] each, swizzled
+constexpr long long kWaitCyclesP = 400000000ll;  // about a fifth of a second
+constexpr float kLog2e = 1.4426950408889634f;
+constexpr float kLazy = 8.f;  // P may reach 2^8 before O is rescaled
+
+enum : uint8_t { kClsZero = 0, kClsMixed = 1, kClsSkip = 2 };
+
+struct __align__(1024) SmemP {
+  uint8_t q[2][kTileBytes];
+  uint8_t k[2][kTileBytes];
+  uint8_t v[2][kTileBytes];
+  uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_ready[2], o_done;
+  uint32_t tmem_base;
+  int n_tiles;
+  volatile int dead;
+  float vs[2][kKeysP];             // scales of the K/V tile, per softmax group
+  float ks[2][kKeysP];
+  uint16_t list[kMaxKTiles];       // K/V tiles with work for a or b, in order
+  uint8_t cls[2][kMaxKTiles];      // class of the list's entry for tile a and b
+};
+
+struct PrefillMaps {
+  CUtensorMap q, k, v, o;
+};
+struct PrefillGeom {
+  const uint8_t* cls;  // null: every tile is mixed (additive mask) or zero (no mask)
+  int n_rows_t;        // row blocks of 128 per query head
+  int n_k;             // K/V tiles
+  int pairs;           // items per KV head
+  int cls_rows, cls_heads, cls_batch;  // extents of the class table (1 where the mask broadcasts)
+  int mask_vec;        // mask rows can be read 16 bytes at a time
+};
+
+__device__ __forceinline__ uint32_t smem_u32p(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void mbar_init_p(uint64_t* bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32p(bar)), "r"(count));
+}
+__device__ __forceinline__ bool mbar_probe_p(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+__device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, volatile int* dead) {
+  const long long t0 = clock64();
+  for (;;) {
+#pragma unroll 1
+    for (int i = 0; i < 16; ++i) {
+      if (mbar_probe_p(bar, parity)) return true;
+    }
+    if (*dead || clock64() - t0 > kWaitCyclesP) {
+      *dead = 1;
+      return false;
+    }
+  }
+}
+// Bounded wait for the phase with the given parity; false when it (or another warp of the CTA) gave up.
+__device__ __forceinline__ bool mbar_wait_p(uint64_t* b, uint32_t parity, SmemP& sm) {
+  const uint32_t bar = smem_u32p(b);
+  return mbar_probe_p(bar, parity) || mbar_wait_slow(bar, parity, &sm.dead);
+}
+__device__ __forceinline__ void mbar_arrive_p(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32p(bar)) : "memory");
+}
+__device__ __forceinline__ void mbar_expect_p(uint64_t* bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32p(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void commit_p(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32p(bar)) : "memory");
+}
+// one bf16 tile (two boxes of 64 dims x 128 rows)
+__device__ __forceinline__ void tma_tile(const void* dst, const CUtensorMap* map, int row, int h, int b, uint64_t* bar) {
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(
+            smem_u32p(dst) + half * (kTileBytes / 2)),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(half * 64), "r"(row), "r"(h), "r"(b), "r"(smem_u32p(bar))
+        : "memory");
+  }
+}
+// K-major operand, 128-byte swizzle: 8-row groups 1024 bytes apart
+__device__ __forceinline__ uint64_t desc_k_major(uint32_t addr) {
+  return (uint64_t)((addr >> 4) & 0x3FFF) | (uint64_t)(1024 >> 4) << 16 | (uint64_t)(1024 >> 4) << 32 | (uint64_t)1 << 46 |
+         (uint64_t)2 << 61;
+}
+// MN-major operand (V as [token][dim]): the 64-dim halves half a tile apart, 8-token groups 1024 bytes apart
+__device__ __forceinline__ uint64_t desc_mn_major(uint32_t addr) {
+  return (uint64_t)((addr >> 4) & 0x3FFF) | (uint64_t)((kTileBytes / 2) >> 4) << 16 | (uint64_t)(1024 >> 4) << 32 |
+         (uint64_t)1 << 46 | (uint64_t)2 << 61;
+}
+// D fp32, A and B bf16, M = 128, N = 128
+constexpr uint32_t kIdescQk = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
+constexpr uint32_t kIdescPv = kIdescQk | (1u << 16);  // B is MN-major
+
+__device__ __forceinline__ void mma_ss(uint32_t d, uint64_t ad, uint64_t bd, uint32_t acc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
+      "l"(ad), "l"(bd), "r"(kIdescQk), "r"(acc)
+      : "memory");
+}
+__device__ __forceinline__ void mma_ts(uint32_t d, uint32_t a, uint64_t bd, uint32_t acc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(d),
+      "r"(a), "l"(bd), "r"(kIdescPv), "r"(acc)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_ld32(uint32_t addr, uint32_t (&v)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+        "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
+        "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
+        "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+      : "r"(addr));
+}
+__device__ __forceinline__ void tmem_st32(uint32_t addr, const uint32_t (&v)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31};\n" ::"r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
+        "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]),
+        "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]),
+        "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31]),
+        "r"(addr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};\n" ::"r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
+        "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]),
+        "r"(addr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void fence_before_p() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void fence_after_p() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ float ex2p(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+  uint32_t r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+  return r;
+}
+__device__ __forceinline__ float lo_f32(uint32_t p) { return __uint_as_float(p << 16); }
+__device__ __forceinline__ float hi_f32(uint32_t p) { return __uint_as_float(p & 0xffff0000u); }
+__device__ __forceinline__ uint32_t mul2(uint32_t x, uint32_t y) {
+  uint32_t r;
+  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(x), "r"(y));
+  return r;
+}
+__device__ __forceinline__ uint32_t add2(uint32_t x, uint32_t y) {
+  uint32_t r;
+  asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(x), "r"(y));
+  return r;
+}
+__device__ __forceinline__ uint32_t max2(uint32_t x, uint32_t y) {
+  uint32_t r;
+  asm("max.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(x), "r"(y));
+  return r;
+}
+__device__ __forceinline__ void group_sync(int group) { asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory"); }
+// barrier of the group's 128 threads; whether `pred` holds in all of them
+__device__ __forceinline__ bool group_all(int group, bool pred) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %2, 0;\n\tbarrier.cta.red.and.pred q, %1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}\n"
+      : "=r"(r)
+      : "r"(1 + group), "r"((uint32_t)pred)
+      : "memory");
+  return r != 0;
+}
+
+// ---------------------------------------------------------------- mask classes
+// One CTA per [128 rows x 128 keys] tile of the mask: all zero, all -inf, or mixed.  Reads the mask once (the bound).
+__global__ void __launch_bounds__(256) mask_class_kernel(AttnArgs a, uint8_t* cls, int rows_per_head, int cls_heads, int vec) {
+  grid_dependency_trigger();
+  const int j = blockIdx.x, tb = blockIdx.y, r = blockIdx.z % cls_heads, b = blockIdx.z / cls_heads;
+  const int t0 = tb * kRowsP, s0 = j * kKeysP;
+  const int nr = min(kRowsP, rows_per_head - t0), nc = min(kKeysP, a.S - s0);
+  const uint16_t* m = static_cast<const uint16_t*>(a.mask) + (int64_t)b * a.mk_b + ((int64_t)r * rows_per_head + t0) * a.mk_r + s0;
+  bool zero = true, inf = true;
+  if (vec && nc == kKeysP) {
+    for (int i = threadIdx.x; i < nr * 16; i += 256) {
+      const uint4 w = __ldg(reinterpret_cast<const uint4*>(m + (int64_t)(i >> 4) * a.mk_r) + (i & 15));
+      const uint32_t x[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        zero = zero && (x[e] & 0x7fff7fffu) == 0u;
+        inf = inf && x[e] == 0xff80ff80u;
+      }
+    }
+  } else {
+    for (int i = threadIdx.x; i < nr * kKeysP; i += 256) {
+      const int c = i & (kKeysP - 1);
+      if (c < nc) {
+        const uint32_t x = m[(int64_t)(i >> 7) * a.mk_r + c];
+        zero = zero && (x & 0x7fffu) == 0u;
+        inf = inf && x == 0xff80u;
+      }
+    }
+  }
+  zero = __syncthreads_and(zero);
+  inf = __syncthreads_and(inf);
+  if (threadIdx.x == 0)
+    cls[(((int64_t)b * cls_heads + r) * gridDim.y + tb) * gridDim.x + j] = zero ? kClsZero : inf ? kClsSkip : kClsMixed;
+}
+
+// ---------------------------------------------------------------- the kernel
+// kRound: dense_attention's logit chain with a bf16 rounding after every step; kScale: per-token K and V scales.
+template <bool kRound, bool kScale>
+__global__ void __launch_bounds__(kThreadsP, 1)
+    prefill_attention_kernel(const __grid_constant__ PrefillMaps maps, const __grid_constant__ AttnArgs a,
+                             const __grid_constant__ PrefillGeom g, int* status) {
+  extern __shared__ __align__(1024) uint8_t smem_raw_p[];
+  SmemP& sm = *reinterpret_cast<SmemP*>(smem_raw_p);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if ((smem_u32p(smem_raw_p) & 1023u) != 0u) {  // (the swizzled tiles need it; the launch has no static shared memory)
+    if (tid == 0) atomicExch(status, 2);
+    return;
+  }
+  const int rep = a.Hq / a.Hkv;
+  const int heads = a.B * a.Hkv;
+  const int pair = g.pairs - 1 - (int)blockIdx.x / heads;  // (the last token blocks, with the most K/V tiles, first)
+  const int bh = (int)blockIdx.x % heads, b = bh / a.Hkv, hkv = bh % a.Hkv;
+  // the item's row tiles: query head and token block of a and b
+  int hq[2], tb[2];
+  bool have[2];
+#pragma unroll
+  for (int t = 0; t < 2; ++t) {
+    const int idx = 2 * pair + t;
+    have[t] = idx < g.n_rows_t * rep;
+    tb[t] = idx / rep;
+    hq[t] = hkv * rep + idx % rep;
+  }
+
+  if (tid == 256) {
+    mbar_init_p(&sm.q_full, 1);
+    mbar_init_p(&sm.o_done, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init_p(&sm.k_full[i], 1);
+      mbar_init_p(&sm.k_empty[i], 1);
+      mbar_init_p(&sm.v_full[i], 1);
+      mbar_init_p(&sm.v_empty[i], 1);
+      mbar_init_p(&sm.s_full[i], 1);
+      mbar_init_p(&sm.p_ready[i], 128);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    sm.dead = 0;
+  }
+  if (warp == 9) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32p(&sm.tmem_base)), "r"(512u)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    fence_before_p();
+  }
+  grid_dependency_wait();
+  grid_dependency_trigger();
+  // ---- the K/V tiles with work, in order (one warp)
+  if (warp == 0) {
+    int count = 0;
+    const uint8_t* row[2] = {nullptr, nullptr};
+    if (g.cls) {
+#pragma unroll
+      for (int t = 0; t < 2; ++t)
+        row[t] = g.cls + (((int64_t)(g.cls_batch > 1 ? b : 0) * g.cls_heads + (g.cls_heads > 1 ? hq[t] % rep : 0)) * g.cls_rows +
+                          (g.cls_rows > 1 ? tb[t] : 0)) * g.n_k;
+    }
+    for (int j0 = 0; j0 < g.n_k; j0 += 32) {
+      const int j = j0 + lane;
+      uint8_t c[2] = {kClsSkip, kClsSkip};
+      if (j < g.n_k) {
+#pragma unroll
+        for (int t = 0; t < 2; ++t)
+          if (have[t]) c[t] = g.cls ? row[t][j] : (a.mask_mode == JPT_MASK_ADD ? (uint8_t)kClsMixed : (uint8_t)kClsZero);
+      }
+      const bool use = c[0] != kClsSkip || c[1] != kClsSkip;
+      const unsigned votes = __ballot_sync(0xffffffffu, use);
+      if (use) {
+        const int at = count + __popc(votes & ((1u << lane) - 1u));
+        sm.list[at] = (uint16_t)j;
+        sm.cls[0][at] = c[0];
+        sm.cls[1][at] = c[1];
+      }
+      count += __popc(votes);
+    }
+    if (lane == 0) sm.n_tiles = count;
+  }
+  __syncthreads();
+  fence_after_p();
+  const uint32_t tmem = sm.tmem_base;
+  const int n = sm.n_tiles;
+
+  if (tid == 256 && n > 0) {
+    // ---- producer
+    mbar_expect_p(&sm.q_full, have[1] ? 2 * kTileBytes : kTileBytes);
+#pragma unroll
+    for (int t = 0; t < 2; ++t)
+      if (have[t]) tma_tile(sm.q[t], &maps.q, tb[t] * kRowsP, hq[t], b, &sm.q_full);
+    for (int i = 0; i < n; ++i) {
+      const int s = i & 1;
+      const uint32_t par = (uint32_t)((i >> 1) - 1) & 1u;
+      if (i >= 2 && !mbar_wait_p(&sm.k_empty[s], par, sm)) break;
+      mbar_expect_p(&sm.k_full[s], kTileBytes);
+      tma_tile(sm.k[s], &maps.k, sm.list[i] * kKeysP, hkv, b, &sm.k_full[s]);
+      if (i >= 2 && !mbar_wait_p(&sm.v_empty[s], par, sm)) break;
+      mbar_expect_p(&sm.v_full[s], kTileBytes);
+      tma_tile(sm.v[s], &maps.v, sm.list[i] * kKeysP, hkv, b, &sm.v_full[s]);
+    }
+    if (sm.dead) {  // (gave up: requests in flight get their time before the CTA leaves)
+      const long long t0 = clock64();
+      while (clock64() - t0 < 2000000) {
+      }
+    }
+  } else if (tid == 288 && n > 0) {
+    // ---- MMA issue
+    bool ok = mbar_wait_p(&sm.q_full, 0, sm);
+    uint32_t cnt[2] = {0, 0};  // products P V issued so far per tile
+    auto qk = [&](int t, int i) {
+      const uint32_t qa = smem_u32p(sm.q[t]), ka = smem_u32p(sm.k[i & 1]);
+#pragma unroll
+      for (int s = 0; s < 8; ++s) {
+        const uint32_t off = (uint32_t)((s >> 2) * (kTileBytes / 2) + (s & 3) * 32);
+        mma_ss(tmem + (uint32_t)(t * 256), desc_k_major(qa + off), desc_k_major(ka + off), s > 0);
+      }
+      commit_p(&sm.s_full[t]);
+    };
+    ok = ok && mbar_wait_p(&sm.k_full[0], 0, sm);
+    if (ok) {
+      fence_after_p();
+#pragma unroll
+      for (int t = 0; t < 2; ++t)
+        if (sm.cls[t][0] != kClsSkip) qk(t, 0);
+      commit_p(&sm.k_empty[0]);
+    }
+    for (int i = 0; i < n && ok; ++i) {
+      ok = mbar_wait_p(&sm.v_full[i & 1], (uint32_t)(i >> 1) & 1u, sm);
+      if (ok && i + 1 < n) ok = mbar_wait_p(&sm.k_full[(i + 1) & 1], (uint32_t)((i + 1) >> 1) & 1u, sm);
+      if (!ok) break;
+      fence_after_p();
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        if (ok && sm.cls[t][i] != kClsSkip) {
+          ok = mbar_wait_p(&sm.p_ready[t], cnt[t] & 1u, sm);
+          fence_after_p();
+          if (ok) {
+            const uint32_t p = tmem + (uint32_t)(t * 256), o = p + 128, va = smem_u32p(sm.v[i & 1]);
+#pragma unroll
+            for (int s = 0; s < 16; ++s)  // (the leading parts, then the rests)
+              mma_ts(o, p + (uint32_t)(8 * s), desc_mn_major(va + (uint32_t)((s & 7) * 2048)), (s > 0 || cnt[t] > 0) ? 1u : 0u);
+            ++cnt[t];
+          }
+        }
+        // S of the next tile goes over the P just read: the tensor core takes the two in order
+        if (ok && i + 1 < n && sm.cls[t][i + 1] != kClsSkip) qk(t, i + 1);
+      }
+      if (!ok) break;
+      if (i + 1 < n) commit_p(&sm.k_empty[(i + 1) & 1]);
+      commit_p(&sm.v_empty[i & 1]);
+    }
+    commit_p(&sm.o_done);
+  } else if (warp < 8) {
+    // ---- softmax of tile t, one query row per thread
+    const int t = warp >> 2, row_in = tid & 127;
+    const uint32_t tl = tmem + (uint32_t)(t * 256) + ((uint32_t)((warp & 3) * 32) << 16);
+    const int trow = (t ? tb[1] : tb[0]) * kRowsP + row_in;  // token of the row
+    const int my_hq = t ? hq[1] : hq[0];
+    const uint16_t* mrow = nullptr;
+    if (a.mask_mode == JPT_MASK_ADD)
+      mrow = static_cast<const uint16_t*>(a.mask) + (int64_t)b * a.mk_b +
+             ((int64_t)(my_hq % rep) * a.Tq + min(trow, a.Tq - 1)) * a.mk_r;
+    float m_ref = -INFINITY, m_true = -INFINITY, l = 0.f;
+    uint32_t cnt = 0;
+    bool ok = true;
+    for (int i = 0; i < n; ++i) {
+      const uint8_t c = sm.cls[t][i];
+      if (c == kClsSkip) continue;
+      const int s0 = sm.list[i] * kKeysP;
+      bool scaled = false;
+      if constexpr (kScale) {
+        const int p = s0 + row_in;
+        float ksv = 1.f, vsv = 1.f;
+        if (p < a.S) {
+          const int64_t idx = (int64_t)b * a.sc_b + (int64_t)p * a.sc_s;
+          ksv = load_scale(a.k_scale, idx, a.scale_is_f32);
+          vsv = load_scale(a.v_scale, idx, a.scale_is_f32);
+        }
+        group_sync(t);  // (everybody is done with the last tile's scales)
+        sm.ks[t][row_in] = ksv;
+        sm.vs[t][row_in] = vsv;
+        scaled = !group_all(t, ksv == 1.f && vsv == 1.f);  // (an unquantised prefill has unit scales)
+      }
+      // (after a wait that gave up the later ones return at once: the loop runs to its end, so that the group's
+      // barriers are met by all of its threads)
+      ok = mbar_wait_p(&sm.s_full[t], cnt & 1u, sm) && ok;
+      __syncwarp();
+      fence_after_p();
+      const int valid = min(kKeysP, a.S - s0);
+      // logits of the row: packed pairs of bf16 (kRound) or fp32
+      uint32_t lg[kRound ? 64 : 128];
+      float mt;
+      {
+        uint32_t mx = 0xff80ff80u;
+        float mxf = -INFINITY;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          uint32_t v[32];
+          tmem_ld32(tl + 32 * q, v);
+          uint32_t mk[16];
+          if (c == kClsMixed) {
+            if (g.mask_vec && valid == kKeysP) {
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const uint4 w = __ldg(reinterpret_cast<const uint4*>(mrow + s0 + 32 * q) + e);
+                mk[4 * e] = w.x, mk[4 * e + 1] = w.y, mk[4 * e + 2] = w.z, mk[4 * e + 3] = w.w;
+              }
+            } else {
+#pragma unroll
+              for (int e = 0; e < 16; ++e) {
+                const int p = 32 * q + 2 * e;
+                const uint32_t x0 = p < valid ? (uint32_t)__ldg(mrow + s0 + p) : 0xff80u;
+                const uint32_t x1 = p + 1 < valid ? (uint32_t)__ldg(mrow + s0 + p + 1) : 0xff80u;
+                mk[e] = x0 | (x1 << 16);
+              }
+            }
+          }
+          tmem_wait_ld();
+#pragma unroll
+          for (int e = 0; e < 16; ++e) {
+            const int p = 32 * q + 2 * e;
+            if constexpr (kRound) {
+              uint32_t x = pack_bf16(__uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1]));  // bf16(q . k)
+              x = pack_bf16(lo_f32(x) * a.sm_scale, hi_f32(x) * a.sm_scale);                      // bf16(. / sqrt(D))
+              if (kScale && scaled) x = pack_bf16(lo_f32(x) * sm.ks[t][p], hi_f32(x) * sm.ks[t][p + 1]);
+              if (c == kClsMixed) x = add2(x, mk[e]);
+              if (c != kClsMixed && valid < kKeysP) {
+                if (p >= valid) x = (x & 0xffff0000u) | 0xff80u;
+                if (p + 1 >= valid) x = (x & 0xffffu) | 0xff800000u;
+              }
+              mx = max2(mx, x);
+              lg[16 * q + e] = x;
+            } else {
+              float f0 = __uint_as_float(v[2 * e]) * a.sm_scale, f1 = __uint_as_float(v[2 * e + 1]) * a.sm_scale;
+              if (kScale && scaled) f0 *= sm.ks[t][p], f1 *= sm.ks[t][p + 1];
+              if (c == kClsMixed) f0 += lo_f32(mk[e]), f1 += hi_f32(mk[e]);
+              if (c != kClsMixed && valid < kKeysP) {
+                if (p >= valid) f0 = -INFINITY;
+                if (p + 1 >= valid) f1 = -INFINITY;
+              }
+              mxf = fmaxf(mxf, fmaxf(f0, f1));
+              lg[(32 * q + 2 * e) & (kRound ? 63 : 127)] = __float_as_uint(f0);
+              lg[(32 * q + 2 * e + 1) & (kRound ? 63 : 127)] = __float_as_uint(f1);
+            }
+          }
+        }
+        mt = kRound ? fmaxf(lo_f32(mx), hi_f32(mx)) : mxf;
+      }
+      m_true = fmaxf(m_true, mt);
+      // raise the reference maximum: on the first tile, later only where P would leave its range
+      float m_new = m_ref;
+      if (m_ref == -INFINITY || (mt - m_ref) * kLog2e > kLazy) m_new = fmaxf(m_ref, mt);
+      const bool raise = m_new > m_ref && cnt > 0;
+      if (__any_sync(0xffffffffu, raise)) {
+        // (S of this tile is there, so the products issued before it are complete: O is at rest)
+        const float f = raise ? ex2p((m_ref - m_new) * kLog2e) : 1.f;
+        l *= f;
+#pragma unroll 1
+        for (int q = 0; q < 4; ++q) {
+          uint32_t v[32];
+          tmem_ld32(tl + 128 + 32 * q, v);
+          tmem_wait_ld();
+#pragma unroll
+          for (int e = 0; e < 32; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) * f);
+          tmem_st32(tl + 128 + 32 * q, v);
+        }
+      }
+      m_ref = m_new;
+      const float off = m_ref == -INFINITY ? 0.f : m_ref * kLog2e;
+      float l0 = 0.f, l1 = 0.f;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        uint32_t hi[16], rest[16];
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+          float f0, f1;
+          if constexpr (kRound) {
+            f0 = lo_f32(lg[16 * q + e]), f1 = hi_f32(lg[16 * q + e]);
+          } else {
+            f0 = __uint_as_float(lg[(32 * q + 2 * e) & (kRound ? 63 : 127)]);
+            f1 = __uint_as_float(lg[(32 * q + 2 * e + 1) & (kRound ? 63 : 127)]);
+          }
+          f0 = ex2p(fmaf(f0, kLog2e, -off)), f1 = ex2p(fmaf(f1, kLog2e, -off));
+          l0 += f0, l1 += f1;
+          if (kScale && scaled) f0 *= sm.vs[t][32 * q + 2 * e], f1 *= sm.vs[t][32 * q + 2 * e + 1];
+          hi[e] = pack_bf16(f0, f1);
+          rest[e] = pack_bf16(f0 - lo_f32(hi[e]), f1 - hi_f32(hi[e]));
+        }
+        tmem_st16(tl + 16 * q, hi);
+        tmem_st16(tl + 64 + 16 * q, rest);
+      }
+      l += l0 + l1;
+      tmem_wait_st();
+      fence_before_p();
+      mbar_arrive_p(&sm.p_ready[t]);
+      ++cnt;
+    }
+    // ---- output rows
+    if (n > 0) ok = mbar_wait_p(&sm.o_done, 0, sm) && ok;
+    __syncwarp();
+    fence_after_p();
+    const float inv = l > 0.f && ok ? 1.f / l : 0.f;
+    const bool any = cnt > 0;
+#pragma unroll 1
+    for (int q = 0; q < 4; ++q) {
+      uint32_t v[32];
+      if (any) {
+        tmem_ld32(tl + 128 + 32 * q, v);
+        tmem_wait_ld();
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        uint32_t w[4];
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          const int i = 8 * e + 2 * x;
+          w[x] = inv > 0.f && any ? pack_bf16(__uint_as_float(v[i]) * inv, __uint_as_float(v[i + 1]) * inv) : 0u;
+        }
+        const int chunk = (q & 1) * 4 + e;  // 16-byte piece of the row's 128-byte half
+        *reinterpret_cast<uint4*>(sm.q[t] + (q >> 1) * (kTileBytes / 2) + row_in * 128 + ((chunk ^ (row_in & 7)) * 16)) =
+            make_uint4(w[0], w[1], w[2], w[3]);
+      }
+    }
+    const bool mine = t ? have[1] : have[0];
+    if (mine && trow < a.Tq && (a.m || a.l)) {
+      const int64_t at = ((int64_t)b * a.Hq + my_hq) * a.Tq + trow;
+      if (a.m) a.m[at] = m_true;
+      if (a.l) a.l[at] = l > 0.f ? l * ex2p((m_ref - m_true) * kLog2e) : 0.f;
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    group_sync(t);
+    if (row_in == 0 && mine) {
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3, %4}], [%5];" ::"l"(
+                         reinterpret_cast<uint64_t>(&maps.o)),
+                     "r"(half * 64), "r"(t ? tb[1] * kRowsP : tb[0] * kRowsP), "r"(my_hq), "r"(b),
+                     "r"(smem_u32p(sm.q[t]) + half * (kTileBytes / 2))
+                     : "memory");
+      }
+      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+      asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    }
+    fence_before_p();
+  }
+  __syncwarp();
+  __syncthreads();
+  if (tid == 0 && sm.dead) atomicExch(status, 1);
+  if (warp == 9) {
+    fence_after_p();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+  }
+}
+
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+// bf16 [batch][head][row][128] with strides in elements; boxes of 64 dims x 128 rows
+bool encode_heads(CUtensorMap* map, const void* base, int64_t rows, int64_t heads, int64_t batch, int64_t s_row, int64_t s_head,
+                  int64_t s_batch) {
+  static EncodeTiledFn fn = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      p = nullptr;
+    return reinterpret_cast<EncodeTiledFn>(p);
+  }();
+  if (!fn) return false;
+  // (the stride of an axis of one entry is never used, but has to be a legal one)
+  if (rows == 1) s_row = kDp;
+  if (heads == 1) s_head = s_row * rows;
+  if (batch == 1) s_batch = s_head * heads;
+  const cuuint64_t dims[4] = {(cuuint64_t)kDp, (cuuint64_t)rows, (cuuint64_t)heads, (cuuint64_t)batch};
+  const cuuint64_t str[3] = {(cuuint64_t)s_row * 2, (cuuint64_t)s_head * 2, (cuuint64_t)s_batch * 2};
+  const cuuint32_t box[4] = {64, (cuuint32_t)kRowsP, 1, 1};
+  const cuuint32_t estr[4] = {1, 1, 1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, str, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Whether the product with sm_scale rounds to the same bf16 values as the division by its reciprocal (the reference
+// divides by sqrt(D)): the quotient of a bf16 number depends on its 128 mantissas only.
+bool product_rounds_like_quotient(float sm_scale) {
+  static std::atomic<uint32_t> known_good{0};
+  uint32_t bits;
+  memcpy(&bits, &sm_scale, 4);
+  if (!(sm_scale > 0.f) || !std::isfinite(sm_scale)) return false;
+  if (known_good.load(std::memory_order_relaxed) == bits) return true;
+  auto bf16 = [](float x) {
+    uint32_t u;
+    memcpy(&u, &x, 4);
+    u += 0x7fffu + ((u >> 16) & 1u);
+    return u >> 16;
+  };
+  const float root = 1.f / sm_scale;
+  for (int m = 0; m < 128; ++m) {
+    const float x = 1.f + (float)m / 128.f;
+    const volatile float prod = x * sm_scale, quot = x / root;
+    if (bf16(prod) != bf16(quot)) return false;
+  }
+  known_good.store(bits, std::memory_order_relaxed);
+  return true;
+}
+
+struct ClassTable {
+  int rows, heads, batch, n_k;
+  size_t bytes() const { return (size_t)rows * heads * batch * n_k; }
+};
+ClassTable class_table(const jpt_attn_params& p) {
+  ClassTable t;
+  t.n_k = (p.S + kKeysP - 1) / kKeysP;
+  t.rows = p.mk_r ? (p.Tq + kRowsP - 1) / kRowsP : 1;
+  t.heads = p.mk_r ? p.Hq / p.Hkv : 1;
+  t.batch = p.mk_b ? p.B : 1;
+  return t;
+}
+bool wants_classes(const jpt_attn_params& p) { return p.mask_mode == JPT_MASK_ADD && (p.S + kKeysP - 1) / kKeysP > kSmallK; }
+
+}  // namespace
+
+bool attention_prefill_eligible(const jpt_attn_params& p, int64_t q_b, int64_t q_h, int64_t q_t) {
+  if (p.D != kDp || p.q_dtype != JPT_BF16 || p.kv_dtype != JPT_BF16 || p.paged) return false;
+  if (p.mask_mode != JPT_MASK_NONE && p.mask_mode != JPT_MASK_ADD) return false;
+  if (p.S > kMaxKTiles * kKeysP) return false;
+  if (!aligned(p.q, 16) || !aligned(p.k, 16) || !aligned(p.v, 16) || !aligned(p.o, 16)) return false;
+  // (tensor maps take positive strides of a multiple of 16 bytes)
+  auto legal = [](int64_t stride, int extent) { return extent == 1 || (stride > 0 && stride % 8 == 0 && stride < (1ll << 38)); };
+  if (!legal(p.kv_b, p.B) || !legal(p.kv_h, p.Hkv) || !legal(p.kv_s, p.S)) return false;
+  if (!legal(q_b, p.B) || !legal(q_h, p.Hq) || !legal(q_t, p.Tq)) return false;
+  if (p.logit_rounding != 0 && !product_rounds_like_quotient(p.sm_scale)) return false;
+  const double items = (double)p.B * p.Hkv * (((double)(p.Tq + kRowsP - 1) / kRowsP) * (p.Hq / p.Hkv) + 1);
+  return items < 1.0e9 && (double)p.B * (p.Hq / p.Hkv) < 65536 && p.Tq <= 65535 * kRowsP;
+}
+
+size_t attention_prefill_workspace_bytes(const jpt_attn_params& p) {
+  return kWorkspaceCounterBytes + (wants_classes(p) ? (class_table(p).bytes() + 255) / 256 * 256 : 0);
+}
+
+int launch_attention_prefill(const jpt_attn_params& p, const AttnArgs& a, int64_t q_b, int64_t q_h, int64_t q_t, cudaStream_t st) {
+  const size_t need = attention_prefill_workspace_bytes(p);
+  JPT_REQUIRE(p.workspace && p.workspace_bytes >= need, JPT_EWORKSPACE, "flash_decode: workspace of %zu bytes needed, %zu given",
+              need, p.workspace_bytes);
+  JPT_REQUIRE(aligned(p.workspace, 256), JPT_EALIGN, "flash_decode: workspace must be 256-byte aligned");
+  char* ws = static_cast<char*>(p.workspace);
+  int* status = reinterpret_cast<int*>(ws + kWorkspaceStatusOffset);
+  static std::atomic<bool> configured[kMaxDevices];
+  if (int rc = configure_once_per_device(configured, "prefill_attention_kernel", [] {
+        cudaError_t e = cudaSuccess;
+        auto set = [&e](auto kernel) {
+          if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemP));
+        };
+        set(prefill_attention_kernel<true, true>);
+        set(prefill_attention_kernel<true, false>);
+        set(prefill_attention_kernel<false, true>);
+        set(prefill_attention_kernel<false, false>);
+        return e;
+      }))
+    return rc;
+  PrefillMaps maps;
+  const int64_t o_h = (int64_t)p.Tq * kDp;
+  JPT_REQUIRE(encode_heads(&maps.q, p.q, p.Tq, p.Hq, p.B, q_t, q_h, q_b) &&
+                  encode_heads(&maps.k, p.k, p.S, p.Hkv, p.B, p.kv_s, p.kv_h, p.kv_b) &&
+                  encode_heads(&maps.v, p.v, p.S, p.Hkv, p.B, p.kv_s, p.kv_h, p.kv_b) &&
+                  encode_heads(&maps.o, p.o, p.Tq, p.Hq, p.B, kDp, o_h, o_h * p.Hq),
+              JPT_EINVAL, "flash_decode: the tensors cannot be described by a tensor map");
+  PrefillGeom g;
+  memset(&g, 0, sizeof(g));
+  const ClassTable t = class_table(p);
+  g.n_rows_t = (p.Tq + kRowsP - 1) / kRowsP;
+  g.n_k = t.n_k;
+  g.pairs = (g.n_rows_t * (p.Hq / p.Hkv) + 1) / 2;
+  g.mask_vec = p.mask_mode == JPT_MASK_ADD && aligned(p.mask, 16) && p.mk_b % 8 == 0 && p.mk_r % 8 == 0;
+  if (wants_classes(p)) {
+    uint8_t* cls = reinterpret_cast<uint8_t*>(ws + kWorkspaceCounterBytes);
+    g.cls = cls;
+    g.cls_rows = t.rows, g.cls_heads = t.heads, g.cls_batch = t.batch;
+    mask_class_kernel<<<dim3(t.n_k, t.rows, t.heads * t.batch), 256, 0, st>>>(a, cls, p.mk_r ? p.Tq : 1, t.heads, g.mask_vec);
+    if (int rc = check_launch("mask_class_kernel")) return rc;
+  }
+  const dim3 grid(g.pairs * p.B * p.Hkv), block(kThreadsP);
+  const size_t smem = sizeof(SmemP);
+  const bool scale = p.k_scale != nullptr;
+  if (a.round_logits) {
+    if (scale) launch_after_previous(prefill_attention_kernel<true, true>, grid, block, smem, st, maps, a, g, status);
+    else launch_after_previous(prefill_attention_kernel<true, false>, grid, block, smem, st, maps, a, g, status);
+  } else {
+    if (scale) launch_after_previous(prefill_attention_kernel<false, true>, grid, block, smem, st, maps, a, g, status);
+    else launch_after_previous(prefill_attention_kernel<false, false>, grid, block, smem, st, maps, a, g, status);
+  }
+  return check_launch("prefill_attention_kernel");
+}
+
+}  // namespace jpt
