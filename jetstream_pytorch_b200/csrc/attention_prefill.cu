@@ -6,16 +6,19 @@
 //
 // Work item of a CTA: two tiles of 128 query rows of one KV head ("a" and "b": two grouped query heads at the same
 // token block where the model groups heads, two consecutive token blocks otherwise), so that a K/V tile read from L2
-// serves 256 rows and the tensor core works on one tile while the other one's 128 threads do their softmax.  Tiles are
+// serves 256 rows and the tensor core works on one tile while the other one's 256 threads do their softmax.  Tiles are
 // made per query head through a tensor map with the caller's strides: a transposed view of the projection needs no copy.
 // Items with the most K/V tiles under a causal mask start first.
 //
-//   warps 0-3, 4-7  softmax of tile a / b: thread = query row = TMEM lane
-//   warp 8          thread 0 requests Q once and K, V tiles through two rings of two 32 KB slots
-//   warp 9          thread 0 issues the MMAs: S_t = Q_t K^T (shared x shared), O_t += P_t V (TMEM x shared)
+//   warps 0-7, 8-15 softmax of tile a / b: thread = query row (TMEM lane) and half of the 128 keys; the two halves
+//                   of a row exchange their maxima through shared memory, one barrier per K/V tile.  (One thread per
+//                   whole row left two warps per scheduler and the chain from S to P was the time: 38.6 us for
+//                   1024 tokens of 32 heads.)
+//   warp 16         thread 0 requests Q once and K, V tiles through two rings of two 32 KB slots
+//   warp 17         thread 0 issues the MMAs: S_t = Q_t K^T (shared x shared), O_t += P_t V (TMEM x shared)
 //
 // P lies over S in tensor memory (S: 128 fp32 columns; P: 64 columns of bf16 pairs for the leading part and 64 for
-// the rest p - bf16(p), so that the probabilities keep 16 bits; two MMAs per step).  S of the next K tile is issued
+// the rest, so that the probabilities keep 16 bits; two MMAs per step).  S of the next K tile is issued
 // behind the PV product that reads P: the tensor core takes them in order.
 // The row maximum is raised lazily (when a tile's maximum is more than 2^8 above the reference in exp2 units): O
 // is rescaled in tensor memory only then, and m, l that go out are those of the true maximum.
@@ -35,7 +38,8 @@ namespace jpt {
 namespace {
 
 constexpr int kDp = 128, kRowsP = 128, kKeysP = 128;
-constexpr int kThreadsP = 320;
+constexpr int kThreadsP = 576, kGroup = 256;  // threads in all, threads of a row tile
+constexpr int kProducerP = 512, kIssuerP = 544;  // the threads that request tiles and issue MMAs
 constexpr int kMaxKTiles = 512;  // K/V tiles of a row (65 536 tokens)
 constexpr int kSmallK = 3;
 constexpr uint32_t kTileBytes = 128 * 128 * 2;  // one bf16 tile: two halves of 64 dims, [128 x 128 B] each, swizzled
@@ -53,8 +57,9 @@ struct __align__(1024) SmemP {
   uint32_t tmem_base;
   int n_tiles;
   volatile int dead;
-  float vs[2][kKeysP];             // scales of the K/V tile, per softmax group
-  float ks[2][kKeysP];
+  float vs[2][2][kKeysP];          // scales of the K/V tile, per row tile and parity of the K/V tile
+  float ks[2][2][kKeysP];
+  float half_max[2][2][2][kRowsP]; // [row tile][parity][half][row]
   uint16_t list[kMaxKTiles];       // K/V tiles with work for a or b, in order
   uint8_t cls[2][kMaxKTiles];      // class of the list's entry for tile a and b
 };
@@ -68,7 +73,7 @@ struct PrefillGeom {
   int n_k;             // K/V tiles
   int pairs;           // items per KV head
   int cls_rows, cls_heads, cls_batch;  // extents of the class table (1 where the mask broadcasts)
-  int mask_vec;        // mask rows can be read 16 bytes at a time
+  int mask_vec, mask_pairs;  // mask rows can be read 16, 4 bytes at a time
 };
 
 __device__ __forceinline__ uint32_t smem_u32p(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -78,9 +83,9 @@ __device__ __forceinline__ void mbar_init_p(uint64_t* bar, uint32_t count) {
 __device__ __forceinline__ bool mbar_probe_p(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
-      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}\n"
+      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.b32 %0, 1, 0, p;\n\t}\n"
       : "=r"(ok)
-      : "r"(bar), "r"(parity)
+      : "r"(bar), "r"(parity), "r"(20000u)  // (may sleep for up to 20 us)
       : "memory");
   return ok != 0;
 }
@@ -122,32 +127,34 @@ __device__ __forceinline__ void tma_tile(const void* dst, const CUtensorMap* map
         : "memory");
   }
 }
-// K-major operand, 128-byte swizzle: 8-row groups 1024 bytes apart
-__device__ __forceinline__ uint64_t desc_k_major(uint32_t addr) {
-  return (uint64_t)((addr >> 4) & 0x3FFF) | (uint64_t)(1024 >> 4) << 16 | (uint64_t)(1024 >> 4) << 32 | (uint64_t)1 << 46 |
-         (uint64_t)2 << 61;
+// Shared-memory descriptors: the low word carries the start address (16-byte units) and the leading byte offset, the
+// high word the stride of 1024 bytes between 8-row groups, the version and the 128-byte swizzle.  K-major operands (Q, K)
+// do not use the leading offset; V as [token][dim] is MN-major, its 64-dim halves lie half a tile apart.
+__device__ __forceinline__ uint32_t desc_lo(uint32_t addr) {
+  return ((addr >> 4) & 0x3FFF) | (uint32_t)((kTileBytes / 2) >> 4) << 16;
 }
-// MN-major operand (V as [token][dim]): the 64-dim halves half a tile apart, 8-token groups 1024 bytes apart
-__device__ __forceinline__ uint64_t desc_mn_major(uint32_t addr) {
-  return (uint64_t)((addr >> 4) & 0x3FFF) | (uint64_t)((kTileBytes / 2) >> 4) << 16 | (uint64_t)(1024 >> 4) << 32 |
-         (uint64_t)1 << 46 | (uint64_t)2 << 61;
+constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ bool elect_one() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(r));
+  return r != 0;
 }
 // D fp32, A and B bf16, M = 128, N = 128
 constexpr uint32_t kIdescQk = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
 constexpr uint32_t kIdescPv = kIdescQk | (1u << 16);  // B is MN-major
 
-__device__ __forceinline__ void mma_ss(uint32_t d, uint64_t ad, uint64_t bd, uint32_t acc) {
+__device__ __forceinline__ void mma_ss(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t acc) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
-      "l"(ad), "l"(bd), "r"(kIdescQk), "r"(acc)
+      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %5, 0;\n\tmov.b64 da, {%1, %3};\n\tmov.b64 db, {%2, %3};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t}\n" ::"r"(d),
+      "r"(a_lo), "r"(b_lo), "r"(kDescHi), "r"(kIdescQk), "r"(acc)
       : "memory");
 }
-__device__ __forceinline__ void mma_ts(uint32_t d, uint32_t a, uint64_t bd, uint32_t acc) {
+__device__ __forceinline__ void mma_ts(uint32_t d, uint32_t a, uint32_t b_lo, uint32_t acc) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(d),
-      "r"(a), "l"(bd), "r"(kIdescPv), "r"(acc)
+      "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\tsetp.ne.b32 p, %5, 0;\n\tmov.b64 db, {%2, %3};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}\n" ::"r"(d),
+      "r"(a), "r"(b_lo), "r"(kDescHi), "r"(kIdescPv), "r"(acc)
       : "memory");
 }
 __device__ __forceinline__ void tmem_ld32(uint32_t addr, uint32_t (&v)[32]) {
@@ -211,12 +218,36 @@ __device__ __forceinline__ uint32_t max2(uint32_t x, uint32_t y) {
   asm("max.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(x), "r"(y));
   return r;
 }
-__device__ __forceinline__ void group_sync(int group) { asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory"); }
-// barrier of the group's 128 threads; whether `pred` holds in all of them
+// two fp32 values in one 64-bit register, and the packed arithmetic on them
+__device__ __forceinline__ uint64_t pack_f32(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack_f32(uint64_t x, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(x));
+}
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t x, uint64_t y) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(y));
+  return r;
+}
+__device__ __forceinline__ uint64_t add_f32x2(uint64_t x, uint64_t y) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(y));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t x, uint64_t y, uint64_t z) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(x), "l"(y), "l"(z));
+  return r;
+}
+__device__ __forceinline__ void group_sync(int group) { asm volatile("bar.sync %0, 256;" ::"r"(1 + group) : "memory"); }
+// barrier of the group's 256 threads; whether `pred` holds in all of them
 __device__ __forceinline__ bool group_all(int group, bool pred) {
   uint32_t r;
   asm volatile(
-      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %2, 0;\n\tbarrier.cta.red.and.pred q, %1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}\n"
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %2, 0;\n\tbarrier.cta.red.and.pred q, %1, 256, p;\n\tselp.u32 %0, 1, 0, q;\n\t}\n"
       : "=r"(r)
       : "r"(1 + group), "r"((uint32_t)pred)
       : "memory");
@@ -258,6 +289,97 @@ __global__ void __launch_bounds__(256) mask_class_kernel(AttnArgs a, uint8_t* cl
     cls[(((int64_t)b * cls_heads + r) * gridDim.y + tb) * gridDim.x + j] = zero ? kClsZero : inf ? kClsSkip : kClsMixed;
 }
 
+// The products of one row (TMEM lane) with 64 keys turned into final logits in place, as fp32: scaled, rounded where the
+// reference rounds, the mask row added; keys from `valid` on get -inf.  ks: the tile's K scales, read when `scaled`.
+template <bool kRound, bool kScale>
+__device__ __noinline__ void final_logits(uint32_t tl, const AttnArgs& a, const float* ks, bool scaled, const uint16_t* mask,
+                                          int valid, bool mask_vec) {
+  const float mul = a.sm_scale;
+#pragma unroll 1
+  for (int q = 0; q < 2; ++q) {
+    uint32_t v[32], mk[16];
+    tmem_ld32(tl + 32 * q, v);
+    if (mask && mask_vec && valid >= kKeysP / 2) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const uint4 w = __ldg(reinterpret_cast<const uint4*>(mask + 32 * q) + e);
+        mk[4 * e] = w.x, mk[4 * e + 1] = w.y, mk[4 * e + 2] = w.z, mk[4 * e + 3] = w.w;
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < 16; ++e) {
+        const int p = 32 * q + 2 * e;
+        const uint32_t x0 = p >= valid ? 0xff80u : mask ? (uint32_t)__ldg(mask + p) : 0u;
+        const uint32_t x1 = p + 1 >= valid ? 0xff80u : mask ? (uint32_t)__ldg(mask + p + 1) : 0u;
+        mk[e] = x0 | (x1 << 16);
+      }
+    }
+    tmem_wait_ld();
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+      const float k0 = kScale && scaled ? ks[32 * q + 2 * e] : 1.f, k1 = kScale && scaled ? ks[32 * q + 2 * e + 1] : 1.f;
+      if constexpr (kRound) {
+        uint32_t x = pack_bf16(__uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1]));
+        x = pack_bf16(lo_f32(x) * mul, hi_f32(x) * mul);
+        if (kScale) x = pack_bf16(lo_f32(x) * k0, hi_f32(x) * k1);
+        x = add2(x, mk[e]);
+        v[2 * e] = __float_as_uint(lo_f32(x)), v[2 * e + 1] = __float_as_uint(hi_f32(x));
+      } else {
+        v[2 * e] = __float_as_uint(fmaf(__uint_as_float(v[2 * e]) * mul, k0, lo_f32(mk[e])));
+        v[2 * e + 1] = __float_as_uint(fmaf(__uint_as_float(v[2 * e + 1]) * mul, k1, hi_f32(mk[e])));
+      }
+    }
+    tmem_st32(tl + 32 * q, v);
+  }
+  tmem_wait_st();
+}
+
+// Bits of the keys a row must not see among its 64: lane r of the warp gets row r's (lo: keys 2 e at bit e, hi: keys
+// 2 e + 1).  The warp reads one row after the other, 128 bytes at a time.  `warp_mask`: the warp's first row at the
+// thread half's first key, null without a mask; rows and keys beyond `rows`, `valid` are not read.  False when the mask
+// holds anything but 0 and -inf.
+// The result: {lo, hi, 1 if so, 0}.
+__device__ __noinline__ uint4 masked_bits(const uint16_t* warp_mask, int64_t mk_r, int rows, int valid, bool pairs) {
+  const int lane = threadIdx.x & 31;
+  const bool in0 = 2 * lane < valid, in1 = 2 * lane + 1 < valid;
+  const uint32_t out_lo = __ballot_sync(0xffffffffu, !in0), out_hi = __ballot_sync(0xffffffffu, !in1);
+  uint32_t lo = out_lo, hi = out_hi;
+  bool odd = false;
+  auto fold = [&](uint32_t x, int r) {
+    const bool inf0 = (x & 0xffffu) == 0xff80u, inf1 = (x >> 16) == 0xff80u;
+    odd = odd || !(inf0 || (x & 0x7fffu) == 0u) || !(inf1 || (x & 0x7fff0000u) == 0u);
+    const uint32_t b0 = __ballot_sync(0xffffffffu, inf0), b1 = __ballot_sync(0xffffffffu, inf1);
+    if (lane == r) lo = out_lo | b0, hi = out_hi | b1;
+  };
+  if (warp_mask && pairs && valid >= kKeysP / 2 && rows >= 32) {
+    // (eight rows in flight, in a short loop: this code runs once per item, and fetching its instructions is most of
+    // its time; one row after the other cost 17 000 cycles a tile)
+#pragma unroll 1
+    for (int r0 = 0; r0 < 32; r0 += 8) {
+      uint32_t x[8];
+#pragma unroll
+      for (int r = 0; r < 8; ++r) x[r] = __ldg(reinterpret_cast<const uint32_t*>(warp_mask + (int64_t)(r0 + r) * mk_r) + lane);
+#pragma unroll
+      for (int r = 0; r < 8; ++r) fold(x[r], r0 + r);
+    }
+  } else if (warp_mask) {
+#pragma unroll 1
+    for (int r0 = 0; r0 < 32 && r0 < rows; r0 += 8) {
+      uint32_t x[8];
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        const uint16_t* p = warp_mask + (int64_t)(r0 + r) * mk_r + 2 * lane;
+        const bool row = r0 + r < rows;
+        const uint32_t x0 = row && in0 ? (uint32_t)__ldg(p) : 0u, x1 = row && in1 ? (uint32_t)__ldg(p + 1) : 0u;
+        x[r] = x0 | (x1 << 16);
+      }
+#pragma unroll
+      for (int r = 0; r < 8; ++r) fold(x[r], r0 + r);
+    }
+  }
+  return make_uint4(lo, hi, __any_sync(0xffffffffu, odd) ? 0u : 1u, 0u);
+}
+
 // ---------------------------------------------------------------- the kernel
 // kRound: dense_attention's logit chain with a bf16 rounding after every step; kScale: per-token K and V scales.
 template <bool kRound, bool kScale>
@@ -286,7 +408,7 @@ __global__ void __launch_bounds__(kThreadsP, 1)
     hq[t] = hkv * rep + idx % rep;
   }
 
-  if (tid == 256) {
+  if (tid == kProducerP) {
     mbar_init_p(&sm.q_full, 1);
     mbar_init_p(&sm.o_done, 1);
     for (int i = 0; i < 2; ++i) {
@@ -295,12 +417,12 @@ __global__ void __launch_bounds__(kThreadsP, 1)
       mbar_init_p(&sm.v_full[i], 1);
       mbar_init_p(&sm.v_empty[i], 1);
       mbar_init_p(&sm.s_full[i], 1);
-      mbar_init_p(&sm.p_ready[i], 128);
+      mbar_init_p(&sm.p_ready[i], kGroup);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     sm.dead = 0;
   }
-  if (warp == 9) {
+  if (warp == kIssuerP / 32) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32p(&sm.tmem_base)), "r"(512u)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -343,7 +465,7 @@ __global__ void __launch_bounds__(kThreadsP, 1)
   const uint32_t tmem = sm.tmem_base;
   const int n = sm.n_tiles;
 
-  if (tid == 256 && n > 0) {
+  if (tid == kProducerP && n > 0) {
     // ---- producer
     mbar_expect_p(&sm.q_full, have[1] ? 2 * kTileBytes : kTileBytes);
 #pragma unroll
@@ -364,42 +486,51 @@ __global__ void __launch_bounds__(kThreadsP, 1)
       while (clock64() - t0 < 2000000) {
       }
     }
-  } else if (tid == 288 && n > 0) {
-    // ---- MMA issue
+  } else if (warp == kIssuerP / 32 && n > 0) {
+    // ---- MMA issue: the whole warp walks the list, one elected thread issues (a branch on the thread index makes the
+    // compiler treat descriptors as per-thread values and move each into uniform registers)
+    const bool elected = elect_one();
     bool ok = mbar_wait_p(&sm.q_full, 0, sm);
     uint32_t cnt[2] = {0, 0};  // products P V issued so far per tile
+    const uint32_t q_lo = desc_lo(smem_u32p(sm.q[0])), k_lo = desc_lo(smem_u32p(sm.k[0])), v_lo = desc_lo(smem_u32p(sm.v[0]));
     auto qk = [&](int t, int i) {
-      const uint32_t qa = smem_u32p(sm.q[t]), ka = smem_u32p(sm.k[i & 1]);
+      if (elected) {
+        const uint32_t qa = q_lo + (uint32_t)t * (kTileBytes >> 4), ka = k_lo + (uint32_t)(i & 1) * (kTileBytes >> 4);
 #pragma unroll
-      for (int s = 0; s < 8; ++s) {
-        const uint32_t off = (uint32_t)((s >> 2) * (kTileBytes / 2) + (s & 3) * 32);
-        mma_ss(tmem + (uint32_t)(t * 256), desc_k_major(qa + off), desc_k_major(ka + off), s > 0);
+        for (int s = 0; s < 8; ++s) {
+          const uint32_t off = ((uint32_t)((s >> 2) * (kTileBytes / 2) + (s & 3) * 32)) >> 4;
+          mma_ss(tmem + (uint32_t)(t * 256), qa + off, ka + off, s > 0);
+        }
+        commit_p(&sm.s_full[t]);
       }
-      commit_p(&sm.s_full[t]);
     };
     ok = ok && mbar_wait_p(&sm.k_full[0], 0, sm);
+    ok = __all_sync(0xffffffffu, ok);
     if (ok) {
       fence_after_p();
 #pragma unroll
       for (int t = 0; t < 2; ++t)
         if (sm.cls[t][0] != kClsSkip) qk(t, 0);
-      commit_p(&sm.k_empty[0]);
+      if (elected) commit_p(&sm.k_empty[0]);
     }
     for (int i = 0; i < n && ok; ++i) {
       ok = mbar_wait_p(&sm.v_full[i & 1], (uint32_t)(i >> 1) & 1u, sm);
       if (ok && i + 1 < n) ok = mbar_wait_p(&sm.k_full[(i + 1) & 1], (uint32_t)((i + 1) >> 1) & 1u, sm);
+      ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       fence_after_p();
 #pragma unroll
       for (int t = 0; t < 2; ++t) {
         if (ok && sm.cls[t][i] != kClsSkip) {
-          ok = mbar_wait_p(&sm.p_ready[t], cnt[t] & 1u, sm);
+          ok = __all_sync(0xffffffffu, mbar_wait_p(&sm.p_ready[t], cnt[t] & 1u, sm));
           fence_after_p();
           if (ok) {
-            const uint32_t p = tmem + (uint32_t)(t * 256), o = p + 128, va = smem_u32p(sm.v[i & 1]);
+            if (elected) {
+              const uint32_t p = tmem + (uint32_t)(t * 256), o = p + 128, va = v_lo + (uint32_t)(i & 1) * (kTileBytes >> 4);
 #pragma unroll
-            for (int s = 0; s < 16; ++s)  // (the leading parts, then the rests)
-              mma_ts(o, p + (uint32_t)(8 * s), desc_mn_major(va + (uint32_t)((s & 7) * 2048)), (s > 0 || cnt[t] > 0) ? 1u : 0u);
+              for (int s = 0; s < 16; ++s)  // (the leading parts, then the rests)
+                mma_ts(o, p + (uint32_t)(8 * s), va + (uint32_t)((s & 7) * (2048 >> 4)), (s > 0 || cnt[t] > 0) ? 1u : 0u);
+            }
             ++cnt[t];
           }
         }
@@ -407,106 +538,141 @@ __global__ void __launch_bounds__(kThreadsP, 1)
         if (ok && i + 1 < n && sm.cls[t][i + 1] != kClsSkip) qk(t, i + 1);
       }
       if (!ok) break;
-      if (i + 1 < n) commit_p(&sm.k_empty[(i + 1) & 1]);
-      commit_p(&sm.v_empty[i & 1]);
+      if (elected) {
+        if (i + 1 < n) commit_p(&sm.k_empty[(i + 1) & 1]);
+        commit_p(&sm.v_empty[i & 1]);
+      }
     }
-    commit_p(&sm.o_done);
-  } else if (warp < 8) {
-    // ---- softmax of tile t, one query row per thread
-    const int t = warp >> 2, row_in = tid & 127;
-    const uint32_t tl = tmem + (uint32_t)(t * 256) + ((uint32_t)((warp & 3) * 32) << 16);
+    if (elected) commit_p(&sm.o_done);
+  } else if (warp < 16) {
+    // ---- softmax of tile t: one query row and 64 keys per thread
+    const int t = warp >> 3, half = (warp >> 2) & 1, row_in = tid & 127;
+    const uint32_t tl = tmem + (uint32_t)(t * 256) + ((uint32_t)((warp & 3) * 32) << 16);  // S, P and behind them O
+    const uint32_t sl = tl + (uint32_t)(64 * half);                                         // this thread's keys
     const int trow = (t ? tb[1] : tb[0]) * kRowsP + row_in;  // token of the row
     const int my_hq = t ? hq[1] : hq[0];
-    const uint16_t* mrow = nullptr;
-    if (a.mask_mode == JPT_MASK_ADD)
-      mrow = static_cast<const uint16_t*>(a.mask) + (int64_t)b * a.mk_b +
-             ((int64_t)(my_hq % rep) * a.Tq + min(trow, a.Tq - 1)) * a.mk_r;
+    // this row's mask at this thread's half of the keys, and the warp's first row
+    const uint16_t *mrow = nullptr, *mwarp = nullptr;
+    const int wrow = (t ? tb[1] : tb[0]) * kRowsP + (warp & 3) * 32;
+    if (a.mask_mode == JPT_MASK_ADD) {
+      const uint16_t* base = static_cast<const uint16_t*>(a.mask) + (int64_t)b * a.mk_b + (int64_t)(my_hq % rep) * a.Tq * a.mk_r + 64 * half;
+      mrow = base + (int64_t)min(trow, a.Tq - 1) * a.mk_r;
+      mwarp = base + (int64_t)min(wrow, a.Tq - 1) * a.mk_r;
+    }
     float m_ref = -INFINITY, m_true = -INFINITY, l = 0.f;
     uint32_t cnt = 0;
-    bool ok = true;
-    for (int i = 0; i < n; ++i) {
+    bool ok = true, scaled = false;
+    // a scale of list entry i (lower half of the threads: K, upper half: V)
+    auto scale_of = [&](int i) {
+      const int p = sm.list[i] * kKeysP + row_in;
+      return p < a.S ? load_scale(half ? a.v_scale : a.k_scale, (int64_t)b * a.sc_b + (int64_t)p * a.sc_s, a.scale_is_f32) : 1.f;
+    };
+    auto keep_scale = [&](float x, uint32_t par) { (half ? sm.vs : sm.ks)[t][par][row_in] = x; };
+    auto next_of = [&](int i) {
+      while (i < n && sm.cls[t][i] == kClsSkip) ++i;
+      return i;
+    };
+    int i = next_of(0);
+    if constexpr (kScale) {
+      if (i < n) {
+        const float x = scale_of(i);
+        keep_scale(x, 0);
+        scaled = !group_all(t, x == 1.f);  // (an unquantised prefill has unit scales)
+      }
+    }
+    while (i < n) {
       const uint8_t c = sm.cls[t][i];
-      if (c == kClsSkip) continue;
-      const int s0 = sm.list[i] * kKeysP;
-      bool scaled = false;
+      const int s0 = sm.list[i] * kKeysP, nxt = next_of(i + 1);
+      const uint32_t par = cnt & 1u;
+      float next_scale = 1.f;
       if constexpr (kScale) {
-        const int p = s0 + row_in;
-        float ksv = 1.f, vsv = 1.f;
-        if (p < a.S) {
-          const int64_t idx = (int64_t)b * a.sc_b + (int64_t)p * a.sc_s;
-          ksv = load_scale(a.k_scale, idx, a.scale_is_f32);
-          vsv = load_scale(a.v_scale, idx, a.scale_is_f32);
-        }
-        group_sync(t);  // (everybody is done with the last tile's scales)
-        sm.ks[t][row_in] = ksv;
-        sm.vs[t][row_in] = vsv;
-        scaled = !group_all(t, ksv == 1.f && vsv == 1.f);  // (an unquantised prefill has unit scales)
+        if (nxt < n) next_scale = scale_of(nxt);
       }
       // (after a wait that gave up the later ones return at once: the loop runs to its end, so that the group's
       // barriers are met by all of its threads)
-      ok = mbar_wait_p(&sm.s_full[t], cnt & 1u, sm) && ok;
+      ok = mbar_wait_p(&sm.s_full[t], par, sm) && ok;
       __syncwarp();
       fence_after_p();
-      const int valid = min(kKeysP, a.S - s0);
+      // Keys that the row must not see (0 / -inf masks, keys behind the last one) are struck out of the logits below.  A
+      // tile with other mask values or with scales to multiply by first turns its products into final logits in tensor
+      // memory, in a function of its own: spelled out inside the main path these cases cost every tile their
+      // predicated instructions (54 instead of 39 us for 1024 tokens of 32 heads).
+      const int valid = a.S - s0 - 64 * half;
+      float mul = a.sm_scale;
+      uint32_t out_lo = 0u, out_hi = 0u;
+      bool strike = false;
+      if (c == kClsMixed || valid < kKeysP / 2 || (kScale && scaled)) {
+        const uint16_t* mw = c == kClsMixed ? mwarp + s0 : nullptr;
+        const uint4 bits = masked_bits(mw, a.mk_r, a.Tq - wrow, valid, g.mask_pairs != 0);
+        out_lo = bits.x, out_hi = bits.y, strike = bits.z != 0u;
+        if (!strike || (kScale && scaled)) {
+          final_logits<kRound, kScale>(sl, a, sm.ks[t][par] + 64 * half, kScale && scaled, c == kClsMixed ? mrow + s0 : nullptr,
+                                       valid, g.mask_vec != 0);
+          mul = 1.f;
+          strike = false;
+        }
+      }
       // logits of the row: packed pairs of bf16 (kRound) or fp32
-      uint32_t lg[kRound ? 64 : 128];
+      uint32_t lg[kRound ? 32 : 64];
       float mt;
       {
+        const uint64_t mul2x = pack_f32(mul, mul);
         uint32_t mx = 0xff80ff80u;
         float mxf = -INFINITY;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          uint32_t v[32];
-          tmem_ld32(tl + 32 * q, v);
-          uint32_t mk[16];
-          if (c == kClsMixed) {
-            if (g.mask_vec && valid == kKeysP) {
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const uint4 w = __ldg(reinterpret_cast<const uint4*>(mrow + s0 + 32 * q) + e);
-                mk[4 * e] = w.x, mk[4 * e + 1] = w.y, mk[4 * e + 2] = w.z, mk[4 * e + 3] = w.w;
-              }
-            } else {
-#pragma unroll
-              for (int e = 0; e < 16; ++e) {
-                const int p = 32 * q + 2 * e;
-                const uint32_t x0 = p < valid ? (uint32_t)__ldg(mrow + s0 + p) : 0xff80u;
-                const uint32_t x1 = p + 1 < valid ? (uint32_t)__ldg(mrow + s0 + p + 1) : 0xff80u;
-                mk[e] = x0 | (x1 << 16);
-              }
-            }
-          }
+        for (int q = 0; q < 2; ++q) {
+          uint32_t v[32];  // (both halves at once would not fit the 96 registers of a thread)
+          tmem_ld32(sl + 32 * q, v);
           tmem_wait_ld();
 #pragma unroll
           for (int e = 0; e < 16; ++e) {
-            const int p = 32 * q + 2 * e;
+            const float d0 = __uint_as_float(v[2 * e]), d1 = __uint_as_float(v[2 * e + 1]);
+            float f0, f1;
             if constexpr (kRound) {
-              uint32_t x = pack_bf16(__uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1]));  // bf16(q . k)
-              x = pack_bf16(lo_f32(x) * a.sm_scale, hi_f32(x) * a.sm_scale);                      // bf16(. / sqrt(D))
-              if (kScale && scaled) x = pack_bf16(lo_f32(x) * sm.ks[t][p], hi_f32(x) * sm.ks[t][p + 1]);
-              if (c == kClsMixed) x = add2(x, mk[e]);
-              if (c != kClsMixed && valid < kKeysP) {
-                if (p >= valid) x = (x & 0xffff0000u) | 0xff80u;
-                if (p + 1 >= valid) x = (x & 0xffffu) | 0xff800000u;
-              }
+              uint32_t x = pack_bf16(d0, d1);  // bf16(q . k)
+              unpack_f32(mul_f32x2(pack_f32(lo_f32(x), hi_f32(x)), mul2x), f0, f1);
+              x = pack_bf16(f0, f1);  // bf16(. / sqrt(D))
               mx = max2(mx, x);
               lg[16 * q + e] = x;
             } else {
-              float f0 = __uint_as_float(v[2 * e]) * a.sm_scale, f1 = __uint_as_float(v[2 * e + 1]) * a.sm_scale;
-              if (kScale && scaled) f0 *= sm.ks[t][p], f1 *= sm.ks[t][p + 1];
-              if (c == kClsMixed) f0 += lo_f32(mk[e]), f1 += hi_f32(mk[e]);
-              if (c != kClsMixed && valid < kKeysP) {
-                if (p >= valid) f0 = -INFINITY;
-                if (p + 1 >= valid) f1 = -INFINITY;
-              }
+              unpack_f32(mul_f32x2(pack_f32(d0, d1), mul2x), f0, f1);
               mxf = fmaxf(mxf, fmaxf(f0, f1));
-              lg[(32 * q + 2 * e) & (kRound ? 63 : 127)] = __float_as_uint(f0);
-              lg[(32 * q + 2 * e + 1) & (kRound ? 63 : 127)] = __float_as_uint(f1);
+              lg[(32 * q + 2 * e) & (kRound ? 31 : 63)] = __float_as_uint(f0);
+              lg[(32 * q + 2 * e + 1) & (kRound ? 31 : 63)] = __float_as_uint(f1);
+            }
+          }
+        }
+        if (strike) {
+          mx = 0xff80ff80u;
+          mxf = -INFINITY;
+#pragma unroll
+          for (int e = 0; e < 32; ++e) {
+            if constexpr (kRound) {
+              uint32_t x = lg[e];
+              if ((out_lo >> e) & 1u) x = (x & 0xffff0000u) | 0xff80u;
+              if ((out_hi >> e) & 1u) x = (x & 0xffffu) | 0xff800000u;
+              lg[e] = x;
+              mx = max2(mx, x);
+            } else {
+              if ((out_lo >> e) & 1u) lg[(2 * e) & (kRound ? 31 : 63)] = 0xff800000u;
+              if ((out_hi >> e) & 1u) lg[(2 * e + 1) & (kRound ? 31 : 63)] = 0xff800000u;
+              mxf = fmaxf(mxf, fmaxf(__uint_as_float(lg[(2 * e) & (kRound ? 31 : 63)]),
+                                     __uint_as_float(lg[(2 * e + 1) & (kRound ? 31 : 63)])));
             }
           }
         }
         mt = kRound ? fmaxf(lo_f32(mx), hi_f32(mx)) : mxf;
       }
+      // the row's maximum; every thread of the tile has also read its part of S behind this barrier: P may go over it
+      sm.half_max[t][par][half][row_in] = mt;
+      // (S of this tile is there, so every thread has handed over its P of the last tile and is done with its scales)
+      if constexpr (kScale) keep_scale(next_scale, par ^ 1u);
+      fence_before_p();
+      const bool next_ones = group_all(t, next_scale == 1.f);
+      fence_after_p();
+      const bool scaled_now = scaled;
+      scaled = !next_ones;
+      mt = fmaxf(mt, sm.half_max[t][par][half ^ 1][row_in]);
       m_true = fmaxf(m_true, mt);
       // raise the reference maximum: on the first tile, later only where P would leave its range
       float m_new = m_ref;
@@ -517,56 +683,78 @@ __global__ void __launch_bounds__(kThreadsP, 1)
         const float f = raise ? ex2p((m_ref - m_new) * kLog2e) : 1.f;
         l *= f;
 #pragma unroll 1
-        for (int q = 0; q < 4; ++q) {
+        for (int q = 0; q < 2; ++q) {
           uint32_t v[32];
-          tmem_ld32(tl + 128 + 32 * q, v);
+          tmem_ld32(tl + 128 + 64 * half + 32 * q, v);
           tmem_wait_ld();
 #pragma unroll
           for (int e = 0; e < 32; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) * f);
-          tmem_st32(tl + 128 + 32 * q, v);
+          tmem_st32(tl + 128 + 64 * half + 32 * q, v);
         }
       }
       m_ref = m_new;
       const float off = m_ref == -INFINITY ? 0.f : m_ref * kLog2e;
-      float l0 = 0.f, l1 = 0.f;
+      const uint64_t l2e = pack_f32(kLog2e, kLog2e), noff = pack_f32(-off, -off);
+      uint64_t lsum = pack_f32(0.f, 0.f);
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
+      for (int q = 0; q < 2; ++q) {
         uint32_t hi[16], rest[16];
+        float f[32];
 #pragma unroll
         for (int e = 0; e < 16; ++e) {
-          float f0, f1;
+          uint64_t x;
           if constexpr (kRound) {
-            f0 = lo_f32(lg[16 * q + e]), f1 = hi_f32(lg[16 * q + e]);
+            x = pack_f32(lo_f32(lg[16 * q + e]), hi_f32(lg[16 * q + e]));
           } else {
-            f0 = __uint_as_float(lg[(32 * q + 2 * e) & (kRound ? 63 : 127)]);
-            f1 = __uint_as_float(lg[(32 * q + 2 * e + 1) & (kRound ? 63 : 127)]);
+            x = pack_f32(__uint_as_float(lg[(32 * q + 2 * e) & (kRound ? 31 : 63)]),
+                         __uint_as_float(lg[(32 * q + 2 * e + 1) & (kRound ? 31 : 63)]));
           }
-          f0 = ex2p(fmaf(f0, kLog2e, -off)), f1 = ex2p(fmaf(f1, kLog2e, -off));
-          l0 += f0, l1 += f1;
-          if (kScale && scaled) f0 *= sm.vs[t][32 * q + 2 * e], f1 *= sm.vs[t][32 * q + 2 * e + 1];
-          hi[e] = pack_bf16(f0, f1);
-          rest[e] = pack_bf16(f0 - lo_f32(hi[e]), f1 - hi_f32(hi[e]));
+          unpack_f32(fma_f32x2(x, l2e, noff), f[2 * e], f[2 * e + 1]);
+          f[2 * e] = ex2p(f[2 * e]), f[2 * e + 1] = ex2p(f[2 * e + 1]);
+          lsum = add_f32x2(lsum, pack_f32(f[2 * e], f[2 * e + 1]));
         }
-        tmem_st16(tl + 16 * q, hi);
-        tmem_st16(tl + 64 + 16 * q, rest);
+        if (kScale && scaled_now) {
+#pragma unroll
+          for (int e = 0; e < 32; ++e) f[e] *= sm.vs[t][par][64 * half + 32 * q + e];
+        }
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+          // p cut after its upper 16 bits, and the remainder cut the same way: 16 bits of p are kept, and byte moves do it
+          // (two conversions per pair and the widening back took half of this phase's time)
+          hi[e] = __byte_perm(__float_as_uint(f[2 * e]), __float_as_uint(f[2 * e + 1]), 0x7632);
+          const float r0 = f[2 * e] - __uint_as_float(__float_as_uint(f[2 * e]) & 0xffff0000u);
+          const float r1 = f[2 * e + 1] - __uint_as_float(__float_as_uint(f[2 * e + 1]) & 0xffff0000u);
+          rest[e] = __byte_perm(__float_as_uint(r0), __float_as_uint(r1), 0x7632);
+        }
+        tmem_st16(tl + 32 * half + 16 * q, hi);
+        tmem_st16(tl + 64 + 32 * half + 16 * q, rest);
       }
-      l += l0 + l1;
+      {
+        float l0, l1;
+        unpack_f32(lsum, l0, l1);
+        l += l0 + l1;
+      }
       tmem_wait_st();
       fence_before_p();
       mbar_arrive_p(&sm.p_ready[t]);
       ++cnt;
+      i = nxt;
     }
-    // ---- output rows
+    // ---- output rows: the row's sum over both halves, 64 dims per thread
+    // (the buffer of the parity before the last: everybody is done with it)
+    sm.half_max[t][cnt & 1u][half][row_in] = l;
+    group_sync(t);
+    l = sm.half_max[t][cnt & 1u][0][row_in] + sm.half_max[t][cnt & 1u][1][row_in];
     if (n > 0) ok = mbar_wait_p(&sm.o_done, 0, sm) && ok;
     __syncwarp();
     fence_after_p();
     const float inv = l > 0.f && ok ? 1.f / l : 0.f;
     const bool any = cnt > 0;
 #pragma unroll 1
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < 2; ++q) {
       uint32_t v[32];
       if (any) {
-        tmem_ld32(tl + 128 + 32 * q, v);
+        tmem_ld32(tl + 128 + 64 * half + 32 * q, v);
         tmem_wait_ld();
       }
 #pragma unroll
@@ -574,29 +762,29 @@ __global__ void __launch_bounds__(kThreadsP, 1)
         uint32_t w[4];
 #pragma unroll
         for (int x = 0; x < 4; ++x) {
-          const int i = 8 * e + 2 * x;
-          w[x] = inv > 0.f && any ? pack_bf16(__uint_as_float(v[i]) * inv, __uint_as_float(v[i + 1]) * inv) : 0u;
+          const int d = 8 * e + 2 * x;
+          w[x] = inv > 0.f && any ? pack_bf16(__uint_as_float(v[d]) * inv, __uint_as_float(v[d + 1]) * inv) : 0u;
         }
-        const int chunk = (q & 1) * 4 + e;  // 16-byte piece of the row's 128-byte half
-        *reinterpret_cast<uint4*>(sm.q[t] + (q >> 1) * (kTileBytes / 2) + row_in * 128 + ((chunk ^ (row_in & 7)) * 16)) =
+        const int chunk = q * 4 + e;  // 16-byte piece of the row's 128-byte half
+        *reinterpret_cast<uint4*>(sm.q[t] + half * (kTileBytes / 2) + row_in * 128 + ((chunk ^ (row_in & 7)) * 16)) =
             make_uint4(w[0], w[1], w[2], w[3]);
       }
     }
     const bool mine = t ? have[1] : have[0];
-    if (mine && trow < a.Tq && (a.m || a.l)) {
+    if (mine && half == 0 && trow < a.Tq && (a.m || a.l)) {
       const int64_t at = ((int64_t)b * a.Hq + my_hq) * a.Tq + trow;
       if (a.m) a.m[at] = m_true;
       if (a.l) a.l[at] = l > 0.f ? l * ex2p((m_ref - m_true) * kLog2e) : 0.f;
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     group_sync(t);
-    if (row_in == 0 && mine) {
+    if (row_in == 0 && half == 0 && mine) {
 #pragma unroll
-      for (int half = 0; half < 2; ++half) {
+      for (int h = 0; h < 2; ++h) {
         asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3, %4}], [%5];" ::"l"(
                          reinterpret_cast<uint64_t>(&maps.o)),
-                     "r"(half * 64), "r"(t ? tb[1] * kRowsP : tb[0] * kRowsP), "r"(my_hq), "r"(b),
-                     "r"(smem_u32p(sm.q[t]) + half * (kTileBytes / 2))
+                     "r"(h * 64), "r"(t ? tb[1] * kRowsP : tb[0] * kRowsP), "r"(my_hq), "r"(b),
+                     "r"(smem_u32p(sm.q[t]) + h * (kTileBytes / 2))
                      : "memory");
       }
       asm volatile("cp.async.bulk.commit_group;" ::: "memory");
@@ -607,7 +795,7 @@ __global__ void __launch_bounds__(kThreadsP, 1)
   __syncwarp();
   __syncthreads();
   if (tid == 0 && sm.dead) atomicExch(status, 1);
-  if (warp == 9) {
+  if (warp == kIssuerP / 32) {
     fence_after_p();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
   }
@@ -732,6 +920,7 @@ int launch_attention_prefill(const jpt_attn_params& p, const AttnArgs& a, int64_
   g.n_k = t.n_k;
   g.pairs = (g.n_rows_t * (p.Hq / p.Hkv) + 1) / 2;
   g.mask_vec = p.mask_mode == JPT_MASK_ADD && aligned(p.mask, 16) && p.mk_b % 8 == 0 && p.mk_r % 8 == 0;
+  g.mask_pairs = p.mask_mode == JPT_MASK_ADD && aligned(p.mask, 4) && p.mk_b % 2 == 0 && p.mk_r % 2 == 0 && p.Tq * p.mk_r % 2 == 0;
   if (wants_classes(p)) {
     uint8_t* cls = reinterpret_cast<uint8_t*>(ws + kWorkspaceCounterBytes);
     g.cls = cls;
