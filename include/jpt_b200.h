@@ -158,6 +158,18 @@ int jpt_kv_scatter_rows(const void* src_k, const void* src_v, void* dst_k,
                         int64_t ds_h, int64_t ds_s, void* stream);
 
 /*
+ * `Int8KVCacheGenerate.finalize` of a lazily updated cache in one launch
+ * (jetstream_pt/cache_manager.py:598-657): the kept codes new_k / new_v
+ * [NL,B,H,1,D] to their rows and the kept scales new_ks / new_vs [NL,B] (elements
+ * of scale_bytes) to theirs; positions as in jpt_kv_scatter_rows, clamped.
+ */
+int jpt_kv_finalize_int8(const int8_t* new_k, const int8_t* new_v, int8_t* cache_k, int8_t* cache_v,
+                         const void* new_ks, const void* new_vs, void* k_scaler, void* v_scaler, int scale_bytes,
+                         const int32_t* pos, int pos_count, int pos_host, int NL, int B, int H, int S, int D,
+                         int64_t ds_l, int64_t ds_b, int64_t ds_h, int64_t ds_s, int64_t ss_l, int64_t ss_b,
+                         int64_t ss_s, void* stream);
+
+/*
  * Paged append: cache[h, page_j, tok_j, :] = x[slot_j, h, 0, :] for the n_active
  * entries of page_token_indices.  Replaces PageKVCacheGenerate.update,
  * jetstream_pt/cache_manager.py:681-706 (which gathers and re-scatters whole
@@ -259,6 +271,26 @@ int jpt_prefill_insert_paged(const void* prefix_k, const void* prefix_v,
                              int n_pages, int NL, int H, int L, int P, int ps,
                              int D, int64_t ps_l, int64_t ps_h, int64_t ps_t,
                              int64_t cs_l, int64_t ss_l, void* stream);
+
+/*
+ * Both inserts for layers whose tensors lie anywhere (jetstream_pt/engine.py:
+ * 397-466, 534-561 loops over the layers): one launch for all of them.  Pointers
+ * of layer l in layers[l] (host array; k_scaler / v_scaler may be NULL), the
+ * other arguments as above.  The page list may lie on the host (pages_host, up to
+ * 256 pages; it travels with the launch) instead of the device.
+ */
+typedef struct jpt_layer_tensors {
+  const void *prefix_k, *prefix_v;
+  void *cache_k, *cache_v;
+  void *k_scaler, *v_scaler;
+} jpt_layer_tensors;
+int jpt_prefill_insert_dense_layers(const jpt_layer_tensors* layers, int NL, int in_dtype, int cache_dtype, int slot,
+                                    int pos, int wrap, int H, int L, int S, int D, int64_t ps_h, int64_t ps_t,
+                                    int64_t cs_b, int64_t cs_h, int64_t cs_s, int64_t ss_b, int64_t ss_s,
+                                    void* stream);
+int jpt_prefill_insert_paged_layers(const jpt_layer_tensors* layers, int NL, int in_dtype, int cache_dtype,
+                                    const int32_t* update_indexes, const int32_t* pages_host, int n_pages, int H,
+                                    int L, int P, int ps, int D, int64_t ps_h, int64_t ps_t, void* stream);
 
 /*
  * The KV insert quantiser on its own: quantize_tensor(w, reduce_axis, 8,
@@ -441,6 +473,22 @@ typedef struct jpt_new_token {
 } jpt_new_token;
 
 int jpt_decode_update_attend(const jpt_attn_params* p, const jpt_new_token* nt, void* stream);
+/* The same with the output rows in out_dtype (JPT_BF16 or JPT_F32, what the merge of the unfused step yields). */
+int jpt_decode_update_attend_out(const jpt_attn_params* p, const jpt_new_token* nt, int out_dtype, void* stream);
+
+/*
+ * The step's own token joined to the attention over the cache, for caches that
+ * take it later (jetstream_pt/layers.py:525-550): flash attention over that one
+ * token (m = q . k * sm_scale, l = 1, o = v) and the merge below in one launch,
+ * which also keeps the token for finalize (keep_k / keep_v, may be NULL).
+ * q, o1 [B,Hq,D] in q_dtype (JPT_BF16 or JPT_F32); xk, xv, keep_k, keep_v
+ * [B,Hkv,D] in q_dtype, or int8 codes with scales xks, xvs [B] in scale_dtype;
+ * m1, l1 [B,Hq]; out fp32 [B,Hq,D].
+ */
+int jpt_attend_new_token(const void* q, int q_dtype, const void* xk, const void* xv, int token_dtype, const void* xks,
+                         const void* xvs, int scale_dtype, const void* o1, const float* m1, const float* l1,
+                         void* keep_k, void* keep_v, float* out, int B, int Hq, int Hkv, int D, float sm_scale,
+                         void* stream);
 
 /*
  * Merge two softmax partials: g = max(m1,m2); o = (l1 e^{m1-g} o1 + l2 e^{m2-g}
@@ -541,6 +589,38 @@ int jpt_w8a16_linear_tp(const void* x, const void* w, const void* w_scale, void*
                         int M, int N, int K, void* workspace, size_t workspace_bytes,
                         const jpt_tp_sum* tp, void* stream);
 int jpt_w8a16_tp_status(const jpt_tp_sum* tp, void* stream);
+
+/* ------------------------------------------------------------------------- */
+/* The engine's bookkeeping                                                  */
+/* ------------------------------------------------------------------------- */
+
+/*
+ * In front of a decode step: the block tables of
+ * `precompute_ragged_block_indices` (jetstream_pt/engine.py:674-729) for start,
+ * input_pos int32 [B], next_b / next_i int32 [B, S / block] out, and, with mask
+ * != NULL ([B,S] in mask_dtype, row stride mask_stride), this step's position
+ * opened in it (774-779): `pos` for every slot when `ring`, else input_pos[b].
+ */
+int jpt_engine_begin(const int32_t* start, const int32_t* input_pos, int B, int S, int block, int32_t* next_b,
+                     int32_t* next_i, void* mask, int mask_dtype, int64_t mask_stride, int ring, int pos, void* stream);
+/*
+ * Behind it: greedy sampling (283-297: argmax of the logits [B,V] in dtype, row
+ * stride row_stride; the first of equal values, NaN above all), the advance of
+ * lens and input_pos (807-818: every slot when `ring`, else idle slots stay 0),
+ * the result rows data [B,3] = {tokens, 1, new lens}, and the mask as above.
+ */
+int jpt_engine_end(const void* logits, int dtype, int64_t row_stride, int V, const int32_t* tokens, const int32_t* lens,
+                   const int32_t* input_pos, int B, int S, int ring, int pos, int32_t* next_token, int32_t* lens_out,
+                   int32_t* pos_out, int32_t* data, void* mask, int mask_dtype, int64_t mask_stride, void* stream);
+/*
+ * The rows of one slot after an insert (386-395, 506-524): mask[slot] (0 on
+ * [pos, cur), or with wrap and cur <= pos outside [cur, pos); -inf elsewhere),
+ * start[slot], input_pos[slot] = seq_len, lens[slot] = 1, tokens[slot] = *token
+ * (int32 or int64).  NULL pointers are left out.
+ */
+int jpt_engine_insert_slot(void* mask, int mask_dtype, int64_t mask_stride, int S, int slot, int pos, int cur, int wrap,
+                           int start_value, int seq_len, int32_t* start, int32_t* input_pos, int32_t* lens,
+                           int32_t* tokens, const void* token, int token_bytes, void* stream);
 
 #ifdef __cplusplus
 }

@@ -33,6 +33,12 @@ class PeerExchangeStruct(ctypes.Structure):
               ("wait_cycles", ctypes.c_longlong)]
 
 
+class LayerTensors(ctypes.Structure):
+  """Mirror of `struct jpt_layer_tensors`."""
+  _fields_ = [("prefix_k", c_void_p), ("prefix_v", c_void_p), ("cache_k", c_void_p), ("cache_v", c_void_p),
+              ("k_scaler", c_void_p), ("v_scaler", c_void_p)]
+
+
 class TpSumStruct(ctypes.Structure):
   """Mirror of `struct jpt_tp_sum`."""
   _fields_ = [("rank", c_int), ("world", c_int), ("buffers", c_void_p * 8), ("buffer_bytes", c_size_t),
@@ -88,6 +94,7 @@ _SIGNATURES = {
                                         + [c_void_p, c_void_p]),
     "jpt_kv_scatter_rows": (c_int, [c_void_p] * 4 + [c_int, c_void_p, c_int, c_int, c_int]
                             + [c_int] * 5 + [c_i64] * 4 + [c_void_p]),
+    "jpt_kv_finalize_int8": (c_int, [c_void_p] * 8 + [c_int, c_void_p] + [c_int] * 7 + [c_i64] * 7 + [c_void_p]),
     "jpt_kv_append_paged": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
                                     c_void_p, c_i64, c_int, c_void_p] + [c_int] * 5 + [c_void_p]),
     "jpt_page_token_indices": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p,
@@ -96,6 +103,9 @@ _SIGNATURES = {
                                          c_void_p] + [c_int] * 8 + [c_i64] * 10 + [c_void_p]),
     "jpt_prefill_insert_paged": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p,
                                          c_void_p, c_void_p] + [c_int] * 7 + [c_i64] * 5 + [c_void_p]),
+    "jpt_prefill_insert_dense_layers": (c_int, [ctypes.POINTER(LayerTensors)] + [c_int] * 10 + [c_i64] * 7 + [c_void_p]),
+    "jpt_prefill_insert_paged_layers": (c_int, [ctypes.POINTER(LayerTensors)] + [c_int] * 3 + [c_void_p, c_void_p]
+                                        + [c_int] * 6 + [c_i64] * 2 + [c_void_p]),
     "jpt_enable_peer_access": (c_int, [c_int, c_int]),
     "jpt_w8a16_linear_workspace_bytes": (c_size_t, [c_int, c_int, c_int]),
     "jpt_w8a16_linear": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_size_t, c_void_p]),
@@ -113,6 +123,14 @@ _SIGNATURES = {
     "jpt_flash_attend_strided_q_ok": (c_int, [ctypes.POINTER(AttnParams), c_i64, c_i64, c_i64]),
     "jpt_flash_decode_static": (c_int, [ctypes.POINTER(AttnParams), c_void_p]),
     "jpt_decode_update_attend": (c_int, [ctypes.POINTER(AttnParams), ctypes.POINTER(NewTokenStruct), c_void_p]),
+    "jpt_decode_update_attend_out": (c_int, [ctypes.POINTER(AttnParams), ctypes.POINTER(NewTokenStruct), c_int, c_void_p]),
+    "jpt_attend_new_token": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int]
+                             + [c_void_p] * 6 + [c_int] * 4 + [c_float, c_void_p]),
+    "jpt_engine_begin": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_i64,
+                                 c_int, c_int, c_void_p]),
+    "jpt_engine_end": (c_int, [c_void_p, c_int, c_i64, c_int] + [c_void_p] * 3 + [c_int] * 4 + [c_void_p] * 5
+                       + [c_int, c_i64, c_void_p]),
+    "jpt_engine_insert_slot": (c_int, [c_void_p, c_int, c_i64] + [c_int] * 7 + [c_void_p] * 5 + [c_int, c_void_p]),
     "jpt_flash_decode_workspace_bytes": (c_size_t, [ctypes.POINTER(AttnParams)]),
     "jpt_flash_decode_workspace_init": (c_int, [c_void_p, c_size_t, c_void_p]),
     "jpt_flash_decode_status": (c_int, [c_void_p, c_void_p]),
@@ -139,6 +157,28 @@ def lib():
       fn.restype, fn.argtypes = res, args
     _lib = handle
   return _lib
+
+
+class _Native:
+  """The extension module `_native` (csrc/host.cpp: the host side of a call), loaded on first use so that importing the
+  package needs no built library.  Raises if it has not been built."""
+
+  def __getattr__(self, name):
+    lib()  # (the same message when nothing has been built)
+    try:
+      from jetstream_pytorch_b200 import _native
+    except ImportError as e:
+      raise RuntimeError(
+          f"the extension module _native cannot be loaded ({e}): build it with `python -m jetstream_pytorch_b200.build` "
+          "(there is no CPU or eager fallback)"
+      ) from e
+    for k in dir(_native):
+      if not k.startswith("__"):
+        setattr(self, k, getattr(_native, k))  # (later look-ups find the function itself)
+    return getattr(_native, name)
+
+
+native = _Native()
 
 
 def check(rc):

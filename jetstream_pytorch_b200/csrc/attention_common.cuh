@@ -31,6 +31,7 @@ struct AttnArgs {
   int mask_mode, scale_is_f32;
   int nsplit;
   float sm_scale;
+  int o_f32;         // the output rows are fp32 (they have q's dtype otherwise)
   int round_logits;  // dense_attention with bf16 tensors: every step of the logit chain is rounded to bf16
 };
 
@@ -45,6 +46,14 @@ __device__ __forceinline__ float rounded_logit(float dot, float sqrt_d, float ks
   s = bf16_round(__fdiv_rn(s, sqrt_d));
   if (quantised) s = bf16_round(s * ks);
   return bf16_round(s + mask_value);
+}
+
+// One element of an output row.
+__device__ __forceinline__ void store_o(const AttnArgs& a, int64_t i, float x) {
+  if (a.o_f32)
+    static_cast<float*>(a.o)[i] = x;
+  else
+    static_cast<__nv_bfloat16*>(a.o)[i] = __float2bfloat16_rn(x);
 }
 
 // Valid range of one sequence in "logical" token order: logical token j

@@ -194,6 +194,38 @@ __global__ void merge_partials_kernel(const TI* o1, const float* m1, const float
   }
 }
 
+// The step's own token joined to a finished attention over the cache, and kept for finalize: for one key the softmax
+// is 1, so the token's partial is (o, m, l) = (v, q . k * sm_scale, 1), and the result is the two-partial merge.  One
+// warp per query row; what it reads and writes is a few KB per slot, so it is a launch and a round trip to L2.  Stands
+// for two copies, an attention launch over one token and the merge launch (four launches of about 2 us each).
+template <typename TQ, typename TX>
+__global__ void __launch_bounds__(128) attend_new_token_kernel(const TQ* q, const TX* xk, const TX* xv, const void* xks, const void* xvs,
+                                                               int scale_is_f32, const TQ* o1, const float* m1, const float* l1,
+                                                               TX* keep_k, TX* keep_v, float* out, int rows, int hq, int rep, int D,
+                                                               float sm_scale) {
+  grid_dependency_wait();
+  grid_dependency_trigger();
+  const int row = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (row >= rows) return;
+  const int64_t qo = (int64_t)row * D, ko = (int64_t)(row / rep) * D;
+  const float ks = xks ? load_scale(xks, row / hq, scale_is_f32) : 1.f, vs = xvs ? load_scale(xvs, row / hq, scale_is_f32) : 1.f;
+  float s = 0.f;
+  for (int d = lane; d < D; d += 32) s += to_f32<TQ>(q[qo + d]) * to_f32<TX>(xk[ko + d]);
+  const float m2 = warp_sum(s) * sm_scale * ks;
+  const float a1 = m1[row], d1 = l1[row];
+  const float g = fmaxf(a1, m2);
+  const float alpha = a1 == -INFINITY ? 0.f : expf(a1 - g) * d1, beta = expf(m2 - g);
+  const float inv = 1.f / (alpha + beta);
+  for (int d = lane; d < D; d += 32) {
+    const TX v = xv[ko + d];
+    out[qo + d] = (alpha * to_f32<TQ>(o1[qo + d]) + beta * (to_f32<TX>(v) * vs)) * inv;
+    if (keep_k && row % rep == 0) {
+      keep_k[ko + d] = xk[ko + d];
+      keep_v[ko + d] = v;
+    }
+  }
+}
+
 template <typename TQ>
 int launch_generic_kv(const jpt_attn_params& p, const AttnArgs& a, cudaStream_t st) {
   const int rcs = (a.R + kRowTile - 1) / kRowTile;
@@ -304,6 +336,11 @@ static AttnArgs attn_args_of(const jpt_attn_params& p) {
 }
 
 extern "C" int jpt_decode_update_attend(const jpt_attn_params* pp, const jpt_new_token* nt, void* stream) {
+  return jpt_decode_update_attend_out(pp, nt, JPT_BF16, stream);
+}
+
+extern "C" int jpt_decode_update_attend_out(const jpt_attn_params* pp, const jpt_new_token* nt, int out_dtype, void* stream) {
+  JPT_REQUIRE(out_dtype == JPT_BF16 || out_dtype == JPT_F32, JPT_EINVAL, "decode_update_attend: the output must be bf16 or f32");
   JPT_REQUIRE(pp && nt, JPT_EINVAL, "decode_update_attend: null argument");
   const jpt_attn_params& p = *pp;
   if (int rc = validate(p)) return rc;
@@ -347,6 +384,7 @@ extern "C" int jpt_decode_update_attend(const jpt_attn_params* pp, const jpt_new
   }
   AttnArgs a = attn_args_of(p);
   a.nsplit = 1;
+  a.o_f32 = out_dtype == JPT_F32;
   return launch_attention_umma(p, a, static_cast<cudaStream_t>(stream), &n);
 }
 
@@ -479,6 +517,31 @@ extern "C" int jpt_flash_decode_status(const void* workspace, void* stream) {
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return fail((int)e, "flash_decode_status: %s", cudaGetErrorString(e));
   return status;
+}
+
+extern "C" int jpt_attend_new_token(const void* q, int q_dtype, const void* xk, const void* xv, int token_dtype, const void* xks,
+                                    const void* xvs, int scale_dtype, const void* o1, const float* m1, const float* l1, void* keep_k,
+                                    void* keep_v, float* out, int B, int Hq, int Hkv, int D, float sm_scale, void* stream) {
+  JPT_REQUIRE(q && xk && xv && o1 && m1 && l1 && out, JPT_EINVAL, "attend_new_token: null tensor");
+  JPT_REQUIRE((keep_k == nullptr) == (keep_v == nullptr) && (xks == nullptr) == (xvs == nullptr), JPT_EINVAL,
+              "attend_new_token: K and V arguments come together");
+  JPT_REQUIRE(B > 0 && Hq > 0 && Hkv > 0 && Hq % Hkv == 0 && D > 0, JPT_EINVAL, "attend_new_token: bad shape");
+  JPT_REQUIRE(q_dtype == JPT_BF16 || q_dtype == JPT_F32, JPT_EINVAL, "attend_new_token: q must be bf16 or f32");
+  JPT_REQUIRE(token_dtype == q_dtype || (token_dtype == JPT_INT8 && xks), JPT_EINVAL,
+              "attend_new_token: the token has q's dtype, or is int8 with scales");
+  const int rows = B * Hq;
+  const dim3 grid((rows + 3) / 4), block(128);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+#define JPT_NEW_TOKEN(TQ, TX)                                                                                                  \
+  launch_after_previous(attend_new_token_kernel<TQ, TX>, grid, block, 0, st, static_cast<const TQ*>(q), static_cast<const TX*>(xk), \
+                        static_cast<const TX*>(xv), xks, xvs, (int)(scale_dtype == JPT_F32), static_cast<const TQ*>(o1), m1, l1,   \
+                        static_cast<TX*>(keep_k), static_cast<TX*>(keep_v), out, rows, Hq, Hq / Hkv, D, sm_scale)
+  if (q_dtype == JPT_BF16 && token_dtype == JPT_BF16) JPT_NEW_TOKEN(__nv_bfloat16, __nv_bfloat16);
+  else if (q_dtype == JPT_BF16) JPT_NEW_TOKEN(__nv_bfloat16, int8_t);
+  else if (token_dtype == JPT_F32) JPT_NEW_TOKEN(float, float);
+  else JPT_NEW_TOKEN(float, int8_t);
+#undef JPT_NEW_TOKEN
+  return check_launch("attend_new_token_kernel");
 }
 
 extern "C" int jpt_merge_partials(const void* o1, const float* m1, const float* l1, const void* o2,

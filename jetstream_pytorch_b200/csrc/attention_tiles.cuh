@@ -143,7 +143,6 @@ static __device__ __forceinline__ void merge_rows(const AttnArgs& a, const MmaSc
     L[r] = __shfl_sync(0xffffffffu, Lr, r);
   }
   hook(M, L, acc);
-  __nv_bfloat16* o = static_cast<__nv_bfloat16*>(a.o);
 #pragma unroll
   for (int r = 0; r < kR; ++r) {
     if (r < R) {
@@ -151,7 +150,7 @@ static __device__ __forceinline__ void merge_rows(const AttnArgs& a, const MmaSc
         if (a.m) a.m[row_base + r] = M[r] * kLn2;
         if (a.l) a.l[row_base + r] = L[r];
       }
-      o[(row_base + r) * kD + tid] = __float2bfloat16_rn(L[r] > 0.f ? acc[r] / L[r] : 0.f);
+      store_o(a, (row_base + r) * kD + tid, L[r] > 0.f ? acc[r] / L[r] : 0.f);
     }
   }
 }

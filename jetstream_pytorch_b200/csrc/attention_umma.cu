@@ -597,8 +597,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
       int ua;
       if (seg_range(b, &ua).n == 0) {
         const int64_t r0 = (int64_t)b * a.Hkv * R;
-        __nv_bfloat16* o = static_cast<__nv_bfloat16*>(a.o);
-        for (int i = tid; i < a.Hkv * R * kD; i += kThreads) o[r0 * kD + i] = __float2bfloat16_rn(0.f);
+        for (int i = tid; i < a.Hkv * R * kD; i += kThreads) store_o(a, r0 * kD + i, 0.f);
         for (int i = tid; i < a.Hkv * R; i += kThreads) {
           if (a.m) a.m[r0 + i] = -INFINITY;
           if (a.l) a.l[r0 + i] = 0.f;
@@ -1141,7 +1140,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
           const float L = L8[r], M = M8[r];
           if (is_final) {
             const int64_t row = row_base + r;
-            static_cast<__nv_bfloat16*>(a.o)[row * kD + tid] = __float2bfloat16_rn(L > 0.f ? o[r] / L : 0.f);
+            store_o(a, row * kD + tid, L > 0.f ? o[r] / L : 0.f);
             if (tid == 0) {
               if (a.m) a.m[row] = M * kLn2;
               if (a.l) a.l[row] = L > 0.f ? L : 0.f;

@@ -4,6 +4,7 @@
 #include <stdarg.h>
 #include <stdlib.h>
 
+#include <algorithm>
 #include <atomic>
 
 #include "common.cuh"
@@ -295,10 +296,12 @@ struct ScatterArgs {
   int64_t ds_l, ds_b, ds_h, ds_s;   // bytes
 };
 
-__global__ void scatter_rows_kernel(ScatterArgs a) {
+// `more`: a second set of rows in the same launch (blockIdx.y 2, 3): the scales that go with the rows of a lazy finalize.
+__global__ void scatter_rows_kernel(const __grid_constant__ ScatterArgs first, const __grid_constant__ ScatterArgs more) {
+  const ScatterArgs& a = blockIdx.y < 2 ? first : more;
   const int chunks_per_row = a.row_bytes / a.chunk;
   const int64_t total = (int64_t)a.NL * a.B * a.H * chunks_per_row;
-  const int which = blockIdx.y;
+  const int which = blockIdx.y & 1;
   if (a.src[which] == nullptr) return;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (int64_t)gridDim.x * blockDim.x) {
@@ -403,12 +406,13 @@ __global__ void page_token_indices_kernel(const int32_t* lens, const int32_t* pa
       int col = len / ps;
       if (col >= max_pages) col = max_pages - 1;
       // Rows of the compacted table are B wide so the layout does not depend
-      // on the (device-side) count; entries past n_active are left untouched.
+      // on the (device-side) count; entries past n_active are zero.
       pti[j] = page_indices[(int64_t)tid * max_pages + col];
       pti[B + j] = j * ps + len % ps;
       pti[2 * B + j] = tid;
     }
   }
+  if (tid >= total && tid < B) pti[tid] = pti[B + tid] = pti[2 * B + tid] = 0;
   if (tid == 0) *n_active = total;
 }
 
@@ -512,10 +516,10 @@ extern "C" int jpt_peer_exchange_status(const void* own_buffer, void* stream) {
   return (int)st3[2];
 }
 
-extern "C" int jpt_kv_scatter_rows(const void* src_k, const void* src_v, void* dst_k, void* dst_v,
-                                   int elem_bytes, const int32_t* pos, int pos_count, int pos_host,
-                                   int clamp, int NL, int B, int H, int S, int D, int64_t ds_l,
-                                   int64_t ds_b, int64_t ds_h, int64_t ds_s, void* stream) {
+// Shared by the two entry points below: the arguments of one set of rows.
+static int scatter_args(ScatterArgs& a, const void* src_k, const void* src_v, void* dst_k, void* dst_v, int elem_bytes,
+                        const int32_t* pos, int pos_count, int pos_host, int clamp, int NL, int B, int H, int S, int D, int64_t ds_l,
+                        int64_t ds_b, int64_t ds_h, int64_t ds_s) {
   JPT_REQUIRE(src_k && dst_k, JPT_EINVAL, "kv_scatter_rows: null tensor");
   JPT_REQUIRE((src_v == nullptr) == (dst_v == nullptr), JPT_EINVAL, "kv_scatter_rows: src_v/dst_v mismatch");
   JPT_REQUIRE(elem_bytes == 1 || elem_bytes == 2 || elem_bytes == 4, JPT_EINVAL,
@@ -523,7 +527,7 @@ extern "C" int jpt_kv_scatter_rows(const void* src_k, const void* src_v, void* d
   JPT_REQUIRE(NL > 0 && B > 0 && H > 0 && D > 0 && S > 0, JPT_EINVAL, "kv_scatter_rows: bad shape");
   JPT_REQUIRE(pos == nullptr || pos_count == 1 || pos_count == B, JPT_EINVAL,
               "kv_scatter_rows: pos_count must be 1 or B");
-  ScatterArgs a{};
+  a = ScatterArgs{};
   a.src[0] = static_cast<const char*>(src_k); a.src[1] = static_cast<const char*>(src_v);
   a.dst[0] = static_cast<char*>(dst_k); a.dst[1] = static_cast<char*>(dst_v);
   a.pos = pos; a.pos_count = pos_count; a.pos_host = pos_host; a.clamp = clamp;
@@ -534,12 +538,38 @@ extern "C" int jpt_kv_scatter_rows(const void* src_k, const void* src_v, void* d
              a.ds_s % 16 == 0 && aligned(src_k, 16) && aligned(dst_k, 16) && aligned(src_v, 16) &&
              aligned(dst_v, 16);
   a.chunk = v16 ? 16 : elem_bytes;
-  const int64_t total = (int64_t)NL * B * H * (a.row_bytes / a.chunk);
-  int blocks = (int)((total + 255) / 256);
-  if (blocks > 148 * 16) blocks = 148 * 16;
-  dim3 grid(blocks, src_v ? 2 : 1);
-  scatter_rows_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(a);
+  return 0;
+}
+static int launch_scatter(const ScatterArgs& a, const ScatterArgs* more, cudaStream_t st) {
+  int64_t total = (int64_t)a.NL * a.B * a.H * (a.row_bytes / a.chunk);
+  if (more) total = std::max(total, (int64_t)more->NL * more->B * more->H * (more->row_bytes / more->chunk));
+  int blocks = (int)std::min<int64_t>((total + 255) / 256, 148 * 16);
+  scatter_rows_kernel<<<dim3(blocks, more ? 4 : a.src[1] ? 2 : 1), 256, 0, st>>>(a, more ? *more : a);
   return check_launch("scatter_rows_kernel");
+}
+
+extern "C" int jpt_kv_scatter_rows(const void* src_k, const void* src_v, void* dst_k, void* dst_v,
+                                   int elem_bytes, const int32_t* pos, int pos_count, int pos_host,
+                                   int clamp, int NL, int B, int H, int S, int D, int64_t ds_l,
+                                   int64_t ds_b, int64_t ds_h, int64_t ds_s, void* stream) {
+  ScatterArgs a;
+  if (int rc = scatter_args(a, src_k, src_v, dst_k, dst_v, elem_bytes, pos, pos_count, pos_host, clamp, NL, B, H, S, D, ds_l, ds_b,
+                            ds_h, ds_s))
+    return rc;
+  return launch_scatter(a, nullptr, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int jpt_kv_finalize_int8(const int8_t* new_k, const int8_t* new_v, int8_t* cache_k, int8_t* cache_v, const void* new_ks,
+                                    const void* new_vs, void* k_scaler, void* v_scaler, int scale_bytes, const int32_t* pos,
+                                    int pos_count, int pos_host, int NL, int B, int H, int S, int D, int64_t ds_l, int64_t ds_b,
+                                    int64_t ds_h, int64_t ds_s, int64_t ss_l, int64_t ss_b, int64_t ss_s, void* stream) {
+  ScatterArgs a, sc;
+  if (int rc = scatter_args(a, new_k, new_v, cache_k, cache_v, 1, pos, pos_count, pos_host, 1, NL, B, H, S, D, ds_l, ds_b, ds_h, ds_s))
+    return rc;
+  if (int rc = scatter_args(sc, new_ks, new_vs, k_scaler, v_scaler, scale_bytes, pos, pos_count, pos_host, 1, NL, B, 1, S, 1, ss_l,
+                            ss_b, 0, ss_s))
+    return rc;
+  return launch_scatter(a, &sc, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int jpt_kv_append_paged(const void* xk, const void* xv, int in_dtype, void* cache_k,

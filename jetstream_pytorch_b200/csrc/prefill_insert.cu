@@ -6,18 +6,22 @@
 namespace jpt {
 namespace {
 
+constexpr int kMaxLayers = 48, kMaxPages = 256;  // (the arguments stay below 4 KB)
+
 struct InsertArgs {
-  const void* prefix[2];
-  void* cache[2];
-  void* scaler[2];  // may be null
-  const int32_t* upd;  // paged: page ids
+  // the layers of the launch: their tensors lie where they lie (32 separately allocated layers are one launch, not 32)
+  const void* prefix[2][kMaxLayers];
+  void* cache[2][kMaxLayers];
+  void* scaler[2][kMaxLayers];  // may be null
+  const int32_t* upd;           // paged: page ids on the device, or null: the list below
+  int32_t pages[kMaxPages];     // page ids that travel with the launch (no copy to the device in front of it)
   int paged, wrap;
   int ntensors;  // 2 = K and V, 1 = a single tensor
   int slot, pos;
   int NL, H, L, Ltot, S, D, P, ps;
-  int64_t ps_l, ps_h, ps_t;        // prefix strides (elements)
-  int64_t cs_l, cs_b, cs_h, cs_s;  // cache strides (elements)
-  int64_t ss_l, ss_b, ss_s;        // scaler strides (elements)
+  int64_t ps_h, ps_t;        // prefix strides (elements)
+  int64_t cs_b, cs_h, cs_s;  // cache strides (elements)
+  int64_t ss_b, ss_s;        // scaler strides (elements)
 };
 
 struct Dest {
@@ -27,15 +31,15 @@ struct Dest {
   bool ok;
 };
 
-__device__ __forceinline__ Dest resolve(const InsertArgs& a, int l, int t) {
+__device__ __forceinline__ Dest resolve(const InsertArgs& a, int t) {
   Dest d;
   d.ok = true;
   if (a.paged) {
-    const int page = a.upd[t / a.ps], tok = t % a.ps;
+    const int tok = t % a.ps, page = a.upd ? a.upd[t / a.ps] : a.pages[t / a.ps];
     if (page < 0 || page >= a.P) d.ok = false;
-    d.row0 = l * a.cs_l + ((int64_t)page * a.ps + tok) * a.D;
+    d.row0 = ((int64_t)page * a.ps + tok) * a.D;
     d.hstep = (int64_t)a.P * a.ps * a.D;
-    d.sidx = l * a.ss_l + (int64_t)page * a.ps + tok;
+    d.sidx = (int64_t)page * a.ps + tok;
   } else {
     int s;
     if (a.wrap) {
@@ -45,9 +49,9 @@ __device__ __forceinline__ Dest resolve(const InsertArgs& a, int l, int t) {
       s = a.pos + t;  // pos already clamped on the host
       if (s < 0 || s >= a.S) d.ok = false;
     }
-    d.row0 = l * a.cs_l + (int64_t)a.slot * a.cs_b + (int64_t)s * a.cs_s;
+    d.row0 = (int64_t)a.slot * a.cs_b + (int64_t)s * a.cs_s;
     d.hstep = a.cs_h;
-    d.sidx = l * a.ss_l + (int64_t)a.slot * a.ss_b + (int64_t)s * a.ss_s;
+    d.sidx = (int64_t)a.slot * a.ss_b + (int64_t)s * a.ss_s;
   }
   return d;
 }
@@ -79,13 +83,13 @@ __device__ __forceinline__ void load_vec(const T* p, float (&v)[VEC]) {
 
 // grid (Ltot, 2, NL); one block per token of one tensor of one layer.
 template <typename T, int VEC, int NV>
-__global__ void __launch_bounds__(256) insert_quant_kernel(InsertArgs a) {
+__global__ void __launch_bounds__(256) insert_quant_kernel(const __grid_constant__ InsertArgs a) {
   __shared__ float red[33];
   const int t = blockIdx.x, which = blockIdx.y, l = blockIdx.z;
   const int HD = a.H * a.D;
-  const Dest dst = resolve(a, l, t);
-  int8_t* cache = static_cast<int8_t*>(a.cache[which]);
-  T* scaler = static_cast<T*>(a.scaler[which]);
+  const Dest dst = resolve(a, t);
+  int8_t* cache = static_cast<int8_t*>(a.cache[which][l]);
+  T* scaler = static_cast<T*>(a.scaler[which][l]);
   if (t >= a.L) {  // page tail: code 0, scale 0
     if (!dst.ok) return;
     for (int n = 0; n < NV; ++n) {
@@ -103,7 +107,7 @@ __global__ void __launch_bounds__(256) insert_quant_kernel(InsertArgs a) {
     if (threadIdx.x == 0 && scaler) scaler[dst.sidx] = from_f32<T>(0.f);
     return;
   }
-  const T* src = static_cast<const T*>(a.prefix[which]) + l * a.ps_l + (int64_t)t * a.ps_t;
+  const T* src = static_cast<const T*>(a.prefix[which][l]) + (int64_t)t * a.ps_t;
   float v[NV][VEC];
   float amax = 0.f;
 #pragma unroll
@@ -145,13 +149,13 @@ __global__ void __launch_bounds__(256) insert_quant_kernel(InsertArgs a) {
 // block barrier) and every lane has NVW independent loads in flight.  Used
 // when H*D is a multiple of 512.
 template <typename T, int NVW>
-__global__ void __launch_bounds__(256) insert_quant_warp_kernel(InsertArgs a) {
+__global__ void __launch_bounds__(256) insert_quant_warp_kernel(const __grid_constant__ InsertArgs a) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = blockIdx.x * 8 + warp, which = blockIdx.y, l = blockIdx.z;
   if (t >= a.Ltot) return;
-  const Dest dst = resolve(a, l, t);
-  int8_t* cache = static_cast<int8_t*>(a.cache[which]);
-  T* scaler = static_cast<T*>(a.scaler[which]);
+  const Dest dst = resolve(a, t);
+  int8_t* cache = static_cast<int8_t*>(a.cache[which][l]);
+  T* scaler = static_cast<T*>(a.scaler[which][l]);
   if (t >= a.L) {  // page tail: code 0, scale 0
     if (!dst.ok) return;
 #pragma unroll
@@ -163,7 +167,7 @@ __global__ void __launch_bounds__(256) insert_quant_warp_kernel(InsertArgs a) {
     if (lane == 0 && scaler) scaler[dst.sidx] = from_f32<T>(0.f);
     return;
   }
-  const T* src = static_cast<const T*>(a.prefix[which]) + l * a.ps_l + (int64_t)t * a.ps_t;
+  const T* src = static_cast<const T*>(a.prefix[which][l]) + (int64_t)t * a.ps_t;
   if constexpr (sizeof(T) == 2) {
     // bf16 tokens: the reference's chain is a chain of bf16 operations, which the packed bf16
     // instructions perform exactly (|x| and max are exact; the product of two bf16 values rounded
@@ -248,13 +252,13 @@ __global__ void __launch_bounds__(256) insert_quant_warp_kernel(InsertArgs a) {
 }
 
 // Same-dtype copy: one thread per chunk of `chunk` bytes.
-__global__ void insert_copy_kernel(InsertArgs a, int elem_bytes, int chunk) {
+__global__ void insert_copy_kernel(const __grid_constant__ InsertArgs a, int elem_bytes, int chunk) {
   const int which = blockIdx.y, l = blockIdx.z;
   const int row_bytes = a.D * elem_bytes;
   const int cpr = row_bytes / chunk;
   const int64_t total = (int64_t)a.Ltot * a.H * cpr;
-  const char* src = static_cast<const char*>(a.prefix[which]);
-  char* cache = static_cast<char*>(a.cache[which]);
+  const char* src = static_cast<const char*>(a.prefix[which][l]);
+  char* cache = static_cast<char*>(a.cache[which][l]);
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (int64_t)gridDim.x * blockDim.x) {
     // chunk fastest, then token, then head: consecutive threads walk one
@@ -263,10 +267,10 @@ __global__ void insert_copy_kernel(InsertArgs a, int elem_bytes, int chunk) {
     int64_t r = i / cpr;
     const int t = (int)(r % a.Ltot);
     const int h = (int)(r / a.Ltot);
-    const Dest dst = resolve(a, l, t);
+    const Dest dst = resolve(a, t);
     if (!dst.ok) continue;
     char* d = cache + (dst.row0 + h * dst.hstep) * elem_bytes + (int64_t)c * chunk;
-    const char* s = src + (l * a.ps_l + h * a.ps_h + (int64_t)t * a.ps_t) * elem_bytes + (int64_t)c * chunk;
+    const char* s = src + (h * a.ps_h + (int64_t)t * a.ps_t) * elem_bytes + (int64_t)c * chunk;
     const bool pad = t >= a.L;
     if (chunk == 16) {
       *reinterpret_cast<uint4*>(d) = pad ? make_uint4(0, 0, 0, 0) : *reinterpret_cast<const uint4*>(s);
@@ -280,12 +284,19 @@ __global__ void insert_copy_kernel(InsertArgs a, int elem_bytes, int chunk) {
   }
 }
 
+bool layers_aligned(const InsertArgs& a) {
+  for (int w = 0; w < a.ntensors; ++w)
+    for (int l = 0; l < a.NL; ++l)
+      if (!aligned(a.prefix[w][l], 16) || !aligned(a.cache[w][l], 16)) return false;
+  return true;
+}
+
 template <typename T>
 int launch_quant(const InsertArgs& a, cudaStream_t st) {
   const int HD = a.H * a.D;
-  bool vec_ok = a.D % 16 == 0 && a.ps_l % 8 == 0 && a.ps_h % 8 == 0 && a.ps_t % 8 == 0 &&
-                a.cs_l % 16 == 0 && a.cs_b % 16 == 0 && a.cs_h % 16 == 0 && a.cs_s % 16 == 0;
-  for (int w = 0; w < a.ntensors; ++w) vec_ok = vec_ok && aligned(a.prefix[w], 16) && aligned(a.cache[w], 16);
+  bool vec_ok = a.D % 16 == 0 && a.ps_h % 8 == 0 && a.ps_t % 8 == 0 &&
+                a.cs_b % 16 == 0 && a.cs_h % 16 == 0 && a.cs_s % 16 == 0;
+  vec_ok = vec_ok && layers_aligned(a);
   dim3 grid(a.Ltot, a.ntensors, a.NL);
   if (vec_ok && (HD == 512 || HD == 1024 || HD == 2048)) {
     const dim3 wgrid((a.Ltot + 7) / 8, a.ntensors, a.NL);
@@ -309,8 +320,7 @@ int launch_quant(const InsertArgs& a, cudaStream_t st) {
   return check_launch("insert_quant_kernel");
 }
 
-int launch_insert(InsertArgs& a, int in_dtype, int cache_dtype, cudaStream_t st) {
-  JPT_REQUIRE(a.prefix[0] && a.cache[0] && (a.ntensors == 1 || (a.prefix[1] && a.cache[1])), JPT_EINVAL, "prefill_insert: null tensor");
+int launch_layers(InsertArgs& a, int in_dtype, int cache_dtype, cudaStream_t st) {
   JPT_REQUIRE(a.NL > 0 && a.H > 0 && a.L >= 0 && a.D > 0, JPT_EINVAL, "prefill_insert: bad shape");
   if (a.Ltot == 0) return 0;
   if (cache_dtype == JPT_INT8 && in_dtype != JPT_INT8) {
@@ -323,9 +333,9 @@ int launch_insert(InsertArgs& a, int in_dtype, int cache_dtype, cudaStream_t st)
   JPT_REQUIRE(eb > 0, JPT_EINVAL, "prefill_insert: bad dtype");
   const int row_bytes = a.D * eb;
   bool v16 = row_bytes % 16 == 0;
-  const int64_t strides[] = {a.ps_l, a.ps_h, a.ps_t, a.cs_l, a.cs_b, a.cs_h, a.cs_s};
+  const int64_t strides[] = {a.ps_h, a.ps_t, a.cs_b, a.cs_h, a.cs_s};
   for (int64_t s : strides) v16 = v16 && (s * eb) % 16 == 0;
-  for (int w = 0; w < a.ntensors; ++w) v16 = v16 && aligned(a.prefix[w], 16) && aligned(a.cache[w], 16);
+  v16 = v16 && layers_aligned(a);
   const int chunk = v16 ? 16 : eb;
   const int64_t total = (int64_t)a.Ltot * a.H * (row_bytes / chunk);
   int blocks = (int)((total + 255) / 256);
@@ -334,10 +344,67 @@ int launch_insert(InsertArgs& a, int in_dtype, int cache_dtype, cudaStream_t st)
   return check_launch("insert_copy_kernel");
 }
 
+// The tensors of layer l of a call.
+struct LayerTensors {
+  const void *pk, *pv;
+  void *ck, *cv, *ks, *vs;
+};
+// Every layer of a call in launches of up to kMaxLayers; `at(l)` gives a layer's tensors.
+template <typename F>
+int launch_insert(InsertArgs& a, int NL, int in_dtype, int cache_dtype, cudaStream_t st, F at) {
+  JPT_REQUIRE(NL > 0, JPT_EINVAL, "prefill_insert: bad shape");
+  for (int l0 = 0; l0 < NL; l0 += kMaxLayers) {
+    a.NL = NL - l0 < kMaxLayers ? NL - l0 : kMaxLayers;
+    for (int l = 0; l < a.NL; ++l) {
+      const LayerTensors t = at(l0 + l);
+      JPT_REQUIRE(t.pk && t.ck && (a.ntensors == 1 || (t.pv && t.cv)), JPT_EINVAL, "prefill_insert: null tensor");
+      a.prefix[0][l] = t.pk, a.prefix[1][l] = t.pv;
+      a.cache[0][l] = t.ck, a.cache[1][l] = t.cv;
+      a.scaler[0][l] = t.ks, a.scaler[1][l] = t.vs;
+    }
+    if (int rc = launch_layers(a, in_dtype, cache_dtype, st)) return rc;
+  }
+  return 0;
+}
+inline const void* at_stride(const void* p, int64_t elements, int bytes) {
+  return p ? static_cast<const char*>(p) + elements * bytes : nullptr;
+}
+inline void* at_stride(void* p, int64_t elements, int bytes) { return p ? static_cast<char*>(p) + elements * bytes : nullptr; }
+
 }  // namespace
 }  // namespace jpt
 
 using namespace jpt;
+
+static int dense_args(InsertArgs& a, int slot, int pos, int wrap, int H, int L, int S, int D, int64_t ps_h, int64_t ps_t, int64_t cs_b,
+                      int64_t cs_h, int64_t cs_s, int64_t ss_b, int64_t ss_s) {
+  JPT_REQUIRE(S > 0 && slot >= 0, JPT_EINVAL, "prefill_insert_dense: bad slot or cache length");
+  JPT_REQUIRE(wrap || L <= S, JPT_ERANGE, "prefill_insert_dense: prefix longer than the cache (L=%d, S=%d)", L, S);
+  a.paged = 0; a.wrap = wrap; a.slot = slot; a.ntensors = 2;
+  if (!wrap) pos = pos < 0 ? 0 : (pos > S - L ? S - L : pos);  // dynamic_update_slice clamps
+  a.pos = pos;
+  a.H = H; a.L = L; a.Ltot = L; a.S = S; a.D = D;
+  a.ps_h = ps_h; a.ps_t = ps_t;
+  a.cs_b = cs_b; a.cs_h = cs_h; a.cs_s = cs_s;
+  a.ss_b = ss_b; a.ss_s = ss_s;
+  return 0;
+}
+static int paged_args(InsertArgs& a, const int32_t* update_indexes, const int32_t* pages_host, int n_pages, int H, int L, int P, int ps,
+                      int D, int64_t ps_h, int64_t ps_t) {
+  JPT_REQUIRE(update_indexes != nullptr || pages_host != nullptr || n_pages == 0, JPT_EINVAL, "prefill_insert_paged: null page list");
+  JPT_REQUIRE(P > 0 && ps > 0 && n_pages >= 0, JPT_EINVAL, "prefill_insert_paged: bad pool shape");
+  JPT_REQUIRE((int64_t)n_pages * ps >= L, JPT_ERANGE,
+              "prefill_insert_paged: %d pages of %d tokens cannot hold a prefix of %d", n_pages, ps, L);
+  if (!update_indexes) {
+    JPT_REQUIRE(n_pages <= kMaxPages, JPT_ERANGE, "prefill_insert_paged: a page list on the host holds up to %d pages", kMaxPages);
+    for (int i = 0; i < n_pages; ++i) a.pages[i] = pages_host[i];
+  }
+  a.upd = update_indexes;
+  a.paged = 1; a.ntensors = 2;
+  a.H = H; a.L = L; a.Ltot = n_pages * ps; a.D = D; a.P = P; a.ps = ps;
+  a.ps_h = ps_h; a.ps_t = ps_t;
+  return 0;
+}
 
 extern "C" int jpt_prefill_insert_dense(const void* prefix_k, const void* prefix_v, int in_dtype,
                                         void* cache_k, void* cache_v, int cache_dtype, void* k_scaler,
@@ -345,20 +412,25 @@ extern "C" int jpt_prefill_insert_dense(const void* prefix_k, const void* prefix
                                         int S, int D, int64_t ps_l, int64_t ps_h, int64_t ps_t,
                                         int64_t cs_l, int64_t cs_b, int64_t cs_h, int64_t cs_s,
                                         int64_t ss_l, int64_t ss_b, int64_t ss_s, void* stream) {
-  JPT_REQUIRE(S > 0 && slot >= 0, JPT_EINVAL, "prefill_insert_dense: bad slot or cache length");
-  JPT_REQUIRE(wrap || L <= S, JPT_ERANGE, "prefill_insert_dense: prefix longer than the cache (L=%d, S=%d)", L, S);
   InsertArgs a{};
-  a.prefix[0] = prefix_k; a.prefix[1] = prefix_v;
-  a.cache[0] = cache_k; a.cache[1] = cache_v;
-  a.scaler[0] = k_scaler; a.scaler[1] = v_scaler;
-  a.paged = 0; a.wrap = wrap; a.slot = slot; a.ntensors = 2;
-  if (!wrap) pos = pos < 0 ? 0 : (pos > S - L ? S - L : pos);  // dynamic_update_slice clamps
-  a.pos = pos;
-  a.NL = NL; a.H = H; a.L = L; a.Ltot = L; a.S = S; a.D = D;
-  a.ps_l = ps_l; a.ps_h = ps_h; a.ps_t = ps_t;
-  a.cs_l = cs_l; a.cs_b = cs_b; a.cs_h = cs_h; a.cs_s = cs_s;
-  a.ss_l = ss_l; a.ss_b = ss_b; a.ss_s = ss_s;
-  return launch_insert(a, in_dtype, cache_dtype, static_cast<cudaStream_t>(stream));
+  if (int rc = dense_args(a, slot, pos, wrap, H, L, S, D, ps_h, ps_t, cs_b, cs_h, cs_s, ss_b, ss_s)) return rc;
+  const int ib = dtype_bytes(in_dtype), cb = dtype_bytes(cache_dtype);
+  return launch_insert(a, NL, in_dtype, cache_dtype, static_cast<cudaStream_t>(stream), [&](int l) {
+    return LayerTensors{at_stride(prefix_k, l * ps_l, ib), at_stride(prefix_v, l * ps_l, ib), at_stride(cache_k, l * cs_l, cb),
+                        at_stride(cache_v, l * cs_l, cb), at_stride(k_scaler, l * ss_l, ib), at_stride(v_scaler, l * ss_l, ib)};
+  });
+}
+
+extern "C" int jpt_prefill_insert_dense_layers(const jpt_layer_tensors* layers, int NL, int in_dtype, int cache_dtype, int slot, int pos,
+                                               int wrap, int H, int L, int S, int D, int64_t ps_h, int64_t ps_t, int64_t cs_b,
+                                               int64_t cs_h, int64_t cs_s, int64_t ss_b, int64_t ss_s, void* stream) {
+  JPT_REQUIRE(layers, JPT_EINVAL, "prefill_insert_dense_layers: null list");
+  InsertArgs a{};
+  if (int rc = dense_args(a, slot, pos, wrap, H, L, S, D, ps_h, ps_t, cs_b, cs_h, cs_s, ss_b, ss_s)) return rc;
+  return launch_insert(a, NL, in_dtype, cache_dtype, static_cast<cudaStream_t>(stream), [&](int l) {
+    const jpt_layer_tensors& t = layers[l];
+    return LayerTensors{t.prefix_k, t.prefix_v, t.cache_k, t.cache_v, t.k_scaler, t.v_scaler};
+  });
 }
 
 extern "C" int jpt_prefill_insert_paged(const void* prefix_k, const void* prefix_v, int in_dtype,
@@ -367,20 +439,25 @@ extern "C" int jpt_prefill_insert_paged(const void* prefix_k, const void* prefix
                                         int NL, int H, int L, int P, int ps, int D, int64_t ps_l,
                                         int64_t ps_h, int64_t ps_t, int64_t cs_l, int64_t ss_l,
                                         void* stream) {
-  JPT_REQUIRE(update_indexes != nullptr || n_pages == 0, JPT_EINVAL, "prefill_insert_paged: null page list");
-  JPT_REQUIRE(P > 0 && ps > 0 && n_pages >= 0, JPT_EINVAL, "prefill_insert_paged: bad pool shape");
-  JPT_REQUIRE((int64_t)n_pages * ps >= L, JPT_ERANGE,
-              "prefill_insert_paged: %d pages of %d tokens cannot hold a prefix of %d", n_pages, ps, L);
   InsertArgs a{};
-  a.prefix[0] = prefix_k; a.prefix[1] = prefix_v;
-  a.cache[0] = cache_k; a.cache[1] = cache_v;
-  a.scaler[0] = k_scale_pool; a.scaler[1] = v_scale_pool;
-  a.upd = update_indexes;
-  a.paged = 1; a.ntensors = 2;
-  a.NL = NL; a.H = H; a.L = L; a.Ltot = n_pages * ps; a.D = D; a.P = P; a.ps = ps;
-  a.ps_l = ps_l; a.ps_h = ps_h; a.ps_t = ps_t;
-  a.cs_l = cs_l; a.ss_l = ss_l;
-  return launch_insert(a, in_dtype, cache_dtype, static_cast<cudaStream_t>(stream));
+  if (int rc = paged_args(a, update_indexes, nullptr, n_pages, H, L, P, ps, D, ps_h, ps_t)) return rc;
+  const int ib = dtype_bytes(in_dtype), cb = dtype_bytes(cache_dtype);
+  return launch_insert(a, NL, in_dtype, cache_dtype, static_cast<cudaStream_t>(stream), [&](int l) {
+    return LayerTensors{at_stride(prefix_k, l * ps_l, ib), at_stride(prefix_v, l * ps_l, ib), at_stride(cache_k, l * cs_l, cb),
+                        at_stride(cache_v, l * cs_l, cb), at_stride(k_scale_pool, l * ss_l, ib), at_stride(v_scale_pool, l * ss_l, ib)};
+  });
+}
+
+extern "C" int jpt_prefill_insert_paged_layers(const jpt_layer_tensors* layers, int NL, int in_dtype, int cache_dtype,
+                                               const int32_t* update_indexes, const int32_t* pages_host, int n_pages, int H, int L,
+                                               int P, int ps, int D, int64_t ps_h, int64_t ps_t, void* stream) {
+  JPT_REQUIRE(layers, JPT_EINVAL, "prefill_insert_paged_layers: null list");
+  InsertArgs a{};
+  if (int rc = paged_args(a, update_indexes, pages_host, n_pages, H, L, P, ps, D, ps_h, ps_t)) return rc;
+  return launch_insert(a, NL, in_dtype, cache_dtype, static_cast<cudaStream_t>(stream), [&](int l) {
+    const jpt_layer_tensors& t = layers[l];
+    return LayerTensors{t.prefix_k, t.prefix_v, t.cache_k, t.cache_v, t.k_scaler, t.v_scaler};
+  });
 }
 
 extern "C" int jpt_quantize_tokens(const void* w, int in_dtype, int token_major, int H, int L, int D,
@@ -389,18 +466,16 @@ extern "C" int jpt_quantize_tokens(const void* w, int in_dtype, int token_major,
   JPT_REQUIRE(in_dtype == JPT_BF16 || in_dtype == JPT_F32, JPT_EINVAL, "quantize_tokens: bad dtype");
   InsertArgs a{};
   a.ntensors = 1;
-  a.prefix[0] = w;
-  a.cache[0] = codes;
-  a.scaler[0] = scales;
   a.paged = 0; a.wrap = 0; a.slot = 0; a.pos = 0;
-  a.NL = 1; a.H = H; a.L = L; a.Ltot = L; a.S = L; a.D = D;
+  a.H = H; a.L = L; a.Ltot = L; a.S = L; a.D = D;
   if (token_major) {
     a.ps_h = D; a.ps_t = (int64_t)H * D; a.cs_h = D; a.cs_s = (int64_t)H * D;
   } else {
     a.ps_h = (int64_t)L * D; a.ps_t = D; a.cs_h = (int64_t)L * D; a.cs_s = D;
   }
   a.ss_s = 1;
-  return launch_insert(a, in_dtype, JPT_INT8, static_cast<cudaStream_t>(stream));
+  return launch_insert(a, 1, in_dtype, JPT_INT8, static_cast<cudaStream_t>(stream),
+                       [&](int) { return LayerTensors{w, nullptr, codes, nullptr, scales, nullptr}; });
 }
 
 // Lets kernels launched on `device` read the memory of `peer` (NVLink peer loads): what a decode GPU needs
