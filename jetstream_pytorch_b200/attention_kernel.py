@@ -9,7 +9,6 @@ The block-skipping tables `ragged_batch_index` / `ragged_block_index`
 bounds skip invalid blocks by themselves.
 """
 
-import ctypes
 import math
 
 import numpy as np
@@ -18,34 +17,6 @@ import torch
 from jetstream_pytorch_b200 import _lib
 
 DEFAULT_MASK_VALUE = -0.7 * float(np.finfo(np.dtype("float32")).max)
-
-_workspaces = {}  # (device, stream handle or None) -> grow-only scratch tensor
-
-
-def _workspace(device, nbytes):
-  """Grow-only attention scratch, allocated by torch and owned here, cleared
-  once when it is created as the kernel's arrival counters require.
-
-  Two launches that share a workspace must not overlap on the GPU, so every
-  stream gets its own.  CUDA graph captures run on a stream of their own and
-  must not allocate: they use one more workspace per device (key `None`) that
-  every eager call keeps at least as large as its own, so a shape that ran once
-  eagerly can be captured.  Graphs captured on one device share that
-  workspace: replay them on one stream, or on streams ordered by events."""
-  capturing = torch.cuda.is_current_stream_capturing()
-  stream = torch.cuda.current_stream(device)
-  keys = [(device, None)] if capturing else [(device, stream.cuda_stream), (device, None)]
-  for key in keys:
-    ws = _workspaces.get(key)
-    if ws is None or ws.numel() < nbytes:
-      if capturing:
-        raise RuntimeError("the attention workspace for CUDA graphs is too small and cannot grow during capture; "
-                           "call the same shape once before capturing")
-      ws = torch.empty(max(nbytes, 8 << 20), dtype=torch.uint8, device=device)
-      _lib.check(_lib.lib().jpt_flash_decode_workspace_init(_lib.ptr(ws), ws.numel(), stream.cuda_stream))
-      _workspaces[key] = ws
-  return _workspaces[keys[0]]
-
 
 def kernel_status(device=None):
   """0 if no attention kernel on `device` ever gave up on a bounded wait, else
@@ -56,8 +27,9 @@ def kernel_status(device=None):
   lib = _lib.lib()
   worst = 0
   devices = set()
-  for (dev, stream), ws in _workspaces.items():
-    if device is not None and torch.device(device) != dev:
+  for index, stream, ws in _lib.native.attention_workspaces():
+    dev = torch.device("cuda", index)
+    if device is not None and torch.device(device) not in (dev, torch.device("cuda")):
       continue
     devices.add(dev)
     with torch.cuda.device(dev):
@@ -86,13 +58,8 @@ def _flash_decode(q, k, v, *, paged=False, page_table=None, page_size=0, k_scale
                   scale_strides=(0, 0), mask_mode=_lib.MASK_NONE, start=None, end=None, mask=None,
                   mask_strides=(0, 0), sm_scale=1.0, kv_strides=(0, 0, 0), n_kv_heads=None, seq=None,
                   want_ml=True, num_splits=0, force_generic=False, static_scratch=False, out=None,
-                  logit_rounding=False, new_token=None):
-  """q [B,Hq,Tq,D] contiguous.  Returns o (q's shape and dtype), m, l float32
-  [B,Hq,Tq] (or None, None).
-
-  `new_token` (a `_lib.NewTokenStruct`, optional) routes the call through
-  `jpt_decode_update_attend`: the step's new K/V token is quantised, written
-  and attended to in the same launch (see `Int8KVCacheGenerate.update_and_attend`).
+                  logit_rounding=False):
+  """q [B,Hq,Tq,D].  Returns o (q's shape and dtype), m, l float32 [B,Hq,Tq] (or None, None).
 
   `out=(o, m, l)` (m, l may be None) makes the call write into tensors the
   caller already owns instead of creating new ones: a step loop that keeps its
@@ -102,101 +69,16 @@ def _flash_decode(q, k, v, *, paged=False, page_table=None, page_size=0, k_scale
   workspace tensor is created or passed, the kernels use the scratch array
   built into the library (for callers that must not allocate at this point;
   shapes needing more than its 16 MiB raise ValueError)."""
-  # (a transposed view of a prompt's projection stays as it is where the prefill kernel takes its strides: see below)
-  strided = q.shape[2] > 1 and q.shape[3] == 128 and not q.is_contiguous() and q.stride(3) == 1
-  if not strided:
-    q = q.contiguous()
-  b, hq, tq, d = q.shape
   dev = q.device
-  if dev.index is not None and dev.index != torch.cuda.current_device():
-    # launches go to the current device's stream and kernel attributes are per device
-    with torch.cuda.device(dev):
-      return _flash_decode(q, k, v, paged=paged, page_table=page_table, page_size=page_size, k_scale=k_scale,
-                           v_scale=v_scale, scale_strides=scale_strides, mask_mode=mask_mode, start=start, end=end,
-                           mask=mask, mask_strides=mask_strides, sm_scale=sm_scale, kv_strides=kv_strides,
-                           n_kv_heads=n_kv_heads, seq=seq, want_ml=want_ml, num_splits=num_splits,
-                           force_generic=force_generic, static_scratch=static_scratch, out=out,
-                           logit_rounding=logit_rounding, new_token=new_token)
-  for t in (k, v, k_scale, v_scale, mask):
-    if t is not None and t.device != dev:
-      raise ValueError(f"attention operands live on {t.device} and {dev}")
-  p = _lib.AttnParams()
-  p.q, p.q_dtype = _lib.ptr(q), _lib.dt(q)
-  p.B, p.Hq, p.Hkv, p.Tq, p.D = b, hq, n_kv_heads, tq, d
-  p.k, p.v, p.kv_dtype = _lib.ptr(k), _lib.ptr(v), _lib.dt(k)
-  p.paged = int(paged)
-  keep = [q, k, v]
-  if paged:
-    page_table = _lib.as_i32(page_table, dev).contiguous()
-    keep.append(page_table)
-    p.page_table, p.max_pages, p.page_size = _lib.ptr(page_table), page_table.shape[1], page_size
-    p.S = page_table.shape[1] * page_size
-    p.kv_h, p.kv_page = k.stride(0), k.stride(1)
-  else:
-    p.S = seq
-    p.kv_b, p.kv_h, p.kv_s = kv_strides
-  if k_scale is not None:
-    if k_scale.dtype != v_scale.dtype:
-      raise ValueError("k and v scales must share a dtype")
-    p.k_scale, p.v_scale, p.scale_dtype = _lib.ptr(k_scale), _lib.ptr(v_scale), _lib.dt(k_scale)
-    p.sc_b, p.sc_s = scale_strides
-    keep += [k_scale, v_scale]
-  p.mask_mode = mask_mode
-  if start is not None:
-    start = _lib.as_i32(start, dev).contiguous()
-    p.start = _lib.ptr(start)
-    keep.append(start)
-  if end is not None:
-    end = _lib.as_i32(end, dev).contiguous()
-    p.end = _lib.ptr(end)
-    keep.append(end)
-  if mask is not None:
-    p.mask = _lib.ptr(mask)
-    p.mk_b, p.mk_r = mask_strides
-    keep.append(mask)
-  p.sm_scale = sm_scale
-  m = l = None
-  if out is not None:
-    o, m, l = out
-    if o.shape != q.shape or o.dtype != q.dtype or o.device != dev or not o.is_contiguous():
-      raise ValueError("out[0] must be a contiguous tensor of the query's shape, dtype and device")
-    for t in (m, l):
-      if t is not None and (t.numel() != b * hq * tq or t.dtype != torch.float32 or t.device != dev
-                            or not t.is_contiguous()):
-        raise ValueError("out[1], out[2] must be contiguous float32 tensors of B*Hq*Tq elements")
-  else:
-    o = torch.empty((b, hq, tq, d), dtype=q.dtype, device=dev)
-    if want_ml:
-      m = torch.empty((b, hq, tq), dtype=torch.float32, device=dev)
-      l = torch.empty((b, hq, tq), dtype=torch.float32, device=dev)
-  p.o = _lib.ptr(o)
-  if m is not None and l is not None:
-    p.m, p.l = _lib.ptr(m), _lib.ptr(l)
-  p.num_splits, p.force_generic = num_splits, int(force_generic)
-  p.logit_rounding = int(logit_rounding)
-  lib = _lib.lib()
-  if strided and (static_scratch or new_token is not None
-                  or not lib.jpt_flash_attend_strided_q_ok(ctypes.byref(p), q.stride(0), q.stride(1), q.stride(2))):
-    q, strided = q.contiguous(), False
-    p.q = _lib.ptr(q)
-    keep.append(q)
-  if static_scratch:
-    if new_token is not None:
-      raise ValueError("the fused update needs a workspace that keeps its contents between calls")
-    _lib.check(lib.jpt_flash_decode_static(ctypes.byref(p), _lib.stream()))
-  else:
-    need = lib.jpt_flash_decode_workspace_bytes(ctypes.byref(p))
-    if need:
-      ws = _workspace(dev, need)
-      p.workspace, p.workspace_bytes = _lib.ptr(ws), ws.numel()
-    if strided:
-      _lib.check(lib.jpt_flash_attend_strided_q(ctypes.byref(p), q.stride(0), q.stride(1), q.stride(2), _lib.stream()))
-    elif new_token is not None:
-      _lib.check(lib.jpt_decode_update_attend(ctypes.byref(p), ctypes.byref(new_token), _lib.stream()))
-    else:
-      _lib.check(lib.jpt_flash_decode(ctypes.byref(p), _lib.stream()))
-  del keep
-  return o, m, l
+  return _lib.native.attend(q, k, v, k_scale, v_scale, _tensor_i32(page_table, dev) if paged else None,
+                            _tensor_i32(start, dev), _tensor_i32(end, dev), mask, mask_mode, *kv_strides, *scale_strides,
+                            *mask_strides, n_kv_heads, seq or 0, page_size, sm_scale, want_ml, logit_rounding, num_splits,
+                            int(force_generic), static_scratch, out)
+
+
+def _tensor_i32(x, device):
+  """Positions, lengths, tables as the native calls take them: tensors as they are, everything else as int32 on `device`."""
+  return x if x is None or isinstance(x, torch.Tensor) else _lib.as_i32(x, device)
 
 
 def _dense_kv(keys, values, layer):
@@ -267,6 +149,8 @@ def _mask_args(mask, q, s, n_kv_heads):
 def dense_attention(xq, keys, values, k_scaler=None, v_scaler=None, mask=None, **kw):
   """attention_kernel.py:605-633: masked softmax attention over the whole cache
   row; `mask` holds 0 / -inf (or any additive values).  Returns [B,Hq,T,D]."""
+  if not kw:
+    return _lib.native.dense(xq, keys, values, k_scaler, v_scaler, mask)
   k, v, strides, hkv, s = _dense_kv(keys, values, 0)
   ks, vs, sst = _dense_scales(k_scaler, v_scaler, 0)
   mode, mask, mst = _mask_args(mask, xq, s, hkv)
@@ -284,13 +168,8 @@ def flash_attention(xq, keys, values, layer, k_scaler=None, v_scaler=None, mask=
   """attention_kernel.py:636-710.  Returns o [B,Hq,T,D], (m, l) [B,Hq,T,1]
   float32: the row max of the logits and the softmax denominator (the v scale
   is applied to the numerator only)."""
-  k, v, strides, hkv, s = _dense_kv(keys, values, layer)
-  ks, vs, sst = _dense_scales(k_scaler, v_scaler, layer)
-  mode, mask, mst = _mask_args(mask, xq, s, hkv)
-  sm = 1.0 / math.sqrt(k.shape[-1]) if normalize_var else 1.0
-  o, m, l = _flash_decode(xq, k, v, k_scale=ks, v_scale=vs, scale_strides=sst, mask_mode=mode, mask=mask,
-                          mask_strides=mst, sm_scale=sm, kv_strides=strides, n_kv_heads=hkv, seq=s)
-  return o, (m.unsqueeze(-1), l.unsqueeze(-1))
+  o, m, l = _lib.native.flash(xq, keys, values, layer, k_scaler, v_scaler, mask, normalize_var)
+  return o, (m, l)
 
 
 def _ragged_per_head(q, k, v, layer, start, end, k_scaler, v_scaler, normalize_var, mode, **kw):
@@ -347,6 +226,10 @@ def ragged_mha(q, k, v, layer, start, end, ragged_batch_index=None, ragged_block
   `ring=True` selects the [start, end) ring semantics of `ragged_mqa` instead.
   """
   del ragged_batch_index, ragged_block_index, bk, mask_value, q_shard_axis, kv_shard_axis, testing
+  if not kw:
+    o, m, l = _lib.native.ragged(q, k, v, layer, _tensor_i32(start, q.device) if ring else None, _tensor_i32(end, q.device),
+                                 k_scaler, v_scaler, normalize_var, ring)
+    return o, (m, l)
   assert k.shape[-1] == q.shape[-1]
   assert k.shape[-4] == q.shape[-4]
   kk, vv, strides, hkv, s = _dense_kv(k, v, layer)
@@ -400,6 +283,9 @@ def call_paged_attention(env, xq, keys, values, seq_lens, page_indices, sm_scale
   hkv, _, ps, d = keys.shape
   if sm_scale is None:
     sm_scale = 1.0 / math.sqrt(d)
+  if not kw:
+    return _lib.native.paged(xq, keys, values, _tensor_i32(seq_lens, xq.device), _tensor_i32(page_indices, xq.device), sm_scale,
+                             k_scaler, v_scaler)
   o, _, _ = _flash_decode(xq.unsqueeze(2), keys, values, paged=True, page_table=page_indices, page_size=ps,
                           k_scale=k_scaler, v_scale=v_scaler, mask_mode=_lib.MASK_LENGTH, end=seq_lens,
                           sm_scale=sm_scale, n_kv_heads=hkv, want_ml=False, **kw)

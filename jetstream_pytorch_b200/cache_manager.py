@@ -7,9 +7,9 @@ Cache layouts (unchanged from the reference): dense [B,H,S,D] or stacked
 [NL,B,H,S,D]; int8 scalers [B,1,S,1] / [NL,B,1,S,1]; page pools [H,P,ps,D].
 """
 
-import numpy as np
 import ctypes
 
+import numpy as np
 import torch
 
 from jetstream_pytorch_b200 import _lib
@@ -51,40 +51,17 @@ class KVCachePrefill:
     return
 
 
-def _pos_args(input_pos, device, batch):
-  """(device int32 tensor or None, count, host value) for the C ABI."""
-  if isinstance(input_pos, torch.Tensor):
-    t = _lib.as_i32(input_pos.reshape(-1), device).contiguous()
-    n = t.numel()
-  elif isinstance(input_pos, (int, np.integer)):
-    return None, 1, int(input_pos), None
-  else:
-    arr = np.asarray(input_pos).reshape(-1)
-    if arr.size == 1:
-      return None, 1, int(arr[0]), None
-    t = _lib.as_i32(arr, device)
-    n = t.numel()
-  if n not in (1, batch):
-    raise ValueError(f"input_pos has {n} entries, expected 1 or {batch}")
-  return _lib.ptr(t), n, 0, t  # keep `t` alive until the launch is enqueued
+def _pos(input_pos, device):
+  """A step's position(s) as the native calls take them: an int for all slots, or a tensor."""
+  if isinstance(input_pos, (torch.Tensor, int)):
+    return input_pos
+  arr = np.asarray(input_pos).reshape(-1)
+  return int(arr[0]) if arr.size == 1 else _lib.as_i32(arr, device)
 
 
-def _scatter_rows(src_k, src_v, dst_k, dst_v, input_pos, clamp, nl, b, h, s, d, strides):
+def _scatter_rows(src_k, src_v, dst_k, dst_v, input_pos, clamp):
   """dst[l, b, h, pos_b, :] = src[l, b, h, :] for K and V (C ABI jpt_kv_scatter_rows)."""
-  p, n, host, keep = _pos_args(input_pos, dst_k.device, b)
-  ds_l, ds_b, ds_h, ds_s = strides
-  _lib.check(_lib.lib().jpt_kv_scatter_rows(
-      _lib.ptr(src_k), _lib.ptr(src_v), _lib.ptr(dst_k), _lib.ptr(dst_v), dst_k.element_size(),
-      p, n, host, int(clamp), nl, b, h, s, d, ds_l, ds_b, ds_h, ds_s, _lib.stream()))
-  del keep
-
-
-def _dense_strides(cache):
-  if cache.stride(-1) != 1:
-    raise ValueError("cache head_dim axis must be contiguous")
-  if cache.ndim == 5:
-    return cache.stride(0), cache.stride(1), cache.stride(2), cache.stride(3)
-  return 0, cache.stride(0), cache.stride(1), cache.stride(2)
+  _lib.native.scatter_rows(src_k, src_v, dst_k, dst_v, _pos(input_pos, dst_k.device), clamp)
 
 
 class KVCacheGenerate:
@@ -114,9 +91,12 @@ class KVCacheGenerate:
 
   def _write(self, cache_k, cache_v, key, value, clamp=False):
     """One row per (slot, head) into an unstacked [B,H,S,D] view."""
-    b, h, s, d = cache_k.shape
-    _scatter_rows(key.contiguous(), value.contiguous(), cache_k, cache_v, self.input_pos, clamp, 1, b, h, s, d,
-                  _dense_strides(cache_k))
+    _scatter_rows(key, value, cache_k, cache_v, self.input_pos, clamp)
+
+  def keeps_stacked(self, xq, xk, xv):
+    """True when the step's token is kept in the stacked `new_ks`, `new_vs` as it is and finalized later, so that
+    attention over the cache and the new token can keep it on the way."""
+    return isinstance(self.new_ks, torch.Tensor) and xk.dtype == xv.dtype == xq.dtype == self.cache_k.dtype and self.new_ks.ndim == 5
 
   def update(self, key, value, layer_id: int):
     """cache_manager.py:227-293."""
@@ -153,10 +133,8 @@ class KVCacheGenerate:
       self._write(self.cache_k, self.cache_v, self.new_ks, self.new_vs)
       return
     if env.generate_cache_stacked:
-      nl, b, h, s, d = self.cache_k.shape
       if env.new_cache_stacked:
-        _scatter_rows(self.new_ks, self.new_vs, self.cache_k, self.cache_v, self.input_pos, True, nl, b, h, s, d,
-                      _dense_strides(self.cache_k))
+        _scatter_rows(self.new_ks, self.new_vs, self.cache_k, self.cache_v, self.input_pos, True)
       else:
         for i in range(env.num_layers):
           self._write(self.cache_k[i], self.cache_v[i], self.new_ks[i], self.new_vs[i])
@@ -207,13 +185,9 @@ class Int8KVCacheGenerate:
     self.stacked = env.generate_cache_stacked
     if env.lazy_cache_update:
       if env.generate_cache_stacked:
-        layer, batch, heads, _, dim = cache_k.shape
-        dev = cache_k.device
         if env.new_cache_stacked:
-          self.new_ks = torch.zeros((layer, batch, heads, 1, dim), dtype=torch.int8, device=dev)
-          self.new_vs = torch.zeros((layer, batch, heads, 1, dim), dtype=torch.int8, device=dev)
-          self.new_k_scaler = torch.zeros((layer, batch, 1, 1, 1), dtype=env.default_type, device=dev)
-          self.new_v_scaler = torch.zeros((layer, batch, 1, 1, 1), dtype=env.default_type, device=dev)
+          self.new_ks, self.new_vs, self.new_k_scaler, self.new_v_scaler = _lib.native.kept_token(
+              cache_k, env.default_type == torch.float32)
         else:
           self.new_ks, self.new_vs, self.new_k_scaler, self.new_v_scaler = [], [], [], []
       else:
@@ -242,47 +216,9 @@ class Int8KVCacheGenerate:
   def _quant_append(self, xk, xv, cache_k, cache_v, k_scaler, v_scaler, outs=None, amax_in=None, peers=None):
     """Quantise the new token of every slot and (when a cache view is given)
     write codes and scale at this step's position: one launch for K and V."""
-    b, h, t, d = xk.shape
-    if t != 1:
-      raise ValueError("the decode cache takes one new token per step")
-    xk, xv = xk.contiguous(), xv.contiguous()
-    if outs is None:
-      kq = torch.empty((b, h, 1, d), dtype=torch.int8, device=xk.device)
-      vq = torch.empty((b, h, 1, d), dtype=torch.int8, device=xk.device)
-      ks = torch.empty((b, 1, 1, 1), dtype=xk.dtype, device=xk.device)
-      vs = torch.empty((b, 1, 1, 1), dtype=xk.dtype, device=xk.device)
-    else:
-      kq, vq, ks, vs = outs
-      if ks.dtype != xk.dtype or vs.dtype != xk.dtype:  # the kernel writes the scale in the input's dtype
-        raise ValueError(f"scale buffers of dtype {ks.dtype} cannot take the scales of {xk.dtype} inputs")
-      if kq.dtype != torch.int8 or vq.dtype != torch.int8:
-        raise ValueError("the buffers for the quantised new token must be int8")
-    p, n, host, keep = (None, 1, 0, None)
-    s = 1
-    cs = (0, 0, 0)
-    ss = (0, 0)
-    if cache_k is not None:
-      if k_scaler.dtype != xk.dtype:
-        raise ValueError(f"scaler dtype {k_scaler.dtype} differs from the input dtype {xk.dtype}")
-      s = cache_k.shape[2]
-      _, cs_b, cs_h, cs_s = _dense_strides(cache_k)
-      cs = (cs_b, cs_h, cs_s)
-      ss = (k_scaler.stride(0), k_scaler.stride(2))
-      p, n, host, keep = _pos_args(self.input_pos, xk.device, b)
-    if peers is not None:
-      if amax_in is not None:
-        raise ValueError("give either the reduced amax or the peer exchange, not both")
-      _lib.check(_lib.lib().jpt_kv_quant_append_dense_peers(
-          _lib.ptr(xk), _lib.ptr(xv), _lib.dt(xk), _lib.ptr(cache_k), _lib.ptr(cache_v), _lib.ptr(k_scaler),
-          _lib.ptr(v_scaler), _lib.ptr(kq), _lib.ptr(vq), _lib.ptr(ks), _lib.ptr(vs), p, n, host, b, h, s, d,
-          cs[0], cs[1], cs[2], ss[0], ss[1], ctypes.byref(peers.struct), _lib.stream()))
-    else:
-      _lib.check(_lib.lib().jpt_kv_quant_append_dense(
-          _lib.ptr(xk), _lib.ptr(xv), _lib.dt(xk), _lib.ptr(cache_k), _lib.ptr(cache_v), _lib.ptr(k_scaler),
-          _lib.ptr(v_scaler), _lib.ptr(kq), _lib.ptr(vq), _lib.ptr(ks), _lib.ptr(vs), p, n, host, b, h, s, d,
-          cs[0], cs[1], cs[2], ss[0], ss[1], _lib.ptr(amax_in), None, _lib.stream()))
-    del keep
-    return kq, vq, ks, vs
+    cache = None if cache_k is None else (cache_k, cache_v, k_scaler, v_scaler)
+    return _lib.native.quant_append(xk, xv, cache, 0, outs, None if cache is None else _pos(self.input_pos, xk.device), amax_in,
+                                    None if peers is None else ctypes.addressof(peers.struct))
 
   def local_amax(self, xk, xv):
     """Phase one of a head-sharded update: this rank's max |x| per slot over
@@ -348,11 +284,7 @@ class Int8KVCacheGenerate:
     """True when `update_and_attend` can run as ONE launch: dense int8 cache
     (not the lazily finalised stacked stash of several layers at once), head_dim
     128, one new token, at most 8 query rows per KV head."""
-    b, hq, tq, d = xq.shape
-    h = xk.shape[1]
-    return (d == 128 and tq == 1 and xk.shape[2] == 1 and hq % h == 0 and hq // h <= 8
-            and xk.dtype in (torch.bfloat16, torch.float32) and xq.dtype == torch.bfloat16
-            and self.k_scaler is not None and self.k_scaler.dtype == xk.dtype)
+    return _lib.native.fused_ok(xq, xk, self.k_scaler)
 
   def update_and_attend(self, xq, xk, xv, layer_id: int, start, end, ring=False, peers=None, out=None):
     """`update(xk, xv, layer_id)` and ragged attention of `xq` over the cache
@@ -386,44 +318,38 @@ class Int8KVCacheGenerate:
       end_all = torch.as_tensor(end).to(xq.device) + 1
       o, ml = ak.ragged_mha(xq, r[0], r[1], layer_id, start, end_all, None, None, r[4], r[5], ring=ring, out=out)
       return r, (o, ml[0], ml[1])
-    b, h, _, d = xk.shape
-    xk, xv = xk.contiguous(), xv.contiguous()
     lazy = env.lazy_cache_update
-    stash = None
-    if lazy and env.new_cache_stacked:
-      stash = (self.new_ks[layer_id], self.new_vs[layer_id], self.new_k_scaler[layer_id], self.new_v_scaler[layer_id])
-      if stash[2].dtype != xk.dtype:
-        raise ValueError(f"scale buffers of dtype {stash[2].dtype} cannot take the scales of {xk.dtype} inputs")
-    if stash is None:
-      stash = (torch.empty((b, h, 1, d), dtype=torch.int8, device=xk.device),
-               torch.empty((b, h, 1, d), dtype=torch.int8, device=xk.device),
-               torch.empty((b, 1, 1, 1), dtype=xk.dtype, device=xk.device),
-               torch.empty((b, 1, 1, 1), dtype=xk.dtype, device=xk.device))
-    kq, vq, ks, vs = stash
-    cache_k, cache_v, k_scaler, v_scaler = self.cache_k, self.cache_v, self.k_scaler, self.v_scaler
-    if cache_k.ndim == 5:
-      cache_k, cache_v, k_scaler, v_scaler = cache_k[layer_id], cache_v[layer_id], k_scaler[layer_id], v_scaler[layer_id]
-    nt = _lib.NewTokenStruct()
-    nt.xk, nt.xv, nt.in_dtype = _lib.ptr(xk), _lib.ptr(xv), _lib.dt(xk)
-    nt.write_cache = 0 if lazy else 1
-    nt.k_quant, nt.v_quant, nt.k_scale, nt.v_scale = _lib.ptr(kq), _lib.ptr(vq), _lib.ptr(ks), _lib.ptr(vs)
-    p, n, host, keep = _pos_args(self.input_pos, xk.device, b)
-    nt.pos, nt.pos_count, nt.pos_host = p, n, host
-    if peers is not None:
-      nt.px = ctypes.pointer(peers.struct)
-    o, (m, l) = ak.ragged_mha(xq, cache_k, cache_v, 0, start, end, None, None, k_scaler, v_scaler, ring=ring, out=out,
-                              new_token=nt)
-    del keep
-    if lazy:
-      if not env.new_cache_stacked:
-        if env.generate_cache_stacked:
-          self.new_ks.append(kq)
-          self.new_vs.append(vq)
-          self.new_k_scaler.append(ks)
-          self.new_v_scaler.append(vs)
-        else:
-          self.new_ks, self.new_vs, self.new_k_scaler, self.new_v_scaler = kq, vq, ks, vs
+    stacked_stash = lazy and env.new_cache_stacked
+    kq, vq, ks, vs, o, m, l = self._fused_step(xq, xk, xv, layer_id, start, end, ring, peers, out, False)
+    if stacked_stash:
+      kq, vq, ks, vs = kq[layer_id], vq[layer_id], ks[layer_id], vs[layer_id]
+    b, hq, tq, d = xq.shape
+    hkv = xk.shape[1]
+    o = o.reshape(b, hkv, hq // hkv * tq, d)
+    if m is not None:
+      m, l = m.reshape(b, hkv, -1), l.reshape(b, hkv, -1)
     return (self.cache_k, self.cache_v, kq, vq, self.k_scaler, self.v_scaler, ks, vs), (o, m, l)
+
+  def _fused_step(self, xq, xk, xv, layer_id, start, end, ring, peers, out, out_f32):
+    """The launch of `update_and_attend` with its bookkeeping: (codes and scales kept, as the stacked tensors where they
+    are stacked; o, m, l)."""
+    env = self.env
+    lazy = env.lazy_cache_update
+    outs = (self.new_ks, self.new_vs, self.new_k_scaler, self.new_v_scaler) if lazy and env.new_cache_stacked else None
+    if not isinstance(end, torch.Tensor):
+      end = _lib.as_i32(end, xq.device)
+    if ring and not isinstance(start, torch.Tensor):
+      start = _lib.as_i32(start, xq.device)
+    r = _lib.native.update_attend(xq, xk, xv, (self.cache_k, self.cache_v, self.k_scaler, self.v_scaler), layer_id, start, end,
+                                  ring, _pos(self.input_pos, xq.device), not lazy, outs, out_f32, out,
+                                  None if peers is None else ctypes.addressof(peers.struct))
+    if lazy and outs is None:
+      if env.generate_cache_stacked:
+        for kept, new in zip((self.new_ks, self.new_vs, self.new_k_scaler, self.new_v_scaler), r):
+          kept.append(new)
+      else:
+        self.new_ks, self.new_vs, self.new_k_scaler, self.new_v_scaler = r[:4]
+    return r
 
   def finalize(self):
     """cache_manager.py:584-657."""
@@ -433,24 +359,17 @@ class Int8KVCacheGenerate:
     if env.ring_buffer:
       # K and V only: the reference does not write the scalers here
       # (cache_manager.py:588-597)
-      b, h, s, d = self.cache_k.shape
-      _scatter_rows(self.new_ks, self.new_vs, self.cache_k, self.cache_v, self.input_pos, False, 1, b, h, s, d,
-                    _dense_strides(self.cache_k))
+      _scatter_rows(self.new_ks, self.new_vs, self.cache_k, self.cache_v, self.input_pos, False)
       return
     if env.generate_cache_stacked:
-      nl, b, h, s, d = self.cache_k.shape
       if env.new_cache_stacked:
         new = (self.new_ks, self.new_vs, self.new_k_scaler, self.new_v_scaler)
       else:
         new = tuple(torch.stack(x) for x in (self.new_ks, self.new_vs, self.new_k_scaler, self.new_v_scaler))
     else:
-      nl = 1
-      b, h, s, d = self.cache_k.shape
       new = (self.new_ks, self.new_vs, self.new_k_scaler, self.new_v_scaler)
-    _scatter_rows(new[0], new[1], self.cache_k, self.cache_v, self.input_pos, True, nl, b, h, s, d,
-                  _dense_strides(self.cache_k))
-    _scatter_rows(new[2], new[3], self.k_scaler, self.v_scaler, self.input_pos, True, nl, b, 1, s, 1,
-                  _dense_strides(self.k_scaler))
+    _lib.native.finalize_int8(*new, self.cache_k, self.cache_v, self.k_scaler, self.v_scaler,
+                              _pos(self.input_pos, self.cache_k.device))
 
 
 class PageKVCacheGenerate:
@@ -477,14 +396,10 @@ class PageKVCacheGenerate:
   def update(self, key, value, layer_id=0):
     """cache[h, page_j, tok_j, :] = key[slot_j, h, 0, :] for every active slot
     (cache_manager.py:681-706); `layer_id` is ignored as in the reference."""
-    h, p, ps, d = self.cache_k.shape
-    b = key.shape[0]
-    pti = _lib.as_i32(self.page_token_indices, key.device).contiguous()
-    n = pti.shape[1]
-    _lib.check(_lib.lib().jpt_kv_append_paged(
-        _lib.ptr(key.contiguous()), _lib.ptr(value.contiguous()), _lib.dt(key), _lib.ptr(self.cache_k),
-        _lib.ptr(self.cache_v), _lib.dt(self.cache_k), _lib.ptr(self.k_scaler), _lib.ptr(self.v_scaler),
-        _lib.ptr(pti), n, n, _lib.ptr(self.n_active_dev), b, h, p, ps, d, _lib.stream()))
+    pti = self.page_token_indices
+    if not isinstance(pti, torch.Tensor):
+      pti = _lib.as_i32(pti, key.device)
+    _lib.native.append_paged(key, value, self.cache_k, self.cache_v, self.k_scaler, self.v_scaler, pti, self.n_active_dev)
     return self.cache_k, self.cache_v
 
   def state(self):

@@ -82,6 +82,8 @@ def precompute_ragged_block_indices(env, start, input_pos):
   outside [start, end) are skipped.  The CUDA kernels skip by their loop bounds
   and ignore these tables; they are produced for callers that pass them on."""
   s, bk = env.cache_len, env.block_size
+  if start.is_cuda and start.dtype == input_pos.dtype == torch.int32 and start.is_contiguous() and input_pos.is_contiguous():
+    return _lib.native.engine_begin(start, input_pos, s, bk, None, False, 0)
   b_count = start.shape[0]
   end = ((start + input_pos) % s).reshape(b_count, 1)
   start = start.reshape(b_count, 1)
@@ -143,16 +145,19 @@ class KVCacheEngine:
     wrap; paged: reserve pages, then scatter) and write the slot's rows of
     tokens, mask, start, input_pos and lens."""
     env = self.env
-    decode_state.tokens[slot] = prefix.token.reshape(-1).to(decode_state.tokens.dtype)
+    ds, token = decode_state, prefix.token
+    if (self._native_step(ds) and token.is_cuda and token.numel() == 1 and token.dtype in (torch.int32, torch.int64)
+        and 0 <= slot < ds.tokens.shape[0] and token.device == ds.tokens.device):
+      rows = dict(tokens=ds.tokens, token=token)
+    else:
+      decode_state.tokens[slot] = prefix.token.reshape(-1).to(decode_state.tokens.dtype)
+      rows = {}
     if env.page_attention:
       insert_ops.insert_page_attention_with_reservation(
           self.page_attention_manager, prefix.caches, prefix.seq_len, decode_state.caches, slot,
           cache_scales=decode_state.cache_scales or None)
-      decode_state.mask[slot] = insert_ops.insert_mask_row(env.cache_len, 0, prefix.seq_len, False,
-                                                           decode_state.mask.device, decode_state.mask.dtype)
-      decode_state.start[slot] = 0
-      decode_state.input_pos[slot] = prefix.seq_len
-      decode_state.lens[slot] = 1
+      insert_ops.write_slot_rows(env.cache_len, slot, 0, prefix.seq_len, False, prefix.seq_len, decode_state.mask,
+                                 decode_state.start, decode_state.input_pos, decode_state.lens, **rows)
       self._host_pos[slot] = prefix.seq_len
       self._pam_device = None
       self.page_attention_manager.lengths_device = None
@@ -160,7 +165,7 @@ class KVCacheEngine:
       return decode_state
     insert_ops.insert(env, prefix.caches, prefix.seq_len, decode_state.caches, decode_state.cache_scales or None, slot,
                       decode_state.current_position, mask=decode_state.mask, start=decode_state.start,
-                      input_pos=decode_state.input_pos, lens=decode_state.lens)
+                      input_pos=decode_state.input_pos, lens=decode_state.lens, **rows)
     return decode_state
 
   # ------------------------------------------------------------------ one decode step
@@ -181,18 +186,32 @@ class KVCacheEngine:
               for (k, v), (ks, vs) in zip(decode_state.caches, scales)]
     return [cache_manager.KVCacheGenerate(k, v, input_indexes, None, env=env) for k, v in decode_state.caches]
 
+  @staticmethod
+  def _native_step(ds):
+    """Whether the step's bookkeeping can run on the state's tensors as they are: int32 rows and a bf16 / fp32 mask on the GPU."""
+    return (all(t.is_cuda and t.dtype == torch.int32 and t.is_contiguous() for t in (ds.tokens, ds.lens, ds.start, ds.input_pos))
+            and ds.tokens.numel() == ds.lens.numel() == ds.input_pos.numel() and ds.mask.is_cuda and ds.mask.ndim == 2
+            and ds.mask.dtype in (torch.bfloat16, torch.float32) and ds.mask.stride(1) == 1)
+
   def generate_impl(self, params: Any, decode_state: DecodeState, sampler=None, page_token_indices=None,
                     n_active_dev=None):
     """engine.py:751-848.  Returns (new DecodeState, result data [B, 3]:
     previous tokens | ones | lens, the layout of the reference's ResultTokens)."""
     env = self.env
     pos = decode_state.current_position
-    input_indexes = [pos] if env.ring_buffer else decode_state.input_pos
-    rbi, rbk = self.precompute_ragged_block_indices(decode_state)
-    rbi, rbk = rbi.reshape(-1), rbk.reshape(-1)
+    ring = bool(env.ring_buffer)
+    input_indexes = [pos] if ring else decode_state.input_pos
     mask = decode_state.mask
-    if not env.lazy_cache_update:
-      mask = update_mask(env, mask, pos, decode_state.input_pos)
+    native = self._native_step(decode_state)
+    if native:
+      # block tables and this step's mask entry in one launch
+      rbi, rbk = _lib.native.engine_begin(decode_state.start, decode_state.input_pos, env.cache_len, env.block_size,
+                                          None if env.lazy_cache_update else mask, ring, pos)
+    else:
+      rbi, rbk = self.precompute_ragged_block_indices(decode_state)
+      if not env.lazy_cache_update:
+        mask = update_mask(env, mask, pos, decode_state.input_pos)
+    rbi, rbk = rbi.reshape(-1), rbk.reshape(-1)
     caches_obj = self.make_caches(decode_state, input_indexes, page_token_indices, n_active_dev)
     logits = self.model_fn(params, decode_state.tokens, decode_state.input_pos, caches_obj,
                            mask.unsqueeze(1).unsqueeze(2), decode_state.start, rbi, rbk)
@@ -204,6 +223,14 @@ class KVCacheEngine:
       new_scales = [c.scalers() for c in caches_obj]
     elif decode_state.cache_scales:
       new_scales = decode_state.cache_scales
+    if native and sampler is None and logits.ndim == 3 and logits.is_cuda and logits.stride(2) == 1 and logits.dtype in (
+        torch.float32, torch.bfloat16) and logits.shape[0] == decode_state.input_pos.numel():
+      # greedy sampling, the advance of the positions, the result rows and (lazy updates) the mask in one launch
+      next_token, lens, input_pos, data = _lib.native.engine_end(
+          logits, decode_state.tokens, decode_state.lens, decode_state.input_pos, env.cache_len,
+          mask if env.lazy_cache_update else None, ring, pos)
+      return DecodeState(next_token, new_caches, new_scales, (pos + 1) % env.cache_len, lens, decode_state.start, input_pos,
+                         mask), data
     if env.lazy_cache_update:
       mask = update_mask(env, mask, pos, decode_state.input_pos)  # after the model: it used flash attention
     next_token = sampler(logits[:, -1]) if sampler else greedy_sampling(logits)

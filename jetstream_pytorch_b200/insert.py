@@ -86,8 +86,29 @@ def insert_mask_row(cache_len, pos, current_pos, wrap, device, dtype=torch.float
   return torch.where(cond, 0.0, float("-inf")).to(dtype)
 
 
+def write_slot_rows(cache_len, slot, pos, cur, wrap, seq_len, mask=None, start=None, input_pos=None, lens=None, tokens=None,
+                    token=None):
+  """The rows of one slot after an insert (those that are given): one launch where the tensors allow it."""
+  given = [t for t in (start, input_pos, lens, tokens) if t is not None]
+  if (all(t.is_cuda and t.dtype == torch.int32 and t.is_contiguous() and slot < t.shape[0] for t in given) and slot >= 0
+      and (mask is None or (mask.is_cuda and mask.ndim == 2 and mask.shape[1] == cache_len and slot < mask.shape[0]
+                            and mask.stride(1) == 1 and mask.dtype in (torch.bfloat16, torch.float32)))):
+    _lib.native.engine_slot(mask, cache_len, slot, pos, cur, wrap, pos % cache_len, seq_len, start, input_pos, lens, tokens, token)
+    return
+  if mask is not None:
+    mask[slot] = insert_mask_row(cache_len, pos, cur, wrap, mask.device, mask.dtype)
+  if start is not None:
+    start[slot] = pos % cache_len
+  if input_pos is not None:
+    input_pos[slot] = seq_len
+  if lens is not None:
+    lens[slot] = 1
+  if tokens is not None:
+    tokens[slot] = token.reshape(-1).to(tokens.dtype)
+
+
 def insert(env, prefix_caches, seq_len, caches, cache_scales, slot, current_position, *, mask=None, start=None,
-           input_pos=None, lens=None):
+           input_pos=None, lens=None, tokens=None, token=None):
   """`PyTorchEngine.insert`, engine.py:627-648, for the dense layouts.
 
   prefix_caches: [(k, v)] per layer, each [1,H,Lpad,D]; caches: [(k, v)] per
@@ -95,7 +116,7 @@ def insert(env, prefix_caches, seq_len, caches, cache_scales, slot, current_posi
   for int8.  Ring buffer: no wrap when 0 <= cur - seq_len and cur - seq_len +
   Lpad < S, else modular positions; left aligned: always position 0.
   Updates (in place, when given) mask[slot], start[slot], input_pos[slot],
-  lens[slot] exactly as engine.py:386-395 / 506-524 do."""
+  lens[slot] (and tokens[slot] from `token`) exactly as engine.py:386-395 / 506-524 do."""
   s = env.cache_len
   lpad = prefix_caches[0][0].shape[2]
   if env.ring_buffer:
@@ -106,20 +127,16 @@ def insert(env, prefix_caches, seq_len, caches, cache_scales, slot, current_posi
   else:
     wrap, pos, cur = False, 0, seq_len
   stacked = env.generate_cache_stacked
+  if _lib.native.insert_dense(prefix_caches, caches, cache_scales or None, slot, pos, wrap, stacked):
+    write_slot_rows(s, slot, pos, cur, wrap, seq_len, mask, start, input_pos, lens, tokens, token)
+    return caches, cache_scales
   for i, (pk, pv) in enumerate(prefix_caches):
     ck, cv = caches[0] if stacked else caches[i]
     ks = vs = None
     if cache_scales:
       ks, vs = cache_scales[0] if stacked else cache_scales[i]
     insert_dense(pk, pv, ck, cv, slot, pos, wrap=wrap, layer=i if stacked else None, k_scaler=ks, v_scaler=vs)
-  if mask is not None:
-    mask[slot] = insert_mask_row(s, pos, cur, wrap, mask.device, mask.dtype)
-  if start is not None:
-    start[slot] = pos % s
-  if input_pos is not None:
-    input_pos[slot] = seq_len
-  if lens is not None:
-    lens[slot] = 1
+  write_slot_rows(s, slot, pos, cur, wrap, seq_len, mask, start, input_pos, lens, tokens, token)
   return caches, cache_scales
 
 

@@ -44,13 +44,9 @@ class _AttentionKernelBase:
     env = self.env
     bsz, num_heads, _, head_dim = xq.shape
     impl = self.ragged_attention_new if keys.ndim == 4 else self.ragged_attention_orig
-    true_len = seqlen
+    # (The reference pads q to two rows for its decode kernels and drops the padded row again,
+    # layers.py:449-457, 619-623; these kernels take one row as it is.)
     paged = (not self.quantized) and env.page_attention
-    # q is padded to two rows unless grouped ragged attention takes it
-    # (layers.py:449-457, 619-623); the padded row is dropped again below.
-    if not (env.ragged_mha and n_rep > 1) and seqlen == 1 and not paged:
-      true_len = 2
-      xq = torch.nn.functional.pad(xq, (0, 0, 0, true_len - seqlen), "constant", 0)
     local_max = local_denom = None
     if env.ragged_mha and seqlen == 1 and keys.shape[-2] > 1:
       local_output, (local_max, local_denom) = impl(xq, keys, values, self.layer_id, start, end,
@@ -70,15 +66,10 @@ class _AttentionKernelBase:
     else:
       local_output = self.dense_attention(xq=xq, keys=keys, values=values, k_scaler=k_scaler,
                                           v_scaler=v_scaler, mask=local_mask)
-    local_output = local_output.reshape(bsz, num_heads, true_len, head_dim)
+    local_output = local_output.reshape(bsz, num_heads, seqlen, head_dim)
     if local_max is not None:
-      local_max = local_max.reshape(bsz, num_heads, true_len, 1)
-      local_denom = local_denom.reshape(bsz, num_heads, true_len, 1)
-    if true_len != seqlen:
-      local_output = local_output[:, :, 0:seqlen, :]
-      if local_max is not None:
-        local_max = local_max[:, :, 0:seqlen, :]
-        local_denom = local_denom[:, :, 0:seqlen, :]
+      local_max = local_max.reshape(bsz, num_heads, seqlen, 1)
+      local_denom = local_denom.reshape(bsz, num_heads, seqlen, 1)
     return local_output, (local_max, local_denom)
 
   @staticmethod
@@ -96,6 +87,12 @@ class AttentionKernel(_AttentionKernelBase):
     _, num_heads, seqlen, _ = xq.shape
     n_rep = num_heads // xk.shape[-3]
     args = (cache, start, end, ragged_batch_index, ragged_block_index, seqlen, n_rep)
+    env = self.env
+    if (env.lazy_cache_update and env.ragged_mha and seqlen == 1 and isinstance(end, torch.Tensor)
+        and getattr(cache, "keeps_stacked", None) and cache.keeps_stacked(xq, xk, xv)):
+      # Two launches instead of two copies + ragged attention + flash attention over the new token + merge (the steps
+      # below): the same softmax over the same tokens.
+      return _lib.native.attend_lazy(xq, xk, xv, cache.cache_k, cache.cache_v, self.layer_id, end, cache.new_ks, cache.new_vs)
     orig_keys, orig_values = cache.update(xk, xv, self.layer_id)
     existing_output, (existing_max, existing_denom) = self._attend(xq, orig_keys, orig_values, None, None, mask,
                                                                    *args)
@@ -116,14 +113,18 @@ class Int8KVAttentionKernel(_AttentionKernelBase):
     bsz, num_heads, seqlen, head_dim = xq.shape
     n_rep = num_heads // xk.shape[-3]
     args = (cache, start, end, ragged_batch_index, ragged_block_index, seqlen, n_rep)
-    if (self.fused_step and self.env.ragged_mha and self.env.lazy_cache_update and n_rep > 1 and seqlen == 1
-        and hasattr(cache, "update_and_attend") and cache.fused_step_supported(xq, xk)):
+    env = self.env
+    if (self.fused_step and env.ragged_mha and env.lazy_cache_update and n_rep > 1 and seqlen == 1
+        and getattr(cache, "fused_step_supported", None) and cache.fused_step_supported(xq, xk)):
       # One launch instead of update + ragged attention over the cache + flash attention over the
-      # new token + merge (the four steps below): the same softmax over the same tokens.
-      _, (out, _, _) = cache.update_and_attend(xq, xk, xv, self.layer_id, start, end)
-      return out.reshape(bsz, num_heads, seqlen, head_dim).float()  # the merge of the four-step form yields float32
+      # new token + merge (the four steps below): the same softmax over the same tokens, in float32 as the merge yields it.
+      return cache._fused_step(xq, xk, xv, self.layer_id, start, end, False, None, None, True)[4]
     (orig_keys, orig_values, new_key, new_value, k_scaler, v_scaler, new_k_scaler,
      new_v_scaler) = cache.update(xk, xv, self.layer_id)
+    if env.lazy_cache_update and env.ragged_mha and seqlen == 1 and isinstance(end, torch.Tensor) and new_key is not None:
+      # the new token's attention and the merge in one launch behind the ragged attention
+      return _lib.native.attend_lazy_int8(xq, (orig_keys, orig_values, k_scaler, v_scaler), self.layer_id, end, new_key, new_value,
+                                          new_k_scaler, new_v_scaler)
     existing_output, (existing_max, existing_denom) = self._attend(xq, orig_keys, orig_values, k_scaler,
                                                                    v_scaler, mask, *args)
     if not self.env.lazy_cache_update or seqlen > 1:
@@ -200,14 +201,15 @@ class WeightOnlyPerChannelQuantizedLinear(torch.nn.Module):
     if inputs.dtype != torch.bfloat16:
       raise NotImplementedError(f"activations must be bfloat16, got {inputs.dtype}")
     k, n = self.in_features, self.out_features
-    x = inputs.reshape(-1, k)
-    m = x.shape[0]
+    if inputs.shape[-1] != k:
+      inputs = inputs.reshape(-1, k)
+    m = inputs.numel() // k
     if m < 1:
       return inputs.new_empty((*inputs.shape[:-1], n))
     if tp is not None:
       if levels is not None or m > ActivationLevels.MAX_ROWS:
         raise NotImplementedError("the row-parallel form takes up to 128 rows of bf16 activations")
-      x = x.contiguous()
+      x = inputs.reshape(-1, k).contiguous()
       lib = _lib.lib()
       need = lib.jpt_w8a16_linear_workspace_bytes(m, n, k)
       if self._workspace is None or self._workspace.numel() < need or self._workspace.device != x.device:
@@ -220,22 +222,10 @@ class WeightOnlyPerChannelQuantizedLinear(torch.nn.Module):
     if levels is not None:
       if (levels.rows, levels.features) != (m, k):
         raise ValueError(f"levels of a [{levels.rows}, {levels.features}] activation given for [{m}, {k}]")
-      y = torch.empty((m, n), dtype=torch.bfloat16, device=x.device)
-      ws = levels.workspace
-      _lib.check(_lib.lib().jpt_w8a16_linear_from_levels(_lib.ptr(ws), ws.numel(), _lib.ptr(self.weight),
-                                                         _lib.ptr(self.weight_scaler), _lib.ptr(y), m, n, k, _lib.stream()))
-      self._workspace = ws  # (kernel_status reads the status word of the workspace last used)
-      return y.reshape(*inputs.shape[:-1], n)
-    if not x.is_contiguous():
-      x = x.contiguous()
-    lib = _lib.lib()
-    need = lib.jpt_w8a16_linear_workspace_bytes(m, n, k)
-    if self._workspace is None or self._workspace.numel() < need or self._workspace.device != x.device:
-      self._workspace = torch.empty((need,), dtype=torch.uint8, device=x.device)
-    y = torch.empty((m, n), dtype=torch.bfloat16, device=x.device)
-    _lib.check(lib.jpt_w8a16_linear(_lib.ptr(x), _lib.ptr(self.weight), _lib.ptr(self.weight_scaler), _lib.ptr(y), m, n,
-                                    k, _lib.ptr(self._workspace), self._workspace.numel(), _lib.stream()))
-    return y.reshape(*inputs.shape[:-1], n)
+      self._workspace = levels.workspace  # (kernel_status reads the status word of the workspace last used)
+      return _lib.native.linear_from_levels(inputs, levels.workspace, self.weight, self.weight_scaler)
+    y, self._workspace = _lib.native.linear(inputs, self.weight, self.weight_scaler, self._workspace)
+    return y
 
 
 class ActivationLevels:
@@ -245,13 +235,20 @@ class ActivationLevels:
 
   MAX_ROWS = 128
 
-  def __init__(self, rows, features, device):
-    if not 1 <= rows <= self.MAX_ROWS or features % 128:
-      raise NotImplementedError(f"levels are kept for 1 .. {self.MAX_ROWS} rows of a multiple of 128 features, "
-                                f"got [{rows}, {features}]")
+  def __init__(self, rows, features, device, workspace=None):
+    self.check(rows, features)
     self.rows, self.features = rows, features
-    need = _lib.lib().jpt_w8a16_linear_workspace_bytes(rows, 1, features)
-    self.workspace = torch.empty((need,), dtype=torch.uint8, device=device)
+    if workspace is None:
+      need = _lib.lib().jpt_w8a16_linear_workspace_bytes(rows, 1, features)
+      workspace = torch.empty((need,), dtype=torch.uint8, device=device)
+    self.workspace = workspace
+
+  @classmethod
+  def check(cls, rows, features):
+    if not 1 <= rows <= cls.MAX_ROWS or features % 128:
+      raise NotImplementedError(f"levels are kept for 1 .. {cls.MAX_ROWS} rows of a multiple of 128 features, "
+                                f"got [{rows}, {features}]")
+    return rows
 
   @classmethod
   def fits(cls, x):
@@ -279,31 +276,24 @@ class RMSNorm(torch.nn.Module):
     """Returns y, or (y, ActivationLevels of y) with `with_levels`."""
     if x.dtype != torch.bfloat16 or self.weight.dtype != torch.bfloat16:
       raise NotImplementedError("RMSNorm is provided for bfloat16 activations and weights")
+    if not with_levels:
+      return _lib.native.rmsnorm(x, self.weight, self.eps, False)[0]
     k = x.shape[-1]
-    x2 = x.reshape(-1, k).contiguous()
-    m = x2.shape[0]
-    y = torch.empty_like(x2)
-    lv = ActivationLevels(m, k, x.device) if with_levels else None
-    _lib.check(_lib.lib().jpt_rmsnorm(_lib.ptr(x2), _lib.ptr(self.weight), float(self.eps), _lib.ptr(y), m, k,
-                                      _lib.ptr(lv.workspace) if lv else None, lv.workspace.numel() if lv else 0,
-                                      _lib.stream()))
-    y = y.reshape(x.shape)
-    return (y, lv) if with_levels else y
+    m = ActivationLevels.check(x.numel() // k, k)
+    y, ws = _lib.native.rmsnorm(x, self.weight, self.eps, True)
+    return y, ActivationLevels(m, k, x.device, ws)
 
 
 def silu_mul(a, b, with_levels=False):
   """bf16(bf16(silu(a)) * b); with `with_levels` also the level split of the result."""
   if a.dtype != torch.bfloat16 or b.dtype != torch.bfloat16 or a.shape != b.shape:
     raise NotImplementedError("silu_mul takes two bfloat16 tensors of one shape")
+  if not with_levels:
+    return _lib.native.silu_mul(a, b, False)[0]
   k = a.shape[-1]
-  a2, b2 = a.reshape(-1, k).contiguous(), b.reshape(-1, k).contiguous()
-  m = a2.shape[0]
-  h = torch.empty_like(a2)
-  lv = ActivationLevels(m, k, a.device) if with_levels else None
-  _lib.check(_lib.lib().jpt_silu_mul(_lib.ptr(a2), _lib.ptr(b2), _lib.ptr(h), m, k, _lib.ptr(lv.workspace) if lv else None,
-                                     lv.workspace.numel() if lv else 0, _lib.stream()))
-  h = h.reshape(a.shape)
-  return (h, lv) if with_levels else h
+  m = ActivationLevels.check(a.numel() // k, k)
+  h, ws = _lib.native.silu_mul(a, b, True)
+  return h, ActivationLevels(m, k, a.device, ws)
 
 
 class FeedForward(torch.nn.Module):
