@@ -507,9 +507,9 @@ int jpt_merge_partials(const void* o1, const float* m1, const float* l1,
  * WeightOnlyPerChannelQuantizedLinear.forward with symmetric weights and
  * without activation quantisation, jetstream_pt/layers.py:141-166:
  *   y = bf16(bf16(x @ W^T) * w_scale)
- *   x        [M, K] bf16, K a multiple of 128, 16-byte aligned; made for decode
- *            batches: up to 128 rows stream the weights once, more rows are
- *            taken in blocks of 128 (each block streams the weights again)
+ *   x        [M, K] bf16, K a multiple of 128, 16-byte aligned; up to 128 rows
+ *            (decode batches) stream the weights once, more rows (prompts) go to
+ *            a compute-bound tile kernel
  *   w        [N, K] int8 (one row per output channel), 16-byte aligned
  *   w_scale  [N] bf16
  *   y        [M, N] bf16 out
@@ -524,6 +524,16 @@ size_t jpt_w8a16_linear_workspace_bytes(int M, int N, int K);
 int jpt_w8a16_linear(const void* x, const void* w, const void* w_scale, void* y,
                      int M, int N, int K, void* workspace,
                      size_t workspace_bytes, void* stream);
+
+/*
+ * The two projections of the feed-forward block and its gate in one launch behind
+ * the level split (third_party/llama/model_exportable.py:84-86, for prompts: any
+ * number of rows): h[m,n] = bf16(bf16(silu(y1)) * y3) with y1, y3 the layers of
+ * (w1, w1_scale) and (w3, w3_scale) as above, h [M,N] bf16.
+ */
+size_t jpt_w8a16_gate_workspace_bytes(int M, int N, int K);
+int jpt_w8a16_gate(const void* x, const void* w1, const void* w1_scale, const void* w3, const void* w3_scale, void* h, int M,
+                   int N, int K, void* workspace, size_t workspace_bytes, void* stream);
 
 /*
  * The same layer in two steps, for activations that feed several layers (wq /

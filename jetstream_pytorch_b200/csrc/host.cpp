@@ -963,6 +963,22 @@ PyObject* linear(Args a, Py_ssize_t n) {
   return tuple(y, ws);
 }
 
+// gate(x [...,K], w1, s1, w3, s3) -> h [...,N], workspace: bf16(silu(x w1)) * (x w3)
+PyObject* gate(Args a, Py_ssize_t n) {
+  expect(n, 5, "gate");
+  const Tensor x = dense(tensor(a[0]));
+  const Tensor &w1 = tensor(a[1]), &s1 = tensor(a[2]), &w3 = tensor(a[3]), &s3 = tensor(a[4]);
+  const c10::Device dev = x.device();
+  OnDevice on(dev);
+  const int64_t out = w1.size(0), k = w1.size(1), m = x.numel() / k;
+  if (w3.sizes() != w1.sizes()) fail(PyExc_ValueError, "gate: w1 and w3 differ in shape");
+  Tensor ws = scratch(nullptr, jpt_w8a16_gate_workspace_bytes((int)m, (int)out, (int)k), dev);
+  Tensor h = empty(with_last(x, out), ScalarType::BFloat16, dev);
+  check(jpt_w8a16_gate(ptr(x), ptr(w1), ptr(s1), ptr(w3), ptr(s3), ptr(h), (int)m, (int)out, (int)k, ptr(ws), (size_t)ws.numel(),
+                       stream_of(dev)));
+  return tuple(h, ws);
+}
+
 // linear_from_levels(x [...,K] for its shape, levels workspace, weight, scale) -> y
 PyObject* linear_from_levels(Args a, Py_ssize_t n) {
   expect(n, 4, "linear_from_levels");
@@ -1038,7 +1054,7 @@ PyMethodDef methods[] = {
     JPT_METHOD("kept_token", kept_token), JPT_METHOD("append_paged", append_paged), JPT_METHOD("page_token_indices", page_token_indices),
     JPT_METHOD("insert_dense", insert_dense), JPT_METHOD("insert_paged", insert_paged), JPT_METHOD("engine_begin", engine_begin),
     JPT_METHOD("engine_end", engine_end), JPT_METHOD("engine_slot", engine_slot), JPT_METHOD("linear", linear),
-    JPT_METHOD("linear_from_levels", linear_from_levels), JPT_METHOD("rmsnorm", rmsnorm), JPT_METHOD("silu_mul", silu_mul),
+    JPT_METHOD("gate", gate), JPT_METHOD("linear_from_levels", linear_from_levels), JPT_METHOD("rmsnorm", rmsnorm), JPT_METHOD("silu_mul", silu_mul),
     JPT_METHOD("attention_workspaces", attention_workspaces), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

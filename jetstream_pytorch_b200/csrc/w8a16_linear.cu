@@ -153,6 +153,17 @@ __device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v));
 }
 
+__device__ __forceinline__ bool elect_sync() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(r));
+  return r != 0;
+}
+__device__ __forceinline__ void tmem_ld_8(uint32_t addr, uint32_t (&v)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "r"(addr));
+}
+
 // 32 consecutive accumulator columns of this thread's lane
 __device__ __forceinline__ void tmem_ld_32(uint32_t addr, uint32_t (&v)[32]) {
   asm volatile(
@@ -167,7 +178,7 @@ __device__ __forceinline__ void tmem_ld_32(uint32_t addr, uint32_t (&v)[32]) {
 
 // ---------------------------------------------------------------- (1) activation levels
 // x [M, K] bf16 -> levels [2 Mp, K] int8 (rows 0 .. M-1: h, rows Mp .. Mp+M-1: l, the others zero)
-// and xs[m] = s_m / 254.
+// and xs[m] = s_m / 254.  More than 128 rows: one such matrix per block of Mp rows, one after the other.
 __global__ void __launch_bounds__(256) x_levels_kernel(const __nv_bfloat16* x, int8_t* lev, float* xs, int* status, int M,
                                                        int Mp, int K, int clear_status, unsigned* launch_counter) {
   __shared__ float red[33];
@@ -175,8 +186,8 @@ __global__ void __launch_bounds__(256) x_levels_kernel(const __nv_bfloat16* x, i
   grid_dependency_trigger();
   if (m == 0 && tid == 0 && clear_status) *status = 0;
   if (m == 0 && tid == 0 && launch_counter) *launch_counter += 1u;  // (one thread, launches in stream order)
-  uint2* hrow = reinterpret_cast<uint2*>(lev + (int64_t)m * K);
-  uint2* lrow = reinterpret_cast<uint2*>(lev + (int64_t)(Mp + m) * K);
+  uint2* hrow = reinterpret_cast<uint2*>(lev + (int64_t)(m + m / Mp * Mp) * K);
+  uint2* lrow = reinterpret_cast<uint2*>(lev + (int64_t)(m + m / Mp * Mp + Mp) * K);
   const int nvec = K / 8;  // eight elements per step: 16 bytes in, 8 + 8 bytes out
   if (m >= M) {  // padding rows of the level matrix
     for (int v = tid; v < nvec; v += 256) hrow[v] = lrow[v] = make_uint2(0u, 0u);
@@ -367,6 +378,14 @@ __global__ void __launch_bounds__(kRowThreads) rmsnorm_levels_kernel(const __nv_
   if (gridDim.x > 1) cluster_sync();  // (no CTA leaves while a peer may still store into its slots)
 }
 
+// One value of the gate: bf16(bf16(silu(a)) * b).  (Fast exponential and division: the quotient is rounded to bf16, and the
+// exact forms are subroutines.)
+__device__ __forceinline__ __nv_bfloat16 gate_value(__nv_bfloat16 a, __nv_bfloat16 b) {
+  const float f = __bfloat162float(a);
+  const float s = __bfloat162float(__float2bfloat16_rn(__fdividef(f, 1.f + __expf(-f))));
+  return __float2bfloat16_rn(s * __bfloat162float(b));
+}
+
 // The feed-forward block's gate (third_party/llama/model_exportable.py:84-86): h = bf16(bf16(silu(a)) * b), and with
 // `lev` the levels of h for the down projection.
 __global__ void __launch_bounds__(kRowThreads) silu_mul_levels_kernel(const __nv_bfloat16* a, const __nv_bfloat16* b, __nv_bfloat16* h,
@@ -391,10 +410,7 @@ __global__ void __launch_bounds__(kRowThreads) silu_mul_levels_kernel(const __nv
     const __nv_bfloat16* eb = reinterpret_cast<const __nv_bfloat16*>(&rb);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const float f = __bfloat162float(ea[j]);
-      // (fast exponential and division: the quotient is rounded to bf16, and the exact forms are subroutines)
-      const float s = __bfloat162float(__float2bfloat16_rn(__fdividef(f, 1.f + __expf(-f))));
-      o[j] = __float2bfloat16_rn(s * __bfloat162float(eb[j]));
+      o[j] = gate_value(ea[j], eb[j]);
     }
   };
   write_row_and_levels(gated, reinterpret_cast<uint4*>(h + (int64_t)m * K), v_lo, nvec, lev != nullptr, hrow, lrow, xs, m, red,
@@ -690,6 +706,201 @@ __global__ void __launch_bounds__(kThreadsL, 1)
   }
 }
 
+// ---------------------------------------------------------------- more than 128 rows (prefill)
+// Bound: the integer MMAs (two levels: 4 M N K operations).  Weights as the M = 128 operand twice (256 channels), a block of up
+// to 128 rows as the N operand (h rows, then l rows), accumulators in all of tensor memory; persistent CTAs, one per SM,
+// walk the tiles with the row blocks fastest, so that the CTAs of a moment share weight tiles in L2.  A tile step (128 bytes
+// of K) reads 64 KB for 1024 cycles of MMA.  The ring keeps filling under the epilogue; the accumulators do not double.
+// The 128-row blocks through the decode kernel that this replaces streamed the weights again for every block and paid its
+// set-up and cluster reduction each time: 27 us per block of 4096 x 14336, where this takes 15.
+//   warp 0 requests tiles, warp 1 issues MMAs, warps 2-9 run the epilogue (a warp owns 32 TMEM lanes = channels and half
+//   of the block's rows).
+// Two forms: a layer (256 channels of one weight matrix), and the feed-forward block's gate (128 channels of w1 and the same 128
+// of w3: the thread that has both writes bf16(silu(a)) * b, so that neither projection goes through memory).
+constexpr int kThreadsT = 320;
+struct __align__(1024) SmemT {
+  uint8_t w[kStages][kTileN * kTileK];
+  uint8_t x[kStages][2 * kMaxM * kTileK];
+  uint64_t full[kStages], empty[kStages], acc_full, acc_empty;
+  uint32_t tmem_base;
+  volatile int dead;
+};
+struct TileMaps {
+  CUtensorMap w0, w1, x;  // w1: the second matrix of the gate form
+};
+struct TileArgs {
+  const float* xs;               // [blocks * Rb]
+  const __nv_bfloat16 *s0, *s1;  // channel scales
+  __nv_bfloat16* y;
+  int M, N, Rb, blocks, k_tiles, tiles;
+};
+
+template <bool kGate>
+__global__ void __launch_bounds__(kThreadsT, 1)
+    w8a16_tiles_kernel(const __grid_constant__ TileMaps maps, const __grid_constant__ TileArgs a, int* status) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  SmemT& sm = *reinterpret_cast<SmemT*>(smem_raw);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if ((smem_addr(smem_raw) & 1023u) != 0u) {
+    grid_dependency_wait();
+    if (tid == 0) atomicExch(status, 2);
+    return;
+  }
+  const int n_mma = 2 * a.Rb;
+  constexpr int kChannels = kGate ? 128 : 256;  // output channels of a tile
+  if (tid == 0) {
+    for (int s = 0; s < kStages; ++s) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&sm.full[s])));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&sm.empty[s])));
+    }
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&sm.acc_full)));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 256;" ::"r"(smem_addr(&sm.acc_empty)));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    sm.dead = 0;
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&sm.tmem_base)),
+                 "r"((uint32_t)kTmemColsL)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  }
+  grid_dependency_wait();
+  grid_dependency_trigger();
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = sm.tmem_base;
+  // a wait that gives up ends the roles of its CTA one after the other (the others see `dead`)
+  auto wait = [&](uint64_t* bar, uint32_t parity) {
+    const uint32_t b = smem_addr(bar);
+    if (mbar_try(b, parity)) return true;
+    const long long t0 = clock64();
+    for (;;) {
+#pragma unroll 1
+      for (int i = 0; i < 16; ++i)
+        if (mbar_try(b, parity)) return true;
+      if (sm.dead || clock64() - t0 > kWaitCyclesL) {
+        sm.dead = 1;
+        return false;
+      }
+    }
+  };
+
+  if (warp == 0) {
+    if (elect_sync()) {
+      uint32_t it = 0;
+      bool ok = true;
+      for (int t = blockIdx.x; t < a.tiles && ok; t += gridDim.x) {
+        const int rb = t % a.blocks, c0 = t / a.blocks * kChannels;
+        for (int k = 0; k < a.k_tiles && ok; ++k, ++it) {
+          const uint32_t s = it % kStages;
+          if (it >= kStages) ok = wait(&sm.empty[s], (it / kStages - 1) & 1u);
+          if (!ok) break;
+          const uint32_t bar = smem_addr(&sm.full[s]);
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
+                       "r"((uint32_t)(kTileN * kTileK + n_mma * kTileK))
+                       : "memory");
+          tma_load_2d(smem_addr(&sm.w[s][0]), &maps.w0, k * kTileK, c0, bar);
+          if constexpr (kGate) tma_load_2d(smem_addr(&sm.w[s][128 * kTileK]), &maps.w1, k * kTileK, c0, bar);
+          tma_load_2d(smem_addr(&sm.x[s][0]), &maps.x, k * kTileK, rb * n_mma, bar);
+        }
+      }
+      if (!ok) {  // (requests in flight get their time before the CTA leaves)
+        const long long t0 = clock64();
+        while (clock64() - t0 < 2000000) {
+        }
+      }
+    }
+  } else if (warp == 1) {
+    const bool elected = elect_sync();
+    const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | (((uint32_t)n_mma >> 3) << 17) | ((128u >> 4) << 24);
+    uint32_t it = 0, done = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < a.tiles && ok; t += gridDim.x, ++done) {
+      if (done > 0) ok = __all_sync(0xffffffffu, wait(&sm.acc_empty, (done - 1) & 1u));
+      for (int k = 0; k < a.k_tiles && ok; ++k, ++it) {
+        const uint32_t s = it % kStages;
+        ok = __all_sync(0xffffffffu, wait(&sm.full[s], (it / kStages) & 1u));
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (elected) {
+          const uint64_t wd = desc_k_major_128b(smem_addr(&sm.w[s][0])), xd = desc_k_major_128b(smem_addr(&sm.x[s][0]));
+#pragma unroll
+          for (int ks = 0; ks < 4; ++ks) {
+            const uint32_t acc = (k > 0 || ks > 0) ? 1u : 0u;
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+              asm volatile(
+                  "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                  "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem + (uint32_t)(half * n_mma)),
+                  "l"(wd + (uint64_t)((half * (128 * kTileK) + 32 * ks) >> 4)), "l"(xd + (uint64_t)((32 * ks) >> 4)), "r"(idesc), "r"(acc)
+                  : "memory");
+            }
+          }
+          asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(&sm.empty[s]))
+                       : "memory");
+        }
+      }
+      if (elected)
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(&sm.acc_full))
+                     : "memory");
+    }
+  } else {
+    // ---- epilogue: warp w owns TMEM lanes 32 (w % 4) .. and rows [r_lo, r_hi) of the block
+    const int part = (warp - 2) >> 2, quad = warp & 3;
+    const int chunks = a.Rb / 8, r_lo = (part ? (chunks + 1) / 2 : 0) * 8, r_hi = (part ? chunks : (chunks + 1) / 2) * 8;
+    const uint32_t lanes = tmem + ((uint32_t)(quad * 32) << 16);
+    uint32_t done = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < a.tiles && ok; t += gridDim.x, ++done) {
+      const int rb = t % a.blocks, c0 = t / a.blocks * kChannels, ch = c0 + quad * 32 + lane;
+      const int ch1 = kGate ? ch : ch + 128;
+      const float sc0 = ch < a.N ? __bfloat162float(a.s0[ch]) : 0.f;
+      const float sc1 = ch1 < a.N ? __bfloat162float((kGate ? a.s1 : a.s0)[ch1]) : 0.f;
+      ok = wait(&sm.acc_full, done & 1u);
+      __syncwarp();
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      for (int r0 = r_lo; r0 < r_hi; r0 += 8) {
+        uint32_t h0[8], l0[8], h1[8], l1[8];
+        tmem_ld_8(lanes + (uint32_t)r0, h0);
+        tmem_ld_8(lanes + (uint32_t)(a.Rb + r0), l0);
+        tmem_ld_8(lanes + (uint32_t)(n_mma + r0), h1);
+        tmem_ld_8(lanes + (uint32_t)(n_mma + a.Rb + r0), l1);
+        const int m0 = rb * a.Rb + r0;
+        float xr[8];
+        const float4 xa = __ldg(reinterpret_cast<const float4*>(a.xs + m0)), xb = __ldg(reinterpret_cast<const float4*>(a.xs + m0) + 1);
+        xr[0] = xa.x, xr[1] = xa.y, xr[2] = xa.z, xr[3] = xa.w, xr[4] = xb.x, xr[5] = xb.y, xr[6] = xb.z, xr[7] = xb.w;
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          if (m0 + r >= a.M) break;
+          // F.linear's bf16 result, then the channel's scale: two bf16 operations
+          const float d0 = __bfloat162float(__float2bfloat16_rn(fmaf((float)(int)h0[r], 254.f, (float)(int)l0[r]) * xr[r]));
+          const float d1 = __bfloat162float(__float2bfloat16_rn(fmaf((float)(int)h1[r], 254.f, (float)(int)l1[r]) * xr[r]));
+          const __nv_bfloat16 y0 = __float2bfloat16_rn(d0 * sc0), y1 = __float2bfloat16_rn(d1 * sc1);
+          __nv_bfloat16* row = a.y + (int64_t)(m0 + r) * a.N;
+          if constexpr (kGate) {
+            if (ch < a.N) row[ch] = gate_value(y0, y1);
+          } else {
+            if (ch < a.N) row[ch] = y0;
+            if (ch1 < a.N) row[ch1] = y1;
+          }
+        }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(&sm.acc_empty)) : "memory");
+    }
+  }
+  __syncwarp();
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (tid == 0 && sm.dead) atomicExch(status, 1);
+  if (warp == 1) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)kTmemColsL) : "memory");
+  }
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -716,10 +927,36 @@ bool encode_2d(CUtensorMap* map, const void* base, int64_t rows, int64_t K, int 
             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-int split_for(int N, int K) {
+int sm_count_l() {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
+  return sms;
+}
+
+// How more than 128 rows are cut into blocks: equal blocks of Rb rows (a multiple of 8), so that no block is mostly padding,
+// and so many of them that the tiles fill whole rounds of the SMs.  Cost of a round in cycles: the tile's steps (MMA 8 Rb, or
+// the step's bytes at about 55 per cycle and SM where the block is narrow) and the epilogue that the next tile's MMAs wait for.
+struct RowBlocks {
+  int Rb, blocks;
+};
+RowBlocks row_blocks(int M, int N, int K, int channels) {
+  static const int sms = sm_count_l();
+  const int ctiles = (N + channels - 1) / channels, k_tiles = K / kTileK;
+  RowBlocks best{0, 0};
+  double best_cost = 0;
+  for (int nb = (M + kMaxM - 1) / kMaxM; nb <= (M + 15) / 16; ++nb) {
+    const int rb = ((M + nb - 1) / nb + 7) / 8 * 8, blocks = (M + rb - 1) / rb;
+    const double step = std::max(8.0 * rb, (32768.0 + 256.0 * rb) / 55.0);
+    const int64_t rounds = ((int64_t)ctiles * blocks + sms - 1) / sms;
+    const double cost = (double)rounds * (k_tiles * step + 2500.0 + 25.0 * rb);
+    if (best.Rb == 0 || cost < best_cost) best_cost = cost, best = RowBlocks{rb, blocks};
+  }
+  return best;
+}
+
+int split_for(int N, int K) {
+  static const int sms = sm_count_l();
   const int tiles = (N + kTileN - 1) / kTileN, k_tiles = K / kTileK;
   // The K splits of a tile are the CTAs of one cluster (1 .. 8; the K steps are dealt out evenly).  The split with
   // the shortest estimated run is taken: CTAs run in waves of one per SM; a CTA costs about 8 us of set-up, first
@@ -739,13 +976,23 @@ int split_for(int N, int K) {
 
 using namespace jpt;
 
+static size_t blocks_workspace_bytes(const RowBlocks& rb, int K) {
+  const size_t rows = (size_t)rb.blocks * rb.Rb;
+  return 256 + (2 * rows * K + 255) / 256 * 256 + (rows * sizeof(float) + 255) / 256 * 256;
+}
+
 extern "C" size_t jpt_w8a16_linear_workspace_bytes(int M, int N, int K) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  const int Mp = (std::min(M, kMaxM) + 7) / 8 * 8;  // (more rows are taken in blocks of 128, one after the other)
+  if (M > kMaxM) return blocks_workspace_bytes(row_blocks(M, N, K, kTileN), K);
+  const int Mp = (M + 7) / 8 * 8;
   const size_t levels = ((size_t)2 * Mp * K + 255) / 256 * 256;
   const size_t xs = 1024;
-  (void)N;
   return 256 + levels + xs;
+}
+
+extern "C" size_t jpt_w8a16_gate_workspace_bytes(int M, int N, int K) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  return blocks_workspace_bytes(row_blocks(M, N, K, 128), K);
 }
 
 namespace jpt {
@@ -822,6 +1069,49 @@ int launch_levels(const void* x, const LevelsView& lv, int M, int K, cudaStream_
   return check_launch("x_levels_kernel");
 }
 
+// More than 128 rows: the level kernel over all of them, then the tiles.
+template <bool kGate>
+int launch_tiles(const void* x, const void* w0, const void* s0, const void* w1, const void* s1, void* y, int M, int N, int K,
+                 void* workspace, cudaStream_t st) {
+  const RowBlocks rb = row_blocks(M, N, K, kGate ? 128 : kTileN);
+  const int rows = rb.blocks * rb.Rb;
+  char* ws = static_cast<char*>(workspace);
+  LevelsView lv;
+  lv.status = reinterpret_cast<int*>(ws);
+  lv.lev = reinterpret_cast<int8_t*>(ws + 256);
+  lv.xs = reinterpret_cast<float*>(ws + 256 + ((size_t)2 * rows * K + 255) / 256 * 256);
+  lv.Mp = rb.Rb;
+  x_levels_kernel<<<rows, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(x), lv.lev, lv.xs, lv.status, M, rb.Rb, K, 1, nullptr);
+  if (int rc = check_launch("x_levels_kernel")) return rc;
+  TileMaps maps;
+  memset(&maps, 0, sizeof(maps));
+  JPT_REQUIRE(encode_2d(&maps.w0, w0, N, K, kGate ? 128 : kTileN) && (!kGate || encode_2d(&maps.w1, w1, N, K, 128)) &&
+                  encode_2d(&maps.x, lv.lev, 2 * (int64_t)rows, K, 2 * rb.Rb),
+              JPT_EINVAL, "w8a16_linear: the tensors cannot be described by a tensor map");
+  static bool configured[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && !configured[dev]) {
+    const cudaError_t e = cudaFuncSetAttribute(w8a16_tiles_kernel<kGate>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemT));
+    if (e != cudaSuccess) return fail((int)e, "w8a16_linear: configuring the kernel: %s", cudaGetErrorString(e));
+    configured[dev] = true;
+  }
+  TileArgs a;
+  memset(&a, 0, sizeof(a));
+  a.xs = lv.xs;
+  a.s0 = static_cast<const __nv_bfloat16*>(s0), a.s1 = static_cast<const __nv_bfloat16*>(s1);
+  a.y = static_cast<__nv_bfloat16*>(y);
+  a.M = M, a.N = N, a.Rb = rb.Rb, a.blocks = rb.blocks, a.k_tiles = K / kTileK;
+  constexpr int kChannels = kGate ? 128 : kTileN;
+  const int64_t tiles = (int64_t)((N + kChannels - 1) / kChannels) * rb.blocks;
+  JPT_REQUIRE(tiles < (1ll << 31), JPT_ERANGE, "w8a16_linear: too many rows");
+  a.tiles = (int)tiles;
+  static const int sms = sm_count_l();
+  launch_after_previous(w8a16_tiles_kernel<kGate>, dim3((unsigned)std::min<int64_t>(tiles, sms)), dim3(kThreadsT), sizeof(SmemT), st, maps, a,
+                        lv.status);
+  return check_launch("w8a16_tiles_kernel");
+}
+
 // CTAs per row of the element-wise producers (a cluster along x): enough of them to fill the GPU
 int row_parts(int rows, int K) {
   const int steps = K / 8;
@@ -872,15 +1162,22 @@ extern "C" int jpt_w8a16_linear(const void* x, const void* w, const void* w_scal
               workspace_bytes);
   JPT_REQUIRE(aligned(workspace, 256), JPT_EALIGN, "w8a16_linear: workspace must be 256-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // More than 128 rows (prefill shapes) go through in blocks of 128 that reuse the workspace in stream order;
-  // every block streams the weights again, which is the wrong trade for a compute-bound shape but a correct one.
-  for (int m0 = 0; m0 < M; m0 += kMaxM) {
-    const int rows = std::min(kMaxM, M - m0);
-    const LevelsView lv = levels_view(workspace, rows, K);
-    if (int rc = launch_levels(static_cast<const char*>(x) + (size_t)m0 * K * 2, lv, rows, K, st, m0 == 0)) return rc;
-    if (int rc = launch_gemm(lv, w, w_scale, static_cast<char*>(y) + (size_t)m0 * N * 2, rows, N, K, st)) return rc;
-  }
-  return 0;
+  if (M > kMaxM) return launch_tiles<false>(x, w, w_scale, nullptr, nullptr, y, M, N, K, workspace, st);
+  const LevelsView lv = levels_view(workspace, M, K);
+  if (int rc = launch_levels(x, lv, M, K, st, true)) return rc;
+  return launch_gemm(lv, w, w_scale, y, M, N, K, st);
+}
+
+extern "C" int jpt_w8a16_gate(const void* x, const void* w1, const void* w1_scale, const void* w3, const void* w3_scale, void* h, int M,
+                              int N, int K, void* workspace, size_t workspace_bytes, void* stream) {
+  JPT_REQUIRE(x && w1 && w1_scale && w3 && w3_scale && h, JPT_EINVAL, "w8a16_gate: null tensor");
+  JPT_REQUIRE(M >= 1 && N >= 1 && K >= kTileK && K % kTileK == 0, JPT_EINVAL, "w8a16_gate: M = %d, K = %d (a multiple of %d)", M, K, kTileK);
+  JPT_REQUIRE(aligned(x, 16) && aligned(w1, 16) && aligned(w3, 16), JPT_EALIGN, "w8a16_gate: x and the weights must be 16-byte aligned");
+  const size_t need = jpt_w8a16_gate_workspace_bytes(M, N, K);
+  JPT_REQUIRE(workspace && workspace_bytes >= need, JPT_EWORKSPACE, "w8a16_gate: workspace of %zu bytes needed, %zu given", need,
+              workspace_bytes);
+  JPT_REQUIRE(aligned(workspace, 256), JPT_EALIGN, "w8a16_gate: workspace must be 256-byte aligned");
+  return launch_tiles<true>(x, w1, w1_scale, w3, w3_scale, h, M, N, K, workspace, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int jpt_w8a16_split_levels(const void* x, int M, int K, void* workspace, size_t workspace_bytes, void* stream) {

@@ -140,8 +140,8 @@ class WeightOnlyPerChannelQuantizedLinear(torch.nn.Module):
   bf16(bf16(inputs @ weight^T) * weight_scaler).
 
   Built: 8-bit symmetric weights, no activation quantisation, `in_features` a
-  multiple of 128.  The kernel is made for decode batches (up to 128 rows of
-  activations stream the weights once); more rows go through in blocks of 128.
+  multiple of 128.  Up to 128 rows of activations (decode batches) stream the
+  weights once; more rows (prompts) go to a compute-bound tile kernel.
   Anything else raises; there is no eager path."""
 
   def __init__(self, in_features, out_features, bias=False, device=None, quant_config=None):
@@ -310,7 +310,11 @@ class FeedForward(torch.nn.Module):
 
   def forward(self, x, levels=None):
     if not ActivationLevels.fits(x):
-      return self.w2(silu_mul(self.w1(x), self.w3(x)))
+      if x.dtype != torch.bfloat16 or x.shape[-1] != self.w1.in_features or x.numel() == 0:
+        return self.w2(silu_mul(self.w1(x), self.w3(x)))
+      # a prompt: both projections and the gate in one launch behind the level split of x
+      h, self.w1._workspace = _lib.native.gate(x, self.w1.weight, self.w1.weight_scaler, self.w3.weight, self.w3.weight_scaler)
+      return self.w2(h)
     if levels is None:
       levels = ActivationLevels.of(x)
     h, h_levels = silu_mul(self.w1(x, levels=levels), self.w3(x, levels=levels), with_levels=True)

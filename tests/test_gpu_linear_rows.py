@@ -1,0 +1,49 @@
+"""The weight-only int8 layers on prompts (more than 128 rows: the tile kernel)
+against the oracle, within the layer's own tolerance."""
+
+import pytest
+import torch
+
+from oracle import linear as ol
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _layer(n, k, g):
+  from jetstream_pytorch_b200.layers import WeightOnlyPerChannelQuantizedLinear
+
+  w, s = ol.quantize_weight(torch.randn(n, k, generator=g) * 0.03)
+  lin = WeightOnlyPerChannelQuantizedLinear(k, n, device=DEV)
+  lin._load_quantized_weights(w, s)
+  return lin, w, s
+
+
+# one row into a second block, row counts that are no multiple of eight, a channel tile with one channel, the shortest K
+@pytest.mark.parametrize("m,k,n", [(129, 128, 256), (130, 384, 257), (257, 640, 100), (1000, 256, 520), (200, 4096, 1280)])
+def test_many_rows_match_the_oracle(m, k, n):
+  g = torch.Generator().manual_seed(m + n)
+  lin, w, s = _layer(n, k, g)
+  x = torch.randn(m, k, generator=g).to(torch.bfloat16)
+  x[5] = 0
+  y = lin(x.to(DEV)).cpu()
+  assert lin.kernel_status() == 0
+  exp = ol.w8a16_linear(x, w, s)
+  err = (y.double() - exp.double()).abs()
+  assert (err <= ol.w8a16_tolerance(x, w, s)).all(), float(err.max())
+  assert (y == exp).float().mean() > 0.95
+  assert not y[5].any()
+
+
+@pytest.mark.parametrize("m,dim,hidden", [(129, 256, 384), (333, 512, 200 * 128), (700, 384, 128)])
+def test_gate_of_a_prompt_equals_the_layers_one_by_one(m, dim, hidden):
+  """The fused projections and gate against the two layers (each checked above) followed by the gate kernel: the same
+  sums, the same roundings, the same bits."""
+  from jetstream_pytorch_b200 import _lib
+  from jetstream_pytorch_b200.layers import silu_mul
+
+  g = torch.Generator().manual_seed(m)
+  w1, w3 = _layer(hidden, dim, g)[0], _layer(hidden, dim, g)[0]
+  x = torch.randn(m, dim, generator=g).to(torch.bfloat16).to(DEV)
+  h, _ = _lib.native.gate(x, w1.weight, w1.weight_scaler, w3.weight, w3.weight_scaler)
+  assert torch.equal(h, silu_mul(w1(x), w3(x)))
