@@ -378,6 +378,51 @@ __global__ void __launch_bounds__(kRowThreads) rmsnorm_levels_kernel(const __nv_
   if (gridDim.x > 1) cluster_sync();  // (no CTA leaves while a peer may still store into its slots)
 }
 
+// RMSNorm without levels for many rows (a prompt): one warp per row, the row held in its registers (K = 256 kVec elements),
+// so that it is read once and nothing waits at a barrier.  A CTA of 1024 threads per row took 18.6 us for [1024, 4096] (16.8 MB).
+template <int kVec>
+__global__ void __launch_bounds__(128) rmsnorm_rows_kernel(const __nv_bfloat16* x, const __nv_bfloat16* weight, float eps,
+                                                           __nv_bfloat16* y, int M, int K) {
+  const int m = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  grid_dependency_wait();
+  grid_dependency_trigger();
+  if (m >= M) return;
+  const uint4* row = reinterpret_cast<const uint4*>(x + (int64_t)m * K);
+  const uint4* wrow = reinterpret_cast<const uint4*>(weight);
+  uint4* out = reinterpret_cast<uint4*>(y + (int64_t)m * K);
+  const int nvec = K / 8;
+  uint4 held[kVec];
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < kVec; ++i) held[i] = lane + 32 * i < nvec ? __ldg(row + lane + 32 * i) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+  for (int i = 0; i < kVec; ++i) {
+    const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&held[i]);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float f = __bfloat162float(e[j]);
+      ss = fmaf(f, f, ss);
+    }
+  }
+  const float rs = 1.f / sqrtf(warp_sum(ss) / (float)K + eps);
+#pragma unroll
+  for (int i = 0; i < kVec; ++i) {
+    if (lane + 32 * i < nvec) {
+      const uint4 wv = __ldg(wrow + lane + 32 * i);
+      const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&held[i]);
+      const __nv_bfloat16* we = reinterpret_cast<const __nv_bfloat16*>(&wv);
+      uint4 o;
+      __nv_bfloat16* oe = reinterpret_cast<__nv_bfloat16*>(&o);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float n = __bfloat162float(__float2bfloat16_rn(__bfloat162float(e[j]) * rs));
+        oe[j] = __float2bfloat16_rn(n * __bfloat162float(we[j]));
+      }
+      out[lane + 32 * i] = o;
+    }
+  }
+}
+
 // One value of the gate: bf16(bf16(silu(a)) * b).  (Fast exponential and division: the quotient is rounded to bf16, and the
 // exact forms are subroutines.)
 __device__ __forceinline__ __nv_bfloat16 gate_value(__nv_bfloat16 a, __nv_bfloat16 b) {
@@ -857,34 +902,53 @@ __global__ void __launch_bounds__(kThreadsT, 1)
       const int ch1 = kGate ? ch : ch + 128;
       const float sc0 = ch < a.N ? __bfloat162float(a.s0[ch]) : 0.f;
       const float sc1 = ch1 < a.N ? __bfloat162float((kGate ? a.s1 : a.s0)[ch1]) : 0.f;
+      // the row scales of this warp's up to 64 rows, a lane each (fetched ahead: read one by one in the loop below they
+      // cost it an L2 round trip per chunk)
+      const int m_lo = rb * a.Rb + r_lo;
+      const float xs_a = r_lo + lane < r_hi ? __ldg(a.xs + m_lo + lane) : 0.f;
+      const float xs_b = r_lo + 32 + lane < r_hi ? __ldg(a.xs + m_lo + 32 + lane) : 0.f;
       ok = wait(&sm.acc_full, done & 1u);
       __syncwarp();
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      for (int r0 = r_lo; r0 < r_hi; r0 += 8) {
-        uint32_t h0[8], l0[8], h1[8], l1[8];
-        tmem_ld_8(lanes + (uint32_t)r0, h0);
-        tmem_ld_8(lanes + (uint32_t)(a.Rb + r0), l0);
-        tmem_ld_8(lanes + (uint32_t)(n_mma + r0), h1);
-        tmem_ld_8(lanes + (uint32_t)(n_mma + a.Rb + r0), l1);
-        const int m0 = rb * a.Rb + r0;
-        float xr[8];
-        const float4 xa = __ldg(reinterpret_cast<const float4*>(a.xs + m0)), xb = __ldg(reinterpret_cast<const float4*>(a.xs + m0) + 1);
-        xr[0] = xa.x, xr[1] = xa.y, xr[2] = xa.z, xr[3] = xa.w, xr[4] = xb.x, xr[5] = xb.y, xr[6] = xb.z, xr[7] = xb.w;
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      __nv_bfloat16* row0 = a.y + (int64_t)m_lo * a.N;
+      const int live = a.M - m_lo;  // rows of this warp that exist
+      uint32_t v[2][4][8];          // [chunk parity][h0, l0, h1, l1][row]
+      auto fetch = [&](int r, uint32_t (&d)[4][8]) {
+        tmem_ld_8(lanes + (uint32_t)(r_lo + r), d[0]);
+        tmem_ld_8(lanes + (uint32_t)(a.Rb + r_lo + r), d[1]);
+        tmem_ld_8(lanes + (uint32_t)(n_mma + r_lo + r), d[2]);
+        tmem_ld_8(lanes + (uint32_t)(n_mma + a.Rb + r_lo + r), d[3]);
+      };
+      auto finish = [&](int r, const uint32_t (&d)[4][8]) {
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
-          if (m0 + r >= a.M) break;
+        for (int j = 0; j < 8; ++j) {
+          const float xr = __shfl_sync(0xffffffffu, r < 32 ? xs_a : xs_b, (r & 31) + j);
           // F.linear's bf16 result, then the channel's scale: two bf16 operations
-          const float d0 = __bfloat162float(__float2bfloat16_rn(fmaf((float)(int)h0[r], 254.f, (float)(int)l0[r]) * xr[r]));
-          const float d1 = __bfloat162float(__float2bfloat16_rn(fmaf((float)(int)h1[r], 254.f, (float)(int)l1[r]) * xr[r]));
+          const float d0 = __bfloat162float(__float2bfloat16_rn(fmaf((float)(int)d[0][j], 254.f, (float)(int)d[1][j]) * xr));
+          const float d1 = __bfloat162float(__float2bfloat16_rn(fmaf((float)(int)d[2][j], 254.f, (float)(int)d[3][j]) * xr));
           const __nv_bfloat16 y0 = __float2bfloat16_rn(d0 * sc0), y1 = __float2bfloat16_rn(d1 * sc1);
-          __nv_bfloat16* row = a.y + (int64_t)(m0 + r) * a.N;
+          __nv_bfloat16* row = row0 + (int64_t)(r + j) * a.N;
+          const bool in = r + j < live;
           if constexpr (kGate) {
-            if (ch < a.N) row[ch] = gate_value(y0, y1);
+            const __nv_bfloat16 g = gate_value(y0, y1);
+            if (in && ch < a.N) row[ch] = g;
           } else {
-            if (ch < a.N) row[ch] = y0;
-            if (ch1 < a.N) row[ch1] = y1;
+            if (in && ch < a.N) row[ch] = y0;
+            if (in && ch1 < a.N) row[ch1] = y1;
           }
+        }
+      };
+      // the next chunk leaves tensor memory while this one is worked on
+      const int nr = r_hi - r_lo;
+      if (nr > 0) fetch(0, v[0]);
+      for (int r = 0; r < nr; r += 16) {
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (r + 8 < nr) fetch(r + 8, v[1]);
+        finish(r, v[0]);
+        if (r + 8 < nr) {
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          if (r + 16 < nr) fetch(r + 16, v[0]);
+          finish(r + 8, v[1]);
         }
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -1202,6 +1266,15 @@ extern "C" int jpt_rmsnorm(const void* x, const void* weight, float eps, void* y
   const __nv_bfloat16* xp = static_cast<const __nv_bfloat16*>(x);
   const __nv_bfloat16* wp = static_cast<const __nv_bfloat16*>(weight);
   if (!levels_workspace) {
+    // (from two rows per SM on, rows of up to 8192 elements: below that a CTA per row has the shorter chain)
+    if (M >= 296 && K <= 8192) {
+      const dim3 grid((M + 3) / 4), block(128);
+      if (K <= 4096)
+        launch_after_previous(rmsnorm_rows_kernel<16>, grid, block, 0, st, xp, wp, eps, static_cast<__nv_bfloat16*>(y), M, K);
+      else
+        launch_after_previous(rmsnorm_rows_kernel<32>, grid, block, 0, st, xp, wp, eps, static_cast<__nv_bfloat16*>(y), M, K);
+      return check_launch("rmsnorm_rows_kernel");
+    }
     return launch_rows("rmsnorm_levels_kernel", rmsnorm_levels_kernel, M, row_parts(M, K), st, xp, wp, eps, static_cast<__nv_bfloat16*>(y),
                        nullptr, nullptr, nullptr, M, M, K);
   }

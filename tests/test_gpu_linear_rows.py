@@ -47,3 +47,18 @@ def test_gate_of_a_prompt_equals_the_layers_one_by_one(m, dim, hidden):
   x = torch.randn(m, dim, generator=g).to(torch.bfloat16).to(DEV)
   h, _ = _lib.native.gate(x, w1.weight, w1.weight_scaler, w3.weight, w3.weight_scaler)
   assert torch.equal(h, silu_mul(w1(x), w3(x)))
+
+
+@pytest.mark.parametrize("m,k", [(296, 4096), (297, 8192), (1000, 264), (301, 5120)])
+def test_rmsnorm_of_a_prompt(m, k):
+  """Equal to a neighbouring bf16 value at most (the fp32 sum is taken in another order)."""
+  from jetstream_pytorch_b200.layers import RMSNorm
+
+  g = torch.Generator().manual_seed(k)
+  norm = RMSNorm(k, device=DEV)
+  w = (1 + 0.1 * torch.randn(k, generator=g)).to(torch.bfloat16)
+  norm.weight.data.copy_(w)
+  x = torch.randn(m, k, generator=g).to(torch.bfloat16)
+  y, exp = norm(x.to(DEV)).cpu(), ol.rmsnorm(x, w, norm.eps)
+  assert torch.allclose(y.float(), exp.float(), rtol=2.0 ** -6, atol=0)
+  assert (y == exp).float().mean() > 0.99
