@@ -13,18 +13,17 @@
 //   y[m, n] = scale[n] * s_m * (S_h[n, m] + S_l[n, m] / 254)
 // with exact int32 sums S_h, S_l in tensor memory.  Nothing is converted in registers.
 //
-// Launches: (1) split of the activations into levels (one CTA per row of x), (2) the GEMM: one CTA
-// per 256 output channels and K split; the CTAs of a tile's K splits form a thread-block cluster.
-// 128 threads: thread 0 requests the tiles of a 3-stage ring of 128-byte-swizzled [256 x 128 B] weight
-// and [2 M x 128 B] activation tiles, thread 32 issues the MMAs, two per K step of 32 bytes, one for
-// each half of the channels, so that an activation tile read from L2 serves 256 channels, and frees
-// the stages through tcgen05.commit.  Epilogue: all four warps read the accumulators out of tensor
-// memory; the rows of the batch are dealt out to the CTAs of the cluster in groups of eight, every
+// Launches: (1) split of the activations into levels (one CTA per row of x), (2) the GEMM: pairs of CTAs
+// (cta_group::2) with up to 256 output channels per CTA; the CTAs of a pair's K splits form a thread-block
+// cluster.  One thread requests the tiles of a ring of 128-byte-swizzled weight and activation tiles, one
+// warp of the pair's first CTA issues the MMAs, two per K step of 32 bytes, one for each half of the channels, and
+// frees the stages through tcgen05.commit.  Epilogue: eight warps read the accumulators out of tensor memory; without a
+// split they finish the result there.  With one, the rows of the batch are dealt out to the splits in groups of eight, every
 // CTA stores its partial sums of a group into the shared memory of the group's owner (the ring is
 // free by then), and the owner adds the partials in the order of the splits, rounds to bf16,
 // multiplies by the channel's scale and rounds again, as the reference's two bf16 operations do.
 // No partial result goes through global memory.  Every wait on data is bounded; a CTA that gives up
-// raises the status word, still meets its cluster at the two cluster barriers, and returns.
+// raises the status word, still meets its cluster at the cluster barriers, and returns.
 //
 // Also here, because they write the same level matrix: RMSNorm and the feed-forward gate (SiLU-mul) as
 // kernels that can leave the level split of their result behind, so that the layers after them start
@@ -43,22 +42,13 @@
 namespace jpt {
 namespace {
 
-constexpr int kTileN = 256;      // output channels per CTA: two accumulators of 128 TMEM lanes
+constexpr int kTileN = 256;      // output channels per CTA at most: two accumulators of 128 TMEM lanes
 constexpr int kTileK = 128;      // int8 elements per stage and row: one 128-byte swizzle atom
 constexpr int kStages = 3;
 constexpr int kMaxM = 128;       // rows of x: the N operand holds 2 * M rows (<= 256)
 constexpr int kTmemColsL = 512;  // two accumulators [128 lanes x 2 M columns]
-constexpr int kThreadsL = 128;
-constexpr int kMaxSplit = 8;     // K splits of a tile = CTAs of a cluster (the portable limit)
+constexpr int kThreadsL = 256;
 constexpr long long kWaitCyclesL = 1000000000ll;
-
-struct __align__(1024) SmemL {
-  uint8_t w[kStages][kTileN * kTileK];        // weight tiles, swizzled
-  uint8_t x[kStages][2 * kMaxM * kTileK];     // activation level tiles (only 2 M rows are filled)
-  uint64_t full[kStages], empty[kStages], done;
-  float xs[kMaxM];  // s_m / 254 of the rows of x
-  uint32_t tmem_base;
-};
 
 struct LinearMaps {
   CUtensorMap w, x;
@@ -130,6 +120,21 @@ __device__ __forceinline__ uint64_t desc_k_major_128b(uint32_t addr) {
   d |= (uint64_t)2 << 61;                 // SWIZZLE_128B
   return d;
 }
+// The box: a number of 128-byte steps of K from step `z` on, each a swizzled tile of rows from `y` on.  (A CTA of a pair: the bytes
+// land in this CTA, the barrier `bar`, a shared::cluster address, may be the other one's.)
+template <bool kPair>
+__device__ __forceinline__ void tma_load_steps(uint32_t dst, const CUtensorMap* map, int y, int z, uint32_t bar) {
+  if constexpr (kPair)
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(y), "r"(z), "r"(bar)
+        : "memory");
+  else
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(y), "r"(z), "r"(bar)
+        : "memory");
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
@@ -158,22 +163,16 @@ __device__ __forceinline__ bool elect_sync() {
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(r));
   return r != 0;
 }
+__device__ __forceinline__ void tmem_ld_16(uint32_t addr, uint32_t (&v)[16]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
+                 "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+               : "r"(addr));
+}
 __device__ __forceinline__ void tmem_ld_8(uint32_t addr, uint32_t (&v)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
                : "r"(addr));
-}
-
-// 32 consecutive accumulator columns of this thread's lane
-__device__ __forceinline__ void tmem_ld_32(uint32_t addr, uint32_t (&v)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
-        "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]),
-        "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]),
-        "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-      : "r"(addr));
 }
 
 // ---------------------------------------------------------------- (1) activation levels
@@ -464,26 +463,67 @@ __global__ void __launch_bounds__(kRowThreads) silu_mul_levels_kernel(const __nv
 }
 
 // ---------------------------------------------------------------- (2) the GEMM
-// grid (ceil(N / 256), ksplit), clusters of (1, ksplit): the rank of a CTA in its cluster is its K split.
+// Two CTAs of a TPC work as a pair (cta_group::2): each holds the weights of its own channels, the activation tile is shared
+// between them (the even CTA loads the h rows, the odd one the l rows, and the tensor cores of both read both halves).  What
+// bounds the K loop besides the HBM read is the L2: at 96 rows a CTA of its own reads 24 KB of activations per 32 KB of
+// weights, a pair half of that.
+// grid (tiles, splits), clusters of (2, splits): blockIdx.x is the channel tile, blockIdx.y the K split.  A tile is as wide as
+// it takes to give every SM one (plan_gemm): the tensor core works on 128 rows whatever the tile's width; the rows behind
+// the tile's, whatever lies there, only feed accumulator lanes that nobody reads.  (Fixed tiles of 256 channels left 36 of
+// 148 SMs idle at 28672 channels.)  A stage holds `kb` steps of 128 bytes of K: the hand-over of a stage between the copy
+// engine, the issuing warp and back costs 0.44 us whatever it holds (64 steps of 32 to 104 channels took 34 us).
+struct GemmArgs {
+  const float* xs;
+  const __nv_bfloat16* scale;
+  __nv_bfloat16* y;
+  int* status;
+  int M, Mp, N, k_steps;  // k_steps: stages' worth of K (the last one may reach beyond K, where the copy engine fills zeros)
+  int tile;               // channels of a CTA
+  int kb, stages, stage_bytes, tail;  // tail: where the ring (and the landing area that takes its place) ends
+};
+constexpr int kMaxStages = 12;
+struct GemmTail {  // behind the ring
+  uint64_t full[kMaxStages], empty[kMaxStages], done;
+  alignas(16) float xs[kMaxM];  // s_m / 254 of the rows of x (read four at a time)
+  uint32_t tmem_base;
+};
+constexpr int kRingBytes = 208 * 1024;
+constexpr int kTailBytes = 16 * 1024;  // (the tail, and what the 128 rows of the ring's last operand reach beyond it)
+static_assert(sizeof(GemmTail) <= kTailBytes && kRingBytes + kTailBytes <= 227 * 1024, "shared memory of a CTA");
+
+template <bool kPair, int kHalves>
 __global__ void __launch_bounds__(kThreadsL, 1)
-    w8a16_gemm_kernel(const __grid_constant__ LinearMaps maps, const float* xs, const __nv_bfloat16* scale, __nv_bfloat16* y,
-                      int M, int Mp, int N, int K, int k_tiles, int* status, const __grid_constant__ TpArgs tp) {
+    w8a16_gemm_kernel(const __grid_constant__ LinearMaps maps, const __grid_constant__ GemmArgs a, const __grid_constant__ TpArgs tp) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  SmemL& sm = *reinterpret_cast<SmemL*>(smem_raw);
-  const int tid = threadIdx.x, warp = tid >> 5;
-  if ((smem_addr(smem_raw) & 1023u) != 0u) {
+  GemmTail& sm = *reinterpret_cast<GemmTail*>(smem_raw + a.tail);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if ((smem_addr(smem_raw) & 1023u) != 0u) {  // (the same in every CTA)
     grid_dependency_wait();  // (the launch before this one clears the status word)
-    if (tid == 0) atomicExch(status, 2);
+    if (tid == 0) atomicExch(a.status, 2);
     return;
   }
-  const int n0 = blockIdx.x * kTileN, split = blockIdx.y;
-  // K steps of this split: the k_tiles steps dealt out as evenly as whole steps allow (the first splits one more)
-  const int nsplit = (int)gridDim.y, k_lo = split * (k_tiles / nsplit) + min(split, k_tiles % nsplit);
-  const int iters = k_tiles / nsplit + (split < k_tiles % nsplit ? 1 : 0), k_begin = k_lo * kTileK;
-  const int n_mma = 2 * Mp;  // columns of the accumulator (a multiple of 16)
+  const int M = a.M, Mp = a.Mp, N = a.N;
+  constexpr int halves = kHalves;  // of the tile, of up to 128 tensor memory lanes each
+  constexpr int kCtas = kPair ? 2 : 1;  // CTAs that an MMA instruction runs on
+  const int pair_rank = kPair ? (int)(blockIdx.x & 1u) : 0, split = (int)blockIdx.y, nsplit = (int)gridDim.y;
+  const int width = a.tile / halves;  // channels of a half
+  const int n0 = (int)blockIdx.x * a.tile;
+  // stages of this split: the k_steps dealt out as evenly as whole ones allow (the first splits one more)
+  const int k_lo = split * (a.k_steps / nsplit) + min(split, a.k_steps % nsplit);
+  const int iters = a.k_steps / nsplit + (split < a.k_steps % nsplit ? 1 : 0);
+  const int n_mma = 2 * Mp;  // columns of an accumulator (a multiple of 32)
+  uint32_t tmem_cols = 32;
+  while ((int)tmem_cols < halves * n_mma) tmem_cols *= 2;
+  // Every CTA of a split reads the same activation tiles: each pair starts at another K step (the sums are exact integers,
+  // their order is free), so that the pairs do not ask the same L2 lines at the same time.
+  const int rot = (int)(blockIdx.x / kCtas % (unsigned)iters);
+  const uint32_t w_bytes = (uint32_t)(a.kb * a.tile * kTileK), x_bytes = (uint32_t)(a.kb * (n_mma / kCtas) * kTileK);
+  const uint32_t leader = (uint32_t)(kCtas * split);  // rank of the pair's even CTA in the cluster: it owns the `full` barriers
+  uint8_t* const ring = smem_raw;
+  const int x_off = (int)w_bytes;
 
   if (tid == 0) {
-    for (int s = 0; s < kStages; ++s) {
+    for (int s = 0; s < a.stages; ++s) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&sm.full[s])));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&sm.empty[s])));
     }
@@ -491,263 +531,311 @@ __global__ void __launch_bounds__(kThreadsL, 1)
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.w)) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.x)) : "memory");
-    // The weights do not depend on the launch before this one (only the activation levels do): the weight
-    // tiles of the first stages are requested before the wait on that launch.  Their bytes are announced to
-    // the stage's barrier without an arrival; the arrival comes with the activation tile's request.
-    const int rot0 = (int)(blockIdx.x % (unsigned)iters);
-    for (int it = 0; it < kStages && it < iters; ++it) {
-      const int kt = it + rot0 < iters ? it + rot0 : it + rot0 - iters;
-      const uint32_t bar = smem_addr(&sm.full[it]);
-      asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"((uint32_t)(kTileN * kTileK)) : "memory");
-      tma_load_2d(smem_addr(&sm.w[it][0]), &maps.w, k_begin + kt * kTileK, n0, bar);
-    }
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&sm.tmem_base)),
-                 "r"((uint32_t)kTmemColsL)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if constexpr (kPair) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&sm.tmem_base)), "r"(tmem_cols)
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&sm.tmem_base)), "r"(tmem_cols)
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  }
+  if constexpr (kPair) {
+    __syncthreads();
+    cluster_sync();  // the barriers of the pair's leader are there
+  }
+  auto full_bar = [&](int s) {
+    const uint32_t bar = smem_addr(&sm.full[s]);
+    return kPair ? remote_smem(bar, (int)leader) : bar;
+  };
+  auto request_w = [&](int it) {
+    const int s = it % a.stages, kt = it + rot < iters ? it + rot : it + rot - iters;
+    tma_load_steps<kPair>(smem_addr(ring + s * a.stage_bytes), &maps.w, n0, (k_lo + kt) * a.kb, full_bar(s));
+  };
+  if (tid == 0) {
+    // The weights do not depend on the launch before this one (only the activation levels do): the weight tiles of the first
+    // stages are requested before the wait on that launch.  Their bytes are announced to the stage's barrier without an
+    // arrival; the arrival comes with the activation tile's request.
+    for (int it = 0; it < a.stages && it < iters; ++it) {
+      if (pair_rank == 0)
+        asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&sm.full[it])), "r"(kCtas * w_bytes) : "memory");
+      request_w(it);
+    }
   }
   grid_dependency_wait();
   grid_dependency_trigger();
   const unsigned tp_epoch = tp.world > 1 ? *reinterpret_cast<volatile unsigned*>(tp.launch_counter) : 0u;
-  sm.xs[tid] = tid < M ? xs[tid] : 0.f;
+  if (tid < kMaxM) sm.xs[tid] = tid < M ? a.xs[tid] : 0.f;
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = sm.tmem_base;
   bool dead = false;
 
-  if (tid == 0) {
-    // ---- producer: tiles of stage s are requested when the MMAs that read its previous contents are done
-    // Every CTA of a K split reads the same activation tiles: each starts at another K step (the sums are
-    // exact integers, their order is free), so that the CTAs do not ask the same L2 lines at the same time.
-    const int rot = (int)(blockIdx.x % (unsigned)iters);
-    const uint32_t w_bytes = (uint32_t)(kTileN * kTileK), x_bytes = (uint32_t)(n_mma * kTileK);
-    for (int it = 0; it < iters && !dead; ++it) {
-      const int s = it % kStages;
-      if (it >= kStages && !mbar_wait_l(smem_addr(&sm.empty[s]), (uint32_t)((it / kStages) - 1) & 1u)) dead = true;
-      if (dead) break;
-      const uint32_t bar = smem_addr(&sm.full[s]);
-      const int kt = it + rot < iters ? it + rot : it + rot - iters;
-      if (it >= kStages) {  // (the weight tiles of the first stages are on their way already)
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(w_bytes + x_bytes) : "memory");
-        tma_load_2d(smem_addr(&sm.w[s][0]), &maps.w, k_begin + kt * kTileK, n0, bar);
-      } else {
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(x_bytes) : "memory");
+  if (warp == 0) {
+    // ---- producer (both CTAs of a pair): tiles of stage s are requested when the MMAs that read its previous contents are
+    // done.  The warp stays together and one lane issues, here and in the MMA warp: addresses and descriptors then live in
+    // uniform registers (issued by a thread of its own, a stage of one step took 0.44 us whatever it held).
+    const bool elected = elect_sync();
+    int s = 0, kt = rot;
+    uint32_t parity = 1;  // of the stage's previous use
+    for (int it = 0; it < iters; ++it) {
+      const bool early = it < a.stages;  // (the weight tiles of the first stages are on their way already)
+      if (!early && !__all_sync(0xffffffffu, mbar_wait_l(smem_addr(&sm.empty[s]), parity))) {
+        dead = true;
+        break;
       }
-      tma_load_2d(smem_addr(&sm.x[s][0]), &maps.x, k_begin + kt * kTileK, 0, bar);
+      if (elected) {
+        if (pair_rank == 0)
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(&sm.full[s])),
+                       "r"(kCtas * (x_bytes + (early ? 0u : w_bytes)))
+                       : "memory");
+        if (!early) tma_load_steps<kPair>(smem_addr(ring + s * a.stage_bytes), &maps.w, n0, (k_lo + kt) * a.kb, full_bar(s));
+        tma_load_steps<kPair>(smem_addr(ring + s * a.stage_bytes + x_off), &maps.x, pair_rank * Mp, (k_lo + kt) * a.kb, full_bar(s));
+      }
+      if (++kt == iters) kt = 0;
+      if (++s == a.stages) s = 0, parity ^= 1u;
     }
-  } else if (tid == 32) {
-    // ---- MMA issue: D_half[128 n x 2 Mp] += W_tile[half][128 x 128 B] . Xl_tile^T, four K steps of 32 bytes per stage
-    const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | (((uint32_t)n_mma >> 3) << 17) | ((128u >> 4) << 24);
-    for (int it = 0; it < iters && !dead; ++it) {
-      const int s = it % kStages;
-      if (!mbar_wait_l(smem_addr(&sm.full[s]), (uint32_t)(it / kStages) & 1u)) {
+  } else if (warp == 1 && pair_rank == 0) {
+    // ---- MMA issue (for the pair): D_half[128 kCtas n x 2 Mp] += W_tile[half] . Xl_tile^T, four K steps of 32 bytes per tile
+    const bool elected = elect_sync();
+    const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | (((uint32_t)n_mma >> 3) << 17) | ((128u * kCtas >> 4) << 24);
+    const uint16_t both = (uint16_t)(3u << leader);
+    auto commit = [&](uint64_t* bar) {  // arrives at this barrier, in both CTAs of a pair
+      if constexpr (kPair)
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_addr(bar)),
+                     "h"(both)
+                     : "memory");
+      else
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(bar)) : "memory");
+    };
+    const uint64_t w_step = (uint64_t)((a.tile * kTileK) >> 4), x_step = (uint64_t)(((n_mma / kCtas) * kTileK) >> 4);
+    const uint64_t w_half = (uint64_t)((width * kTileK) >> 4);
+    int s = 0;
+    uint32_t parity = 0, acc = 0;
+    for (int it = 0; it < iters; ++it) {
+      if (!__all_sync(0xffffffffu, mbar_wait_l(smem_addr(&sm.full[s]), parity))) {
         dead = true;
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t wa = smem_addr(&sm.w[s][0]), xa = smem_addr(&sm.x[s][0]);
+      uint64_t wd = desc_k_major_128b(smem_addr(ring + s * a.stage_bytes)), xd = desc_k_major_128b(smem_addr(ring + s * a.stage_bytes + x_off));
+      for (int kt = 0; kt < a.kb; ++kt) {
+        if (elected) {
 #pragma unroll
-      for (int ks = 0; ks < 4; ++ks) {
-        const uint64_t bd = desc_k_major_128b(xa + 32 * ks);
-        const uint32_t acc = (it > 0 || ks > 0) ? 1u : 0u;
+          for (int ks = 0; ks < 4; ++ks) {
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          const uint64_t ad = desc_k_major_128b(wa + half * (128 * kTileK) + 32 * ks);
-          asm volatile(
-              "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-              "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem + (uint32_t)(half * n_mma)),
-              "l"(ad), "l"(bd), "r"(idesc), "r"(acc)
-              : "memory");
+            for (int half = 0; half < halves; ++half) {
+              const uint32_t d = tmem + (uint32_t)(half * n_mma);
+              const uint64_t wk = wd + (half ? w_half : 0u) + (uint64_t)(2 * ks), xk = xd + (uint64_t)(2 * ks);
+              if constexpr (kPair)
+                asm volatile(
+                    "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                    "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
+                    "l"(wk), "l"(xk), "r"(idesc), "r"(ks ? 1u : acc)
+                    : "memory");
+              else
+                asm volatile(
+                    "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                    "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
+                    "l"(wk), "l"(xk), "r"(idesc), "r"(ks ? 1u : acc)
+                    : "memory");
+            }
+          }
         }
+        acc = 1;
+        wd += w_step, xd += x_step;
       }
-      // the stage is free again when these MMAs have read it
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(&sm.empty[s]))
-                   : "memory");
+      if (elected) commit(&sm.empty[s]);  // the stage is free again when these MMAs have read it
+      if (++s == a.stages) s = 0, parity ^= 1u;
     }
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(&sm.done))
-                 : "memory");
+    if (elected) commit(&sm.done);
   }
   __syncwarp();
-  // ---- epilogue: lane n of accumulator `half` belongs to thread n (output channel n0 + 128 half + n)
-  const int csize = (int)gridDim.y;  // CTAs in the cluster = K splits
-  const int groups = Mp / 8;         // groups of eight rows of the batch; group j belongs to rank j % csize
-  const int owned = (groups + csize - 1) / csize;
-  // landing area in the ring: [source rank][owned group][half][row of the group][thread] fp32
+  // ---- epilogue: thread (half, j) of the 256 owns lane j of accumulator `half`, i.e. channel n0 + half * width + j, and with
+  // one half only every second part of that lane's rows
+  const int groups = Mp / 8;  // groups of eight rows of the batch; group j belongs to split j % nsplit
+  const int owned = (groups + nsplit - 1) / nsplit;
+  const int half = halves == 2 ? warp >> 2 : 0, j = (warp & 3) * 32 + lane;
+  const int c_first = halves == 2 ? 0 : warp >> 2, c_step = halves == 2 ? 1 : 2;  // (sixteen rows at a time)
+  const int n = n0 + half * width + j;
+  const bool live = j < width && n < N;
+  const float sc = live ? __bfloat162float(a.scale[n]) : 0.f;
+  // landing area in the ring: [source split][owned group][half][row of the group][lane] fp32
   float* land = reinterpret_cast<float*>(smem_raw);
   const bool ok = mbar_wait_l(smem_addr(&sm.done), 0u);
   const bool bad = __syncthreads_or(dead || !ok) != 0;
-  if (bad && tid == 0) atomicExch(status, 1);  // (only if the copy engine or the tensor core stopped answering)
+  if (bad && tid == 0) atomicExch(a.status, 1);  // (only if the copy engine or the tensor core stopped answering)
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  cluster_sync();  // every ring of the cluster has been read to the end: the landing areas are free
+  const bool exchange = nsplit > 1 || tp.world > 1;
+  if (exchange) cluster_sync();  // every ring of the cluster has been read to the end: the landing areas are free
+  auto store = [&](int m, float dot32) {
+    const float dot = __bfloat162float(__float2bfloat16_rn(dot32));                  // F.linear's bf16 result
+    if (live && m < M) a.y[(int64_t)m * N + n] = __float2bfloat16_rn(dot * sc);      // * weight_scaler
+  };
   if (!bad) {
-    for (int m0 = 0; m0 < Mp; m0 += 32) {
-      uint32_t h[2][32], l[2][32];
+    const uint32_t lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(half * n_mma);
+    uint32_t v[2][2][16];  // [parity][h, l][row]: the next sixteen rows leave tensor memory while these are worked on
+    auto fetch = [&](int c, uint32_t (&d)[2][16]) {
+      tmem_ld_16(lanes + (uint32_t)(16 * c), d[0]);
+      tmem_ld_16(lanes + (uint32_t)(Mp + 16 * c), d[1]);
+    };
+    auto finish = [&](int c, const uint32_t (&d)[2][16]) {
+      float sum[16];
 #pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(half * n_mma);
-        tmem_ld_32(lane_addr + (uint32_t)m0, h[half]);
-        tmem_ld_32(lane_addr + (uint32_t)(Mp + m0), l[half]);
+      for (int r = 0; r < 16; r += 4) {
+        const float4 x4 = *reinterpret_cast<const float4*>(&sm.xs[16 * c + r]);
+        const float xr[4] = {x4.x, x4.y, x4.z, x4.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) sum[r + e] = fmaf((float)(int)d[0][r + e], 254.f, (float)(int)d[1][r + e]) * xr[e];
       }
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      float xr[32];  // (all loads before the stores: the compiler cannot move them across)
+      if (!exchange) {
 #pragma unroll
-      for (int jj = 0; jj < 32; ++jj) xr[jj] = sm.xs[(m0 + jj) & (kMaxM - 1)];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const int j = m0 / 8 + c;
-        if (j < groups) {
-          const int owner = j % csize, q = j / csize;
-          const uint32_t base = remote_smem(smem_addr(land + ((((int64_t)split * owned + q) * 2) * 8) * kThreadsL + tid), owner);
-#pragma unroll
-          for (int half = 0; half < 2; ++half) {
-#pragma unroll
-            for (int r = 0; r < 8; ++r) {
-              const int jj = 8 * c + r;
-              const float v = fmaf((float)(int)h[half][jj], 254.f, (float)(int)l[half][jj]) * xr[jj];
-              st_cluster_f32(base + (uint32_t)((half * 8 + r) * kThreadsL * 4), v);
-            }
-          }
-        }
+        for (int r = 0; r < 16; ++r) store(16 * c + r, sum[r]);
+        return;
       }
-    }
-  }
-  float sc[2];
 #pragma unroll
-  for (int half = 0; half < 2; ++half) {
-    const int n = n0 + half * 128 + tid;
-    sc[half] = n < N ? __bfloat162float(scale[n]) : 0.f;
-  }
-  cluster_sync();  // all partial sums have landed
-  if (!bad) {
-    auto reduce = [&](auto cs_tag) {
-      constexpr int kCs = decltype(cs_tag)::value;
-      for (int q = 0; q < owned; ++q) {
-        const int j = q * kCs + split;
-        if (j >= groups) break;
-        float acc[2][8];  // (sixteen independent chains; all loads before the stores)
+      for (int part = 0; part < 2; ++part) {
+        const int g = 2 * c + part, q = g / nsplit, owner = kCtas * (g - q * nsplit) + pair_rank;
+        const uint32_t base = remote_smem(smem_addr(land + ((split * owned + q) * halves + half) * 8 * 128 + j), owner);
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-#pragma unroll
-          for (int r = 0; r < 8; ++r) acc[half][r] = land[(((0 * owned + q) * 2 + half) * 8 + r) * kThreadsL + tid];
-        }
-#pragma unroll
-        for (int src = 1; src < kCs; ++src) {
-#pragma unroll
-          for (int half = 0; half < 2; ++half) {
-#pragma unroll
-            for (int r = 0; r < 8; ++r) acc[half][r] += land[(((src * owned + q) * 2 + half) * 8 + r) * kThreadsL + tid];
-          }
-        }
-        if (tp.world > 1) {
-          // this rank's sums of the group go into its own buffer, where the other ranks read them; the roundings
-          // follow below, on the sum over the ranks
-          float* dst = reinterpret_cast<float*>(tp.buffers[tp.rank] + kTpDataOffset) + (int64_t)(tp_epoch & 1u) * kMaxM * N;
-#pragma unroll
-          for (int half = 0; half < 2; ++half) {
-            const int n = n0 + half * 128 + tid;
-#pragma unroll
-            for (int r = 0; r < 8; ++r) {
-              const int m = 8 * j + r;
-              if (m < M && n < N) __stcg(&dst[(int64_t)m * N + n], acc[half][r]);
-            }
-          }
-          continue;
-        }
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          const int n = n0 + half * 128 + tid;
-#pragma unroll
-          for (int r = 0; r < 8; ++r) {
-            const int m = 8 * j + r;
-            const float dot = __bfloat162float(__float2bfloat16_rn(acc[half][r]));            // F.linear's bf16 result
-            if (m < M && n < N) y[(int64_t)m * N + n] = __float2bfloat16_rn(dot * sc[half]);  // * weight_scaler
-          }
-        }
+        for (int r = 0; r < 8; ++r) st_cluster_f32(base + (uint32_t)(r * 128 * 4), sum[8 * part + r]);
       }
     };
-    switch (csize) {
-      case 1: reduce(std::integral_constant<int, 1>{}); break;
-      case 2: reduce(std::integral_constant<int, 2>{}); break;
-      case 3: reduce(std::integral_constant<int, 3>{}); break;
-      case 4: reduce(std::integral_constant<int, 4>{}); break;
-      case 5: reduce(std::integral_constant<int, 5>{}); break;
-      case 6: reduce(std::integral_constant<int, 6>{}); break;
-      case 7: reduce(std::integral_constant<int, 7>{}); break;
-      default: reduce(std::integral_constant<int, 8>{}); break;
-    }
-    if (tp.world > 1 && split < groups) {  // (a CTA without a group of rows has nothing to send or to wait for)
-      // ---- sum over the ranks: tell every rank that this CTA's groups are in this rank's buffer, wait (bounded) for
-      // the same CTA of every rank, read their sums and add them in the order of the ranks
-      const int par = (int)(tp_epoch & 1u);
-      auto flag_of = [&](int buffer_of, int src) {  // the sums of rank `src` are ready, as told to rank `buffer_of`
-        return reinterpret_cast<unsigned*>(tp.buffers[buffer_of] + kTpFlagOffset) +
-               (((size_t)par * 8 + src) * kTpMaxTiles + blockIdx.x) * 8 + split;
-      };
-      __syncthreads();  // every thread's stores are issued ...
-      if (tid < tp.world && tid != tp.rank) {
-        __threadfence_system();  // ... and ordered before the launch number that announces them
-        st_sys_u32(flag_of(tid, tp.rank), tp_epoch);
-        const long long t0c = clock64();
-        while (ld_sys_u32(flag_of(tp.rank, tid)) != tp_epoch) {
-          if (clock64() - t0c > tp.wait_cycles) {  // a rank never came: report, go on with what is there
-            atomicExch(tp.status, 1);
-            break;
-          }
-        }
-        __threadfence_system();
+    const int chunks = Mp / 16;
+    if (c_first < chunks) fetch(c_first, v[0]);
+    for (int c = c_first; c < chunks; c += 2 * c_step) {
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      if (c + c_step < chunks) fetch(c + c_step, v[1]);
+      finish(c, v[0]);
+      if (c + c_step < chunks) {
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (c + 2 * c_step < chunks) fetch(c + 2 * c_step, v[0]);
+        finish(c + c_step, v[1]);
       }
-      __syncthreads();
-      asm volatile("" ::: "memory");  // (the peer loads below carry no memory clobber of their own)
-      const size_t part_off = kTpDataOffset + (size_t)par * kMaxM * N * sizeof(float);
-      // A group is eight rows x 256 channels: 512 pieces of four channels (16 bytes), four per thread.  A thread
-      // has the pieces of up to three groups (twelve loads per rank) in flight at a time.
-      constexpr int kBatch = 12;
-      const int my_groups = (groups - split + csize - 1) / csize;
-      for (int base = 0; base < 4 * my_groups; base += kBatch) {
-        float4 sum[kBatch];
-        int64_t at[kBatch];  // element offset of the piece, -1: none
+    }
+  }
+  if (exchange) {
+    cluster_sync();  // all partial sums have landed
+    if (!bad) {
+      auto reduce = [&](auto cs_tag) {
+        constexpr int kCs = decltype(cs_tag)::value;
+        // (the landing area is written with a lane per channel: with one half the two groups of warps take turns here too)
+        for (int q = c_first; q < owned; q += c_step) {
+          const int g = q * kCs + split;
+          if (g >= groups) break;
+          float acc[8];  // (eight independent chains; all loads before the stores)
 #pragma unroll
-        for (int b = 0; b < kBatch; ++b) {
-          const int idx = base + b, item = (idx & 3) * kThreadsL + tid;
-          const int m = 8 * ((idx >> 2) * csize + split) + (item >> 6), n = n0 + 4 * (item & 63);
-          at[b] = (idx < 4 * my_groups && m < M && n < N) ? (int64_t)m * N + n : -1;
-          sum[b] = make_float4(0.f, 0.f, 0.f, 0.f);
+          for (int r = 0; r < 8; ++r) acc[r] = land[(((0 * owned + q) * halves + half) * 8 + r) * 128 + j];
+#pragma unroll
+          for (int src = 1; src < kCs; ++src) {
+#pragma unroll
+            for (int r = 0; r < 8; ++r) acc[r] += land[(((src * owned + q) * halves + half) * 8 + r) * 128 + j];
+          }
+          if (tp.world > 1) {
+            // this rank's sums of the group go into its own buffer, where the other ranks read them; the roundings
+            // follow below, on the sum over the ranks
+            float* dst = reinterpret_cast<float*>(tp.buffers[tp.rank] + kTpDataOffset) + (int64_t)(tp_epoch & 1u) * kMaxM * N;
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+              const int m = 8 * g + r;
+              if (m < M && live) __stcg(&dst[(int64_t)m * N + n], acc[r]);
+            }
+            continue;
+          }
+#pragma unroll
+          for (int r = 0; r < 8; ++r) store(8 * g + r, acc[r]);
         }
-        for (int src = 0; src < tp.world; ++src) {
-          const float* part = reinterpret_cast<const float*>(tp.buffers[src] + part_off);
-          float4 v[kBatch];
+      };
+      switch (nsplit) {
+        case 1: reduce(std::integral_constant<int, 1>{}); break;
+        case 2: reduce(std::integral_constant<int, 2>{}); break;
+        case 3: reduce(std::integral_constant<int, 3>{}); break;
+        case 4: reduce(std::integral_constant<int, 4>{}); break;
+        case 5: reduce(std::integral_constant<int, 5>{}); break;
+        case 6: reduce(std::integral_constant<int, 6>{}); break;
+        case 7: reduce(std::integral_constant<int, 7>{}); break;
+        default: reduce(std::integral_constant<int, 8>{}); break;
+      }
+      if (tp.world > 1 && split < groups) {  // (a CTA without a group of rows has nothing to send or to wait for)
+        // ---- sum over the ranks: tell every rank that this CTA's groups are in this rank's buffer, wait (bounded) for
+        // the same CTA of every rank, read their sums and add them in the order of the ranks
+        const int par = (int)(tp_epoch & 1u);
+        auto flag_of = [&](int buffer_of, int src) {  // the sums of rank `src` are ready, as told to rank `buffer_of`
+          return reinterpret_cast<unsigned*>(tp.buffers[buffer_of] + kTpFlagOffset) +
+                 (((size_t)par * 8 + src) * kTpMaxTiles + blockIdx.x) * 8 + split;
+        };
+        __syncthreads();  // every thread's stores are issued ...
+        if (tid < tp.world && tid != tp.rank) {
+          __threadfence_system();  // ... and ordered before the launch number that announces them
+          st_sys_u32(flag_of(tid, tp.rank), tp_epoch);
+          const long long t0c = clock64();
+          while (ld_sys_u32(flag_of(tp.rank, tid)) != tp_epoch) {
+            if (clock64() - t0c > tp.wait_cycles) {  // a rank never came: report, go on with what is there
+              atomicExch(tp.status, 1);
+              break;
+            }
+          }
+          __threadfence_system();
+        }
+        __syncthreads();
+        asm volatile("" ::: "memory");  // (the peer loads below carry no memory clobber of their own)
+        const size_t part_off = kTpDataOffset + (size_t)par * kMaxM * N * sizeof(float);
+        // A group is eight rows x `tile` channels, in pieces of four channels (16 bytes; a tile is a multiple of eight
+        // channels).  A thread has twelve pieces (twelve loads per rank) in flight at a time.
+        constexpr int kBatch = 12;
+        const int my_groups = (groups - split + nsplit - 1) / nsplit, per_row = a.tile / 4, pieces = my_groups * 8 * per_row;
+        for (int base = tid; base < pieces; base += kBatch * kThreadsL) {
+          float4 sum[kBatch];
+          int64_t at[kBatch];  // element offset of the piece, -1: none
 #pragma unroll
           for (int b = 0; b < kBatch; ++b) {
-            v[b] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (at[b] >= 0) v[b] = src == tp.rank ? __ldcg(reinterpret_cast<const float4*>(part + at[b])) : ld_sys_f32x4(part + at[b]);
+            const int idx = base + b * kThreadsL, row = idx / per_row;
+            const int m = 8 * ((row >> 3) * nsplit + split) + (row & 7), c = n0 + 4 * (idx % per_row);
+            at[b] = (idx < pieces && m < M && c < N) ? (int64_t)m * N + c : -1;
+            sum[b] = make_float4(0.f, 0.f, 0.f, 0.f);
+          }
+          for (int src = 0; src < tp.world; ++src) {
+            const float* part = reinterpret_cast<const float*>(tp.buffers[src] + part_off);
+            float4 v[kBatch];
+#pragma unroll
+            for (int b = 0; b < kBatch; ++b) {
+              v[b] = make_float4(0.f, 0.f, 0.f, 0.f);
+              if (at[b] >= 0) v[b] = src == tp.rank ? __ldcg(reinterpret_cast<const float4*>(part + at[b])) : ld_sys_f32x4(part + at[b]);
+            }
+#pragma unroll
+            for (int b = 0; b < kBatch; ++b) sum[b].x += v[b].x, sum[b].y += v[b].y, sum[b].z += v[b].z, sum[b].w += v[b].w;
           }
 #pragma unroll
-          for (int b = 0; b < kBatch; ++b) sum[b].x += v[b].x, sum[b].y += v[b].y, sum[b].z += v[b].z, sum[b].w += v[b].w;
-        }
+          for (int b = 0; b < kBatch; ++b) {
+            if (at[b] < 0) continue;
+            const int c = (int)(at[b] % N);
+            const uint2 sraw = __ldg(reinterpret_cast<const uint2*>(a.scale + c));
+            const __nv_bfloat16* sb = reinterpret_cast<const __nv_bfloat16*>(&sraw);
+            const float a4[4] = {sum[b].x, sum[b].y, sum[b].z, sum[b].w};
+            uint2 o;
+            __nv_bfloat16* ob = reinterpret_cast<__nv_bfloat16*>(&o);
 #pragma unroll
-        for (int b = 0; b < kBatch; ++b) {
-          if (at[b] < 0) continue;
-          const int n = (int)(at[b] % N);
-          const uint2 sraw = __ldg(reinterpret_cast<const uint2*>(scale + n));
-          const __nv_bfloat16* sb = reinterpret_cast<const __nv_bfloat16*>(&sraw);
-          const float a4[4] = {sum[b].x, sum[b].y, sum[b].z, sum[b].w};
-          uint2 o;
-          __nv_bfloat16* ob = reinterpret_cast<__nv_bfloat16*>(&o);
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-            ob[e] = __float2bfloat16_rn(__bfloat162float(__float2bfloat16_rn(a4[e])) * __bfloat162float(sb[e]));
-          *reinterpret_cast<uint2*>(y + at[b]) = o;
+            for (int e = 0; e < 4; ++e)
+              ob[e] = __float2bfloat16_rn(__bfloat162float(__float2bfloat16_rn(a4[e])) * __bfloat162float(sb[e]));
+            *reinterpret_cast<uint2*>(a.y + at[b]) = o;
+          }
         }
       }
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if constexpr (kPair) cluster_sync();  // (tensor memory is given back by both CTAs of a pair, when neither reads it any more)
   if (warp == 1) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)kTmemColsL) : "memory");
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if constexpr (kPair)
+      asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols) : "memory");
+    else
+      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols) : "memory");
   }
 }
 
@@ -979,6 +1067,17 @@ EncodeTiledFn encode_fn() {
   }();
   return fn;
 }
+// rows x K bytes, row-major, seen as K / 128 steps of [rows x 128 bytes]; boxes of kb steps of box_rows rows, 128-byte swizzle
+bool encode_steps(CUtensorMap* map, const void* base, int64_t rows, int64_t K, int box_rows, int kb) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return false;
+  const cuuint64_t dims[3] = {(cuuint64_t)kTileK, (cuuint64_t)rows, (cuuint64_t)(K / kTileK)};
+  const cuuint64_t str[2] = {(cuuint64_t)K, (cuuint64_t)kTileK};
+  const cuuint32_t box[3] = {(cuuint32_t)kTileK, (cuuint32_t)box_rows, (cuuint32_t)kb};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), dims, str, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
 // rows x K bytes, row-major; boxes of box_rows x 128 bytes with the 128-byte swizzle
 bool encode_2d(CUtensorMap* map, const void* base, int64_t rows, int64_t K, int box_rows) {
   EncodeTiledFn fn = encode_fn();
@@ -1019,20 +1118,47 @@ RowBlocks row_blocks(int M, int N, int K, int channels) {
   return best;
 }
 
-int split_for(int N, int K) {
-  static const int sms = sm_count_l();
-  const int tiles = (N + kTileN - 1) / kTileN, k_tiles = K / kTileK;
-  // The K splits of a tile are the CTAs of one cluster (1 .. 8; the K steps are dealt out evenly).  The split with
-  // the shortest estimated run is taken: CTAs run in waves of one per SM; a CTA costs about 8 us of set-up, first
-  // fetch and epilogue plus 0.6 us per K step (measured on B200 for 96 rows).
-  int split = 1;
-  float best = 0.f;
-  for (int c = 1; c <= kMaxSplit && c <= k_tiles; ++c) {
-    const int waves = (tiles * c + sms - 1) / sms;
-    const float cost = (float)waves * (8.f + 0.6f * (float)((k_tiles + c - 1) / c));
-    if (c == 1 || cost < best) best = cost, split = c;
+// How the channels and the K steps are dealt out over the SMs.  Clusters of `split` CTAs or pairs; `slots` of them fit the GPU at
+// once (a cluster lies within a group of SMs, so that larger ones leave some SMs over: the driver says how many).  For
+// every form the tile is the narrowest that covers the channels in whole waves of clusters; the plan with the shortest
+// estimated run is taken.  A stage costs its hand-over and its MMAs or bytes (the weights at a share of the memory rate, the
+// activations from L2); a wave costs set-up, first fetch and epilogue.  The constants (us, bytes per us) are fitted to the
+// measured times of up to nine forms each of 9 shapes (1280 to 28672 channels, K of 4096 to 28672) with 7 and 96 rows: the form taken
+// is within 4 % of the fastest of them everywhere and the estimate mostly within 10 %.  Measured, us, 96 rows / 7 rows: pairs on
+// 8192 -> 28672 49.0 / 40.7 (single CTAs 52.1 / 42.4), pairs in two splits on 28672 -> 8192 46.4 / 37.8 (single CTAs in four 51.0 /
+// 42.0), single CTAs in four splits on 14336 -> 4096 17.1 / 12.7 (one pair per tile 31.8 / 18.2).
+struct GemmPlan {
+  int pair, split, tile, halves, tiles, kb;
+};
+constexpr int kMaxCluster = 8;  // CTAs of a cluster: the portable limit
+int cluster_slots(bool pair, int split);
+GemmPlan plan_gemm(int M, int N, int K, bool tp) {
+  const int k_tiles = K / kTileK, Mp = (M + 15) / 16 * 16;
+  GemmPlan best{};
+  float best_cost = 0.f;
+  for (int ctas = 1; ctas <= 2; ++ctas) {
+    const int x_rows = 2 * Mp / ctas;
+    for (int c = 1; c * ctas <= kMaxCluster && c <= k_tiles; ++c) {
+      const int slots = cluster_slots(ctas == 2, c);
+      const int waves = (N + ctas * kTileN * slots - 1) / (ctas * kTileN * slots);
+      int tile = (N + ctas * slots * waves - 1) / (ctas * slots * waves);
+      tile = tile <= 128 ? std::max(32, (tile + 7) / 8 * 8) : (tile + 15) / 16 * 16;
+      if (tp && (N + tile - 1) / tile >= kTpMaxTiles) tile = kTileN;  // (the exchange between the ranks counts its tiles)
+      const int halves = tile <= 128 ? 1 : 2;
+      // Stages of about 32 KB: four to six of them are in flight, and none is so short that its hand-over is what it costs.
+      int kb = 1;
+      while (kb < 8 && 2 * kb * c <= k_tiles && 2 * kb * (tile + x_rows) * kTileK <= 40 * 1024) kb *= 2;
+      const int groups = (N + ctas * tile - 1) / (ctas * tile), rounds = (groups + slots - 1) / slots;
+      const int steps = ((k_tiles + kb - 1) / kb + c - 1) / c;
+      const int active = std::min(groups, slots) * c * ctas;
+      const float mma = (float)halves * std::max(0.11f, 0.0021f * (float)Mp);
+      const float bytes = (float)(tile * kTileK) * (float)active / 8.6e6f + (float)(x_rows * kTileK) / 288e3f + 0.033f * (float)(halves - 1);
+      const float step = 0.063f + (float)kb * std::max(mma, bytes);
+      const float cost = (float)rounds * (4.35f + 0.024f * (float)(Mp * halves) + (ctas == 2 ? 0.7f : 0.f) + (c > 1 ? 0.33f : 0.f) + (float)steps * step);
+      if (best.tiles == 0 || cost < best_cost) best_cost = cost, best = GemmPlan{ctas == 2, c, tile, halves, ctas * groups, kb};
+    }
   }
-  return split;
+  return best;
 }
 
 }  // namespace
@@ -1048,7 +1174,7 @@ static size_t blocks_workspace_bytes(const RowBlocks& rb, int K) {
 extern "C" size_t jpt_w8a16_linear_workspace_bytes(int M, int N, int K) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (M > kMaxM) return blocks_workspace_bytes(row_blocks(M, N, K, kTileN), K);
-  const int Mp = (M + 7) / 8 * 8;
+  const int Mp = (M + 15) / 16 * 16;
   const size_t levels = ((size_t)2 * Mp * K + 255) / 256 * 256;
   const size_t xs = 1024;
   return 256 + levels + xs;
@@ -1070,7 +1196,7 @@ struct LevelsView {
 };
 LevelsView levels_view(void* workspace, int M, int K) {
   LevelsView v;
-  v.Mp = (M + 7) / 8 * 8;
+  v.Mp = (M + 15) / 16 * 16;
   char* ws = static_cast<char*>(workspace);
   v.status = reinterpret_cast<int*>(ws);
   v.lev = reinterpret_cast<int8_t*>(ws + 256);
@@ -1079,48 +1205,82 @@ LevelsView levels_view(void* workspace, int M, int K) {
   return v;
 }
 
-// The GEMM on levels that a launch before this one in the stream wrote.  The launch may start while that one
-// drains (it requests its first weight tiles at once) and waits for its results on the device.
-int launch_gemm(const LevelsView& lv, const void* w, const void* w_scale, void* y, int M, int N, int K, cudaStream_t st,
-                const TpArgs* tp_in = nullptr) {
-  const int ksplit = split_for(N, K);
-  TpArgs tp;
-  memset(&tp, 0, sizeof(tp));
-  tp.world = 1;
-  if (tp_in) tp = *tp_in;
-  static std::mutex mu;
-  LinearMaps maps;
-  memset(&maps, 0, sizeof(maps));
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    JPT_REQUIRE(encode_2d(&maps.w, w, N, K, kTileN) && encode_2d(&maps.x, lv.lev, 2 * lv.Mp, K, 2 * lv.Mp), JPT_EINVAL,
-                "w8a16_linear: the tensors cannot be described by a tensor map");
-  }
-  static bool configured[64];
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev >= 0 && dev < 64 && !configured[dev]) {
-    const cudaError_t e = cudaFuncSetAttribute(w8a16_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemL));
-    if (e != cudaSuccess) return fail((int)e, "w8a16_linear: configuring the kernel: %s", cudaGetErrorString(e));
-    configured[dev] = true;
-  }
+// Clusters of `split` CTAs or pairs that the current device holds at once; the kernels' attributes are set on the way.
+constexpr size_t kGemmSmem = kRingBytes + kTailBytes;
+using GemmKernel = void (*)(const LinearMaps, const GemmArgs, const TpArgs);
+GemmKernel gemm_kernel(bool pair, int halves) {
+  if (pair) return halves == 2 ? w8a16_gemm_kernel<true, 2> : w8a16_gemm_kernel<true, 1>;
+  return halves == 2 ? w8a16_gemm_kernel<false, 2> : w8a16_gemm_kernel<false, 1>;
+}
+cudaLaunchConfig_t gemm_config(dim3 grid, size_t smem, cudaStream_t st, cudaLaunchAttribute (&attr)[2], bool pair, int split) {
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((N + kTileN - 1) / kTileN, ksplit);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3(kThreadsL);
-  cfg.dynamicSmemBytes = sizeof(SmemL);
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 1;
-  attr[0].val.clusterDim.y = ksplit;
+  attr[0].val.clusterDim.x = pair ? 2 : 1;
+  attr[0].val.clusterDim.y = split;
   attr[0].val.clusterDim.z = 1;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+int cluster_slots(bool pair, int split) {
+  static std::mutex mu;
+  static int known[64][2][kMaxCluster + 1];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lock(mu);
+  int& n = known[dev & 63][pair][split];
+  if (n == 0) {
+    cudaLaunchAttribute attr[2];
+    const cudaLaunchConfig_t cfg = gemm_config(dim3(pair ? 2 : 1, split), kGemmSmem, nullptr, attr, pair, split);
+    bool ok = true;
+    for (int halves = 1; halves <= 2; ++halves)
+      ok = ok && cudaFuncSetAttribute(gemm_kernel(pair, halves), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem) == cudaSuccess;
+    if (!ok || cudaOccupancyMaxActiveClusters(&n, gemm_kernel(pair, 2), &cfg) != cudaSuccess || n <= 0) {
+      cudaGetLastError();
+      n = 0;
+      return std::max(1, sm_count_l() / ((pair ? 2 : 1) * split));  // (asked again at the next call; the launch reports what is wrong)
+    }
+  }
+  return n;
+}
+
+// The GEMM on levels that a launch before this one in the stream wrote.  The launch may start while that one
+// drains (it requests its first weight tiles at once) and waits for its results on the device.
+int launch_gemm(const LevelsView& lv, const void* w, const void* w_scale, void* y, int M, int N, int K, cudaStream_t st,
+                const TpArgs* tp_in = nullptr) {
+  const GemmPlan plan = plan_gemm(M, N, K, tp_in != nullptr);
+  const int x_rows = plan.pair ? lv.Mp : 2 * lv.Mp;  // rows of levels that a CTA loads
+  TpArgs tp;
+  memset(&tp, 0, sizeof(tp));
+  tp.world = 1;
+  if (tp_in) tp = *tp_in;
+  LinearMaps maps;
+  memset(&maps, 0, sizeof(maps));
+  JPT_REQUIRE(encode_steps(&maps.w, w, N, K, plan.tile, plan.kb) && encode_steps(&maps.x, lv.lev, 2 * lv.Mp, K, x_rows, plan.kb), JPT_EINVAL,
+              "w8a16_linear: the tensors cannot be described by a tensor map");
+  GemmArgs a;
+  memset(&a, 0, sizeof(a));
+  a.xs = lv.xs;
+  a.scale = static_cast<const __nv_bfloat16*>(w_scale);
+  a.y = static_cast<__nv_bfloat16*>(y);
+  a.status = lv.status;
+  a.M = M, a.Mp = lv.Mp, a.N = N, a.k_steps = (K / kTileK + plan.kb - 1) / plan.kb;
+  a.tile = plan.tile, a.kb = plan.kb;
+  a.stage_bytes = plan.kb * (plan.tile + x_rows) * kTileK;
+  a.stages = std::min(kMaxStages, kRingBytes / a.stage_bytes);
+  // the landing area of the partial sums: [split][groups a split owns][half][8 rows][128 lanes] fp32, at most 23 groups = 184 KB
+  const int landing = plan.split * ((lv.Mp / 8 + plan.split - 1) / plan.split) * plan.halves * 8 * 128 * (int)sizeof(float);
+  a.tail = std::max(a.stages * a.stage_bytes, landing);
+  cudaLaunchAttribute attr[2];
+  cudaLaunchConfig_t cfg = gemm_config(dim3(plan.tiles, plan.split), (size_t)a.tail + kTailBytes, st, attr, plan.pair, plan.split);
   cfg.numAttrs = pdl_enabled() ? 2 : 1;  // (also inside a graph capture: the weight tiles stream in under the level kernel)
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, w8a16_gemm_kernel, maps, static_cast<const float*>(lv.xs),
-                                           static_cast<const __nv_bfloat16*>(w_scale), static_cast<__nv_bfloat16*>(y), M, lv.Mp, N, K,
-                                           K / kTileK, lv.status, tp);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_kernel(plan.pair, plan.halves), maps, a, tp);
   if (e != cudaSuccess) return fail((int)e, "w8a16_gemm_kernel: %s", cudaGetErrorString(e));
   return 0;
 }
