@@ -1152,7 +1152,7 @@ GemmPlan plan_gemm(int M, int N, int K, bool tp) {
       const int steps = ((k_tiles + kb - 1) / kb + c - 1) / c;
       const int active = std::min(groups, slots) * c * ctas;
       const float mma = (float)halves * std::max(0.11f, 0.0021f * (float)Mp);
-      const float bytes = (float)(tile * kTileK) * (float)active / 8.6e6f + (float)(x_rows * kTileK) / 288e3f + 0.033f * (float)(halves - 1);
+      const float bytes = (float)(tile * kTileK) * (float)active / 8.6e6f + (float)(x_rows * kTileK) / 288e3f + 0.045f * (float)(halves - 1);
       const float step = 0.063f + (float)kb * std::max(mma, bytes);
       const float cost = (float)rounds * (4.35f + 0.024f * (float)(Mp * halves) + (ctas == 2 ? 0.7f : 0.f) + (c > 1 ? 0.33f : 0.f) + (float)steps * step);
       if (best.tiles == 0 || cost < best_cost) best_cost = cost, best = GemmPlan{ctas == 2, c, tile, halves, ctas * groups, kb};
