@@ -257,6 +257,13 @@ struct TmaMaps {
 };
 constexpr int kTmaNone = 0, kTmaDense = 1, kTmaPaged = 2;
 
+// true in one lane of a converged warp, always the same one
+__device__ __forceinline__ bool elect_sync() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(r));
+  return r != 0;
+}
+
 // maximum over the 32 lanes in one instruction
 __device__ __forceinline__ float warp_max(float x) {
   float r;
@@ -302,6 +309,10 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
   }
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // Instructions of the tensor core and the copy engine are issued by the elected lane of a warp: the compiler takes their operands
+  // out of uniform registers, and under any other condition (tid == 0) wraps every one of them in a loop over the lanes. (B200,
+  // 96 sequences of 8 KV heads and 1 to 2047 tokens: 62.3 -> 59.4 us with the new token; paged, 512 to 2047: 62.7 -> 59.3.)
+  const bool elected = elect_sync();
   // slots charged per segment on top of its tiles (with the new token: one more for its quantisation)
   constexpr int kPieceCost = kFused ? JPT_PIECE_COST_FUSED : kPieceCostU;
   const int R = a.R;
@@ -751,8 +762,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
   // records and requests the K rows, warp 2 requests the V rows, warp 3 issues the O^T MMAs
   // (44.1 us per launch on the bench workload against 45.2 with everything in thread 0).
   constexpr bool kSpread = kTma && !kFused;
-  constexpr int kWalkerWarp = kSpread ? 1 : 0, kWalkerThread = 32 * kWalkerWarp;
-  constexpr int kVRequestThread = kSpread ? 64 : 0, kPvThread = kSpread ? 96 : 0;
+  constexpr int kWalkerWarp = kSpread ? 1 : 0, kVRequestWarp = kSpread ? 2 : 0, kPvWarp = kSpread ? 3 : 0;
   auto issue_k = [&](int seq) {
     if constexpr (kSpread) {
       if (warp != kWalkerWarp) {  // (the others keep their count of copy groups in step)
@@ -766,7 +776,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
       rg.first = pfirst;
       int pos, cnt;
       tile_rows(rg, a.S, pt, &pos, &cnt);
-      if (tid == kWalkerThread) {
+      if (warp == kWalkerWarp && elected) {
         TileMeta mt;
         mt.b = pb; mt.h = ph; mt.t = pt; mt.T = pT; mt.n = pn; mt.first = pfirst; mt.use_add = puse_add;
         mt.first_cta = pfirst_cta; mt.parts = pparts;
@@ -782,7 +792,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
         if (pext && pt == pT - 1) stage_new_token(seq, pb, ph);  // the segment's last tile takes the new token
       }
       advance();
-    } else if (tid == kWalkerThread) {
+    } else if (warp == kWalkerWarp && elected) {
       sm.meta[seq & 3].t = -1;
     }
     cp_async_commit();
@@ -800,7 +810,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
     const int cnt = sm.meta[seq & 3].pad[0], pos = sm.meta[seq & 3].pad[1];
     if (mtile >= 0) {
       if constexpr (kTma) {
-        if (tid == kVRequestThread) request_rows(smem_u32(&sm.v[seq & 1][0]), &maps.v, smem_u32(&sm.bar_v[seq & 1]), mb, mh, pos, cnt);
+        if (warp == kVRequestWarp && elected) request_rows(smem_u32(&sm.v[seq & 1][0]), &maps.v, smem_u32(&sm.bar_v[seq & 1]), mb, mh, pos, cnt);
       } else {
         copy_rows(smem_u32(&sm.v[seq & 1][0]), vbase, mb, mh, pos, cnt);
       }
@@ -903,16 +913,19 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
         __syncthreads();
       }
     }
-    if (tid == 0) {
+    if (warp == 0) {
       if constexpr (kTma) {
         if (!mbar_wait(smem_u32(&sm.bar_k[seq & 1]), (uint32_t)(seq >> 1) & 1u)) dead = true;
       }
+      __syncwarp();
       tc_fence_after();
-      const uint32_t k_addr = smem_u32(&sm.k[seq & 1][0]);
+      if (elected) {
+        const uint64_t kd = umma_desc(smem_u32(&sm.k[seq & 1][0])), qd = umma_desc(q_desc_addr);
 #pragma unroll
-      for (int ks = 0; ks < 4; ++ks)
-        umma_i8(tmem, umma_desc(k_addr + 32 * ks), umma_desc(q_desc_addr + 32 * ks), kIdescS, ks > 0);
-      umma_commit(bar_s);
+        for (int ks = 0; ks < 4; ++ks) umma_i8(tmem, kd + (uint64_t)(2 * ks), qd + (uint64_t)(2 * ks), kIdescS, ks > 0);
+        umma_commit(bar_s);
+      }
+      __syncwarp();
     }
   };
   // O^T of the tile with the given parity into the accumulators (alpha and cmax are that tile's)
@@ -1067,16 +1080,19 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
     __syncthreads();
 
     // ---------------- O^T = V^T Pl^T on the tensor core
-    if (tid == kPvThread) {
+    if (warp == kPvWarp) {
       if constexpr (kTma) {
         if (!mbar_wait(smem_u32(&sm.bar_v[i & 1]), (uint32_t)(i >> 1) & 1u)) dead = true;
       }
+      __syncwarp();
       tc_fence_after();
-      const uint32_t v_addr = smem_u32(&sm.v[i & 1][0]);
+      if (elected) {
+        const uint64_t vd = umma_desc(smem_u32(&sm.v[i & 1][0])), pd = umma_desc(p_desc_addr);
 #pragma unroll
-      for (int ks = 0; ks < 4; ++ks)
-        umma_i8(tmem + kColO, umma_desc(v_addr + 4096 * ks), umma_desc(p_desc_addr + 32 * ks), kIdescO, ks > 0);
-      umma_commit(bar_o);
+        for (int ks = 0; ks < 4; ++ks) umma_i8(tmem + kColO, vd + (uint64_t)(256 * ks), pd + (uint64_t)(2 * ks), kIdescO, ks > 0);
+        umma_commit(bar_o);
+      }
+      __syncwarp();
     }
 
     // The tile that ends a piece leaves through the epilogue below, after the next tile's S^T has been
