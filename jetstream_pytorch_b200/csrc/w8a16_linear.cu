@@ -599,6 +599,12 @@ __global__ void __launch_bounds__(kThreadsL, 1)
       if (++kt == iters) kt = 0;
       if (++s == a.stages) s = 0, parity ^= 1u;
     }
+    if constexpr (kPair) {  // the last hand-overs, which come from the other CTA, arrive before this one may leave
+      for (int it = iters; it < iters + a.stages && !dead; ++it) {
+        if (it >= a.stages) dead = !__all_sync(0xffffffffu, mbar_wait_l(smem_addr(&sm.empty[s]), parity));
+        if (++s == a.stages) s = 0, parity ^= 1u;
+      }
+    }
   } else if (warp == 1 && pair_rank == 0) {
     // ---- MMA issue (for the pair): D_half[128 kCtas n x 2 Mp] += W_tile[half] . Xl_tile^T, four K steps of 32 bytes per tile
     const bool elected = elect_sync();
