@@ -186,12 +186,15 @@ class KVCacheEngine:
               for (k, v), (ks, vs) in zip(decode_state.caches, scales)]
     return [cache_manager.KVCacheGenerate(k, v, input_indexes, None, env=env) for k, v in decode_state.caches]
 
-  @staticmethod
-  def _native_step(ds):
-    """Whether the step's bookkeeping can run on the state's tensors as they are: int32 rows and a bf16 / fp32 mask on the GPU."""
-    return (all(t.is_cuda and t.dtype == torch.int32 and t.is_contiguous() for t in (ds.tokens, ds.lens, ds.start, ds.input_pos))
-            and ds.tokens.numel() == ds.lens.numel() == ds.input_pos.numel() and ds.mask.is_cuda and ds.mask.ndim == 2
-            and ds.mask.dtype in (torch.bfloat16, torch.float32) and ds.mask.stride(1) == 1)
+  def _native_step(self, ds):
+    """Whether the step's bookkeeping can run on the state's tensors as they are: int32 rows of one length and a bf16 / fp32
+    mask [slots, cache_len], all on one GPU."""
+    rows = (ds.tokens, ds.lens, ds.start, ds.input_pos)
+    slots = ds.input_pos.numel()
+    return (all(t.is_cuda and t.dtype == torch.int32 and t.is_contiguous() and t.numel() == slots and t.device == ds.mask.device
+                for t in rows)
+            and ds.mask.shape == (slots, self.env.cache_len) and ds.mask.dtype in (torch.bfloat16, torch.float32)
+            and ds.mask.stride(1) == 1)
 
   def generate_impl(self, params: Any, decode_state: DecodeState, sampler=None, page_token_indices=None,
                     n_active_dev=None):
