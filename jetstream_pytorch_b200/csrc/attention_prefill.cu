@@ -237,11 +237,6 @@ __device__ __forceinline__ uint64_t add_f32x2(uint64_t x, uint64_t y) {
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(y));
   return r;
 }
-__device__ __forceinline__ uint64_t fma_f32x2(uint64_t x, uint64_t y, uint64_t z) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(x), "l"(y), "l"(z));
-  return r;
-}
 __device__ __forceinline__ void group_sync(int group) { asm volatile("bar.sync %0, 256;" ::"r"(1 + group) : "memory"); }
 // barrier of the group's 256 threads; whether `pred` holds in all of them
 __device__ __forceinline__ bool group_all(int group, bool pred) {
@@ -693,7 +688,10 @@ __global__ void __launch_bounds__(kThreadsP, 1)
         }
       }
       m_ref = m_new;
-      const float off = m_ref == -INFINITY ? 0.f : m_ref * kLog2e;
+      // The reference maximum is subtracted before the product with log2 e: one fused step x log2 e - (m_ref log2 e) carries the
+      // rounding of the second product, which for finite masks of large magnitude (-1e10, the lowest bf16) exceeds the range
+      // of the exponential.
+      const float off = m_ref == -INFINITY ? 0.f : m_ref;
       const uint64_t l2e = pack_f32(kLog2e, kLog2e), noff = pack_f32(-off, -off);
       uint64_t lsum = pack_f32(0.f, 0.f);
 #pragma unroll
@@ -709,7 +707,7 @@ __global__ void __launch_bounds__(kThreadsP, 1)
             x = pack_f32(__uint_as_float(lg[(32 * q + 2 * e) & (kRound ? 31 : 63)]),
                          __uint_as_float(lg[(32 * q + 2 * e + 1) & (kRound ? 31 : 63)]));
           }
-          unpack_f32(fma_f32x2(x, l2e, noff), f[2 * e], f[2 * e + 1]);
+          unpack_f32(mul_f32x2(add_f32x2(x, noff), l2e), f[2 * e], f[2 * e + 1]);
           f[2 * e] = ex2p(f[2 * e]), f[2 * e + 1] = ex2p(f[2 * e + 1]);
           lsum = add_f32x2(lsum, pack_f32(f[2 * e], f[2 * e + 1]));
         }
