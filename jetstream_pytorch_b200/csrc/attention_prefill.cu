@@ -18,7 +18,11 @@
 //   warp 17         thread 0 issues the MMAs: S_t = Q_t K^T (shared x shared), O_t += P_t V (TMEM x shared)
 //
 // P lies over S in tensor memory (S: 128 fp32 columns; P: 64 columns of bf16 pairs for the leading part and 64 for
-// the rest, so that the probabilities keep 16 bits; two MMAs per step).  S of the next K tile is issued
+// the rest, so that the probabilities keep 17 bits; two MMAs per step).  Measured against fp64 over 24 causal prompts of
+// 24 to 1024 tokens, relative error in the 2-norm and signed: 1.562775e-3 and -2.4e-6, the scalar kernel with fp32
+// probabilities 1.562775e-3 and -2.2e-6 (both parts cut instead of rounded: 1.562789e-3 and -6.8e-6).  With the logits
+// rounded to bf16 1.5635e-3 against 1.5621e-3: the fp32 sums of the tensor core (1.2e-7 of the rms) put a few more logits
+// on the other side of a rounding boundary than those of the scalar kernel (5e-8).  S of the next K tile is issued
 // behind the PV product that reads P: the tensor core takes them in order.
 // The row maximum is raised lazily (when a tile's maximum is more than 2^8 above the reference in exp2 units): O
 // is rescaled in tensor memory only then, and m, l that go out are those of the true maximum.
@@ -717,12 +721,10 @@ __global__ void __launch_bounds__(kThreadsP, 1)
         }
 #pragma unroll
         for (int e = 0; e < 16; ++e) {
-          // p cut after its upper 16 bits, and the remainder cut the same way: 16 bits of p are kept, and byte moves do it
-          // (two conversions per pair and the widening back took half of this phase's time)
-          hi[e] = __byte_perm(__float_as_uint(f[2 * e]), __float_as_uint(f[2 * e + 1]), 0x7632);
-          const float r0 = f[2 * e] - __uint_as_float(__float_as_uint(f[2 * e]) & 0xffff0000u);
-          const float r1 = f[2 * e + 1] - __uint_as_float(__float_as_uint(f[2 * e + 1]) & 0xffff0000u);
-          rest[e] = __byte_perm(__float_as_uint(r0), __float_as_uint(r1), 0x7632);
+          // p rounded to bf16 and the remainder rounded to bf16 again: both to the nearest, so that what is left out (below 2^-17
+          // of p) has no side
+          hi[e] = pack_bf16(f[2 * e], f[2 * e + 1]);
+          rest[e] = pack_bf16(f[2 * e] - lo_f32(hi[e]), f[2 * e + 1] - hi_f32(hi[e]));
         }
         tmem_st16(tl + 32 * half + 16 * q, hi);
         tmem_st16(tl + 64 + 32 * half + 16 * q, rest);
