@@ -81,3 +81,37 @@ def test_probabilities_are_rounded_to_both_sides():
                                kv_strides=k.stride()[:3], n_kv_heads=hkv, seq=t, force_generic=force_generic)
     bias.append(float(((o.double() - want) * want.sign()).sum() / want.abs().sum()))
   assert abs(bias[0] - bias[1]) <= 1.5e-6, bias
+
+
+@pytest.mark.parametrize("hq,hkv,t,s", [(8, 2, 100, 320), (2, 2, 130, 700)])
+@pytest.mark.parametrize("rounded", [True, False])
+@pytest.mark.parametrize("scaled", [False, True])
+def test_values_that_are_not_finite(hq, hkv, t, s, rounded, scaled):
+  """Masked keys may hold anything; an attended infinity or NaN reaches the rows that see it and no others.  Against the
+  scalar kernel: the same rows finite, and within the tolerance where they are."""
+  q, k, v = _inputs(hq, hkv, t, s)
+  q = q.transpose(1, 2).contiguous().transpose(1, 2)  # (strided, as a model hands it over)
+  from jetstream_pytorch_b200 import _lib
+
+  m = torch.full((t, s), float("-inf"), device=DEV).triu(1 + s - t)
+  m[:, :100] = float("-inf")
+  mask = m.to(torch.bfloat16).repeat(hq // hkv, 1)[None, None]
+  v[:, :, :60, 5] = float("nan")  # masked for every row, in a tile that the rows read
+  v[:, :, 60:100] = float("inf")
+  v[:, 0, s - 20, 70] = float("inf")  # seen by the last 20 queries of the first group
+  v[:, 0, s - 10, 3] = float("nan")
+  v[:, hkv - 1, s - 30, 100] = float("-inf")
+  scales = (0.5 + torch.rand((2, 1, 1, s, 1), device=DEV)) if scaled else (None, None)
+  outs = []
+  for force_generic in (0, 1):
+    o, _, _ = ak._flash_decode(q, k, v, k_scale=scales[0], v_scale=scales[1], scale_strides=(s, 1), mask_mode=_lib.MASK_ADD, mask=mask,
+                               mask_strides=(0, s), sm_scale=1 / math.sqrt(128), kv_strides=k.stride()[:3], n_kv_heads=hkv, seq=s,
+                               force_generic=force_generic, logit_rounding=rounded)
+    outs.append(o.float())
+  assert ak.kernel_status(DEV) == 0
+  got, want = outs
+  bad = ~torch.isfinite(want)
+  assert 0 < int(bad.sum()) < want.numel() // 100
+  assert torch.equal(torch.nan_to_num(got[bad], nan=7.0), torch.nan_to_num(want[bad], nan=7.0))
+  assert bool(torch.isfinite(got[~bad]).all())
+  _check(torch.where(bad, torch.zeros_like(got), got), torch.where(bad, torch.zeros_like(want), want).double())
