@@ -599,6 +599,15 @@ int jpt_w8a16_linear_tp(const void* x, const void* w, const void* w_scale, void*
                         int M, int N, int K, void* workspace, size_t workspace_bytes,
                         const jpt_tp_sum* tp, void* stream);
 int jpt_w8a16_tp_status(const jpt_tp_sum* tp, void* stream);
+/*
+ * How the GEMM of up to 128 rows deals out its channels and K steps: plan =
+ * {pairs of CTAs, K splits, channels per CTA, tiles, 128-byte steps per stage}.
+ * `slots` [2][9] (clusters of single CTAs and of pairs, by K splits, that a GPU
+ * holds at once) or NULL for the current device.  The row-parallel form ignores
+ * them: the ranks exchange their sums by tile and split, so all of them have to
+ * come to the same plan for the same shape.
+ */
+int jpt_w8a16_plan(int M, int N, int K, int row_parallel, const int* slots, int* plan);
 
 /* ------------------------------------------------------------------------- */
 /* The engine's bookkeeping                                                  */

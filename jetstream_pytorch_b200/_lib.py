@@ -114,6 +114,7 @@ _SIGNATURES = {
     "jpt_w8a16_split_levels": (c_int, [c_void_p, c_int, c_int, c_void_p, c_size_t, c_void_p]),
     "jpt_w8a16_linear_from_levels": (c_int, [c_void_p, c_size_t, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),
     "jpt_w8a16_tp_buffer_bytes": (c_size_t, [c_int, c_int]),
+    "jpt_w8a16_plan": (c_int, [c_int] * 4 + [c_void_p, c_void_p]),
     "jpt_w8a16_linear_tp": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_size_t,
                                     ctypes.POINTER(TpSumStruct), c_void_p]),
     "jpt_w8a16_tp_status": (c_int, [ctypes.POINTER(TpSumStruct), c_void_p]),

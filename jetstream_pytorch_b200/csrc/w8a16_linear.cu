@@ -1137,15 +1137,23 @@ struct GemmPlan {
   int pair, split, tile, halves, tiles, kb;
 };
 constexpr int kMaxCluster = 8;  // CTAs of a cluster: the portable limit
-int cluster_slots(bool pair, int split);
-GemmPlan plan_gemm(int M, int N, int K, bool tp) {
+// Clusters of single CTAs [0] and of pairs [1] by their number of splits that fit the GPU at once.
+struct ClusterSlots {
+  int n[2][kMaxCluster + 1];
+};
+// The row-parallel form (`tp`) exchanges its sums by tile and split, so every rank has to come to the same plan: it is made for
+// these counts (of a B200 with 148 SMs), whatever the rank's own GPU holds.  How many clusters fit differs from GPU to GPU with
+// the SMs that each of them has switched off; a GPU that holds fewer runs the same plan in one more wave.
+constexpr ClusterSlots kTpSlots = {{{0, 148, 74, 48, 36, 28, 24, 20, 16}, {0, 74, 36, 24, 16, 0, 0, 0, 0}}};
+GemmPlan plan_gemm(int M, int N, int K, bool tp, const ClusterSlots& own_slots) {
+  const ClusterSlots& all_slots = tp ? kTpSlots : own_slots;
   const int k_tiles = K / kTileK, Mp = (M + 15) / 16 * 16;
   GemmPlan best{};
   float best_cost = 0.f;
   for (int ctas = 1; ctas <= 2; ++ctas) {
     const int x_rows = 2 * Mp / ctas;
     for (int c = 1; c * ctas <= kMaxCluster && c <= k_tiles; ++c) {
-      const int slots = cluster_slots(ctas == 2, c);
+      const int slots = all_slots.n[ctas - 1][c];
       const int waves = (N + ctas * kTileN * slots - 1) / (ctas * kTileN * slots);
       int tile = (N + ctas * slots * waves - 1) / (ctas * slots * waves);
       tile = tile <= 128 ? std::max(32, (tile + 7) / 8 * 8) : (tile + 15) / 16 * 16;
@@ -1211,7 +1219,7 @@ LevelsView levels_view(void* workspace, int M, int K) {
   return v;
 }
 
-// Clusters of `split` CTAs or pairs that the current device holds at once; the kernels' attributes are set on the way.
+// Clusters that the current device holds at once; the kernels' attributes are set on the way.
 constexpr size_t kGemmSmem = kRingBytes + kTailBytes;
 using GemmKernel = void (*)(const LinearMaps, const GemmArgs, const TpArgs);
 GemmKernel gemm_kernel(bool pair, int halves) {
@@ -1234,33 +1242,42 @@ cudaLaunchConfig_t gemm_config(dim3 grid, size_t smem, cudaStream_t st, cudaLaun
   cfg.numAttrs = 1;
   return cfg;
 }
-int cluster_slots(bool pair, int split) {
+// (filled on first use per device; a query that failed is made again at the next call, and the launch reports what is wrong)
+const ClusterSlots& device_slots() {
   static std::mutex mu;
-  static int known[64][2][kMaxCluster + 1];
+  static ClusterSlots known[64];
+  static thread_local ClusterSlots guess;
   int dev = 0;
   cudaGetDevice(&dev);
   std::lock_guard<std::mutex> lock(mu);
-  int& n = known[dev & 63][pair][split];
-  if (n == 0) {
-    cudaLaunchAttribute attr[2];
-    const cudaLaunchConfig_t cfg = gemm_config(dim3(pair ? 2 : 1, split), kGemmSmem, nullptr, attr, pair, split);
-    bool ok = true;
-    for (int halves = 1; halves <= 2; ++halves)
-      ok = ok && cudaFuncSetAttribute(gemm_kernel(pair, halves), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem) == cudaSuccess;
-    if (!ok || cudaOccupancyMaxActiveClusters(&n, gemm_kernel(pair, 2), &cfg) != cudaSuccess || n <= 0) {
-      cudaGetLastError();
-      n = 0;
-      return std::max(1, sm_count_l() / ((pair ? 2 : 1) * split));  // (asked again at the next call; the launch reports what is wrong)
+  ClusterSlots& slots = known[dev & 63];
+  bool all = true;
+  for (int pair = 0; pair < 2; ++pair) {
+    for (int split = 1; split * (pair + 1) <= kMaxCluster; ++split) {
+      int& n = slots.n[pair][split];
+      if (n == 0) {
+        cudaLaunchAttribute attr[2];
+        const cudaLaunchConfig_t cfg = gemm_config(dim3(pair ? 2 : 1, split), kGemmSmem, nullptr, attr, pair, split);
+        bool ok = true;
+        for (int halves = 1; halves <= 2; ++halves)
+          ok = ok && cudaFuncSetAttribute(gemm_kernel(pair, halves), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem) == cudaSuccess;
+        if (!ok || cudaOccupancyMaxActiveClusters(&n, gemm_kernel(pair, 2), &cfg) != cudaSuccess || n <= 0) {
+          cudaGetLastError();
+          n = 0;
+          all = false;
+        }
+      }
+      guess.n[pair][split] = n > 0 ? n : std::max(1, sm_count_l() / ((pair ? 2 : 1) * split));
     }
   }
-  return n;
+  return all ? slots : guess;
 }
 
 // The GEMM on levels that a launch before this one in the stream wrote.  The launch may start while that one
 // drains (it requests its first weight tiles at once) and waits for its results on the device.
 int launch_gemm(const LevelsView& lv, const void* w, const void* w_scale, void* y, int M, int N, int K, cudaStream_t st,
                 const TpArgs* tp_in = nullptr) {
-  const GemmPlan plan = plan_gemm(M, N, K, tp_in != nullptr);
+  const GemmPlan plan = plan_gemm(M, N, K, tp_in != nullptr, device_slots());
   const int x_rows = plan.pair ? lv.Mp : 2 * lv.Mp;  // rows of levels that a CTA loads
   TpArgs tp;
   memset(&tp, 0, sizeof(tp));
@@ -1465,6 +1482,15 @@ extern "C" int jpt_silu_mul(const void* a, const void* b, void* h, int M, int K,
   const LevelsView lv = levels_view(levels_workspace, M, K);
   return launch_rows("silu_mul_levels_kernel", silu_mul_levels_kernel, lv.Mp, row_parts(lv.Mp, K), st, ap, bp,
                      static_cast<__nv_bfloat16*>(h), lv.lev, lv.xs, lv.status, M, lv.Mp, K);
+}
+
+extern "C" int jpt_w8a16_plan(int M, int N, int K, int row_parallel, const int* slots, int* plan) {
+  JPT_REQUIRE(M >= 1 && M <= kMaxM && N >= 1 && K >= kTileK && K % kTileK == 0 && plan, JPT_EINVAL, "w8a16_plan: bad arguments");
+  ClusterSlots given;
+  if (slots) memcpy(&given, slots, sizeof(given));
+  const GemmPlan p = plan_gemm(M, N, K, row_parallel != 0, slots ? given : device_slots());
+  plan[0] = p.pair, plan[1] = p.split, plan[2] = p.tile, plan[3] = p.tiles, plan[4] = p.kb;
+  return 0;
 }
 
 extern "C" size_t jpt_w8a16_tp_buffer_bytes(int N, int world) {
