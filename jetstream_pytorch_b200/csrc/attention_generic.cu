@@ -280,10 +280,27 @@ static int resolve_splits(const jpt_attn_params& p, int R) {
   return auto_splits_generic(p, R);
 }
 
-// The prefill kernel on contiguous queries (its strided form has an entry point of its own).
+// Whether the prefill kernel takes a call that it can take.  A few query rows of few KV heads over many keys are better off in the
+// scalar kernel: it splits the keys over the SMs, while the prefill kernel has one CTA walk them for every two row tiles.  Estimates
+// in us, within 15 % of the times measured for 22 shapes: 2.5 per K/V tile of 128 keys (both row tiles), in waves of one CTA per SM;
+// 1.8 per key of a warp, or 1.35 ns per key and four rows where the SMs are full.  Measured, prefill / scalar: 40 rows of one KV head
+// 16 / 58 over 512 keys, 167 / 134 over 8192; 24 rows 26 / 60 over 1024 keys, 86 / 68 over 4096, 326 / 160 over 16384; 32 rows of
+// eight KV heads over 8192 keys 167 / 705.
+static bool prefill_taken(const jpt_attn_params& p, int64_t q_b, int64_t q_h, int64_t q_t) {
+  if (p.force_generic != 0 || !attention_prefill_eligible(p, q_b, q_h, q_t)) return false;
+  if (p.S <= 128) return true;  // (one tile)
+  const int rep = p.Hq / p.Hkv, R = rep * p.Tq;
+  const double heads = (double)p.B * p.Hkv, four_rows = heads * ((R + kRowTile - 1) / kRowTile);
+  const double items = heads * (((p.Tq + 127) / 128 * rep + 1) / 2);
+  const double prefill = 6.0 + 2.5 * ((p.S + 127) / 128) * ceil(items / 148.0);
+  const int splits = auto_splits_generic(p, R);
+  const double scalar = fmax(1.8 * ((p.S + splits - 1) / splits / 4), 1.35e-3 * four_rows * p.S);
+  return prefill <= scalar;
+}
+// (contiguous queries; the strided form has an entry point of its own)
 static bool prefill_eligible(const jpt_attn_params& p) {
   const int64_t q_h = (int64_t)p.Tq * p.D;
-  return p.force_generic == 0 && attention_prefill_eligible(p, q_h * p.Hq, q_h, p.D);
+  return prefill_taken(p, q_h * p.Hq, q_h, p.D);
 }
 
 static int validate(const jpt_attn_params& p) {
@@ -424,7 +441,7 @@ extern "C" int jpt_flash_decode(const jpt_attn_params* pp, void* stream) {
 }
 
 extern "C" int jpt_flash_attend_strided_q_ok(const jpt_attn_params* p, int64_t q_b, int64_t q_h, int64_t q_t) {
-  return p && validate(*p) == 0 && p->force_generic == 0 && !attention_mma_eligible(*p) && attention_prefill_eligible(*p, q_b, q_h, q_t);
+  return p && validate(*p) == 0 && !attention_mma_eligible(*p) && prefill_taken(*p, q_b, q_h, q_t);
 }
 
 extern "C" int jpt_flash_attend_strided_q(const jpt_attn_params* pp, int64_t q_b, int64_t q_h, int64_t q_t, void* stream) {
