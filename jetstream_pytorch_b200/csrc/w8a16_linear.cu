@@ -1142,9 +1142,9 @@ struct ClusterSlots {
   int n[2][kMaxCluster + 1];
 };
 // The row-parallel form (`tp`) exchanges its sums by tile and split, so every rank has to come to the same plan: it is made for
-// these counts (of a B200 with 148 SMs), whatever the rank's own GPU holds.  How many clusters fit differs from GPU to GPU with
+// these counts (what the driver said of one B200 with 148 SMs), whatever the rank's own GPU holds.  How many clusters fit differs from GPU to GPU with
 // the SMs that each of them has switched off; a GPU that holds fewer runs the same plan in one more wave.
-constexpr ClusterSlots kTpSlots = {{{0, 148, 74, 48, 36, 28, 24, 20, 16}, {0, 74, 36, 24, 16, 0, 0, 0, 0}}};
+constexpr ClusterSlots kTpSlots = {{{0, 148, 74, 45, 33, 26, 22, 15, 15}, {0, 74, 33, 22, 15, 0, 0, 0, 0}}};
 GemmPlan plan_gemm(int M, int N, int K, bool tp, const ClusterSlots& own_slots) {
   const ClusterSlots& all_slots = tp ? kTpSlots : own_slots;
   const int k_tiles = K / kTileK, Mp = (M + 15) / 16 * 16;

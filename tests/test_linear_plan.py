@@ -5,8 +5,8 @@ import ctypes
 
 import pytest
 
-# clusters that a GPU holds at once, [single CTAs, pairs] by K splits: with its SMs in even groups, and with one group short
-EVEN = [[0, 148, 74, 48, 36, 28, 24, 20, 16], [0, 74, 36, 24, 16, 0, 0, 0, 0]]
+# clusters that a GPU holds at once, [single CTAs, pairs] by K splits: of one B200, and with a group of SMs short
+EVEN = [[0, 148, 74, 45, 33, 26, 22, 15, 15], [0, 74, 33, 22, 15, 0, 0, 0, 0]]
 SHORT = [[0, 132, 64, 42, 30, 24, 20, 16, 12], [0, 60, 28, 16, 10, 0, 0, 0, 0]]
 
 
