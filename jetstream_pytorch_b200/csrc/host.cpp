@@ -338,6 +338,28 @@ void head_check(const Tensor& q, const Tensor& k) {
   if (k.dim() != 4 && k.dim() != 5) fail(PyExc_ValueError, "caches are [B,H,S,D] or [NL,B,H,S,D]");
 }
 
+// What the kernels of a call over a whole cache take on trust: as many sequences and dims as the queries have, and a scale per token.
+void cache_check(const Tensor& q, const Tensor& k) {
+  head_check(q, k);
+  if (k.size(-1) != q.size(-1) || k.size(-4) != q.size(0)) fail(PyExc_AssertionError, "queries and cache differ in batch or head_dim");
+}
+void scale_check(const Call& c) {
+  if (!c.ks.defined()) return;
+  const int64_t o = c.sc_off || c.ks.dim() == 5 || (c.ks.dim() == 4 && c.ks.size(3) != 1) ? 1 : 0;
+  if (c.ks.size(o) != c.q.size(0) || c.ks.size(o + 2) != c.seq) fail(PyExc_AssertionError, "scales do not match the cache");
+}
+// ... and of a step's token: one per sequence and KV head, on the queries' GPU.
+void token_check(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& xk, const Tensor& xv) {
+  cache_check(q, k);
+  if (v.sizes() != k.sizes()) fail(PyExc_ValueError, "K and V caches differ in shape");
+  if (q.size(2) != 1) fail(PyExc_ValueError, "a step has one query token, got %lld", (long long)q.size(2));
+  const int64_t want[4] = {q.size(0), k.size(-3), 1, q.size(3)};
+  for (const Tensor* x : {&xk, &xv})
+    if (x->sizes() != at::IntArrayRef(want, 4) || x->device() != q.device())
+      fail(PyExc_ValueError, "the step's token must be [%lld, %lld, 1, %lld] on %s", (long long)want[0], (long long)want[1],
+           (long long)want[3], q.device().str().c_str());
+}
+
 // attend(q, k, v, k_scale, v_scale, page_table, start, end, mask, mask_mode, kv strides (b, h, s), scale strides (b, s), mask
 // strides (b, r), hkv, seq, page_size, sm_scale, want_ml, rounding, num_splits, force_generic, static_scratch, out)
 PyObject* attend(Args a, Py_ssize_t n) {
@@ -370,16 +392,12 @@ PyObject* ragged(Args a, Py_ssize_t n) {
   Call c;
   c.q = tensor(a[0]);
   const Tensor &k = tensor(a[1]), &v = tensor(a[2]);
-  head_check(c.q, k);
+  cache_check(c.q, k);
   const int64_t layer = integer(a[3]);
   const bool ring = truth(a[9]);
-  if (k.size(-1) != c.q.size(-1) || k.size(-4) != c.q.size(0)) fail(PyExc_AssertionError, "queries and cache differ in batch or head_dim");
   take_kv(c, k, v, layer);
   take_scales(c, maybe(a[6]), maybe(a[7]), layer);
-  if (c.ks.defined()) {
-    const int64_t o = c.sc_off || c.ks.dim() == 5 || (c.ks.dim() == 4 && c.ks.size(3) != 1) ? 1 : 0;
-    if (c.ks.size(o) != c.q.size(0) || c.ks.size(o + 2) != c.seq) fail(PyExc_AssertionError, "scales do not match the cache");
-  }
+  scale_check(c);
   if (ring) c.start = tensor(a[4]);
   c.end = tensor(a[5]);
   c.mask_mode = ring ? JPT_MASK_RING : JPT_MASK_LENGTH;
@@ -498,6 +516,10 @@ Stash stash(PyObject* outs, PyObject* layer, int64_t b, int64_t h, int64_t d, Sc
     fail(PyExc_ValueError, "scale buffers of dtype %s cannot take the scales of %s inputs", c10::toString(s.ks.scalar_type()), c10::toString(type));
   if (s.kq.scalar_type() != ScalarType::Char || s.vq.scalar_type() != ScalarType::Char)
     fail(PyExc_ValueError, "the buffers for the quantised new token must be int8");
+  const int64_t layers = s.kq.dim() == 5 ? s.kq.size(0) : 1;
+  for (const Tensor* t : {&s.kq, &s.vq, &s.ks, &s.vs})
+    if (t->numel() != layers * b * (t == &s.kq || t == &s.vq ? h * d : 1) || !t->is_contiguous() || t->device() != dev)
+      fail(PyExc_ValueError, "the buffers for the quantised new token must be contiguous, of %lld sequences and %lld heads", (long long)b, (long long)h);
   if (s.kq.dim() == 5) {
     const int64_t l = layer_index(integer(layer), s.kq.size(0));
     s.q_off = l * s.kq.stride(0), s.s_off = l * s.ks.stride(0);
@@ -550,10 +572,11 @@ PyObject* update_attend(Args a, Py_ssize_t n) {
   const c10::Device dev = c.q.device();
   OnDevice on(dev);
   const Tensor &k = tensor(PyTuple_GET_ITEM(a[3], 0)), &v = tensor(PyTuple_GET_ITEM(a[3], 1));
-  head_check(c.q, k);
+  token_check(c.q, k, v, xk, xv);
   const int64_t layer = integer(a[4]);
   take_kv(c, k, v, layer);
   take_scales(c, maybe(PyTuple_GET_ITEM(a[3], 2)), maybe(PyTuple_GET_ITEM(a[3], 3)), layer);
+  scale_check(c);
   const bool ring = truth(a[7]);
   if (ring) c.start = tensor(a[5]);
   c.end = tensor(a[6]);
@@ -606,7 +629,7 @@ PyObject* attend_lazy(Args a, Py_ssize_t n) {
   c.q = dense(tensor(a[0]));
   const Tensor xk = dense(tensor(a[1])), xv = dense(tensor(a[2]));
   const Tensor &k = tensor(a[3]), &v = tensor(a[4]);
-  head_check(c.q, k);
+  token_check(c.q, k, v, xk, xv);
   const c10::Device dev = c.q.device();
   OnDevice on(dev);
   const int64_t layer = integer(a[5]);
@@ -616,9 +639,14 @@ PyObject* attend_lazy(Args a, Py_ssize_t n) {
   const int64_t b = c.q.size(0), hq = c.q.size(1), d = c.q.size(3);
   c.sm_scale = 1.0 / std::sqrt((double)d);
   const Tensor *kk = maybe(a[7]), *kv = maybe(a[8]);
+  if ((kk == nullptr) != (kv == nullptr)) fail(PyExc_ValueError, "attend_lazy: kept K and V come together");
   if (xk.scalar_type() != c.q.scalar_type() || xv.scalar_type() != c.q.scalar_type() ||
-      (kk && (kk->scalar_type() != xk.scalar_type() || !kk->is_contiguous() || !kv->is_contiguous())))
+      (kk && (kk->scalar_type() != xk.scalar_type() || kv->scalar_type() != xk.scalar_type())))
     fail(PyExc_ValueError, "attend_lazy: queries, token and kept rows share a dtype");
+  for (const Tensor* t : {kk, kv})
+    if (kk && (t->dim() != 5 || t->numel() != t->size(0) * xk.numel() || !t->is_contiguous() || t->device() != dev))
+      fail(PyExc_ValueError, "attend_lazy: the kept rows must be contiguous tensors [layers, %lld, %lld, 1, %lld]", (long long)b,
+           (long long)xk.size(1), (long long)d);
   const int64_t keep = kk ? layer_index(layer, kk->size(0)) * kk->stride(0) : 0;
   run_attention(c, {b, hq, 1, d}, {b, hq});
   Tensor out = empty({b, hq, 1, d}, ScalarType::Float, dev);
@@ -636,15 +664,19 @@ PyObject* attend_lazy_int8(Args a, Py_ssize_t n) {
   Call c;
   c.q = dense(tensor(a[0]));
   const Tensor &k = tensor(PyTuple_GET_ITEM(a[1], 0)), &v = tensor(PyTuple_GET_ITEM(a[1], 1));
-  head_check(c.q, k);
   const c10::Device dev = c.q.device();
   OnDevice on(dev);
+  const Tensor kq = dense(tensor(a[4])), vq = dense(tensor(a[5])), ks = dense(tensor(a[6])), vs = dense(tensor(a[7]));
+  token_check(c.q, k, v, kq, vq);
+  for (const Tensor* t : {&ks, &vs})
+    if (t->numel() != c.q.size(0) || t->device() != dev || t->scalar_type() != ks.scalar_type())
+      fail(PyExc_ValueError, "attend_lazy_int8: the token has a scale per sequence");
   const int64_t layer = integer(a[2]);
   take_kv(c, k, v, layer);
   take_scales(c, maybe(PyTuple_GET_ITEM(a[1], 2)), maybe(PyTuple_GET_ITEM(a[1], 3)), layer);
+  scale_check(c);
   c.end = tensor(a[3]);
   c.mask_mode = JPT_MASK_LENGTH;
-  const Tensor kq = dense(tensor(a[4])), vq = dense(tensor(a[5])), ks = dense(tensor(a[6])), vs = dense(tensor(a[7]));
   const int64_t b = c.q.size(0), hq = c.q.size(1), d = c.q.size(3);
   c.sm_scale = 1.0 / std::sqrt((double)d);
   run_attention(c, {b, hq, 1, d}, {b, hq});

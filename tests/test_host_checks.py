@@ -1,0 +1,66 @@
+"""CPU: the checks of the native host side.  Shapes are looked at before devices, so a CPU tensor of the right
+shape is refused for its device and one of the wrong shape for its shape."""
+
+import pytest
+import torch
+
+BF = torch.bfloat16
+B, HQ, H, S, D = 3, 8, 2, 16, 128
+
+
+def _native():
+  from jetstream_pytorch_b200 import _lib
+
+  return _lib.native
+
+
+def _step(dtype=BF):
+  return (torch.zeros(B, HQ, 1, D, dtype=BF), torch.zeros(B, H, 1, D, dtype=dtype), torch.zeros(B, H, 1, D, dtype=dtype))
+
+
+def _calls():
+  """name -> (call(q, xk, xv, batch, heads, dim, scale tokens, kept batch)), each with the shapes of the cache as given"""
+
+  def int8_cache(b, h, d, s):
+    return tuple(torch.zeros(b, h, S, d, dtype=torch.int8) for _ in range(2)) + tuple(torch.ones(b, 1, s, 1, dtype=BF) for _ in range(2))
+
+  end = torch.zeros(B, dtype=torch.int32)
+
+  def fused(q, xk, xv, b=B, h=H, d=D, s=S, kept=B):
+    outs = tuple(torch.zeros(2, kept, H, 1, D, dtype=torch.int8) for _ in range(2)) + tuple(torch.zeros(2, kept, 1, 1, 1, dtype=BF) for _ in range(2))
+    _native().update_attend(q, xk, xv, int8_cache(b, h, d, s), 0, None, end, False, 0, False, outs, True, None, None)
+
+  def lazy(q, xk, xv, b=B, h=H, d=D, s=S, kept=B):
+    keep = [torch.zeros(2, kept, H, 1, D, dtype=BF) for _ in range(2)]
+    k, v = (torch.zeros(2, b, h, S, d, dtype=BF) for _ in range(2))
+    _native().attend_lazy(q, xk, xv, k, v, 1, end, *keep)
+
+  def lazy_int8(q, xk, xv, b=B, h=H, d=D, s=S, kept=B):
+    scale = torch.ones(kept, dtype=BF)
+    _native().attend_lazy_int8(q, int8_cache(b, h, d, s), 0, end, xk.to(torch.int8), xv.to(torch.int8), scale, scale)
+
+  return {"update_attend": fused, "attend_lazy": lazy, "attend_lazy_int8": lazy_int8}
+
+
+@pytest.mark.parametrize("name", ["update_attend", "attend_lazy", "attend_lazy_int8"])
+def test_step_shapes(name):
+  call = _calls()[name]
+  q, xk, xv = _step()
+  with pytest.raises(ValueError, match="CUDA tensors only"):
+    call(q, xk, xv)  # all shapes agree
+  for wrong in (dict(b=B - 1), dict(d=64)):
+    with pytest.raises(AssertionError, match="batch or head_dim"):
+      call(q, xk, xv, **wrong)
+  with pytest.raises(ValueError, match="token must be"):
+    call(q, xk, xv, h=H * 2)  # more KV heads than the token has
+  with pytest.raises(ValueError, match="token must be"):
+    call(q, xk[:1], xv[:1])
+  with pytest.raises(ValueError, match="token must be"):
+    call(q, xk, xv[:, :1])
+  with pytest.raises(ValueError, match="one query token"):
+    call(torch.zeros(B, HQ, 2, D, dtype=BF), xk, xv)
+  with pytest.raises(ValueError):
+    call(q, xk, xv, kept=B - 1)
+  if name != "attend_lazy":
+    with pytest.raises(AssertionError, match="scales"):
+      call(q, xk, xv, s=S - 1)
