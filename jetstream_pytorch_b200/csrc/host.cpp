@@ -929,6 +929,10 @@ PyObject* engine_begin(Args a, Py_ssize_t n) {
   const c10::Device dev = start.device();
   OnDevice on(dev);
   const int64_t b = start.size(0), s = integer(a[2]), block = integer(a[3]);
+  if (start.numel() != b || pos.numel() != b || pos.device() != dev) fail(PyExc_ValueError, "engine_begin: start and input_pos are one row per slot");
+  if (block < 1) fail(PyExc_ValueError, "engine_begin: blocks of %lld tokens", (long long)block);
+  if (a[4] != Py_None && (tensor(a[4]).dim() != 2 || tensor(a[4]).size(0) != b || tensor(a[4]).size(1) != s || tensor(a[4]).device() != dev))
+    fail(PyExc_ValueError, "engine_begin: the mask is [%lld, %lld]", (long long)b, (long long)s);
   Tensor nb = empty({b, s / block}, ScalarType::Int, dev), ni = empty({b, s / block}, ScalarType::Int, dev);
   const MaskArg m = mask_arg(a[4]);
   check(jpt_engine_begin(i32(start, "start"), i32(pos, "input_pos"), (int)b, (int)s, (int)block, i32(nb, ""), i32(ni, ""), m.p, m.dtype,

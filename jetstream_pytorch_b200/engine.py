@@ -82,7 +82,8 @@ def precompute_ragged_block_indices(env, start, input_pos):
   outside [start, end) are skipped.  The CUDA kernels skip by their loop bounds
   and ignore these tables; they are produced for callers that pass them on."""
   s, bk = env.cache_len, env.block_size
-  if start.is_cuda and start.dtype == input_pos.dtype == torch.int32 and start.is_contiguous() and input_pos.is_contiguous():
+  if (start.is_cuda and start.dtype == input_pos.dtype == torch.int32 and start.is_contiguous() and input_pos.is_contiguous()
+      and start.numel() == start.shape[0] == input_pos.numel() and start.device == input_pos.device):
     return _lib.native.engine_begin(start, input_pos, s, bk, None, False, 0)
   b_count = start.shape[0]
   end = ((start + input_pos) % s).reshape(b_count, 1)

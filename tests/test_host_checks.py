@@ -64,3 +64,44 @@ def test_step_shapes(name):
   if name != "attend_lazy":
     with pytest.raises(AssertionError, match="scales"):
       call(q, xk, xv, s=S - 1)
+
+
+def test_block_tables_need_one_row_per_slot():
+  i32 = dict(dtype=torch.int32)
+  begin = _native().engine_begin
+  with pytest.raises(ValueError, match="one row per slot"):
+    begin(torch.zeros(4, **i32), torch.zeros(1, **i32), 64, 16, None, False, 0)
+  with pytest.raises(ValueError, match="one row per slot"):
+    begin(torch.zeros(2, 2, **i32), torch.zeros(4, **i32), 64, 16, None, False, 0)
+  with pytest.raises(ValueError, match="the mask is"):
+    begin(torch.zeros(4, **i32), torch.zeros(4, **i32), 64, 16, torch.zeros(3, 64), False, 0)
+
+
+def test_block_tables_of_a_broadcast_position_go_through_tensor_operations(monkeypatch):
+  """One `input_pos` for all slots: the tensor operations broadcast it, the launch reads one per slot."""
+  from types import SimpleNamespace
+
+  from jetstream_pytorch_b200 import _lib, engine
+
+  class OnGpu:  # (a CPU tensor that says that it lies on a GPU)
+    def __init__(self, t):
+      self.t = t
+
+    is_cuda = True
+
+    def __getattr__(self, name):
+      return getattr(self.t, name)
+
+    def __add__(self, other):
+      return self.t + other.t
+
+  taken = []
+  monkeypatch.setattr(_lib, "native", SimpleNamespace(engine_begin=lambda *a: taken.append(a)))
+  env = SimpleNamespace(cache_len=64, block_size=16)
+  start, pos = torch.tensor([0, 5, 60], dtype=torch.int32), torch.tensor([7], dtype=torch.int32)
+  got = engine.precompute_ragged_block_indices(env, OnGpu(start), OnGpu(pos))
+  want = engine.precompute_ragged_block_indices(env, start, pos.expand(3).contiguous())
+  assert not taken
+  assert all(torch.equal(x, y) for x, y in zip(got, want))
+  engine.precompute_ragged_block_indices(env, OnGpu(start), OnGpu(pos.expand(3).contiguous()))
+  assert len(taken) == 1
