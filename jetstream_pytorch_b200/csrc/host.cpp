@@ -947,8 +947,10 @@ PyObject* engine_end(Args a, Py_ssize_t n) {
   const c10::Device dev = lg.device();
   OnDevice on(dev);
   const int64_t b = lg.size(0);
-  if (lg.dim() != 3 || lg.stride(2) != 1 || tokens.numel() != b || lens.numel() != b || pos.numel() != b)
+  if (lg.dim() != 3 || lg.size(1) < 1 || lg.stride(2) != 1 || tokens.numel() != b || lens.numel() != b || pos.numel() != b)
     fail(PyExc_ValueError, "engine_end: logits are [B,T,V] with contiguous rows");
+  if (tokens.device() != dev || lens.device() != dev || pos.device() != dev || (a[5] != Py_None && tensor(a[5]).device() != dev))
+    fail(PyExc_ValueError, "engine_end: logits on %s, the state elsewhere", dev.str().c_str());
   Tensor next = empty({b, 1}, ScalarType::Int, dev), lo = empty(lens.sizes(), ScalarType::Int, dev),
          po = empty(pos.sizes(), ScalarType::Int, dev), data = empty({b, 3}, ScalarType::Int, dev);
   const MaskArg m = mask_arg(a[5]);

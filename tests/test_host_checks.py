@@ -105,3 +105,11 @@ def test_block_tables_of_a_broadcast_position_go_through_tensor_operations(monke
   assert all(torch.equal(x, y) for x, y in zip(got, want))
   engine.precompute_ragged_block_indices(env, OnGpu(start), OnGpu(pos.expand(3).contiguous()))
   assert len(taken) == 1
+
+
+def test_end_of_a_step_needs_a_token_of_logits():
+  i32 = [torch.zeros(2, dtype=torch.int32) for _ in range(3)]
+  with pytest.raises(ValueError, match="logits are"):  # (the row before the first one would be read)
+    _native().engine_end(torch.zeros(2, 0, 5), *i32, 64, None, False, 0)
+  with pytest.raises(ValueError, match="elsewhere"):
+    _native().engine_end(torch.zeros(2, 1, 5), *(t.to("meta") for t in i32), 64, None, False, 0)
