@@ -536,6 +536,16 @@ int jpt_w8a16_gate(const void* x, const void* w1, const void* w1_scale, const vo
                    int N, int K, void* workspace, size_t workspace_bytes, void* stream);
 
 /*
+ * Both with the status word at `status` instead of the workspace's start (NULL: as
+ * above), so that a workspace as large as a prompt can be given back, in stream
+ * order, as soon as the call has returned, and the status read later.
+ */
+int jpt_w8a16_linear_reporting(const void* x, const void* w, const void* w_scale, void* y, int M, int N, int K, void* workspace,
+                               size_t workspace_bytes, int32_t* status, void* stream);
+int jpt_w8a16_gate_reporting(const void* x, const void* w1, const void* w1_scale, const void* w3, const void* w3_scale, void* h, int M,
+                             int N, int K, void* workspace, size_t workspace_bytes, int32_t* status, void* stream);
+
+/*
  * The same layer in two steps, for activations that feed several layers (wq /
  * wk / wv after the attention norm, w1 / w3 after the ffn norm): the level
  * split once into a workspace (M <= 128 rows), then one GEMM per layer on the

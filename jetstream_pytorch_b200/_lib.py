@@ -111,6 +111,8 @@ _SIGNATURES = {
     "jpt_w8a16_linear": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_size_t, c_void_p]),
     "jpt_w8a16_gate_workspace_bytes": (c_size_t, [c_int, c_int, c_int]),
     "jpt_w8a16_gate": (c_int, [c_void_p] * 6 + [c_int] * 3 + [c_void_p, c_size_t, c_void_p]),
+    "jpt_w8a16_linear_reporting": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_size_t, c_void_p, c_void_p]),
+    "jpt_w8a16_gate_reporting": (c_int, [c_void_p] * 6 + [c_int] * 3 + [c_void_p, c_size_t, c_void_p, c_void_p]),
     "jpt_w8a16_split_levels": (c_int, [c_void_p, c_int, c_int, c_void_p, c_size_t, c_void_p]),
     "jpt_w8a16_linear_from_levels": (c_int, [c_void_p, c_size_t, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),
     "jpt_w8a16_tp_buffer_bytes": (c_size_t, [c_int, c_int]),

@@ -987,7 +987,13 @@ std::vector<int64_t> with_last(const Tensor& x, int64_t last) {
   return s;
 }
 
-// linear(x [...,K], weight [N,K], scale [N], workspace or None) -> y [...,N], workspace
+// What a layer keeps between its calls is the workspace of up to kKeptRows rows, whose first word its kernels report to.  The scratch of a
+// longer prompt (2 M K bytes) goes back to the allocator behind the call, in stream order: kept by every layer it was
+// several GB of a model.
+constexpr int64_t kKeptRows = 128;
+constexpr size_t kStatusBytes = 256;
+
+// linear(x [...,K], weight [N,K], scale [N], workspace or None) -> y [...,N], workspace to keep
 PyObject* linear(Args a, Py_ssize_t n) {
   expect(n, 4, "linear");
   const Tensor x = dense(tensor(a[0]));
@@ -995,26 +1001,30 @@ PyObject* linear(Args a, Py_ssize_t n) {
   const c10::Device dev = x.device();
   OnDevice on(dev);
   const int64_t out = w.size(0), k = w.size(1), m = x.numel() / k;
-  Tensor ws = scratch(maybe(a[3]), jpt_w8a16_linear_workspace_bytes((int)m, (int)out, (int)k), dev);
+  const size_t need = jpt_w8a16_linear_workspace_bytes((int)m, (int)out, (int)k);
+  Tensor kept = scratch(maybe(a[3]), m > kKeptRows ? kStatusBytes : need, dev);
+  Tensor ws = m > kKeptRows ? scratch(nullptr, need, dev) : kept;
   Tensor y = empty(with_last(x, out), ScalarType::BFloat16, dev);
-  check(jpt_w8a16_linear(ptr(x), ptr(w), ptr(sc), ptr(y), (int)m, (int)out, (int)k, ptr(ws), (size_t)ws.numel(), stream_of(dev)));
-  return tuple(y, ws);
+  check(jpt_w8a16_linear_reporting(ptr(x), ptr(w), ptr(sc), ptr(y), (int)m, (int)out, (int)k, ptr(ws), (size_t)ws.numel(),
+                                   static_cast<int32_t*>(ptr(kept)), stream_of(dev)));
+  return tuple(y, kept);
 }
 
-// gate(x [...,K], w1, s1, w3, s3) -> h [...,N], workspace: bf16(silu(x w1)) * (x w3)
+// gate(x [...,K], w1, s1, w3, s3[, workspace or None]) -> h [...,N], workspace to keep: bf16(silu(x w1)) * (x w3)
 PyObject* gate(Args a, Py_ssize_t n) {
-  expect(n, 5, "gate");
+  if (n != 5) expect(n, 6, "gate");
   const Tensor x = dense(tensor(a[0]));
   const Tensor &w1 = tensor(a[1]), &s1 = tensor(a[2]), &w3 = tensor(a[3]), &s3 = tensor(a[4]);
   const c10::Device dev = x.device();
   OnDevice on(dev);
   const int64_t out = w1.size(0), k = w1.size(1), m = x.numel() / k;
   if (w3.sizes() != w1.sizes()) fail(PyExc_ValueError, "gate: w1 and w3 differ in shape");
+  Tensor kept = scratch(n == 6 ? maybe(a[5]) : nullptr, kStatusBytes, dev);
   Tensor ws = scratch(nullptr, jpt_w8a16_gate_workspace_bytes((int)m, (int)out, (int)k), dev);
   Tensor h = empty(with_last(x, out), ScalarType::BFloat16, dev);
-  check(jpt_w8a16_gate(ptr(x), ptr(w1), ptr(s1), ptr(w3), ptr(s3), ptr(h), (int)m, (int)out, (int)k, ptr(ws), (size_t)ws.numel(),
-                       stream_of(dev)));
-  return tuple(h, ws);
+  check(jpt_w8a16_gate_reporting(ptr(x), ptr(w1), ptr(s1), ptr(w3), ptr(s3), ptr(h), (int)m, (int)out, (int)k, ptr(ws), (size_t)ws.numel(),
+                                 static_cast<int32_t*>(ptr(kept)), stream_of(dev)));
+  return tuple(h, kept);
 }
 
 // linear_from_levels(x [...,K] for its shape, levels workspace, weight, scale) -> y

@@ -1319,12 +1319,12 @@ int launch_levels(const void* x, const LevelsView& lv, int M, int K, cudaStream_
 // More than 128 rows: the level kernel over all of them, then the tiles.
 template <bool kGate>
 int launch_tiles(const void* x, const void* w0, const void* s0, const void* w1, const void* s1, void* y, int M, int N, int K,
-                 void* workspace, cudaStream_t st) {
+                 void* workspace, int* status, cudaStream_t st) {
   const RowBlocks rb = row_blocks(M, N, K, kGate ? 128 : kTileN);
   const int rows = rb.blocks * rb.Rb;
   char* ws = static_cast<char*>(workspace);
   LevelsView lv;
-  lv.status = reinterpret_cast<int*>(ws);
+  lv.status = status ? status : reinterpret_cast<int*>(ws);
   lv.lev = reinterpret_cast<int8_t*>(ws + 256);
   lv.xs = reinterpret_cast<float*>(ws + 256 + ((size_t)2 * rows * K + 255) / 256 * 256);
   lv.Mp = rb.Rb;
@@ -1400,6 +1400,11 @@ int check_levels_args(const char* who, int M, int K, const void* workspace, size
 
 extern "C" int jpt_w8a16_linear(const void* x, const void* w, const void* w_scale, void* y, int M, int N, int K,
                                 void* workspace, size_t workspace_bytes, void* stream) {
+  return jpt_w8a16_linear_reporting(x, w, w_scale, y, M, N, K, workspace, workspace_bytes, nullptr, stream);
+}
+
+extern "C" int jpt_w8a16_linear_reporting(const void* x, const void* w, const void* w_scale, void* y, int M, int N, int K,
+                                          void* workspace, size_t workspace_bytes, int32_t* status, void* stream) {
   JPT_REQUIRE(x && w && w_scale && y, JPT_EINVAL, "w8a16_linear: null tensor");
   JPT_REQUIRE(M >= 1, JPT_EINVAL, "w8a16_linear: M = %d rows", M);
   JPT_REQUIRE(N >= 1 && K >= kTileK && K % kTileK == 0, JPT_EINVAL, "w8a16_linear: K = %d must be a multiple of %d", K, kTileK);
@@ -1409,14 +1414,20 @@ extern "C" int jpt_w8a16_linear(const void* x, const void* w, const void* w_scal
               workspace_bytes);
   JPT_REQUIRE(aligned(workspace, 256), JPT_EALIGN, "w8a16_linear: workspace must be 256-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (M > kMaxM) return launch_tiles<false>(x, w, w_scale, nullptr, nullptr, y, M, N, K, workspace, st);
-  const LevelsView lv = levels_view(workspace, M, K);
+  if (M > kMaxM) return launch_tiles<false>(x, w, w_scale, nullptr, nullptr, y, M, N, K, workspace, status, st);
+  LevelsView lv = levels_view(workspace, M, K);
+  if (status) lv.status = status;
   if (int rc = launch_levels(x, lv, M, K, st, true)) return rc;
   return launch_gemm(lv, w, w_scale, y, M, N, K, st);
 }
 
 extern "C" int jpt_w8a16_gate(const void* x, const void* w1, const void* w1_scale, const void* w3, const void* w3_scale, void* h, int M,
                               int N, int K, void* workspace, size_t workspace_bytes, void* stream) {
+  return jpt_w8a16_gate_reporting(x, w1, w1_scale, w3, w3_scale, h, M, N, K, workspace, workspace_bytes, nullptr, stream);
+}
+
+extern "C" int jpt_w8a16_gate_reporting(const void* x, const void* w1, const void* w1_scale, const void* w3, const void* w3_scale, void* h,
+                                        int M, int N, int K, void* workspace, size_t workspace_bytes, int32_t* status, void* stream) {
   JPT_REQUIRE(x && w1 && w1_scale && w3 && w3_scale && h, JPT_EINVAL, "w8a16_gate: null tensor");
   JPT_REQUIRE(M >= 1 && N >= 1 && K >= kTileK && K % kTileK == 0, JPT_EINVAL, "w8a16_gate: M = %d, K = %d (a multiple of %d)", M, K, kTileK);
   JPT_REQUIRE(aligned(x, 16) && aligned(w1, 16) && aligned(w3, 16), JPT_EALIGN, "w8a16_gate: x and the weights must be 16-byte aligned");
@@ -1424,7 +1435,7 @@ extern "C" int jpt_w8a16_gate(const void* x, const void* w1, const void* w1_scal
   JPT_REQUIRE(workspace && workspace_bytes >= need, JPT_EWORKSPACE, "w8a16_gate: workspace of %zu bytes needed, %zu given", need,
               workspace_bytes);
   JPT_REQUIRE(aligned(workspace, 256), JPT_EALIGN, "w8a16_gate: workspace must be 256-byte aligned");
-  return launch_tiles<true>(x, w1, w1_scale, w3, w3_scale, h, M, N, K, workspace, static_cast<cudaStream_t>(stream));
+  return launch_tiles<true>(x, w1, w1_scale, w3, w3_scale, h, M, N, K, workspace, status, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int jpt_w8a16_split_levels(const void* x, int M, int K, void* workspace, size_t workspace_bytes, void* stream) {

@@ -313,7 +313,8 @@ class FeedForward(torch.nn.Module):
       if x.dtype != torch.bfloat16 or x.shape[-1] != self.w1.in_features or x.numel() == 0:
         return self.w2(silu_mul(self.w1(x), self.w3(x)))
       # a prompt: both projections and the gate in one launch behind the level split of x
-      h, self.w1._workspace = _lib.native.gate(x, self.w1.weight, self.w1.weight_scaler, self.w3.weight, self.w3.weight_scaler)
+      h, self.w1._workspace = _lib.native.gate(x, self.w1.weight, self.w1.weight_scaler, self.w3.weight, self.w3.weight_scaler,
+                                               self.w1._workspace)
       return self.w2(h)
     if levels is None:
       levels = ActivationLevels.of(x)

@@ -62,3 +62,21 @@ def test_rmsnorm_of_a_prompt(m, k):
   y, exp = norm(x.to(DEV)).cpu(), ol.rmsnorm(x, w, norm.eps)
   assert torch.allclose(y.float(), exp.float(), rtol=2.0 ** -6, atol=0)
   assert (y == exp).float().mean() > 0.99
+
+
+def test_a_prompt_leaves_no_scratch_behind():
+  """What a layer keeps is the workspace of at most 128 rows, whatever came before; its status word reports the last call."""
+  from jetstream_pytorch_b200 import _lib, layers
+
+  k, n = 512, 640
+  block = layers.FeedForward(k, n, device="cuda")
+  most = {m: _lib.lib().jpt_w8a16_linear_workspace_bytes(128, m.out_features, m.in_features) for m in (block.w1, block.w2, block.w3)}
+  small, large = (torch.randn(rows, k, device="cuda").to(torch.bfloat16) for rows in (5, 3000))
+  want = block.w1(small)
+  for x in (large, small, large):
+    assert block(x).shape == x.shape
+    assert block.w1(x).shape == (x.shape[0], n)
+    for layer, limit in most.items():
+      assert layer._workspace is None or layer._workspace.numel() <= limit
+    assert block.w1.kernel_status() == 0 and block.w2.kernel_status() == 0
+  assert torch.equal(block.w1(small), want)  # (the short call grows what a prompt left it)
