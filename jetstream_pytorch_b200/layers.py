@@ -296,6 +296,14 @@ def silu_mul(a, b, with_levels=False):
   return h, ActivationLevels(m, k, a.device, ws)
 
 
+def _as_built(layer):
+  """Whether calling `layer` is nothing but its own kernel on its weights: no other module put in its place, no hook, no
+  replaced `forward`.  Only then may a fused launch read its weights instead of calling it."""
+  hooks = torch.nn.modules.module
+  return (type(layer) is WeightOnlyPerChannelQuantizedLinear and "forward" not in vars(layer)
+          and not (layer._forward_hooks or layer._forward_pre_hooks or hooks._global_forward_hooks or hooks._global_forward_pre_hooks))
+
+
 class FeedForward(torch.nn.Module):
   """third_party/llama/model_exportable.py:32-86 with weight-only int8 linear
   layers: w2(silu(w1(x)) * w3(x)).  For a decode batch the level split of x is
@@ -310,7 +318,8 @@ class FeedForward(torch.nn.Module):
 
   def forward(self, x, levels=None):
     if not ActivationLevels.fits(x):
-      if x.dtype != torch.bfloat16 or x.shape[-1] != self.w1.in_features or x.numel() == 0:
+      if (x.dtype != torch.bfloat16 or x.shape[-1] != self.w1.in_features or x.numel() == 0
+          or not (_as_built(self.w1) and _as_built(self.w3))):
         return self.w2(silu_mul(self.w1(x), self.w3(x)))
       # a prompt: both projections and the gate in one launch behind the level split of x
       h, self.w1._workspace = _lib.native.gate(x, self.w1.weight, self.w1.weight_scaler, self.w3.weight, self.w3.weight_scaler,

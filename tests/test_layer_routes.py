@@ -1,0 +1,72 @@
+"""CPU: which launches the layers ask for, with the native host side replaced by a recorder."""
+
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+BF = torch.bfloat16
+
+
+@pytest.fixture
+def calls(monkeypatch):
+  from jetstream_pytorch_b200 import _lib
+
+  names = []
+
+  def record(name, result):
+    def call(*args):
+      names.append(name)
+      return result(*args)
+
+    return call
+
+  fake = SimpleNamespace(
+      gate=record("gate", lambda x, w1, *a: (x.new_zeros(*x.shape[:-1], w1.shape[0]), None)),
+      linear=record("linear", lambda x, w, *a: (x.new_zeros(*x.shape[:-1], w.shape[0]), None)),
+      silu_mul=record("silu_mul", lambda a, b, levels: (a, None)))
+  monkeypatch.setattr(_lib, "native", fake)
+  return names
+
+
+def _block():
+  from jetstream_pytorch_b200 import layers
+
+  return layers.FeedForward(128, 256, device="cpu"), torch.zeros(200, 128, dtype=BF)
+
+
+def test_a_prompt_takes_the_fused_gate(calls):
+  block, x = _block()
+  block(x)
+  assert calls == ["gate", "linear"]
+
+
+@pytest.mark.parametrize("change", ["hook", "pre_hook", "global_hook", "subclass", "forward"])
+def test_projections_that_do_more_are_called(calls, change):
+  from jetstream_pytorch_b200 import layers
+
+  block, x = _block()
+  seen, handle = [], None
+  if change == "hook":
+    block.w1.register_forward_hook(lambda m, a, y: seen.append("w1"))
+  elif change == "pre_hook":
+    block.w3.register_forward_pre_hook(lambda m, a: seen.append("w3"))
+  elif change == "global_hook":
+    handle = torch.nn.modules.module.register_module_forward_hook(lambda m, a, y: seen.append("any"))
+  elif change == "subclass":
+
+    class Adapted(layers.WeightOnlyPerChannelQuantizedLinear):
+      def forward(self, x, **kw):
+        seen.append("adapted")
+        return super().forward(x, **kw)
+
+    block.w3 = Adapted(128, 256, device="cpu")
+  else:
+    inner = block.w1.forward
+    block.w1.forward = lambda x, **kw: (seen.append("w1"), inner(x, **kw))[1]
+  try:
+    block(x)
+  finally:
+    if handle:
+      handle.remove()
+  assert seen and calls == ["linear", "linear", "silu_mul", "linear"]
