@@ -201,8 +201,8 @@ class WeightOnlyPerChannelQuantizedLinear(torch.nn.Module):
     if inputs.dtype != torch.bfloat16:
       raise NotImplementedError(f"activations must be bfloat16, got {inputs.dtype}")
     k, n = self.in_features, self.out_features
-    if inputs.shape[-1] != k:
-      inputs = inputs.reshape(-1, k)
+    if inputs.shape[-1] != k and inputs.numel() > 0:
+      raise RuntimeError(f"activations {tuple(inputs.shape)} given to a layer of {k} input features")
     m = inputs.numel() // k
     if m < 1:
       return inputs.new_empty((*inputs.shape[:-1], n))

@@ -70,3 +70,15 @@ def test_projections_that_do_more_are_called(calls, change):
     if handle:
       handle.remove()
   assert seen and calls == ["linear", "linear", "silu_mul", "linear"]
+
+
+def test_activations_of_another_width_are_refused(calls):
+  from jetstream_pytorch_b200 import layers
+
+  layer = layers.WeightOnlyPerChannelQuantizedLinear(128, 64, device="cpu")
+  for shape in [(2, 256), (256, 64), (3, 100)]:
+    with pytest.raises(RuntimeError, match="128 input features"):
+      layer(torch.zeros(shape, dtype=BF))
+  assert not calls
+  assert layer(torch.zeros(3, 0, 128, dtype=BF)).shape == (3, 0, 64)
+  assert layer(torch.zeros(5, 4, 128, dtype=BF)).shape == (5, 4, 64) and calls == ["linear"]
