@@ -186,8 +186,15 @@ class Int8KVCacheGenerate:
     if env.lazy_cache_update:
       if env.generate_cache_stacked:
         if env.new_cache_stacked:
-          self.new_ks, self.new_vs, self.new_k_scaler, self.new_v_scaler = _lib.native.kept_token(
-              cache_k, env.default_type == torch.float32)
+          if cache_k.is_cuda and env.default_type in (torch.bfloat16, torch.float32):
+            self.new_ks, self.new_vs, self.new_k_scaler, self.new_v_scaler = _lib.native.kept_token(
+                cache_k, env.default_type == torch.float32)
+          else:
+            layer, batch, heads, _, dim = cache_k.shape
+            self.new_ks, self.new_vs = (
+                torch.zeros((layer, batch, heads, 1, dim), dtype=torch.int8, device=cache_k.device) for _ in range(2))
+            self.new_k_scaler, self.new_v_scaler = (
+                torch.zeros((layer, batch, 1, 1, 1), dtype=env.default_type, device=cache_k.device) for _ in range(2))
         else:
           self.new_ks, self.new_vs, self.new_k_scaler, self.new_v_scaler = [], [], [], []
       else:

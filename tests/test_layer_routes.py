@@ -82,3 +82,15 @@ def test_activations_of_another_width_are_refused(calls):
   assert not calls
   assert layer(torch.zeros(3, 0, 128, dtype=BF)).shape == (3, 0, 64)
   assert layer(torch.zeros(5, 4, 128, dtype=BF)).shape == (5, 4, 64) and calls == ["linear"]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32, torch.float16])
+def test_kept_token_has_the_default_type(dtype):
+  from jetstream_pytorch_b200.cache_manager import Int8KVCacheGenerate
+
+  env = SimpleNamespace(generate_cache_stacked=True, lazy_cache_update=True, new_cache_stacked=True, default_type=dtype)
+  cache, scales = torch.zeros(2, 3, 4, 16, 128, dtype=torch.int8), torch.ones(2, 3, 1, 16, 1, dtype=dtype)
+  kept = Int8KVCacheGenerate(cache, cache.clone(), scales, scales.clone(), None, env=env)
+  assert kept.new_ks.shape == kept.new_vs.shape == (2, 3, 4, 1, 128) and kept.new_ks.dtype == torch.int8
+  assert kept.new_k_scaler.shape == (2, 3, 1, 1, 1) and kept.new_k_scaler.dtype == kept.new_v_scaler.dtype == dtype
+  assert not kept.new_ks.any() and not kept.new_v_scaler.any()
