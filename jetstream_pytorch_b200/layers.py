@@ -89,7 +89,8 @@ class AttentionKernel(_AttentionKernelBase):
     args = (cache, start, end, ragged_batch_index, ragged_block_index, seqlen, n_rep)
     env = self.env
     if (env.lazy_cache_update and env.ragged_mha and seqlen == 1 and isinstance(end, torch.Tensor)
-        and getattr(cache, "keeps_stacked", None) and cache.keeps_stacked(xq, xk, xv)):
+        and getattr(cache, "keeps_stacked", None) and cache.keeps_stacked(xq, xk, xv)
+        and cache.cache_k.shape[-2] > 1):  # (over a cache of one token `_attend` takes flash attention under the mask)
       # Two launches instead of two copies + ragged attention + flash attention over the new token + merge (the steps
       # below): the same softmax over the same tokens.
       return _lib.native.attend_lazy(xq, xk, xv, cache.cache_k, cache.cache_v, self.layer_id, end, cache.new_ks, cache.new_vs)
@@ -121,7 +122,8 @@ class Int8KVAttentionKernel(_AttentionKernelBase):
       return cache._fused_step(xq, xk, xv, self.layer_id, start, end, False, None, None, True)[4]
     (orig_keys, orig_values, new_key, new_value, k_scaler, v_scaler, new_k_scaler,
      new_v_scaler) = cache.update(xk, xv, self.layer_id)
-    if env.lazy_cache_update and env.ragged_mha and seqlen == 1 and isinstance(end, torch.Tensor) and new_key is not None:
+    if (env.lazy_cache_update and env.ragged_mha and seqlen == 1 and isinstance(end, torch.Tensor) and new_key is not None
+        and orig_keys.shape[-2] > 1):
       # the new token's attention and the merge in one launch behind the ragged attention
       return _lib.native.attend_lazy_int8(xq, (orig_keys, orig_values, k_scaler, v_scaler), self.layer_id, end, new_key, new_value,
                                           new_k_scaler, new_v_scaler)

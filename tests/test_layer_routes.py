@@ -94,3 +94,36 @@ def test_kept_token_has_the_default_type(dtype):
   assert kept.new_ks.shape == kept.new_vs.shape == (2, 3, 4, 1, 128) and kept.new_ks.dtype == torch.int8
   assert kept.new_k_scaler.shape == (2, 3, 1, 1, 1) and kept.new_k_scaler.dtype == kept.new_v_scaler.dtype == dtype
   assert not kept.new_ks.any() and not kept.new_v_scaler.any()
+
+
+@pytest.mark.parametrize("int8", [False, True])
+@pytest.mark.parametrize("tokens", [1, 2])
+def test_a_cache_of_one_token_keeps_its_mask(monkeypatch, int8, tokens):
+  """A lazy step over a cache of one token is flash attention under the step's mask and not ragged attention up to `end`."""
+  from jetstream_pytorch_b200 import _lib, layers
+
+  env = SimpleNamespace(lazy_cache_update=True, ragged_mha=True, flash_attention=True, page_attention=False, shard_on_batch=False,
+                        generate_cache_stacked=True, block_size=16)
+  b, h, d = 2, 4, 16
+  k = torch.zeros(1, b, h, tokens, d, dtype=torch.int8 if int8 else BF)
+  out = torch.zeros(b, h, 1, d)
+  native = []
+  fake = lambda name: lambda *a: (native.append(name), out)[1]
+  monkeypatch.setattr(_lib, "native", SimpleNamespace(attend_lazy=fake("lazy"), attend_lazy_int8=fake("lazy_int8")))
+  cache = SimpleNamespace(cache_k=k, cache_v=k, new_ks=k, new_vs=k, keeps_stacked=lambda *a: True, fused_step_supported=lambda *a: False)
+  cache.update = (lambda xk, xv, i: (k, k, xk, xv, None, None, None, None)) if int8 else (lambda xk, xv, i: (k[i], k[i]))
+  kernel = (layers.Int8KVAttentionKernel if int8 else layers.AttentionKernel)(env, 0)
+  masks = []
+
+  def flash(xq, keys, values, layer, k_scaler, v_scaler, mask):
+    masks.append(mask)
+    return out.to(BF), (torch.zeros(b, h, 1, 1), torch.ones(b, h, 1, 1))
+
+  kernel.flash_attention = flash
+  kernel._merge = lambda *a: out
+  x = torch.zeros(b, h, 1, d, dtype=BF)
+  kernel(x, x, x, "mask", cache, start=torch.zeros(b, dtype=torch.int32), end=torch.ones(b, dtype=torch.int32))
+  if tokens == 1:
+    assert native == [] and masks[0] == "mask"
+  else:
+    assert native == ["lazy_int8" if int8 else "lazy"] and not masks
