@@ -11,12 +11,12 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <cuda_runtime_api.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
-#include <exception>
 #include <optional>
 #include <string>
 #include <vector>
@@ -1082,17 +1082,19 @@ PyObject* attention_workspaces(Args, Py_ssize_t n) {
   return list;
 }
 
+// (exceptions of torch's own calls become the Python types that its operators raise: OutOfMemoryError, IndexError and so on)
 template <PyObject* (*F)(Args, Py_ssize_t)>
 PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
   try {
     return F(args, n);
   } catch (const PyFail& f) {
     PyErr_SetString(f.type, f.text.c_str());
+    return nullptr;
   } catch (const PySet&) {
-  } catch (const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
+    return nullptr;
   }
-  return nullptr;
+  END_HANDLE_TH_ERRORS
 }
 #define JPT_METHOD(name, fn) {name, (PyCFunction)(void (*)(void))entry<fn>, METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {

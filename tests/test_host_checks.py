@@ -113,3 +113,16 @@ def test_end_of_a_step_needs_a_token_of_logits():
     _native().engine_end(torch.zeros(2, 0, 5), *i32, 64, None, False, 0)
   with pytest.raises(ValueError, match="elsewhere"):
     _native().engine_end(torch.zeros(2, 1, 5), *(t.to("meta") for t in i32), 64, None, False, 0)
+
+
+def test_exceptions_of_tensor_calls_keep_their_types():
+  with pytest.raises(IndexError):
+    _native().rmsnorm(torch.zeros((), dtype=BF), torch.zeros(8, dtype=BF), 1e-6, False)
+
+
+@pytest.mark.gpu
+def test_out_of_memory_is_torchs():
+  """2 TB: refused by the allocator, nothing is launched."""
+  x = torch.zeros(1, 8, dtype=BF, device="cuda").expand(1 << 37, 8)
+  with pytest.raises(torch.OutOfMemoryError):
+    _native().silu_mul(x, x, False)
