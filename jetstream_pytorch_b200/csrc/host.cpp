@@ -92,6 +92,7 @@ Tensor as_i32(const Tensor& t, c10::Device dev) {
 }
 Tensor dense(const Tensor& t) { return t.is_contiguous() ? t : t.contiguous(); }
 Tensor empty(at::IntArrayRef sizes, ScalarType type, c10::Device dev) {
+  if (!dev.is_cuda()) fail(PyExc_ValueError, "libjpt_b200 works on CUDA tensors only; got a tensor on %s", dev.str().c_str());
   return Tensor(at::detail::empty_cuda(sizes, type, dev, std::nullopt));
 }
 cudaStream_t stream_of(c10::Device dev) { return c10::cuda::getCurrentCUDAStream(dev.index()).stream(); }
@@ -282,6 +283,7 @@ void take_kv(Call& c, const Tensor& k, const Tensor& v, int64_t layer) {
   if (o == 1) c.k_off = layer_index(layer, c.k.size(0)) * c.k.stride(0);
   c.kv_b = c.k.stride(o), c.kv_h = c.k.stride(o + 1), c.kv_s = c.k.stride(o + 2);
   c.hkv = c.k.size(o + 1), c.seq = c.k.size(o + 2);
+  if (c.hkv < 1) fail(PyExc_ValueError, "a cache without KV heads");
 }
 // Scales [B,1,S,1] or [B,1,S]; stacked: a leading NL.
 void take_scales(Call& c, const Tensor* ks, const Tensor* vs, int64_t layer) {
@@ -456,6 +458,7 @@ PyObject* paged(Args a, Py_ssize_t n) {
   c.end = tensor(a[3]), c.table = tensor(a[4]);
   c.paged = true;
   c.hkv = c.k.size(0), c.page_size = c.k.size(2);
+  if (c.hkv < 1) fail(PyExc_ValueError, "page pools without KV heads");
   c.sm_scale = real(a[5]);
   if (auto t = maybe(a[6])) c.ks = *t, c.vs = tensor(a[7]);
   c.mask_mode = JPT_MASK_LENGTH;
@@ -615,7 +618,7 @@ PyObject* fused_ok(Args a, Py_ssize_t n) {
   expect(n, 3, "fused_ok");
   const Tensor &q = tensor(a[0]), &k = tensor(a[1]);
   const Tensor* sc = maybe(a[2]);
-  const bool ok = q.dim() == 4 && k.dim() == 4 && q.size(3) == 128 && q.size(2) == 1 && k.size(2) == 1 && q.size(1) % k.size(1) == 0 &&
+  const bool ok = q.dim() == 4 && k.dim() == 4 && q.size(3) == 128 && q.size(2) == 1 && k.size(2) == 1 && k.size(1) > 0 && q.size(1) % k.size(1) == 0 &&
                   q.size(1) / k.size(1) <= 8 && (k.scalar_type() == ScalarType::BFloat16 || k.scalar_type() == ScalarType::Float) &&
                   q.scalar_type() == ScalarType::BFloat16 && sc && sc->scalar_type() == k.scalar_type();
   return PyBool_FromLong(ok);
@@ -987,6 +990,11 @@ std::vector<int64_t> with_last(const Tensor& x, int64_t last) {
   return s;
 }
 
+// Rows of k features in x.
+int64_t rows_of(const Tensor& x, int64_t k) {
+  if (k < 1 || x.dim() < 1) fail(PyExc_ValueError, "activations of %lld features", (long long)k);
+  return x.numel() / k;
+}
 // What a layer keeps between its calls is the workspace of up to kKeptRows rows, whose first word its kernels report to.  The scratch of a
 // longer prompt (2 M K bytes) goes back to the allocator behind the call, in stream order: kept by every layer it was
 // several GB of a model.
@@ -1000,7 +1008,7 @@ PyObject* linear(Args a, Py_ssize_t n) {
   const Tensor &w = tensor(a[1]), &sc = tensor(a[2]);
   const c10::Device dev = x.device();
   OnDevice on(dev);
-  const int64_t out = w.size(0), k = w.size(1), m = x.numel() / k;
+  const int64_t out = w.size(0), k = w.size(1), m = rows_of(x, k);
   const size_t need = jpt_w8a16_linear_workspace_bytes((int)m, (int)out, (int)k);
   Tensor kept = scratch(maybe(a[3]), m > kKeptRows ? kStatusBytes : need, dev);
   Tensor ws = m > kKeptRows ? scratch(nullptr, need, dev) : kept;
@@ -1017,7 +1025,7 @@ PyObject* gate(Args a, Py_ssize_t n) {
   const Tensor &w1 = tensor(a[1]), &s1 = tensor(a[2]), &w3 = tensor(a[3]), &s3 = tensor(a[4]);
   const c10::Device dev = x.device();
   OnDevice on(dev);
-  const int64_t out = w1.size(0), k = w1.size(1), m = x.numel() / k;
+  const int64_t out = w1.size(0), k = w1.size(1), m = rows_of(x, k);
   if (w3.sizes() != w1.sizes()) fail(PyExc_ValueError, "gate: w1 and w3 differ in shape");
   Tensor kept = scratch(n == 6 ? maybe(a[5]) : nullptr, kStatusBytes, dev);
   Tensor ws = scratch(nullptr, jpt_w8a16_gate_workspace_bytes((int)m, (int)out, (int)k), dev);
@@ -1033,7 +1041,7 @@ PyObject* linear_from_levels(Args a, Py_ssize_t n) {
   const Tensor &x = tensor(a[0]), &ws = tensor(a[1]), &w = tensor(a[2]), &sc = tensor(a[3]);
   const c10::Device dev = ws.device();
   OnDevice on(dev);
-  const int64_t out = w.size(0), k = w.size(1), m = x.numel() / k;
+  const int64_t out = w.size(0), k = w.size(1), m = rows_of(x, k);
   Tensor y = empty(with_last(x, out), ScalarType::BFloat16, dev);
   check(jpt_w8a16_linear_from_levels(ptr(ws), (size_t)ws.numel(), ptr(w), ptr(sc), ptr(y), (int)m, (int)out, (int)k, stream_of(dev)));
   return wrap(y);
@@ -1046,7 +1054,7 @@ PyObject* rmsnorm(Args a, Py_ssize_t n) {
   const Tensor& w = tensor(a[1]);
   const c10::Device dev = x.device();
   OnDevice on(dev);
-  const int64_t k = x.size(-1), m = x.numel() / k;
+  const int64_t k = x.size(-1), m = rows_of(x, k);
   Tensor y = empty(x.sizes(), ScalarType::BFloat16, dev), ws;
   if (truth(a[3])) ws = scratch(nullptr, jpt_w8a16_linear_workspace_bytes((int)m, 1, (int)k), dev);
   check(jpt_rmsnorm(ptr(x), ptr(w), (float)real(a[2]), ptr(y), (int)m, (int)k, ws.defined() ? ptr(ws) : nullptr,
@@ -1060,7 +1068,7 @@ PyObject* silu_mul(Args a, Py_ssize_t n) {
   const Tensor x = dense(tensor(a[0])), g = dense(tensor(a[1]));
   const c10::Device dev = x.device();
   OnDevice on(dev);
-  const int64_t k = x.size(-1), m = x.numel() / k;
+  const int64_t k = x.size(-1), m = rows_of(x, k);
   Tensor h = empty(x.sizes(), ScalarType::BFloat16, dev), ws;
   if (truth(a[2])) ws = scratch(nullptr, jpt_w8a16_linear_workspace_bytes((int)m, 1, (int)k), dev);
   check(jpt_silu_mul(ptr(x), ptr(g), ptr(h), (int)m, (int)k, ws.defined() ? ptr(ws) : nullptr, ws.defined() ? (size_t)ws.numel() : 0,

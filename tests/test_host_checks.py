@@ -126,3 +126,30 @@ def test_out_of_memory_is_torchs():
   x = torch.zeros(1, 8, dtype=BF, device="cuda").expand(1 << 37, 8)
   with pytest.raises(torch.OutOfMemoryError):
     _native().silu_mul(x, x, False)
+
+
+def test_empty_extents_are_refused():
+  """(an integer division by zero would end the process)"""
+  n, e = _native(), torch.zeros(4, 0, dtype=BF)
+  w, sc = torch.zeros(8, 0, dtype=torch.int8), torch.zeros(8, dtype=BF)
+  for call in (lambda: n.rmsnorm(e, e[0], 1e-6, False), lambda: n.silu_mul(e, e, False), lambda: n.linear(e, w, sc, None),
+               lambda: n.gate(e, w, sc, w, sc, None), lambda: n.linear_from_levels(e, e, w, sc)):
+    with pytest.raises(ValueError, match="0 features"):
+      call()
+  q, k = torch.zeros(2, 8, 1, D, dtype=BF), torch.zeros(2, 0, S, D, dtype=BF)
+  end, mask = torch.zeros(2, dtype=torch.int32), torch.zeros(2, 1, 1, S, dtype=BF)
+  for call in (lambda: n.ragged(q, k, k, 0, None, end, None, None, True, False), lambda: n.dense(q, k, k, None, None, mask),
+               lambda: n.paged(q[:, :, 0], k.reshape(0, 2, S, D), k.reshape(0, 2, S, D), end, end.reshape(2, 1), 1.0, None, None)):
+    with pytest.raises(ValueError, match="without KV heads"):
+      call()
+  assert n.fused_ok(q, torch.zeros(2, 0, 1, D, dtype=BF), None) is False
+  with pytest.raises(ValueError, match="blocks of 0"):
+    n.engine_begin(end, end, 64, 0, None, False, 0)
+
+
+def test_cpu_tensors_are_refused_with_one_message():
+  n, x = _native(), torch.zeros(4, 128, dtype=BF)
+  w, sc = torch.zeros(8, 128, dtype=torch.int8), torch.zeros(8, dtype=BF)
+  for call in (lambda: n.rmsnorm(x, x[0], 1e-6, False), lambda: n.silu_mul(x, x, True), lambda: n.linear(x, w, sc, None)):
+    with pytest.raises(ValueError, match="CUDA tensors only"):
+      call()
