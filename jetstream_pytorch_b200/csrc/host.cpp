@@ -117,42 +117,55 @@ PyObject* tuple(const Ts&... ts) {
 // ---------------------------------------------------------------- attention workspaces
 // Grow-only attention scratch, one per stream (two launches that share one must not overlap) and one more per device for
 // CUDA graph captures, which run on a stream of their own and must not allocate: every eager call keeps that one at
-// least as large as its own.  Cleared once when created, as the kernels' arrival counters require.
+// least as large as its own.  Cleared once when created, as the kernels' arrival counters require.  A graph holds the address
+// of the scratch that it was captured with, so one that a capture has been given stays allocated when a larger one takes
+// its place; each is at least twice as large as the one before, so that all retired ones together are smaller than it.
 struct Workspace {
   c10::DeviceIndex device;
   bool graph;
   cudaStream_t stream;
   Tensor mem;
+  bool captured = false, retired = false;  // (graph)
 };
 std::vector<Workspace>& workspaces() {
   static auto* list = new std::vector<Workspace>();  // (never destroyed: the CUDA context may be gone by then)
   return *list;
 }
-Tensor& workspace_for(c10::Device dev, cudaStream_t st, bool graph, bool may_grow, size_t bytes) {
-  Workspace* w = nullptr;
+Workspace* find_workspace(c10::Device dev, cudaStream_t st, bool graph) {
   for (Workspace& e : workspaces())
-    if (e.device == dev.index() && e.graph == graph && (graph || e.stream == st)) w = &e;
-  if (w && (size_t)w->mem.numel() >= bytes) return w->mem;
-  if (!may_grow)
-    fail(PyExc_RuntimeError,
-         "the attention workspace for CUDA graphs is too small and cannot grow during capture; call the same shape once before "
-         "capturing");
-  Tensor mem = empty({(int64_t)std::max<size_t>(bytes, 8u << 20)}, ScalarType::Byte, dev);
+    if (e.device == dev.index() && e.graph == graph && !e.retired && (graph || e.stream == st)) return &e;
+  return nullptr;
+}
+Workspace& grown_workspace(c10::Device dev, cudaStream_t st, bool graph, size_t bytes) {
+  Workspace* w = find_workspace(dev, st, graph);
+  if (w && (size_t)w->mem.numel() >= bytes) return *w;
+  size_t size = std::max<size_t>(bytes, 8u << 20);
+  if (w && w->captured) size = std::max<size_t>(size, 2 * (size_t)w->mem.numel());
+  Tensor mem = empty({(int64_t)size}, ScalarType::Byte, dev);
   check(jpt_flash_decode_workspace_init(mem.data_ptr(), (size_t)mem.numel(), st));
-  if (w) {
+  if (w && !w->captured) {
     w->mem = mem;
-    return w->mem;
+    return *w;
   }
+  if (w) w->retired = true;
   workspaces().push_back({dev.index(), graph, st, mem});
-  return workspaces().back().mem;
+  return workspaces().back();
 }
 Tensor workspace(c10::Device dev, cudaStream_t st, size_t bytes) {
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess) capturing = cudaStreamCaptureStatusNone;
-  if (capturing != cudaStreamCaptureStatusNone) return workspace_for(dev, st, true, false, bytes);
-  Tensor own = workspace_for(dev, st, false, true, bytes);
-  workspace_for(dev, st, true, true, bytes);
-  return own;
+  if (capturing == cudaStreamCaptureStatusNone) {
+    Tensor own = grown_workspace(dev, st, false, bytes).mem;
+    grown_workspace(dev, st, true, bytes);
+    return own;
+  }
+  Workspace* w = find_workspace(dev, st, true);
+  if (!w || (size_t)w->mem.numel() < bytes)
+    fail(PyExc_RuntimeError,
+         "the attention workspace for CUDA graphs is too small and cannot grow during capture; call the same shape once before "
+         "capturing");
+  w->captured = true;
+  return w->mem;
 }
 
 // ---------------------------------------------------------------- attention
