@@ -775,15 +775,17 @@ PyObject* append_paged(Args a, Py_ssize_t n) {
   Py_RETURN_NONE;
 }
 
-// page_token_indices(lens, page_table, page_size) -> pti int32 [3,B], n_active [1], new_lengths [B]
+// page_token_indices(lens, page_table, page_size, slots, pages per slot) -> pti int32 [3,B], n_active [1], new_lengths [B]
 PyObject* page_token_indices(Args a, Py_ssize_t n) {
-  expect(n, 3, "page_token_indices");
+  expect(n, 5, "page_token_indices");
   const c10::Device dev = tensor(a[0]).device();
   OnDevice on(dev);
+  const int64_t b = integer(a[3]), pages = integer(a[4]);
+  if (tensor(a[0]).numel() < b || tensor(a[1]).numel() < b * pages)
+    fail(PyExc_ValueError, "page_token_indices: lengths of %lld slots and a table of %lld pages each are needed", (long long)b, (long long)pages);
   const Tensor lens = as_i32(tensor(a[0]), dev), table = as_i32(tensor(a[1]), dev);
-  const int64_t b = table.size(0);
   Tensor pti = empty({3, b}, ScalarType::Int, dev), active = empty({1}, ScalarType::Int, dev), lengths = empty({b}, ScalarType::Int, dev);
-  check(jpt_page_token_indices(static_cast<const int32_t*>(ptr(lens)), static_cast<const int32_t*>(ptr(table)), (int)b, (int)table.size(1),
+  check(jpt_page_token_indices(static_cast<const int32_t*>(ptr(lens)), static_cast<const int32_t*>(ptr(table)), (int)b, (int)pages,
                                (int)integer(a[2]), static_cast<int32_t*>(ptr(pti)), static_cast<int32_t*>(ptr(active)),
                                static_cast<int32_t*>(ptr(lengths)), stream_of(dev)));
   return tuple(pti, active, lengths);

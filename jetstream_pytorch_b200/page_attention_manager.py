@@ -107,7 +107,8 @@ class PageAttentionManager:
     rows compacted over active slots, n_active int32 [1], new_lengths int32
     [B]).  The caller remains responsible for page reservation
     (`fill_new_pages`) on the host."""
-    return _lib.native.page_token_indices(lens_dev, page_indices_dev, self.paged_attention_page_size)
+    return _lib.native.page_token_indices(lens_dev, page_indices_dev, self.paged_attention_page_size, self.batch_size,
+                                          self.max_pages_per_sequence)
 
   def prefill_cache_padding(self, caches, seq_len: int, num_pages: int):
     """page_attention_manager.py:67-81 (zero-pad the sequence axis to whole pages)."""

@@ -153,3 +153,21 @@ def test_cpu_tensors_are_refused_with_one_message():
   for call in (lambda: n.rmsnorm(x, x[0], 1e-6, False), lambda: n.silu_mul(x, x, True), lambda: n.linear(x, w, sc, None)):
     with pytest.raises(ValueError, match="CUDA tensors only"):
       call()
+
+
+def test_page_table_walk_takes_the_managers_extents(monkeypatch):
+  """As many slots and pages as the manager has, not as many as the table happens to have rows and columns."""
+  from types import SimpleNamespace
+
+  from jetstream_pytorch_b200 import _lib
+  from jetstream_pytorch_b200.page_attention_manager import PageAttentionManager
+
+  lens, table = torch.zeros(4, dtype=torch.int32), torch.zeros(3, 6, dtype=torch.int32)
+  walk = _native().page_token_indices
+  for few in ((lens[:2], table), (lens, table[:2])):
+    with pytest.raises(ValueError, match="lengths of 3 slots"):
+      walk(*few, 16, 3, 6)
+  seen = []
+  monkeypatch.setattr(_lib, "native", SimpleNamespace(page_token_indices=lambda *a: seen.append(a[2:])))
+  PageAttentionManager(3, 20, 16, 6).get_page_token_indices_device(lens, table)
+  assert seen == [(16, 3, 6)]
