@@ -171,3 +171,11 @@ def test_page_table_walk_takes_the_managers_extents(monkeypatch):
   monkeypatch.setattr(_lib, "native", SimpleNamespace(page_token_indices=lambda *a: seen.append(a[2:])))
   PageAttentionManager(3, 20, 16, 6).get_page_token_indices_device(lens, table)
   assert seen == [(16, 3, 6)]
+
+
+def test_stacked_insert_needs_a_scale_per_layer():
+  """Scalers of fewer layers than the prefix: left to the loop over the layers, which raises IndexError for the missing one."""
+  prefix = [(torch.zeros(1, H, 5, D, dtype=BF),) * 2 for _ in range(3)]
+  caches = [(torch.zeros(3, B, H, S, D, dtype=torch.int8),) * 2]
+  assert _native().insert_dense(prefix, caches, [(torch.ones(2, B, 1, S, 1, dtype=BF),) * 2], 0, 0, False, True) is False
+  assert _native().insert_dense(prefix, caches, [(torch.ones(B, 1, S, 1, dtype=BF),) * 2], 0, 0, False, True) is False
