@@ -151,10 +151,12 @@ Workspace& grown_workspace(c10::Device dev, cudaStream_t st, bool graph, size_t 
   workspaces().push_back({dev.index(), graph, st, mem});
   return workspaces().back();
 }
-Tensor workspace(c10::Device dev, cudaStream_t st, size_t bytes) {
+bool is_capturing(cudaStream_t st) {
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess) capturing = cudaStreamCaptureStatusNone;
-  if (capturing == cudaStreamCaptureStatusNone) {
+  return cudaStreamIsCapturing(st, &capturing) == cudaSuccess && capturing != cudaStreamCaptureStatusNone;
+}
+Tensor workspace(c10::Device dev, cudaStream_t st, size_t bytes) {
+  if (!is_capturing(st)) {
     Tensor own = grown_workspace(dev, st, false, bytes).mem;
     grown_workspace(dev, st, true, bytes);
     return own;
@@ -265,6 +267,17 @@ void run_attention(Call& c, at::IntArrayRef out_shape, at::IntArrayRef ml_shape)
   }
   Tensor ws;
   if (const size_t need = jpt_flash_decode_workspace_bytes(&p)) {
+    if (!c.nt && is_capturing(st)) {
+      // A prompt captured before anything ran: the prefill kernel wants only a status word and its table of mask classes, which the
+      // scratch built into the library has (the scalar kernel that took such calls before mostly needed none).
+      const Workspace* w = find_workspace(dev, st, true);
+      if ((!w || (size_t)w->mem.numel() < need) && jpt_flash_attend_strided_q_ok(&p, hq * tq * d, tq * d, d)) {
+        c.q = dense(c.q);
+        p.q = ptr(c.q);
+        check(jpt_flash_decode_static(&p, st));
+        return;
+      }
+    }
     ws = workspace(dev, st, need);
     p.workspace = ws.data_ptr(), p.workspace_bytes = (size_t)ws.numel();
   }

@@ -49,3 +49,30 @@ def test_a_graph_keeps_the_scratch_it_was_captured_with():
   torch.cuda.synchronize()
   assert torch.equal(out, want) and ak.kernel_status(DEV) == 0
   assert all(bool((f == 7).all()) for f in fill)
+
+
+_FIRST = """
+import torch
+from jetstream_pytorch_b200 import attention_kernel as ak
+g = torch.Generator(device="cuda").manual_seed(0)
+q, k, v = (torch.randn((1, 700, h, 128), generator=g, device="cuda", dtype=torch.bfloat16).transpose(1, 2) for h in (16, 4, 4))
+mask = torch.full((700, 700), float("-inf"), device="cuda").triu(1).to(torch.bfloat16).repeat(4, 1)[None, None]
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+  out = ak.dense_attention(q, k, v, None, None, mask)
+graph.replay()
+torch.cuda.synchronize()
+got = out.clone()
+assert torch.equal(got, ak.dense_attention(q, k, v, None, None, mask)) and ak.kernel_status("cuda") == 0
+print("captured first")
+"""
+
+
+def test_a_prompt_can_be_captured_before_anything_ran():
+  import os
+  import subprocess
+  import sys
+
+  root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+  run = subprocess.run([sys.executable, "-c", _FIRST], cwd=root, capture_output=True, text=True, timeout=300)
+  assert run.returncode == 0 and "captured first" in run.stdout, run.stderr[-2000:]
