@@ -29,7 +29,8 @@
 //
 // An additive mask is classified beforehand, one byte per [128 x 128] tile: all zero (no mask work), all -inf (tile
 // skipped), mixed (added value by value).  With up to kSmallK tiles per row every tile counts as mixed and that launch
-// (2 us and more) is saved.  Keys and values of masked keys may hold anything (plain_rows).  Every wait is bounded; a CTA that gives up raises the workspace's status word.
+// (2 us and more) is saved.  The values of masked keys may hold anything, NaN and infinities too (plain_rows).  Every wait is
+// bounded; a CTA that gives up raises the workspace's status word.
 #include <cuda.h>
 #include <string.h>
 

@@ -846,7 +846,8 @@ __global__ void __launch_bounds__(kThreadsL, 1)
 }
 
 // ---------------------------------------------------------------- more than 128 rows (prefill)
-// Bound: the integer MMAs (two levels: 4 M N K operations).  Weights as the M = 128 operand twice (256 channels), a block of up
+// Bound: the integer MMAs (two levels: 4 M N K operations) where a tile has many steps of K (tensor pipe 0.88 of the active cycles with
+// 112), and the epilogue between the tiles where it has few (0.62 with the gate's 32).  Weights as the M = 128 operand twice (256 channels), a block of up
 // to 128 rows as the N operand (h rows, then l rows), accumulators in all of tensor memory; persistent CTAs, one per SM,
 // walk the tiles with the row blocks fastest, so that the CTAs of a moment share weight tiles in L2.  A tile step (128 bytes
 // of K) reads 64 KB for 1024 cycles of MMA.  The ring keeps filling under the epilogue; the accumulators do not double.
@@ -1129,8 +1130,10 @@ RowBlocks row_blocks(int M, int N, int K, int channels) {
 // every form the tile is the narrowest that covers the channels in whole waves of clusters; the plan with the shortest
 // estimated run is taken.  A stage costs its hand-over and its MMAs or bytes (the weights at a share of the memory rate, the
 // activations from L2); a wave costs set-up, first fetch and epilogue.  The constants (us, bytes per us) are fitted to the
-// measured times of up to nine forms each of 9 shapes (1280 to 28672 channels, K of 4096 to 28672) with 7 and 96 rows: the form taken
-// is within 4 % of the fastest of them everywhere and the estimate mostly within 10 %.  Measured, us, 96 rows / 7 rows: pairs on
+// measured times of up to nine forms each of 9 shapes (1280 to 28672 channels, K of 4096 to 28672) with 7 and 96 rows, the estimate
+// mostly within 10 %.  Against every form timed for 10 such shapes with 1, 7, 16, 32, 48, 64, 80, 96 and 128 rows the form taken is
+// within 5 % of the fastest in 87 of the 90 and within 9 % in all (3584 -> 8192 with 32 rows: 10.9 against 10.0 for pairs in two
+// splits).  Measured, us, 96 rows / 7 rows: pairs on
 // 8192 -> 28672 49.0 / 40.7 (single CTAs 52.1 / 42.4), pairs in two splits on 28672 -> 8192 46.4 / 37.8 (single CTAs in four 51.0 /
 // 42.0), single CTAs in four splits on 14336 -> 4096 17.1 / 12.7 (one pair per tile 31.8 / 18.2).
 struct GemmPlan {
