@@ -167,6 +167,7 @@ class WeightOnlyPerChannelQuantizedLinear(torch.nn.Module):
     self.n_bit = 8
     self.quantize_activation = False
     self._workspace = None
+    self._status = None  # the tensor whose first word the last call reports to
 
   def _load_quantized_weights(self, w_q, scale, zp=None):
     """layers.py:114-120 with `load_q_weight_helper` (quantize.py:86-93)."""
@@ -190,7 +191,7 @@ class WeightOnlyPerChannelQuantizedLinear(torch.nn.Module):
 
   def kernel_status(self):
     """0, or 1 if a bounded wait inside the last launch gave up (synchronises)."""
-    return 0 if self._workspace is None else int(self._workspace[:4].view(torch.int32).item())
+    return 0 if self._status is None else int(self._status[:4].view(torch.int32).item())
 
   def forward(self, inputs, levels=None, tp=None):
     """`levels` (an `ActivationLevels` of `inputs`, from `RMSNorm`, `FeedForward`
@@ -216,6 +217,7 @@ class WeightOnlyPerChannelQuantizedLinear(torch.nn.Module):
       need = lib.jpt_w8a16_linear_workspace_bytes(m, n, k)
       if self._workspace is None or self._workspace.numel() < need or self._workspace.device != x.device:
         self._workspace = torch.empty((need,), dtype=torch.uint8, device=x.device)
+      self._status = self._workspace
       y = torch.empty((m, n), dtype=torch.bfloat16, device=x.device)
       _lib.check(lib.jpt_w8a16_linear_tp(_lib.ptr(x), _lib.ptr(self.weight), _lib.ptr(self.weight_scaler), _lib.ptr(y), m, n, k,
                                          _lib.ptr(self._workspace), self._workspace.numel(), ctypes.byref(tp.struct),
@@ -224,9 +226,10 @@ class WeightOnlyPerChannelQuantizedLinear(torch.nn.Module):
     if levels is not None:
       if (levels.rows, levels.features) != (m, k):
         raise ValueError(f"levels of a [{levels.rows}, {levels.features}] activation given for [{m}, {k}]")
-      self._workspace = levels.workspace  # (kernel_status reads the status word of the workspace last used)
+      self._status = levels.workspace  # (not a workspace of this layer's: other layers read these levels)
       return _lib.native.linear_from_levels(inputs, levels.workspace, self.weight, self.weight_scaler)
     y, self._workspace = _lib.native.linear(inputs, self.weight, self.weight_scaler, self._workspace)
+    self._status = self._workspace
     return y
 
 
@@ -326,6 +329,7 @@ class FeedForward(torch.nn.Module):
       # a prompt: both projections and the gate in one launch behind the level split of x
       h, self.w1._workspace = _lib.native.gate(x, self.w1.weight, self.w1.weight_scaler, self.w3.weight, self.w3.weight_scaler,
                                                self.w1._workspace)
+      self.w1._status = self.w1._workspace
       return self.w2(h)
     if levels is None:
       levels = ActivationLevels.of(x)

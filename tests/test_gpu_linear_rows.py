@@ -80,3 +80,18 @@ def test_a_prompt_leaves_no_scratch_behind():
       assert layer._workspace is None or layer._workspace.numel() <= limit
     assert block.w1.kernel_status() == 0 and block.w2.kernel_status() == 0
   assert torch.equal(block.w1(small), want)  # (the short call grows what a prompt left it)
+
+
+def test_levels_outlive_another_call_of_a_layer_that_read_them():
+  """One level split for two layers, with a call on other activations in between."""
+  from jetstream_pytorch_b200 import layers
+
+  g = torch.Generator().manual_seed(3)
+  w1, w3 = (_layer(320, 256, g)[0] for _ in range(2))
+  x, other = (torch.randn(9, 256, generator=g).to(torch.bfloat16).to(DEV) for _ in range(2))
+  want = w3(x)
+  levels = layers.ActivationLevels.of(x)
+  w1(x, levels=levels)
+  assert w1.kernel_status() == 0
+  w1(other)
+  assert torch.equal(w3(x, levels=levels), want)
