@@ -227,8 +227,8 @@ class KVCacheEngine:
       new_scales = [c.scalers() for c in caches_obj]
     elif decode_state.cache_scales:
       new_scales = decode_state.cache_scales
-    if (native and sampler is None and logits.ndim == 3 and logits.device == decode_state.tokens.device and logits.stride(2) == 1
-        and logits.dtype in (torch.float32, torch.bfloat16) and logits.shape[0] == decode_state.input_pos.numel() and logits.shape[1] > 0):
+    if (native and sampler is None and logits.ndim == 3 and logits.is_cuda and logits.stride(2) == 1
+        and logits.dtype in (torch.float32, torch.bfloat16) and logits.shape[0] == decode_state.input_pos.numel() and logits.shape[1]):
       # greedy sampling, the advance of the positions, the result rows and (lazy updates) the mask in one launch
       next_token, lens, input_pos, data = _lib.native.engine_end(
           logits, decode_state.tokens, decode_state.lens, decode_state.input_pos, env.cache_len,

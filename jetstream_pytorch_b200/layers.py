@@ -193,6 +193,10 @@ class WeightOnlyPerChannelQuantizedLinear(torch.nn.Module):
     """0, or 1 if a bounded wait inside the last launch gave up (synchronises)."""
     return 0 if self._status is None else int(self._status[:4].view(torch.int32).item())
 
+  def _keep(self, workspace):
+    """What the last call left: its scratch, whose first word is its status.  (Module.__setattr__ takes over 1 us.)"""
+    self.__dict__["_workspace"] = self.__dict__["_status"] = workspace
+
   def forward(self, inputs, levels=None, tp=None):
     """`levels` (an `ActivationLevels` of `inputs`, from `RMSNorm`, `FeedForward`
     or `ActivationLevels.of`): the layer starts at its GEMM.
@@ -217,7 +221,7 @@ class WeightOnlyPerChannelQuantizedLinear(torch.nn.Module):
       need = lib.jpt_w8a16_linear_workspace_bytes(m, n, k)
       if self._workspace is None or self._workspace.numel() < need or self._workspace.device != x.device:
         self._workspace = torch.empty((need,), dtype=torch.uint8, device=x.device)
-      self._status = self._workspace
+      self._keep(self._workspace)
       y = torch.empty((m, n), dtype=torch.bfloat16, device=x.device)
       _lib.check(lib.jpt_w8a16_linear_tp(_lib.ptr(x), _lib.ptr(self.weight), _lib.ptr(self.weight_scaler), _lib.ptr(y), m, n, k,
                                          _lib.ptr(self._workspace), self._workspace.numel(), ctypes.byref(tp.struct),
@@ -226,10 +230,10 @@ class WeightOnlyPerChannelQuantizedLinear(torch.nn.Module):
     if levels is not None:
       if (levels.rows, levels.features) != (m, k):
         raise ValueError(f"levels of a [{levels.rows}, {levels.features}] activation given for [{m}, {k}]")
-      self._status = levels.workspace  # (not a workspace of this layer's: other layers read these levels)
+      self.__dict__["_status"] = levels.workspace  # (not a workspace of this layer's: other layers read these levels)
       return _lib.native.linear_from_levels(inputs, levels.workspace, self.weight, self.weight_scaler)
-    y, self._workspace = _lib.native.linear(inputs, self.weight, self.weight_scaler, self._workspace)
-    self._status = self._workspace
+    y, kept = _lib.native.linear(inputs, self.weight, self.weight_scaler, self._workspace)
+    self._keep(kept)
     return y
 
 
@@ -327,9 +331,8 @@ class FeedForward(torch.nn.Module):
           or not (_as_built(self.w1) and _as_built(self.w3))):
         return self.w2(silu_mul(self.w1(x), self.w3(x)))
       # a prompt: both projections and the gate in one launch behind the level split of x
-      h, self.w1._workspace = _lib.native.gate(x, self.w1.weight, self.w1.weight_scaler, self.w3.weight, self.w3.weight_scaler,
-                                               self.w1._workspace)
-      self.w1._status = self.w1._workspace
+      h, kept = _lib.native.gate(x, self.w1.weight, self.w1.weight_scaler, self.w3.weight, self.w3.weight_scaler, self.w1._workspace)
+      self.w1._keep(kept)
       return self.w2(h)
     if levels is None:
       levels = ActivationLevels.of(x)
