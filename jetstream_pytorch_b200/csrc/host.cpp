@@ -851,7 +851,7 @@ bool take_layers(Layers& r, PyObject* prefixes, PyObject* caches, PyObject* scal
       r.pk = pk, r.ck = ck;
       if (ks) r.ks = *ks;
       if (ck.dim() != (stacked ? 5 : 4) || (stacked && ck.size(0) < n)) return false;
-      if (ks && (ks->dim() != ck.dim() || (stacked && ks->size(0) < n))) return false;
+      if (ks && (ks->dim() != ck.dim() || (stacked && vs && (ks->size(0) < n || vs->size(0) < n)))) return false;
     }
     if (pk.dim() != 4 || pv.sizes() != pk.sizes() || pk.sizes() != r.pk.sizes() || pk.strides() != r.pk.strides() ||
         pk.scalar_type() != r.pk.scalar_type() || pv.scalar_type() != pk.scalar_type() || pk.device() != r.pk.device() ||
@@ -859,7 +859,7 @@ bool take_layers(Layers& r, PyObject* prefixes, PyObject* caches, PyObject* scal
         cv.strides() != ck.strides() || ck.scalar_type() != r.ck.scalar_type() || cv.scalar_type() != ck.scalar_type() ||
         ck.device() != r.ck.device() || cv.device() != ck.device() || (ks != nullptr) != r.ks.defined() || (ks != nullptr) != (vs != nullptr))
       return false;
-    if (ks && (ks->sizes() != r.ks.sizes() || ks->strides() != r.ks.strides() || vs->sizes() != ks->sizes() || vs->strides() != ks->strides() || ks->scalar_type() != pk.scalar_type() ||
+    if (ks && (ks->strides() != r.ks.strides() || vs->strides() != ks->strides() || ks->scalar_type() != pk.scalar_type() ||
                vs->scalar_type() != pk.scalar_type()) && ck.scalar_type() == ScalarType::Char)
       return false;
     const int64_t co = stacked ? i * ck.stride(0) : 0, so = stacked && ks ? i * ks->stride(0) : 0;
