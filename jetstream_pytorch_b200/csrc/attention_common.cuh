@@ -48,6 +48,17 @@ __device__ __forceinline__ float rounded_logit(float dot, float sqrt_d, float ks
   return bf16_round(s + mask_value);
 }
 
+// The same with the reciprocal of sqrt_d (rounded to nearest) at hand: the quotient's first guess and one correction by the exact
+// remainder give the correctly rounded quotient (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", 1990) in three instructions.
+__device__ __forceinline__ float rounded_logit(float dot, float sqrt_d, float inv_sqrt_d, float ks, bool quantised, float mask_value) {
+  float s = bf16_round(dot);
+  const float guess = s * inv_sqrt_d;
+  s = bf16_round(fmaf(fmaf(-guess, sqrt_d, s), inv_sqrt_d, guess));
+  if (quantised) s = bf16_round(s * ks);
+  return bf16_round(s + mask_value);
+}
+
 // One element of an output row.
 __device__ __forceinline__ void store_o(const AttnArgs& a, int64_t i, float x) {
   if (a.o_f32)
@@ -62,14 +73,16 @@ struct SeqRange {
   int n, first;
 };
 
+// kL2: the bounds are read past L1 (before the kernel in front has completed: a guess, to be checked behind it).
+template <bool kL2 = false>
 __device__ __forceinline__ SeqRange seq_range(const AttnArgs& a, int b) {
   SeqRange r;
   r.first = 0;
   if (a.mask_mode == JPT_MASK_LENGTH) {
-    int e = a.end[b];
+    int e = kL2 ? __ldcg(a.end + b) : a.end[b];
     r.n = e < 0 ? 0 : (e > a.S ? a.S : e);
   } else if (a.mask_mode == JPT_MASK_RING) {
-    int st = a.start[b], en = a.end[b];
+    int st = kL2 ? __ldcg(a.start + b) : a.start[b], en = kL2 ? __ldcg(a.end + b) : a.end[b];
     st = st < 0 ? 0 : (st >= a.S ? a.S - 1 : st);
     en = en < 0 ? 0 : (en > a.S ? a.S : en);
     r.first = st;
@@ -112,6 +125,7 @@ __device__ __forceinline__ float load_scale(const void* base, int64_t idx, int i
 constexpr size_t kWorkspaceCounterBytes = 256 * 1024;
 constexpr size_t kWorkspaceStatusOffset = kWorkspaceCounterBytes - 256;
 constexpr size_t kWorkspaceExchangeOffset = 192 * 1024;
+constexpr size_t kWorkspaceTicketOffset = kWorkspaceExchangeOffset + 32;  // in the exchange state's 64 bytes, which use the first 12
 constexpr size_t kWorkspaceExchangeBytes = kWorkspaceStatusOffset - kWorkspaceExchangeOffset;
 constexpr size_t kWorkspaceMaxSegments = kWorkspaceExchangeOffset / sizeof(unsigned);  // (sequence, head) pairs
 

@@ -810,7 +810,7 @@ __global__ void __launch_bounds__(kThreads, kRows16 ? 2 : (kBf16 ? 3 : 4))
         __syncthreads();
         if (s_flag) {
           __threadfence();
-          merge_segment(a, x, mt.first_cta, mt.parts, row_base);
+          merge_segment(a, x, PartSlots{2 * mt.first_cta + 1, 2}, mt.parts, row_base);
         }
       }
       // The next iteration's barrier orders these reads before the stage is refilled.
@@ -831,6 +831,8 @@ __global__ void __launch_bounds__(kThreads, kRows16 ? 2 : (kBf16 ? 3 : 4))
 // finite entries are zero the mask itself is not needed any more.  Any other
 // row keeps the whole cache length and the additive term.
 __global__ void __launch_bounds__(kThreads) mask_ranges_kernel(AttnArgs a, MmaScratch x) {
+  grid_dependency_wait();  // the mask, and the ranges of the launch before this one, which may still read them
+  grid_dependency_trigger();
   const int b = blockIdx.x, tid = threadIdx.x;
   const __nv_bfloat16* mask = static_cast<const __nv_bfloat16*>(a.mask) + (int64_t)b * a.mk_b;
   int cnt = 0, lo = INT_MAX, hi = -1, bad_lo = INT_MAX, bad_hi = -1, nonzero = 0;
@@ -883,7 +885,7 @@ __global__ void __launch_bounds__(kThreads) mask_ranges_kernel(AttnArgs a, MmaSc
 }  // namespace
 
 int launch_mask_ranges(const AttnArgs& a, const MmaScratch& x, cudaStream_t st) {
-  mask_ranges_kernel<<<a.B, kThreads, 0, st>>>(a, x);
+  launch_after_previous(mask_ranges_kernel, dim3(a.B), dim3(kThreads), 0, st, a, x);
   return check_launch("mask_ranges_kernel");
 }
 
@@ -928,6 +930,8 @@ int launch_attention_mma(const jpt_attn_params& p, const AttnArgs& a, cudaStream
   x.part_t = reinterpret_cast<float*>(ws + lay.part_t);
   x.part_o = reinterpret_cast<float*>(ws + lay.part_o);
   x.num_ctas = lay.num_ctas;
+  x.ticket = reinterpret_cast<unsigned*>(ws + kWorkspaceTicketOffset);
+  x.early = 0;
 
   static std::atomic<bool> configured[kMaxDevices];
   if (int rc = configure_once_per_device(configured, "flash_decode_kernel", [] {

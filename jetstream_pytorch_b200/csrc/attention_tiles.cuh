@@ -23,11 +23,13 @@ constexpr float kLn2 = 0.6931471805599453f;
 struct MmaScratch {
   unsigned* counters;  // [B * Hkv] wrapping arrival counters, zero between launches
   int32_t* seqinfo;    // [B][4] (first, n, use_add, -) for additive masks
+  unsigned* ticket;    // the next item of the work list; wraps to zero by the end of the launch
   float* part_o;       // [num_ctas][2][16][128] unnormalised partial outputs
   float* part_m;       // [num_ctas][2][16] reference maximum (log2 domain)
   float* part_l;       // [num_ctas][2][16] sum of exp2(x - reference)
   float* part_t;       // [num_ctas][2][16] true maximum (log2 domain)
   int num_ctas;
+  int early;           // launched under the kernel before it (programmatic launch)
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -60,40 +62,40 @@ struct TileMeta {
   int pad[3];
 };
 
+// Where a segment's partial results lie: the first in slot `first`, piece p > 0 in slot first + 1 + (p - 1) * stride.
+struct PartSlots {
+  int first, stride;
+  __device__ __forceinline__ int of(int piece) const { return piece == 0 ? first : first + 1 + (piece - 1) * stride; }
+};
+
 // Valid range of a sequence for every mask mode (additive masks have been
 // reduced to ranges by mask_ranges_kernel).
+template <bool kL2 = false>
 __device__ __forceinline__ SeqRange seq_range_x(const AttnArgs& a, const MmaScratch& x, int b, int* use_add) {
   *use_add = 0;
   if (a.mask_mode == JPT_MASK_ADD) {
     SeqRange r;
+    if (kL2) {
+      const int4 info = __ldcg(reinterpret_cast<const int4*>(x.seqinfo) + b);
+      r.first = min(max(info.x, 0), a.S - 1);  // (scratch that no launch may have written yet)
+      r.n = min(max(info.y, 0), a.S);
+      return r;
+    }
     r.first = x.seqinfo[4 * b];
     r.n = x.seqinfo[4 * b + 1];
     *use_add = x.seqinfo[4 * b + 2];
     return r;
   }
-  return seq_range(a, b);
+  return seq_range<kL2>(a, b);
 }
 
-// Combine the `parts` partials of one segment (CTAs first .. first+parts-1) and
-// write its R final rows.  Called by 128 threads (threadIdx.x 0..127): thread t
-// owns head-dim index t of every row
-// and the rows' statistics travel by warp shuffles, so there is no staging in
-// shared memory and no barrier; two pieces are combined per step with all of
-// their loads in flight at once (one L2 round trip for the usual two pieces).
-struct NoMergeHook {
-  template <typename A>
-  __device__ __forceinline__ void operator()(A&, A&, A&) const {}
-};
-
-// `hook(M, L, acc)` runs after the pieces are combined and before the rows are
-// written: M[r] the maximum (log2 domain) and L[r] the denominator of row r
-// (equal in every thread), acc[r] this thread's head-dim component of the
-// unnormalised output.  It may change all three, the same way in every thread
-// (the tcgen05 kernel adds the decode step's new token there), and is called by
-// all 128 threads.
-template <int kR, typename Hook>
-static __device__ __forceinline__ void merge_rows(const AttnArgs& a, const MmaScratch& x, int first, int parts, int64_t row_base,
-                                                  Hook& hook) {
+// Combine the `parts` partials of one segment and write its R final rows.  Called by 128 threads
+// (threadIdx.x 0..127): thread t owns head-dim index t of every row and the rows' statistics travel by
+// warp shuffles, so there is no staging in shared memory and no barrier; `kStep` pieces are combined per
+// step with all of their loads in flight at once (four of up to 8 rows: one L2 round trip for nearly
+// every segment).
+template <int kR, int kStep>
+static __device__ __forceinline__ void merge_rows(const AttnArgs& a, const MmaScratch& x, PartSlots at, int parts, int64_t row_base) {
   const int tid = threadIdx.x, lane = tid & 31, R = a.R;
   // Lane r of every warp keeps row r's statistics (reference maximum, denominator relative to
   // it, true maximum) and hands the weights to the other lanes by shuffles.
@@ -102,67 +104,216 @@ static __device__ __forceinline__ void merge_rows(const AttnArgs& a, const MmaSc
   float acc[kR];
 #pragma unroll
   for (int r = 0; r < kR; ++r) acc[r] = 0.f;
-  for (int pi = 0; pi < parts; pi += 2) {
-    const bool two = pi + 1 < parts;
-    const int64_t i0 = ((int64_t)(first + pi) * 2 + (pi == 0 ? 1 : 0)) * kMaxRows;
-    const int64_t i1 = ((int64_t)(first + pi + 1) * 2) * kMaxRows;
-    const float m0 = mine ? __ldcg(x.part_m + i0 + lane) : -INFINITY;
-    const float l0 = mine ? __ldcg(x.part_l + i0 + lane) : 0.f;
-    const float t0 = mine ? __ldcg(x.part_t + i0 + lane) : -INFINITY;
-    const float m1 = (mine && two) ? __ldcg(x.part_m + i1 + lane) : -INFINITY;
-    const float l1 = (mine && two) ? __ldcg(x.part_l + i1 + lane) : 0.f;
-    const float t1 = (mine && two) ? __ldcg(x.part_t + i1 + lane) : -INFINITY;
-    float v0[kR], v1[kR];
+  for (int pi = 0; pi < parts; pi += kStep) {
+    float m[kStep], l[kStep], t[kStep], v[kStep][kR];
 #pragma unroll
-    for (int r = 0; r < kR; ++r) {
-      v0[r] = r < R ? __ldcg(x.part_o + (i0 + r) * kD + tid) : 0.f;
-      v1[r] = (two && r < R) ? __ldcg(x.part_o + (i1 + r) * kD + tid) : 0.f;
+    for (int z = 0; z < kStep; ++z) {
+      const bool there = pi + z < parts;
+      const int64_t i0 = (int64_t)at.of(there ? pi + z : pi) * kMaxRows;
+      m[z] = (mine && there) ? __ldcg(x.part_m + i0 + lane) : -INFINITY;
+      l[z] = (mine && there) ? __ldcg(x.part_l + i0 + lane) : 0.f;
+      t[z] = (mine && there) ? __ldcg(x.part_t + i0 + lane) : -INFINITY;
+#pragma unroll
+      for (int r = 0; r < kR; ++r) v[z][r] = (there && r < R) ? __ldcg(x.part_o + (i0 + r) * kD + tid) : 0.f;
     }
-    const float mn = fmaxf(Mr, fmaxf(m0, m1));
-    const float s = Mr == -INFINITY ? 0.f : fast_exp2(Mr - mn);
-    const float w0 = m0 == -INFINITY ? 0.f : fast_exp2(m0 - mn);
-    const float w1 = m1 == -INFINITY ? 0.f : fast_exp2(m1 - mn);
-    Lr = Lr * s + w0 * l0 + w1 * l1;
-    Mr = mn;
-    Tr = fmaxf(Tr, fmaxf(t0, t1));
+    float mn = Mr;
 #pragma unroll
-    for (int r = 0; r < kR; ++r) {
-      const float S = __shfl_sync(0xffffffffu, s, r), W0 = __shfl_sync(0xffffffffu, w0, r), W1 = __shfl_sync(0xffffffffu, w1, r);
-      acc[r] = acc[r] * S + W0 * v0[r] + W1 * v1[r];
+    for (int z = 0; z < kStep; ++z) {
+      mn = fmaxf(mn, m[z]);
+      Tr = fmaxf(Tr, t[z]);
+    }
+    const float s = Mr == -INFINITY ? 0.f : fast_exp2(Mr - mn);
+    Lr *= s;
+    Mr = mn;
+#pragma unroll
+    for (int r = 0; r < kR; ++r) acc[r] *= __shfl_sync(0xffffffffu, s, r);
+#pragma unroll
+    for (int z = 0; z < kStep; ++z) {
+      const float w = m[z] == -INFINITY ? 0.f : fast_exp2(m[z] - mn);
+      Lr = fmaf(w, l[z], Lr);
+#pragma unroll
+      for (int r = 0; r < kR; ++r) acc[r] = fmaf(__shfl_sync(0xffffffffu, w, r), v[z][r], acc[r]);
     }
   }
   // the denominator and the output relative to the true maximum, which is what gets reported
   const float c = Lr > 0.f ? fast_exp2(Mr - Tr) : 0.f;
   Lr *= c;
   Mr = Tr;
-  float M[kR], L[kR];
 #pragma unroll
   for (int r = 0; r < kR; ++r) {
-    acc[r] *= __shfl_sync(0xffffffffu, c, r);
-    M[r] = __shfl_sync(0xffffffffu, Mr, r);
-    L[r] = __shfl_sync(0xffffffffu, Lr, r);
+    const float L = __shfl_sync(0xffffffffu, Lr, r);
+    const float o = acc[r] * __shfl_sync(0xffffffffu, c, r);
+    if (r < R) store_o(a, (row_base + r) * kD + tid, L > 0.f ? o / L : 0.f);
   }
-  hook(M, L, acc);
-#pragma unroll
-  for (int r = 0; r < kR; ++r) {
-    if (r < R) {
-      if (tid == r) {
-        if (a.m) a.m[row_base + r] = M[r] * kLn2;
-        if (a.l) a.l[row_base + r] = L[r];
-      }
-      store_o(a, (row_base + r) * kD + tid, L[r] > 0.f ? acc[r] / L[r] : 0.f);
-    }
+  if (tid < R) {
+    if (a.m) a.m[row_base + tid] = Mr * kLn2;
+    if (a.l) a.l[row_base + tid] = Lr;
   }
 }
 
-template <typename Hook = NoMergeHook>
-static __device__ void merge_segment(const AttnArgs& a, const MmaScratch& x, int first, int parts, int64_t row_base,
-                                     Hook hook = Hook()) {
+static __device__ void merge_segment(const AttnArgs& a, const MmaScratch& x, PartSlots at, int parts, int64_t row_base) {
   if (a.R <= 8) {
-    merge_rows<8>(a, x, first, parts, row_base, hook);
+    merge_rows<8, 4>(a, x, at, parts, row_base);
   } else {
-    merge_rows<kMaxRows>(a, x, first, parts, row_base, hook);
+    merge_rows<kMaxRows, 2>(a, x, at, parts, row_base);
   }
+}
+
+// ------------------------------------------------------------------ the work list
+// The (sequence, KV head) segments of a launch as a list of items, longest first: a whole segment, or one of `parts`
+// equal runs of its tiles.  CTA i starts with item i and takes further ones as it finishes (one ticket counter), so
+// long segments start first and the short ones fill up the end of the launch.  Against equal contiguous shares of one
+// tile list (which cut nearly every CTA's first and last segment) far fewer segments are cut: every cut costs a
+// partial result, an arrival and a merge.
+// Sequences are sorted by their number of tiles ("bins"): a counting sort, since comparing all pairs took 3 us with the
+// 12 warps of an SM at it.
+constexpr int kPlanSeqs = 2 * kThreads;  // more sequences than this, or longer ones: equal shares
+constexpr int kPlanBins = kThreads;      // tiles of a sequence: 1 .. kPlanBins - 2
+struct __align__(16) WorkList {
+  uint16_t prefix[kPlanBins];  // items in front of the bin's first one (0xffff: the bin is empty)
+  uint8_t seq0[kPlanBins];     // the bin's first entry of `order`
+  uint8_t parts[kPlanBins];
+  uint8_t order[kPlanSeqs];    // sequences, bin by bin
+};
+struct __align__(16) PlanScratch {  // while planning only
+  uint32_t count[2][kPlanBins];     // sequences of the bin: one byte per warp, [128 of the sequences]
+  uint2 bin[kPlanBins];             // x: sort key, y: items << 16 | sequences
+};
+
+// Before the first plan_items of a launch, by all threads, with a barrier behind it.
+static __device__ __forceinline__ void plan_clear(PlanScratch& ps) {
+  ps.count[0][threadIdx.x] = 0u;
+  ps.count[1][threadIdx.x] = 0u;
+}
+__device__ __forceinline__ int ceil_div_by(int t, float inv) { return (int)(((float)t - 0.5f) * inv) + 1; }  // t >= 1, both below 2^15
+
+// All 128 threads; `tiles(b)` = tiles of sequence b, `T` takes those of this thread's sequences.  Returns the number of items of the
+// list left in `wl`, or -1 when equal shares are expected to be faster (or the list is too long to sort).  `red`: 8 ints of shared
+// memory.  The estimate is in tiles: a piece costs kPiece more, an end that is cut kCut more than that.  Among the longest pieces c
+// (32 candidates from the mean load of a CTA up to whole segments) the cheapest is taken: with at most one item per CTA
+// the longest piece, else the mean load plus one for the uneven end.  The caller's barrier publishes `wl`.
+template <typename Tiles>
+static __device__ __forceinline__ int plan_items(int B, int Hkv, int n, const Tiles& tiles, int (&T)[2], PlanScratch& ps,
+                                                 int* red, WorkList& wl, float kPiece, float kCut) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (B > kPlanSeqs) return -1;
+  const int groups = B > kThreads ? 2 : 1;
+  int nth[2] = {0, 0};  // which of its warp's sequences in the bin
+  T[0] = T[1] = 0;
+  for (int z = 0; z < groups; ++z) {
+    const int b = tid + kThreads * z;
+    T[z] = b < B ? min(tiles(b), kPlanBins - 1) : 0;
+    const unsigned same = __match_any_sync(0xffffffffu, T[z]);
+    nth[z] = __popc(same & ((1u << lane) - 1u));
+    if (nth[z] == 0) reinterpret_cast<uint8_t*>(&ps.count[z][T[z]])[warp] = (uint8_t)__popc(same);
+  }
+  if (tid < 8) red[tid] = 0;
+  __syncthreads();
+  auto in_bin = [&](int t) {
+    unsigned v = __dp4a(ps.count[0][t], 0x01010101u, 0u);
+    if (groups > 1) v = __dp4a(ps.count[1][t], 0x01010101u, v);
+    return (int)v;
+  };
+  int W = 0, segs = 0, longest = 0;
+#pragma unroll
+  for (int z = 0; z < kPlanBins / 32; ++z) {
+    const int t = lane + 32 * z, h = t > 0 ? in_bin(t) : 0;
+    W += t * h;
+    segs += h;
+    if (h > 0) longest = t;
+  }
+  W = Hkv * __reduce_add_sync(0xffffffffu, W);
+  segs = Hkv * __reduce_add_sync(0xffffffffu, segs);
+  longest = __reduce_max_sync(0xffffffffu, longest);
+  if (W == 0) return 0;
+  if (longest == kPlanBins - 1) return -1;
+  const float inv_n = 1.f / (float)n;
+  int c;
+  float cost;
+  {
+    const int c0 = min(longest, (W + n - 1) / n), step = (longest - c0) / 31 + 1;
+    const int mine = min(longest, c0 + lane * step);
+    const float rc = 1.f / (float)mine;
+    int N = 0, cut = 0;
+#pragma unroll 4
+    for (int t = 1; t <= longest; ++t) {
+      const int parts = ceil_div_by(t, rc), items = parts * in_bin(t);
+      N += items;
+      cut += parts > 1 ? items : 0;
+    }
+    N *= Hkv;
+    cut *= Hkv;
+    float e = (float)mine + kPiece + (cut ? kCut : 0.f);
+    if (N > n) {
+      e = fmaxf(e, ((float)W + kPiece * (float)N + kCut * (float)cut) * inv_n + 1.f);
+      if (cut && N > 2 * n) e = 1.0e6f;  // partial results have two slots per CTA
+    }
+    const unsigned best = __reduce_min_sync(0xffffffffu, ((unsigned)(e * 16.f) << 5) | (unsigned)lane);
+    c = min(longest, c0 + (int)(best & 31u) * step);
+    cost = (float)(best >> 5) * (1.f / 16.f);
+  }
+  // thread t: bin t; longer pieces first, then the longer sequences
+  const int h = tid > 0 ? in_bin(tid) : 0;
+  const int parts = h > 0 ? ceil_div_by(tid, 1.f / (float)c) : 0, size = h > 0 ? (tid + parts - 1) / parts : 0;
+  const uint32_t key = (uint32_t)(size << 8 | tid);
+  ps.bin[tid] = make_uint2(key, (uint32_t)(h * parts) << 16 | (uint32_t)h);
+  __syncthreads();
+  uint32_t before = 0u;  // sums of both halves: items < 2^16 (at most two a CTA, or one a sequence), sequences <= 256
+#pragma unroll 4
+  for (int t = 1; t <= longest; ++t) {
+    const uint2 o = ps.bin[t];
+    before += o.x > key ? o.y : 0u;
+  }
+  const int lo = (int)(before >> 16) * Hkv, hi = lo + h * parts * Hkv;
+  if (h > 0) {
+    // lengths of the items that share a CTA when the n longest are one to each: n - 1 and n, 2 n, 3 n
+    if (lo <= n - 1 && n - 1 < hi) red[0] = size;
+#pragma unroll
+    for (int m = 1; m < 4; ++m)
+      if (lo <= m * n && m * n < hi) red[m] = size;
+    atomicMax(&red[4], hi);
+  }
+  wl.prefix[tid] = (uint16_t)(h > 0 ? lo : 0xffff);
+  wl.seq0[tid] = (uint8_t)(before & 0xffu);  // (256 only behind the last sequence)
+  wl.parts[tid] = (uint8_t)parts;
+  __syncthreads();
+  for (int z = 0; z < groups; ++z) {
+    const int b = tid + kThreads * z;
+    if (b < B && T[z] > 0) {
+      // in the order of the sequences: those of the first group, then of the warps before, then of this warp
+      int at = wl.seq0[T[z]] + nth[z] + (int)__dp4a(ps.count[z][T[z]] & ((1u << (8 * warp)) - 1u), 0x01010101u, 0u);
+      if (z > 0) at += (int)__dp4a(ps.count[0][T[z]], 0x01010101u, 0u);
+      wl.order[at] = (uint8_t)b;
+    }
+  }
+  // n + 1 items of about one length take two rounds, whatever the mean says
+  cost = fmaxf(cost, red[1] > 0 ? (float)(red[0] + red[1]) + 2.f * kPiece : 0.f);
+  cost = fmaxf(cost, fmaxf(red[2] > 0 ? 3.f * ((float)red[2] + kPiece) : 0.f, red[3] > 0 ? 4.f * ((float)red[3] + kPiece) : 0.f));
+  const float shares = ((float)W + kPiece * (float)segs) * inv_n + kPiece + 2.f * kCut;
+  return cost <= shares ? red[4] : -1;
+}
+
+// Item k of the list, by a whole warp: sequence, head and part.
+struct WorkItem {
+  int b, h, part, parts;
+};
+static __device__ __forceinline__ WorkItem find_item(const WorkList& wl, int Hkv, int k) {
+  const int lane = threadIdx.x & 31;
+  const uint2 p = *reinterpret_cast<const uint2*>(&wl.prefix[4 * lane]);
+  const int v[4] = {(int)(p.x & 0xffffu), (int)(p.x >> 16), (int)(p.y & 0xffffu), (int)(p.y >> 16)};
+  int best = -1;  // the last bin that starts at or in front of item k
+#pragma unroll
+  for (int e = 0; e < 4; ++e)
+    if (v[e] <= k) best = max(best, v[e] << 8 | (4 * lane + e));
+  best = __reduce_max_sync(0xffffffffu, best);
+  const int t = best & 255, j = k - (best >> 8);
+  WorkItem it;
+  it.parts = wl.parts[t];
+  const int per_seq = it.parts * Hkv, s = j / per_seq, r = j - s * per_seq;
+  it.b = wl.order[wl.seq0[t] + s];
+  it.h = r / it.parts;
+  it.part = r - it.h * it.parts;
+  return it;
 }
 
 // Per-device facts are kept per device ordinal: a process may drive several GPUs.

@@ -130,6 +130,14 @@ __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepco
 __device__ __forceinline__ void grid_dependency_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 bool pdl_enabled();
+// Whether launch_after_previous() starts kernels of this stream early.  Inside a CUDA graph the launch gaps are already
+// short and the early start measured slower (59.1 against 57.0 us per decode layer); eager launches gain from it (12 %
+// end to end).
+inline bool starts_early(cudaStream_t st) {
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess) capturing = cudaStreamCaptureStatusNone;
+  return pdl_enabled() && capturing == cudaStreamCaptureStatusNone;
+}
 
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_after_previous(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
@@ -143,11 +151,7 @@ inline cudaError_t launch_after_previous(void (*kernel)(KArgs...), dim3 grid, di
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  // Inside a CUDA graph the launch gaps are already short and the early start measured slower
-  // (59.1 against 57.0 us per decode layer); eager launches gain from it (12 % end to end).
-  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess) capturing = cudaStreamCaptureStatusNone;
-  cfg.numAttrs = (pdl_enabled() && capturing == cudaStreamCaptureStatusNone) ? 1 : 0;
+  cfg.numAttrs = starts_early(st) ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
 
