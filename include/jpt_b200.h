@@ -157,6 +157,9 @@ int jpt_kv_scatter_rows(const void* src_k, const void* src_v, void* dst_k,
                         int H, int S, int D, int64_t ds_l, int64_t ds_b,
                         int64_t ds_h, int64_t ds_s, void* stream);
 
+/* `bytes` (a multiple of 16) zeroes at the 16-byte aligned p, as a kernel that starts under the one before it. */
+int jpt_zero(void* p, size_t bytes, void* stream);
+
 /*
  * `Int8KVCacheGenerate.finalize` of a lazily updated cache in one launch
  * (jetstream_pt/cache_manager.py:598-657): the kept codes new_k / new_v

@@ -150,6 +150,8 @@ __global__ void __launch_bounds__(kThreads, kRows16 ? 2 : (kBf16 ? 3 : 4))
   extern __shared__ __align__(128) uint8_t smem_raw[];
   Smem<kRows16, kBf16>& sm = *reinterpret_cast<Smem<kRows16, kBf16>*>(smem_raw);
 
+  grid_dependency_wait();
+  grid_dependency_trigger();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, c = lane & 3;
   const int R = a.R;
@@ -953,12 +955,13 @@ int launch_attention_mma(const jpt_attn_params& p, const AttnArgs& a, cudaStream
     if (int rc = launch_mask_ranges(a, x, st)) return rc;
   }
   const bool bf16 = p.kv_dtype == JPT_BF16;
+  const dim3 grid(lay.num_ctas), block(kThreads);
   if (a.R > 8) {
-    if (bf16) flash_decode_kernel<true, true><<<lay.num_ctas, kThreads, sizeof(Smem<true, true>), st>>>(a, x);
-    else flash_decode_kernel<true, false><<<lay.num_ctas, kThreads, sizeof(Smem<true, false>), st>>>(a, x);
+    if (bf16) launch_after_previous(flash_decode_kernel<true, true>, grid, block, sizeof(Smem<true, true>), st, a, x);
+    else launch_after_previous(flash_decode_kernel<true, false>, grid, block, sizeof(Smem<true, false>), st, a, x);
   } else {
-    if (bf16) flash_decode_kernel<false, true><<<lay.num_ctas, kThreads, sizeof(Smem<false, true>), st>>>(a, x);
-    else flash_decode_kernel<false, false><<<lay.num_ctas, kThreads, sizeof(Smem<false, false>), st>>>(a, x);
+    if (bf16) launch_after_previous(flash_decode_kernel<false, true>, grid, block, sizeof(Smem<false, true>), st, a, x);
+    else launch_after_previous(flash_decode_kernel<false, false>, grid, block, sizeof(Smem<false, false>), st, a, x);
   }
   return check_launch("flash_decode_kernel");
 }

@@ -259,6 +259,7 @@ __device__ __forceinline__ bool group_all(int group, bool pred) {
 // One CTA per [128 rows x 128 keys] tile of the mask: all zero, all -inf, or mixed.  Reads the mask once (the bound).
 __global__ void __launch_bounds__(256) mask_class_kernel(AttnArgs a, uint8_t* cls, int rows_per_head, int cls_heads, int vec) {
   grid_dependency_trigger();
+  grid_dependency_wait();
   const int j = blockIdx.x, tb = blockIdx.y, r = blockIdx.z % cls_heads, b = blockIdx.z / cls_heads;
   const int t0 = tb * kRowsP, s0 = j * kKeysP;
   const int nr = min(kRowsP, rows_per_head - t0), nc = min(kKeysP, a.S - s0);
@@ -1032,7 +1033,8 @@ int launch_attention_prefill(const jpt_attn_params& p, const AttnArgs& a, int64_
     uint8_t* cls = reinterpret_cast<uint8_t*>(ws + kWorkspaceCounterBytes);
     g.cls = cls;
     g.cls_rows = t.rows, g.cls_heads = t.heads, g.cls_batch = t.batch;
-    mask_class_kernel<<<dim3(t.n_k, t.rows, t.heads * t.batch), 256, 0, st>>>(a, cls, p.mk_r ? p.Tq : 1, t.heads, g.mask_vec);
+    launch_after_previous(mask_class_kernel, dim3(t.n_k, t.rows, t.heads * t.batch), dim3(256), 0, st, a, cls, (int)(p.mk_r ? p.Tq : 1),
+                          (int)t.heads, (int)g.mask_vec);
     if (int rc = check_launch("mask_class_kernel")) return rc;
   }
   const dim3 grid(g.pairs * p.B * p.Hkv), block(kThreadsP);

@@ -126,6 +126,8 @@ __global__ void __launch_bounds__(kEndThreads) engine_end_kernel(const T* logits
 // The rows of one slot after an insert: mask (0 on the prefix's positions, -inf elsewhere), token, start, length, count.
 __global__ void engine_slot_kernel(MaskRef mask, int S, int slot, int pos, int cur, int wrap, int start_value, int seq_len,
                                    int32_t* start, int32_t* input_pos, int32_t* lens, int32_t* tokens, const void* token, int token_bytes) {
+  grid_dependency_wait();
+  grid_dependency_trigger();
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < S && mask.p; s += gridDim.x * blockDim.x) {
     const bool in = !wrap ? s >= pos && s < cur : cur > pos ? s >= pos && s < cur : s >= pos || s < cur;
     mask_put(mask, slot, s, in ? 0.f : -INFINITY);
@@ -171,13 +173,15 @@ extern "C" int jpt_engine_end(const void* logits, int dtype, int64_t row_stride,
   cfg.gridDim = dim3(kEndCtas, B);
   cfg.blockDim = dim3(kEndThreads);
   cfg.stream = static_cast<cudaStream_t>(stream);
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = kEndCtas;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = starts_early(cfg.stream) ? 2 : 1;
   const cudaError_t e =
       dtype == JPT_F32
           ? cudaLaunchKernelEx(&cfg, engine_end_kernel<float>, static_cast<const float*>(logits), row_stride, V, vec, tokens, lens,
@@ -196,7 +200,7 @@ extern "C" int jpt_engine_insert_slot(void* mask, int mask_dtype, int64_t mask_s
   JPT_REQUIRE(!tokens || (token && (token_bytes == 4 || token_bytes == 8)), JPT_EINVAL, "engine_insert_slot: the token must be int32 or int64");
   const MaskRef m{mask, mask_dtype == JPT_F32, mask_stride};
   const int blocks = mask ? (S + 255) / 256 : 1;
-  engine_slot_kernel<<<blocks > 148 ? 148 : blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      m, S, slot, pos, cur, wrap, start_value, seq_len, start, input_pos, lens, tokens, token, token_bytes);
+  launch_after_previous(engine_slot_kernel, dim3(blocks > 148 ? 148 : blocks), dim3(256), 0, static_cast<cudaStream_t>(stream), m, S, slot, pos,
+                        cur, wrap, start_value, seq_len, start, input_pos, lens, tokens, token, token_bytes);
   return check_launch("engine_slot_kernel");
 }

@@ -751,7 +751,7 @@ PyObject* finalize_int8(Args a, Py_ssize_t n) {
 }
 
 // kept_token(cache_k [NL,B,H,S,D], scale dtype of a tensor) -> zeroed new_k, new_v [NL,B,H,1,D] int8 and new_ks, new_vs [NL,B,1,1,1]:
-// one allocation and one memset for the four
+// one allocation and one launch for the four
 PyObject* kept_token(Args a, Py_ssize_t n) {
   expect(n, 2, "kept_token");
   const Tensor& ck = tensor(a[0]);
@@ -762,8 +762,7 @@ PyObject* kept_token(Args a, Py_ssize_t n) {
   const ScalarType st = f32 ? ScalarType::Float : ScalarType::BFloat16;
   const int64_t rows = (nl * b * h * d + 255) / 256 * 256, es = f32 ? 4 : 2, scales = (nl * b * es + 255) / 256 * 256;
   Tensor all = empty({2 * rows + 2 * scales}, ScalarType::Char, dev);
-  const cudaError_t e = cudaMemsetAsync(all.data_ptr(), 0, (size_t)all.numel(), stream_of(dev));
-  if (e != cudaSuccess) fail(PyExc_RuntimeError, "clearing the kept token: %s", cudaGetErrorString(e));
+  check(jpt_zero(all.data_ptr(), (size_t)all.numel(), stream_of(dev)));
   auto part = [&](int64_t byte, at::IntArrayRef sizes, ScalarType type, int64_t bytes_each) {
     Tensor t = empty({0}, type, dev);
     t.set_(all.storage(), byte / bytes_each, sizes, {});

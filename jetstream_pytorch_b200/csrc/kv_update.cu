@@ -298,6 +298,8 @@ struct ScatterArgs {
 
 // `more`: a second set of rows in the same launch (blockIdx.y 2, 3): the scales that go with the rows of a lazy finalize.
 __global__ void scatter_rows_kernel(const __grid_constant__ ScatterArgs first, const __grid_constant__ ScatterArgs more) {
+  grid_dependency_wait();
+  grid_dependency_trigger();
   const ScatterArgs& a = blockIdx.y < 2 ? first : more;
   const int chunks_per_row = a.row_bytes / a.chunk;
   const int64_t total = (int64_t)a.NL * a.B * a.H * chunks_per_row;
@@ -346,6 +348,8 @@ struct PagedCopyArgs {
 };
 
 __global__ void paged_append_copy_kernel(PagedCopyArgs a) {
+  grid_dependency_wait();
+  grid_dependency_trigger();
   const int chunks_per_row = a.row_bytes / a.chunk;
   const int n_act = a.n_active_dev ? *a.n_active_dev : a.n_active;
   const int64_t total = (int64_t)n_act * a.H * chunks_per_row;
@@ -380,6 +384,8 @@ __global__ void paged_append_copy_kernel(PagedCopyArgs a) {
 __global__ void page_token_indices_kernel(const int32_t* lens, const int32_t* page_indices, int B,
                                           int max_pages, int ps, int32_t* pti, int32_t* n_active,
                                           int32_t* new_lengths) {
+  grid_dependency_wait();
+  grid_dependency_trigger();
   __shared__ int s_warp[33];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int len = tid < B ? lens[tid] : 0;
@@ -544,7 +550,7 @@ static int launch_scatter(const ScatterArgs& a, const ScatterArgs* more, cudaStr
   int64_t total = (int64_t)a.NL * a.B * a.H * (a.row_bytes / a.chunk);
   if (more) total = std::max(total, (int64_t)more->NL * more->B * more->H * (more->row_bytes / more->chunk));
   int blocks = (int)std::min<int64_t>((total + 255) / 256, 148 * 16);
-  scatter_rows_kernel<<<dim3(blocks, more ? 4 : a.src[1] ? 2 : 1), 256, 0, st>>>(a, more ? *more : a);
+  launch_after_previous(scatter_rows_kernel, dim3(blocks, more ? 4 : a.src[1] ? 2 : 1), dim3(256), 0, st, a, more ? *more : a);
   return check_launch("scatter_rows_kernel");
 }
 
@@ -557,6 +563,24 @@ extern "C" int jpt_kv_scatter_rows(const void* src_k, const void* src_v, void* d
                             ds_h, ds_s))
     return rc;
   return launch_scatter(a, nullptr, static_cast<cudaStream_t>(stream));
+}
+
+// Zeroes in the chain of early starts: a memset in a decode step holds back the launch behind it until it is complete, and starts itself only
+// when everything in front is (about 3 us of a step).
+static __global__ void __launch_bounds__(256) zero_kernel(uint4* p, int64_t n) {
+  grid_dependency_wait();
+  grid_dependency_trigger();
+  for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) p[i] = make_uint4(0u, 0u, 0u, 0u);
+}
+
+extern "C" int jpt_zero(void* p, size_t bytes, void* stream) {
+  JPT_REQUIRE(p || bytes == 0, JPT_EINVAL, "zero: null pointer");
+  JPT_REQUIRE(aligned(p, 16) && bytes % 16 == 0, JPT_EALIGN, "zero: 16-byte units");
+  if (bytes == 0) return 0;
+  const int64_t n = (int64_t)(bytes / 16);
+  launch_after_previous(zero_kernel, dim3((unsigned)std::min<int64_t>((n + 255) / 256, 148 * 8)), dim3(256), 0, static_cast<cudaStream_t>(stream),
+                        static_cast<uint4*>(p), n);
+  return check_launch("zero_kernel");
 }
 
 extern "C" int jpt_kv_finalize_int8(const int8_t* new_k, const int8_t* new_v, int8_t* cache_k, int8_t* cache_v, const void* new_ks,
@@ -598,7 +622,7 @@ extern "C" int jpt_kv_append_paged(const void* xk, const void* xv, int in_dtype,
     const int64_t total = (int64_t)n_active * H * (a.row_bytes / a.chunk);
     int blocks = (int)((total + 255) / 256);
     if (blocks > 148 * 16) blocks = 148 * 16;
-    paged_append_copy_kernel<<<dim3(blocks, 2), 256, 0, st>>>(a);
+    launch_after_previous(paged_append_copy_kernel, dim3(blocks, 2), dim3(256), 0, st, a);
     return check_launch("paged_append_copy_kernel");
   }
   JPT_REQUIRE(cache_dtype == JPT_INT8 && (in_dtype == JPT_BF16 || in_dtype == JPT_F32), JPT_EINVAL,
@@ -623,8 +647,8 @@ extern "C" int jpt_page_token_indices(const int32_t* lens, const int32_t* page_i
   JPT_REQUIRE(B > 0 && B <= 1024 && max_pages > 0 && ps > 0, JPT_ERANGE,
               "page_token_indices: need 0 < B <= 1024");
   const int threads = ((B + 31) / 32) * 32;
-  page_token_indices_kernel<<<1, threads, 0, static_cast<cudaStream_t>(stream)>>>(
-      lens, page_indices, B, max_pages, ps, pti, n_active, new_lengths);
+  launch_after_previous(page_token_indices_kernel, dim3(1), dim3(threads), 0, static_cast<cudaStream_t>(stream), lens, page_indices, B,
+                        max_pages, ps, pti, n_active, new_lengths);
   return check_launch("page_token_indices_kernel");
 }
 

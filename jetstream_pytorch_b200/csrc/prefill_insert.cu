@@ -84,6 +84,8 @@ __device__ __forceinline__ void load_vec(const T* p, float (&v)[VEC]) {
 // grid (Ltot, 2, NL); one block per token of one tensor of one layer.
 template <typename T, int VEC, int NV>
 __global__ void __launch_bounds__(256) insert_quant_kernel(const __grid_constant__ InsertArgs a) {
+  grid_dependency_wait();
+  grid_dependency_trigger();
   __shared__ float red[33];
   const int t = blockIdx.x, which = blockIdx.y, l = blockIdx.z;
   const int HD = a.H * a.D;
@@ -150,6 +152,8 @@ __global__ void __launch_bounds__(256) insert_quant_kernel(const __grid_constant
 // when H*D is a multiple of 512.
 template <typename T, int NVW>
 __global__ void __launch_bounds__(256) insert_quant_warp_kernel(const __grid_constant__ InsertArgs a) {
+  grid_dependency_wait();
+  grid_dependency_trigger();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = blockIdx.x * 8 + warp, which = blockIdx.y, l = blockIdx.z;
   if (t >= a.Ltot) return;
@@ -253,6 +257,8 @@ __global__ void __launch_bounds__(256) insert_quant_warp_kernel(const __grid_con
 
 // Same-dtype copy: one thread per chunk of `chunk` bytes.
 __global__ void insert_copy_kernel(const __grid_constant__ InsertArgs a, int elem_bytes, int chunk) {
+  grid_dependency_wait();
+  grid_dependency_trigger();
   const int which = blockIdx.y, l = blockIdx.z;
   const int row_bytes = a.D * elem_bytes;
   const int cpr = row_bytes / chunk;
@@ -300,22 +306,22 @@ int launch_quant(const InsertArgs& a, cudaStream_t st) {
   dim3 grid(a.Ltot, a.ntensors, a.NL);
   if (vec_ok && (HD == 512 || HD == 1024 || HD == 2048)) {
     const dim3 wgrid((a.Ltot + 7) / 8, a.ntensors, a.NL);
-    if (HD == 512) insert_quant_warp_kernel<T, 1><<<wgrid, 256, 0, st>>>(a);
-    else if (HD == 1024) insert_quant_warp_kernel<T, 2><<<wgrid, 256, 0, st>>>(a);
-    else insert_quant_warp_kernel<T, 4><<<wgrid, 256, 0, st>>>(a);
+    if (HD == 512) launch_after_previous(insert_quant_warp_kernel<T, 1>, wgrid, dim3(256), 0, st, a);
+    else if (HD == 1024) launch_after_previous(insert_quant_warp_kernel<T, 2>, wgrid, dim3(256), 0, st, a);
+    else launch_after_previous(insert_quant_warp_kernel<T, 4>, wgrid, dim3(256), 0, st, a);
     return check_launch("insert_quant_warp_kernel");
   }
   if (vec_ok && HD <= 16 * 256 * 2) {
     const int nvec = HD / 16;
     if (nvec <= 256) {
-      insert_quant_kernel<T, 16, 1><<<grid, ((nvec + 31) / 32) * 32, 0, st>>>(a);
+      launch_after_previous(insert_quant_kernel<T, 16, 1>, grid, dim3(((nvec + 31) / 32) * 32), 0, st, a);
     } else {
-      insert_quant_kernel<T, 16, 2><<<grid, 256, 0, st>>>(a);
+      launch_after_previous(insert_quant_kernel<T, 16, 2>, grid, dim3(256), 0, st, a);
     }
   } else {
     JPT_REQUIRE(HD <= 256 * 32, JPT_ERANGE, "prefill_insert: H*D = %d too large for the scalar path", HD);
     const int threads = HD < 256 ? ((HD + 31) / 32) * 32 : 256;
-    insert_quant_kernel<T, 1, 32><<<grid, threads, 0, st>>>(a);
+    launch_after_previous(insert_quant_kernel<T, 1, 32>, grid, dim3(threads), 0, st, a);
   }
   return check_launch("insert_quant_kernel");
 }
@@ -340,7 +346,7 @@ int launch_layers(InsertArgs& a, int in_dtype, int cache_dtype, cudaStream_t st)
   const int64_t total = (int64_t)a.Ltot * a.H * (row_bytes / chunk);
   int blocks = (int)((total + 255) / 256);
   if (blocks > 148 * 8) blocks = 148 * 8;
-  insert_copy_kernel<<<dim3(blocks, a.ntensors, a.NL), 256, 0, st>>>(a, eb, chunk);
+  launch_after_previous(insert_copy_kernel, dim3(blocks, a.ntensors, a.NL), dim3(256), 0, st, a, eb, chunk);
   return check_launch("insert_copy_kernel");
 }
 

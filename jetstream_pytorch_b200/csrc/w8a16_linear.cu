@@ -183,6 +183,7 @@ __global__ void __launch_bounds__(256) x_levels_kernel(const __nv_bfloat16* x, i
   __shared__ float red[33];
   const int m = blockIdx.x, tid = threadIdx.x;  // one CTA per row of the padded batch
   grid_dependency_trigger();
+  grid_dependency_wait();
   if (m == 0 && tid == 0 && clear_status) *status = 0;
   if (m == 0 && tid == 0 && launch_counter) *launch_counter += 1u;  // (one thread, launches in stream order)
   uint2* hrow = reinterpret_cast<uint2*>(lev + (int64_t)(m + m / Mp * Mp) * K);
@@ -1314,8 +1315,8 @@ int launch_gemm(const LevelsView& lv, const void* w, const void* w_scale, void* 
 // (the level kernel also clears the status word and the padding rows of the level matrix)
 int launch_levels(const void* x, const LevelsView& lv, int M, int K, cudaStream_t st, bool clear_status,
                   unsigned* launch_counter = nullptr) {
-  x_levels_kernel<<<lv.Mp, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(x), lv.lev, lv.xs, lv.status, M, lv.Mp, K,
-                                         clear_status ? 1 : 0, launch_counter);
+  launch_after_previous(x_levels_kernel, dim3(lv.Mp), dim3(256), 0, st, static_cast<const __nv_bfloat16*>(x), lv.lev, lv.xs, lv.status, M,
+                        lv.Mp, K, clear_status ? 1 : 0, launch_counter);
   return check_launch("x_levels_kernel");
 }
 
@@ -1331,7 +1332,8 @@ int launch_tiles(const void* x, const void* w0, const void* s0, const void* w1, 
   lv.lev = reinterpret_cast<int8_t*>(ws + 256);
   lv.xs = reinterpret_cast<float*>(ws + 256 + ((size_t)2 * rows * K + 255) / 256 * 256);
   lv.Mp = rb.Rb;
-  x_levels_kernel<<<rows, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(x), lv.lev, lv.xs, lv.status, M, rb.Rb, K, 1, nullptr);
+  launch_after_previous(x_levels_kernel, dim3(rows), dim3(256), 0, st, static_cast<const __nv_bfloat16*>(x), lv.lev, lv.xs, lv.status, M, rb.Rb,
+                        K, 1, static_cast<unsigned*>(nullptr));
   if (int rc = check_launch("x_levels_kernel")) return rc;
   TileMaps maps;
   memset(&maps, 0, sizeof(maps));
