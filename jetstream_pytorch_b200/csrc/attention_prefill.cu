@@ -6,7 +6,8 @@
 //
 // Work item of a CTA: two tiles of 128 query rows of one KV head ("a" and "b": two grouped query heads at the same
 // token block where the model groups heads, two consecutive token blocks otherwise), so that a K/V tile read from L2
-// serves 256 rows and the tensor core works on one tile while the other one's 256 threads do their softmax.  Tiles are
+// serves 256 rows and the tensor core works on one tile while the other one's 256 threads do their softmax (grids of one wave: see
+// row_tile).  Tiles are
 // made per query head through a tensor map with the caller's strides: a transposed view of the projection needs no copy.
 // Items with the most K/V tiles under a causal mask start first.
 //
@@ -77,10 +78,24 @@ struct PrefillGeom {
   int n_rows_t;        // row blocks of 128 per query head
   int n_k;             // K/V tiles
   int pairs;           // items per KV head
+  int fold;            // how row tiles make items: see row_tile
   int cls_rows, cls_heads, cls_batch;  // extents of the class table (1 where the mask broadcasts)
   int mask_vec, mask_pairs;  // mask rows can be read 16, 4 bytes at a time
   int64_t q_b, q_h, q_t;     // strides of the queries
 };
+
+// Row tile t (0: a, 1: b) of item `item` of a KV head: token block index / rep, grouped query head index % rep.  Under a causal mask a
+// tile has as many K/V tiles as blocks up to its own.
+// Folded: the longest with the shortest, the second longest with the second shortest, ..., so that every item has about
+// as much work; for grids of one wave, whose time is that of the longest item (1024 tokens, 32 / 8 heads: 42.6 -> 41.0 us
+// with the mask classes; a step of one tile alone takes nearly as long as one of two).  Else neighbours, the longest
+// items first, which fill up the end of several waves: items of one length would take whole waves.
+__device__ __forceinline__ int row_tile(const PrefillGeom& g, int rep, int item, int t, bool* have) {
+  const int tiles = g.n_rows_t * rep;
+  const int idx = g.fold ? (t == 0 ? tiles - 1 - item : item) : 2 * (g.pairs - 1 - item) + t;
+  *have = g.fold ? t == 0 || item < tiles - 1 - item : idx < tiles;
+  return idx;
+}
 
 __device__ __forceinline__ uint32_t smem_u32p(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init_p(uint64_t* bar, uint32_t count) {
@@ -396,7 +411,8 @@ __device__ __noinline__ void plain_rows(const AttnArgs& a, const PrefillGeom& g,
   constexpr int kKeys = 4, kDims = 32;  // at a time
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = warp >> 3, half = (warp >> 2) & 1;
   const int rep = a.Hq / a.Hkv, heads = a.B * a.Hkv, bh = (int)blockIdx.x % heads, b = bh / a.Hkv, hkv = bh % a.Hkv;
-  const int idx = 2 * (g.pairs - 1 - (int)blockIdx.x / heads) + t, hq = hkv * rep + idx % rep;
+  bool have;
+  const int idx = row_tile(g, rep, (int)blockIdx.x / heads, t, &have), hq = hkv * rep + idx % rep;
   const int token = min(idx / rep * kRowsP + (warp & 3) * 32 + lane, a.Tq - 1);
   // (all tiles of the item are done: the rings are free.  The query rows read once a key from global memory, a line per lane,
   // were most of the time.)
@@ -496,15 +512,13 @@ __global__ void __launch_bounds__(kThreadsP, 1)
   }
   const int rep = a.Hq / a.Hkv;
   const int heads = a.B * a.Hkv;
-  const int pair = g.pairs - 1 - (int)blockIdx.x / heads;  // (the last token blocks, with the most K/V tiles, first)
   const int bh = (int)blockIdx.x % heads, b = bh / a.Hkv, hkv = bh % a.Hkv;
   // the item's row tiles: query head and token block of a and b
   int hq[2], tb[2];
   bool have[2];
 #pragma unroll
   for (int t = 0; t < 2; ++t) {
-    const int idx = 2 * pair + t;
-    have[t] = idx < g.n_rows_t * rep;
+    const int idx = row_tile(g, rep, (int)blockIdx.x / heads, t, &have[t]);
     tb[t] = idx / rep;
     hq[t] = hkv * rep + idx % rep;
   }
@@ -1026,6 +1040,7 @@ int launch_attention_prefill(const jpt_attn_params& p, const AttnArgs& a, int64_
   g.n_rows_t = (p.Tq + kRowsP - 1) / kRowsP;
   g.n_k = t.n_k;
   g.pairs = (g.n_rows_t * (p.Hq / p.Hkv) + 1) / 2;
+  g.fold = g.pairs * p.B * p.Hkv <= sm_count();
   g.q_b = q_b, g.q_h = q_h, g.q_t = q_t;
   g.mask_vec = p.mask_mode == JPT_MASK_ADD && aligned(p.mask, 16) && p.mk_b % 8 == 0 && p.mk_r % 8 == 0;
   g.mask_pairs = p.mask_mode == JPT_MASK_ADD && aligned(p.mask, 4) && p.mk_b % 2 == 0 && p.mk_r % 2 == 0 && p.Tq * p.mk_r % 2 == 0;

@@ -64,6 +64,7 @@ def _mask(kind, rep, t, s, g):
     (1, 4, 1, 520, 520, "random", True),      # mixed tiles everywhere, a row without a single key
     (2, 8, 2, 70, 600, "broadcast", True),    # one mask row for all
     (1, 40, 1, 1, 512, "none", False),        # many grouped heads, one token
+    (10, 10, 10, 650, 650, "causal", True),   # more items than SMs, an odd number of row tiles of a head: neighbours share an item
 ])
 @pytest.mark.parametrize("scales", ["none", "ones", "random", "random_f32"])
 def test_dense_attention_matches_the_reference(b, hq, hkv, t, s, kind, transposed, scales):
