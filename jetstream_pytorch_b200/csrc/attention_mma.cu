@@ -321,6 +321,7 @@ __global__ void __launch_bounds__(kThreads, kRows16 ? 2 : (kBf16 ? 3 : 4))
   int pend_stage = -1;
   bool first_issue = true;
 
+  const uint64_t policy = evict_first_policy();
   auto issue_tile = [&](int stage) {
     const int j0 = pt * kTile;
     const bool piece_start = first_issue || pt == 0;
@@ -349,8 +350,8 @@ __global__ void __launch_bounds__(kThreads, kRows16 ? 2 : (kBf16 ? 3 : 4))
       const int8_t* vp = vseg + off * kES;
 #pragma unroll
       for (int i = 0; i < Geo::kPasses; ++i) {
-        cp_async16(kdst + 2048 * i, kp + 2048 * i, true);
-        cp_async16(vdst + 2048 * i, vp + 2048 * i, true);
+        cp_async16(kdst + 2048 * i, kp + 2048 * i, true, policy);
+        cp_async16(vdst + 2048 * i, vp + 2048 * i, true, policy);
       }
     } else {
 #pragma unroll
@@ -370,8 +371,8 @@ __global__ void __launch_bounds__(kThreads, kRows16 ? 2 : (kBf16 ? 3 : 4))
         } else {
           off = (int64_t)pos * kv_s32;
         }
-        cp_async16(kdst + 2048 * i, kseg + off * kES, valid);
-        cp_async16(vdst + 2048 * i, vseg + off * kES, valid);
+        cp_async16(kdst + 2048 * i, kseg + off * kES, valid, policy);
+        cp_async16(vdst + 2048 * i, vseg + off * kES, valid, policy);
       }
     }
     if (piece_start) {

@@ -332,15 +332,8 @@ __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-// L2 policy of the cache rows: read once per step, they leave first and do not push out what the launches share (their
-// instructions, page tables, lengths, the weights of the layers around them).  With the default policy the launches met their own code
-// in DRAM again: two layers of 96 sequences, 8 KV heads, 116.3 -> 108.4 us, paged 112.4 -> 106.8.
-__device__ __forceinline__ uint64_t evict_first_policy() {
-  uint64_t p;
-  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
-  return p;
-}
-// One box of a 4-d tensor map (128 bytes x rows x 1 x 1) into swizzled shared memory of this CTA.
+// One box of a 4-d tensor map (128 bytes x rows x 1 x 1) into swizzled shared memory of this CTA.  (evict_first_policy: with the default
+// one the launches met their own code in DRAM again: two layers of 96 sequences, 8 KV heads, 116.3 -> 108.4 us, paged 112.4 -> 106.8.)
 __device__ __forceinline__ void tma_load_rows(uint32_t dst, const CUtensorMap* map, int row, int c2, int c3, uint32_t bar, uint64_t policy) {
   asm volatile(
       "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3, %4, %5}], [%6], %7;" ::"r"(dst),
