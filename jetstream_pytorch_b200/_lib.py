@@ -94,6 +94,7 @@ _SIGNATURES = {
                                         + [c_void_p, c_void_p]),
     "jpt_kv_scatter_rows": (c_int, [c_void_p] * 4 + [c_int, c_void_p, c_int, c_int, c_int]
                             + [c_int] * 5 + [c_i64] * 4 + [c_void_p]),
+    "jpt_zero": (c_int, [c_void_p, c_size_t, c_void_p]),
     "jpt_kv_finalize_int8": (c_int, [c_void_p] * 8 + [c_int, c_void_p] + [c_int] * 7 + [c_i64] * 7 + [c_void_p]),
     "jpt_kv_append_paged": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
                                     c_void_p, c_i64, c_int, c_void_p] + [c_int] * 5 + [c_void_p]),
