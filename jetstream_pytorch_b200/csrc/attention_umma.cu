@@ -46,8 +46,8 @@
 // the levels of a token are one 16-byte store (16 byte stores before), page ids are looked up a
 // round ahead (the scales' addresses waited 4000 cycles a round for them), a piece's rows leave
 // with the next round's logits, and segments are not cut where they need not be.
-// B200, per launch: 96 sequences of 8 KV heads, 1 .. 2047 tokens, with the new token: 57 -> 50 us;
-// paged, 512 .. 2047 tokens: 58 -> 49.
+// B200, 96 sequences of 8 KV heads, a step of two layers with these changes and the row's L2 policy: 1 .. 2047 tokens with the
+// new token 129.7 -> 108.2 us; paged, 512 .. 2047 tokens, 131.3 -> 106.3.
 //
 // Fused decode update (jpt_decode_update_attend): the launch also takes the
 // step's new K/V token, which becomes the last token of its segment: the
