@@ -10,7 +10,7 @@
 //
 // "Levels" make the small operands 8-bit without losing the precision of the
 // bf16 / fp32 values they stand for:
-//   * a query row q (bf16) is split as q = s (h + l / 254) with s = amax|q| / 127.49
+//   * a query row q (bf16) is split as q = s (h + l / 254) with s = amax|q| / 127 (values of the row's amax are exact)
 //     and h, l signed bytes; rows 0..7 of Ql hold h, rows 8..15 hold l, so the
 //     two partial dot products of a token arrive in the same TMEM lane and
 //     S = s (S_h + S_l / 254) is exact to 2^-16 of the row's amax;
@@ -1148,7 +1148,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
       for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(f[e]));
 #pragma unroll
       for (int sh = 1; sh <= 8; sh <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, sh));
-      const float inv = amax > 0.f ? 127.49f / amax : 0.f;  // (rounds to 127: the whole range of both bytes)
+      const float inv = amax > 0.f ? 127.f / amax : 0.f;
       uint32_t hi[2] = {0u, 0u}, lo[2] = {0u, 0u};
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
@@ -1161,8 +1161,8 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
       *reinterpret_cast<uint2*>(&sm.qlev[swz(row, 8 * ch)]) = make_uint2(hi[0], hi[1]);
       *reinterpret_cast<uint2*>(&sm.qlev[swz(8 + row, 8 * ch)]) = make_uint2(lo[0], lo[1]);
       if (ch == 0) {
-        sm.qsc[row] = amax * (1.f / 127.49f) * unit2 * (1.f / 254.f);
-        if constexpr (kRound) sm.qsr[row] = amax * (1.f / 127.49f) * (1.f / 254.f);
+        sm.qsc[row] = amax * (1.f / 127.f) * unit2 * (1.f / 254.f);
+        if constexpr (kRound) sm.qsr[row] = amax * (1.f / 127.f) * (1.f / 254.f);
       }
       fence_async_smem();
       tc_fence_before();
@@ -1212,11 +1212,10 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
     for (int r = 1; r < kR; ++r) M = lane == r ? m_run[r] : M;
     if (!(M > 0.5f * kNoMax)) M = -INFINITY;  // every logit of the row was masked
     if (is_final) {
-      const float inv = L > 0.f ? __frcp_rn(L) : 0.f;
 #pragma unroll
       for (int r = 0; r < kR; ++r) {
-        const float c = __shfl_sync(0xffffffffu, inv, r);
-        if (r < R) store_o(a, (row_base + r) * kD + tid, c > 0.f ? o[r] * c : 0.f);
+        const float den = __shfl_sync(0xffffffffu, L, r);
+        if (r < R) store_o(a, (row_base + r) * kD + tid, den > 0.f ? o[r] / den : 0.f);
       }
       if (tid < R) {
         if (a.m) a.m[row_base + tid] = M * kLn2;

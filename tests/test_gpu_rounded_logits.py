@@ -1,0 +1,63 @@
+"""The logit chain of dense_attention on bf16 tensors (dot product, / sqrt(D), * K scale, + mask, each rounded to bf16) in the int8
+decode kernel, read from the row maximum of sequences of one token: bit for bit where the dot product is exact in float32."""
+
+import math
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda"
+D, ROWS = 128, 8
+
+
+def _row_maxima(x, codes, sm_scale=1.0 / math.sqrt(D)):
+  """x [B, 8]: query rows of one value each; codes [B, 128] int8: the token of each sequence.  The logits as the kernel has them."""
+  from jetstream_pytorch_b200 import _lib
+  from jetstream_pytorch_b200 import attention_kernel as ak
+
+  b = x.shape[0]
+  q = x[:, :, None, None].expand(b, ROWS, 1, D).contiguous().to(DEV)
+  k = codes.reshape(b, 1, 1, D).to(DEV)
+  one = torch.ones(b, 1, 1, 1, dtype=torch.bfloat16, device=DEV)
+  _, m, _ = ak._flash_decode(q, k, k, k_scale=one, v_scale=one, scale_strides=(1, 1), mask_mode=_lib.MASK_LENGTH,
+                             end=torch.ones(b, dtype=torch.int32), sm_scale=sm_scale, kv_strides=(D, D, D), n_kv_heads=1, seq=1,
+                             logit_rounding=True)
+  return m.reshape(b, ROWS).to(torch.bfloat16).cpu()  # (held as a base-2 logarithm: back within 3e-7)
+
+
+def _codes_of_sum(total, rng):
+  """128 codes of the given sum: equal ones, then pairs moved against each other."""
+  c = np.full(D, total // D)
+  c[: total - c.sum()] += 1
+  move = rng.integers(0, 127 - c.max() + 1, D // 2)
+  c[0::2] += move
+  c[1::2] -= move
+  return c
+
+
+def test_exact_dot_products_next_to_a_tie_are_rounded_as_the_reference_rounds_them():
+  # x m-th of 128 .. 255, codes of sum t: the product m t (below 2^22, exact in float32) lies above a tie of its bf16 rounding by 1e-6 ..
+  # 8e-6 of itself: more than float32 loses on the way (four roundings: 2.4e-7), less than query levels that do not hold the
+  # row's amax exactly.
+  rng = np.random.default_rng(5)
+  m = np.arange(128, 256)
+  xs, codes = [], []
+  while len(xs) < 64:
+    t = int(rng.integers(2000, 12000))
+    p = (m * t).astype(np.int64)
+    ulp = 1 << (np.floor(np.log2(p)).astype(np.int64) - 7)
+    over = p % ulp - ulp // 2
+    near = m[(over > 1e-6 * p) & (over < 8e-6 * p)]
+    if near.size:
+      xs.append(rng.choice(near, ROWS))
+      codes.append(_codes_of_sum(t, rng))
+  x = torch.from_numpy(np.stack(xs)).to(torch.bfloat16)
+  c = torch.from_numpy(np.stack(codes))
+  assert c.abs().max() <= 127
+  dot = (x.float() * c.sum(1, keepdim=True)).to(torch.bfloat16)
+  want = (dot.float() / math.sqrt(D)).to(torch.bfloat16)
+  got = _row_maxima(x, c.to(torch.int8))
+  assert torch.equal(got, want), f"{int((got != want).sum())} of {want.numel()} logits differ"
