@@ -1351,6 +1351,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
     }
     const int info_next = i >= -1 ? info_of(i + 1) : 0;
     if (info_next & kRoundValid) issue_k(i + 1, info_next);
+    else cp_async_commit();  // (an empty group: behind it the V rows of this round are never the youngest group, see below)
     publish(i + 2);
     if constexpr (kFused) {
       if (peers && i == -1) post_amax();
@@ -1418,8 +1419,8 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
           if constexpr (kTma) {
             if (!mbar_wait(smem_u32(&sm.bar_v[half]), half ? (info & kRoundParB ? 1u : 0u) : par)) dead = true;
           } else {
-            cp_async_wait<1>();
-            __syncthreads();  // every thread's copies into this tile have landed
+            cp_async_wait<1>();  // (the younger group: that of the next round's K rows)
+            __syncthreads();     // every thread's copies into this tile have landed
           }
           sm.v[half][swz((half ? rows_b(info) : rows_a(info)) - 1, tid)] = sm.ntv[tid];
         }

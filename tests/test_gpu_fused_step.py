@@ -196,3 +196,31 @@ def test_fused_step_state_survives_other_shapes_on_the_workspace():
     ak.ragged_mha(q3, k3, k3, 0, torch.zeros(3, dtype=torch.int32, device=DEV),
                   torch.full((3,), 1024, dtype=torch.int32, device=DEV), None, None, None, None)
   assert ak.kernel_status() == 0
+
+
+@pytest.mark.parametrize("lazy", [False, True])
+@pytest.mark.parametrize("hkv", [1, 8])
+def test_fused_step_token_in_the_only_or_last_round(hkv, lazy):
+  """Segments that end with the new token in the only or the last 128-token tile and 256-token round of a CTA.  The token has nearly all of
+  the weight, and the cache row at its place (a row of another sequence's past) holds other codes: they must not be attended to."""
+  from jetstream_pytorch_b200 import attention_kernel as ak
+  from jetstream_pytorch_b200.cache_manager import Int8KVCacheGenerate
+
+  existing = torch.tensor([0, 1, 126, 127, 128, 129, 254, 255, 256, 257, 383, 384, 511, 512, 513])
+  b, hq, s, d = len(existing), 4 * hkv, 640, 128
+  g = torch.Generator().manual_seed(407 + hkv)
+  ck, cv = (torch.randint(-127, 128, (b, hkv, s, d), generator=g, dtype=torch.int8) for _ in range(2))
+  ks, vs = (torch.full((b, 1, s, 1), 0.01, dtype=torch.bfloat16) for _ in range(2))
+  q = torch.randn(b, hq, 1, d, generator=g).to(torch.bfloat16)
+  xk = (3 * q.reshape(b, hkv, 4, d).float().mean(2, keepdim=True)).to(torch.bfloat16)
+  xv = torch.randn(b, hkv, 1, d, generator=g).to(torch.bfloat16)
+  env = make_env(batch_size=b, cache_sequence_length=s, ring_buffer=False, lazy_cache_update=lazy)
+  dev = lambda x: x.to(DEV)
+  e = oc.int8_update(ck, cv, ks, vs, xk, xv, existing, ring_buffer=False, lazy=False)
+  eo, _ = oa.ragged_mha(q, e[0], e[1], 0, torch.zeros(b), existing + 1, e[4], e[5], bk=128)
+  for _ in range(20):
+    c = Int8KVCacheGenerate(dev(ck).clone(), dev(cv).clone(), dev(ks).clone(), dev(vs).clone(), dev(existing), env=env)
+    r, (o, _, _) = c.update_and_attend(dev(q), dev(xk), dev(xv), 0, torch.zeros(b, dtype=torch.int32, device=DEV), dev(existing))
+    assert attention_close(o, eo), describe(o, eo)
+    assert torch.equal(c.cache_v.cpu(), cv if lazy else e[1])
+  assert ak.kernel_status() == 0
