@@ -1248,6 +1248,22 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
     }
   };
 
+  // A wait ran out: reported, and the requests of the copy engine that may still be in flight get their (bounded) time: the V rows of
+  // round i, the K rows of the one behind it (`next`: its record's bits, 0 where there is none).
+  auto give_up = [&](int i, int next) {
+    if (tid != 0) return;
+    atomicExch(status, 1);
+    if constexpr (kTma) {
+      auto landed = [&](uint64_t (&bar)[2], int round, int bits) {
+        if (!(bits & kRoundValid)) return;
+        mbar_wait(smem_u32(&bar[0]), (uint32_t)round & 1u);
+        if (rows_b(bits) > 0) mbar_wait(smem_u32(&bar[1]), bits & kRoundParB ? 1u : 0u);
+      };
+      landed(sm.bar_k, i + 1, next);
+      landed(sm.bar_v, i, i >= 0 ? sm.meta[i & 3].info : 0);
+    }
+  };
+
   // The tensor core works one step ahead of the threads: S^T of round i+1 is issued in iteration i, and O^T of round i is
   // collected in iteration i+1, in the same trip to tensor memory as the logits of round i+1 (a piece that ended with round i
   // leaves there), so neither MMA is waited for right after it was issued.
@@ -1291,7 +1307,10 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
       tmem_ld16(tmem_lane, s0);
       tmem_ld16(tmem_lane + 16, s1);
       tmem_ld_wait();
-      if (!more) break;
+      if (!more) {  // what ran out since the last round's barrier: its V rows, its output
+        if (__syncthreads_or(dead)) give_up(i - 1, 0);
+        break;
+      }
     }
     if (info & kRoundStarts) {
 #pragma unroll
@@ -1431,19 +1450,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
     fence_async_smem();
     tc_fence_before();
     if (__syncthreads_or(dead)) {
-      if (tid == 0) {
-        atomicExch(status, 1);
-        if constexpr (kTma) {  // requests of the copy engine that may still be in flight get their (bounded) time
-          if (info_next & kRoundValid) {
-            mbar_wait(smem_u32(&sm.bar_k[0]), (uint32_t)(i + 1) & 1u);
-            if (rows_b(info_next) > 0) mbar_wait(smem_u32(&sm.bar_k[1]), info_next & kRoundParB ? 1u : 0u);
-          }
-          if (filled) {
-            mbar_wait(smem_u32(&sm.bar_v[0]), par);
-            if (rows_b(info) > 0) mbar_wait(smem_u32(&sm.bar_v[1]), info & kRoundParB ? 1u : 0u);
-          }
-        }
-      }
+      give_up(i, info_next);
       if (listed && items > n_ctas && warp == kWalkerWarp && lane == 0 && pmore) {  // the ticket comes round to zero all the same
         if (pt + 2 < pt_end) ticket = atomicInc(x.ticket, (unsigned)items - 1u);
         for (int z = 0; z < items && n_ctas + (int)ticket < items; ++z) ticket = atomicInc(x.ticket, (unsigned)items - 1u);
