@@ -81,11 +81,10 @@ __device__ __forceinline__ void load_vec(const T* p, float (&v)[VEC]) {
   }
 }
 
-// grid (Ltot, 2, NL); one block per token of one tensor of one layer.
+// grid (Ltot, 2, NL); one block per token of one tensor of one layer.  An ordinary launch: with an early start each of its many CTAs of a
+// microsecond waited and triggered first (1900 tokens, 32 layers, 1 or 2 KV heads: 138.5 us, 75.4 without; 64 tokens: 22.9 and 23.7).
 template <typename T, int VEC, int NV>
 __global__ void __launch_bounds__(256) insert_quant_kernel(const __grid_constant__ InsertArgs a) {
-  grid_dependency_wait();
-  grid_dependency_trigger();
   __shared__ float red[33];
   const int t = blockIdx.x, which = blockIdx.y, l = blockIdx.z;
   const int HD = a.H * a.D;
@@ -314,14 +313,14 @@ int launch_quant(const InsertArgs& a, cudaStream_t st) {
   if (vec_ok && HD <= 16 * 256 * 2) {
     const int nvec = HD / 16;
     if (nvec <= 256) {
-      launch_after_previous(insert_quant_kernel<T, 16, 1>, grid, dim3(((nvec + 31) / 32) * 32), 0, st, a);
+      insert_quant_kernel<T, 16, 1><<<grid, ((nvec + 31) / 32) * 32, 0, st>>>(a);
     } else {
-      launch_after_previous(insert_quant_kernel<T, 16, 2>, grid, dim3(256), 0, st, a);
+      insert_quant_kernel<T, 16, 2><<<grid, 256, 0, st>>>(a);
     }
   } else {
     JPT_REQUIRE(HD <= 256 * 32, JPT_ERANGE, "prefill_insert: H*D = %d too large for the scalar path", HD);
     const int threads = HD < 256 ? ((HD + 31) / 32) * 32 : 256;
-    launch_after_previous(insert_quant_kernel<T, 1, 32>, grid, dim3(threads), 0, st, a);
+    insert_quant_kernel<T, 1, 32><<<grid, threads, 0, st>>>(a);
   }
   return check_launch("insert_quant_kernel");
 }

@@ -96,6 +96,31 @@ def test_inserts_of_scattered_layers(nl, quant, paged):
     assert torch.equal(x[0], y[0]) and torch.equal(x[1], y[1])
 
 
+def test_inserts_of_narrow_prefixes_take_no_longer_than_wide_ones():
+  """A prefix of 1 or 2 KV heads has an eighth or a quarter of the bytes of one of 8 and about its time (1.1 of it: a CTA per token); 1.5 leaves
+  room for the clock.  (With a wait at the start of each of those CTAs it was 2.2.)"""
+  from jetstream_pytorch_b200 import _lib
+
+  def best_time(h, n=1900, nl=32):
+    prefix = [tuple(torch.randn(1, n, h, 128, device=DEV, dtype=torch.bfloat16).transpose(1, 2) for _ in range(2)) for _ in range(nl)]
+    caches = [tuple(torch.zeros(1, h, 2048, 128, dtype=torch.int8, device=DEV) for _ in range(2)) for _ in range(nl)]
+    scales = [tuple(torch.ones(1, 1, 2048, 1, dtype=torch.bfloat16, device=DEV) for _ in range(2)) for _ in range(nl)]
+    times = []
+    for _ in range(8):
+      a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+      a.record()
+      for _ in range(20):
+        assert _lib.native.insert_dense(prefix, caches, scales, 0, 0, False, False)
+      b.record()
+      b.synchronize()
+      times.append(a.elapsed_time(b))
+    return min(times)
+
+  wide = best_time(8)
+  for h in (1, 2):
+    assert best_time(h) < 1.5 * wide
+
+
 @pytest.mark.parametrize("b,hq,hkv,d,dt", [(1, 4, 1, 128, torch.bfloat16), (3, 8, 8, 128, torch.bfloat16), (2, 6, 3, 20, torch.float32)])
 @pytest.mark.parametrize("int8", [False, True])
 def test_lazy_token_joins_the_cache(b, hq, hkv, d, dt, int8):
