@@ -48,13 +48,15 @@ __device__ __forceinline__ float rounded_logit(float dot, float sqrt_d, float ks
   return bf16_round(s + mask_value);
 }
 
-// The same with the reciprocal of sqrt_d (rounded to nearest) at hand: the quotient's first guess and one correction by the exact
-// remainder give the correctly rounded quotient (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000
-// processor", 1990) in three instructions.
+// The same with the reciprocal of sqrt_d (rounded to nearest) at hand: the quotient's first guess and one correction by its
+// remainder (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", 1990), three
+// instructions and the test for a quotient that has none because it is infinite.  After the rounding to bf16 it is the division's for every
+// bf16 mantissa and the scales of the tests; a quotient below the normal range may differ in its last place.
 __device__ __forceinline__ float rounded_logit(float dot, float sqrt_d, float inv_sqrt_d, float ks, bool quantised, float mask_value) {
   float s = bf16_round(dot);
   const float guess = s * inv_sqrt_d;
-  s = bf16_round(fmaf(fmaf(-guess, sqrt_d, s), inv_sqrt_d, guess));
+  const float corrected = fmaf(fmaf(-guess, sqrt_d, s), inv_sqrt_d, guess);
+  s = bf16_round(fabsf(guess) < INFINITY ? corrected : guess);
   if (quantised) s = bf16_round(s * ks);
   return bf16_round(s + mask_value);
 }

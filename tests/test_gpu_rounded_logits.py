@@ -61,3 +61,32 @@ def test_exact_dot_products_next_to_a_tie_are_rounded_as_the_reference_rounds_th
   want = (dot.float() / math.sqrt(D)).to(torch.bfloat16)
   got = _row_maxima(x, c.to(torch.int8))
   assert torch.equal(got, want), f"{int((got != want).sum())} of {want.numel()} logits differ"
+
+
+@pytest.mark.parametrize("sm_scale", [1.0 / math.sqrt(D), 1.0 / math.sqrt(96), 1.0 / math.sqrt(160), 0.3, 1.0, 1.7, 3e-3])
+def test_the_quotient_is_the_division(sm_scale):
+  """Every bf16 mantissa at exponents over the range where the quotient is a normal number, both signs."""
+  m = torch.arange(128, 256, dtype=torch.float64)
+  exponents = torch.tensor([-100, -31, -9, -8, -7, -1, 0, 3, 30, 60], dtype=torch.float64)
+  x = (m[None, :] * 2.0 ** exponents[:, None]).to(torch.bfloat16).reshape(-1, ROWS)
+  x[::3] *= -1
+  codes = torch.zeros(x.shape[0], D, dtype=torch.int8)
+  codes[:, 5] = 1  # the dot product is x itself
+  by = np.float32(1) / np.float32(sm_scale)
+  want = torch.from_numpy(x.float().numpy() / by).to(torch.bfloat16)
+  got = _row_maxima(x, codes, sm_scale)
+  assert torch.equal(got, want), f"{int((got != want).sum())} of {want.numel()} logits differ"
+
+
+def test_a_dot_product_beyond_the_range_is_a_logit_of_minus_infinity():
+  """Two tokens, one with a dot product below -3.4e38: it has no weight, and the row is the other token's."""
+  from jetstream_pytorch_b200 import attention_kernel as ak
+
+  q = torch.full((1, 4, 1, D), 3e38, dtype=torch.bfloat16, device=DEV)
+  k = torch.zeros(1, 1, 2, D, dtype=torch.int8, device=DEV)
+  k[0, 0, 0] = -127
+  v = torch.randint(-127, 128, (1, 1, 2, D), dtype=torch.int8, device=DEV)
+  one = torch.ones(1, 1, 2, 1, dtype=torch.bfloat16, device=DEV)
+  mask = torch.zeros(1, 1, 1, 2, dtype=torch.bfloat16, device=DEV)
+  out = ak.dense_attention(q, k, v, one, one, mask)
+  assert torch.equal(out, v[:, :, 1:].to(torch.bfloat16).expand(1, 4, 1, D))
