@@ -1307,6 +1307,10 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
       tmem_ld16(tmem_lane, s0);
       tmem_ld16(tmem_lane + 16, s1);
       tmem_ld_wait();
+      if (rows_b(info) == 0) {  // no second tile: what its columns held before could be beyond what a masked logit may be (infinite)
+#pragma unroll
+        for (int r = 0; r < 16; ++r) s1[r] = 0u;
+      }
       if (!more) {  // what ran out since the last round's barrier: its V rows, its output
         if (__syncthreads_or(dead)) give_up(i - 1, 0);
         break;

@@ -78,15 +78,25 @@ def test_the_quotient_is_the_division(sm_scale):
   assert torch.equal(got, want), f"{int((got != want).sum())} of {want.numel()} logits differ"
 
 
-def test_a_dot_product_beyond_the_range_is_a_logit_of_minus_infinity():
-  """Two tokens, one with a dot product below -3.4e38: it has no weight, and the row is the other token's."""
+@pytest.mark.parametrize("rounded", [True, False])
+def test_a_dot_product_beyond_the_range_is_a_logit_of_minus_infinity(rounded):
+  """Two tokens, one with a dot product below -3.4e38: it has no weight, and the row is the other token's, whatever the launches before left
+  where a second tile's sums would be."""
   from jetstream_pytorch_b200 import attention_kernel as ak
 
-  q = torch.full((1, 4, 1, D), 3e38, dtype=torch.bfloat16, device=DEV)
-  k = torch.zeros(1, 1, 2, D, dtype=torch.int8, device=DEV)
-  k[0, 0, 0] = -127
-  v = torch.randint(-127, 128, (1, 1, 2, D), dtype=torch.int8, device=DEV)
-  one = torch.ones(1, 1, 2, 1, dtype=torch.bfloat16, device=DEV)
-  mask = torch.zeros(1, 1, 1, 2, dtype=torch.bfloat16, device=DEV)
-  out = ak.dense_attention(q, k, v, one, one, mask)
-  assert torch.equal(out, v[:, :, 1:].to(torch.bfloat16).expand(1, 4, 1, D))
+  one = torch.ones(1, 1, 512, 1, dtype=torch.bfloat16, device=DEV)
+  for turn in range(3):
+    k = torch.zeros(1, 1, 2, D, dtype=torch.int8, device=DEV)
+    k[0, 0, 0] = -127
+    v = torch.randint(-127, 128, (1, 1, 2, D), dtype=torch.int8, device=DEV)
+    q = torch.full((1, 4, 1, D), 3e38, dtype=torch.bfloat16, device=DEV)
+    if rounded:
+      out = ak.dense_attention(q, k, v, one[:, :, :2], one[:, :, :2], torch.zeros(1, 1, 1, 2, dtype=torch.bfloat16, device=DEV))
+    else:
+      out = ak.ragged_mha(q, k, v, 0, None, torch.full((1,), 2, dtype=torch.int32, device=DEV), None, None, one[:, :, :2], one[:, :, :2])[0]
+    assert torch.equal(out.reshape(4, D), v[0, 0, 1:].to(torch.bfloat16).expand(4, D)), turn
+    # sums of full tiles in every column of every SM
+    full = torch.full((64, 8, 512, D), 127, dtype=torch.int8, device=DEV)
+    ones = one.expand(64, 1, 512, 1).contiguous()
+    ak.ragged_mha(torch.ones(64, 64, 1, D, dtype=torch.bfloat16, device=DEV), full, full, 0, None,
+                  torch.full((64,), 512, dtype=torch.int32, device=DEV), None, None, ones, ones)
