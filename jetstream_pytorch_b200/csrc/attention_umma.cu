@@ -1055,7 +1055,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
   const bool sc_f32 = a.scale_is_f32 != 0;
   const uint32_t raw_one = sc_f32 ? 0x3f800000u : 0x3f80u;
   auto scale_of = [&](uint32_t raw) { return __uint_as_float(sc_f32 ? raw : raw << 16); };
-  uint32_t nks[2] = {raw_one, raw_one}, nvs[2] = {0u, 0u};
+  uint32_t nks[2] = {0u, 0u}, nvs[2] = {0u, 0u};
   auto issue_k = [&](int seq, int info) {
     const RoundRec& m = sm.meta[seq & 3];
     const int mb = m.b;
@@ -1064,11 +1064,11 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
       for (int ch = tid; ch < R * 16; ch += kThreads) cp_async16(smem_u32(&sm.qraw[0]) + ch * 16, q + ch * 8, true);
     }
     if (!kTma || warp == kWalkerWarp) fetch_rows(seq, info, sm.k, kbase, &maps.k, sm.bar_k);
-    // (a tile that is not there: no rows)
+    // (a tile that is not there: no rows.  Where there is no token the scales are zero: a stale row's product, or the second tile's columns
+    // of tensor memory from before, could be infinite, and minus infinity added to that is no mask.)
     const bool in_a = tid < rows_a(info), in_b = tid < rows_b(info);
-    nks[0] = nks[1] = raw_one;
-    nvs[0] = in_a ? raw_one : 0u;
-    nvs[1] = in_b ? raw_one : 0u;
+    nks[0] = nvs[0] = in_a ? raw_one : 0u;
+    nks[1] = nvs[1] = in_b ? raw_one : 0u;
     if (quant) {
       int64_t at[2];
       if (a.paged) {
@@ -1212,10 +1212,12 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
     for (int r = 1; r < kR; ++r) M = lane == r ? m_run[r] : M;
     if (!(M > 0.5f * kNoMax)) M = -INFINITY;  // every logit of the row was masked
     if (is_final) {
+      // (times the reciprocal: 1e-7 of a row at most, beside 4e-5 from the levels; divisions, or a correction by the remainder, cost 1 % of a step)
+      const float inv = L > 0.f ? __frcp_rn(L) : 0.f;
 #pragma unroll
       for (int r = 0; r < kR; ++r) {
-        const float den = __shfl_sync(0xffffffffu, L, r);
-        if (r < R) store_o(a, (row_base + r) * kD + tid, den > 0.f ? o[r] / den : 0.f);
+        const float c = __shfl_sync(0xffffffffu, inv, r);
+        if (r < R) store_o(a, (row_base + r) * kD + tid, c > 0.f ? o[r] * c : 0.f);
       }
       if (tid < R) {
         if (a.m) a.m[row_base + tid] = M * kLn2;
@@ -1248,22 +1250,6 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
     }
   };
 
-  // A wait ran out: reported, and the requests of the copy engine that may still be in flight get their (bounded) time: the V rows of
-  // round i, the K rows of the one behind it (`next`: its record's bits, 0 where there is none).
-  auto give_up = [&](int i, int next) {
-    if (tid != 0) return;
-    atomicExch(status, 1);
-    if constexpr (kTma) {
-      auto landed = [&](uint64_t (&bar)[2], int round, int bits) {
-        if (!(bits & kRoundValid)) return;
-        mbar_wait(smem_u32(&bar[0]), (uint32_t)round & 1u);
-        if (rows_b(bits) > 0) mbar_wait(smem_u32(&bar[1]), bits & kRoundParB ? 1u : 0u);
-      };
-      landed(sm.bar_k, i + 1, next);
-      landed(sm.bar_v, i, i >= 0 ? sm.meta[i & 3].info : 0);
-    }
-  };
-
   // The tensor core works one step ahead of the threads: S^T of round i+1 is issued in iteration i, and O^T of round i is
   // collected in iteration i+1, in the same trip to tensor memory as the logits of round i+1 (a piece that ended with round i
   // leaves there), so neither MMA is waited for right after it was issued.
@@ -1277,8 +1263,9 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
   for (int r = 0; r < 8; ++r) m_run[r] = l_run[r] = o[r] = alpha[r] = beta[r] = 0.f;
   int info = 0;   // of the round at hand; what is needed less often is read from its record
   bool ended = false;  // the round before ended a piece
+  int i = -2, info_next = 0;
 #pragma unroll 1
-  for (int i = -2;; ++i) {
+  for (;; ++i) {
     const bool more = (info & kRoundValid) != 0, filled = i >= 0 && more;
     const bool pending = i > 0;  // O^T of the round before has not been added yet
     const RoundRec& mt = sm.meta[i & 3];
@@ -1307,14 +1294,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
       tmem_ld16(tmem_lane, s0);
       tmem_ld16(tmem_lane + 16, s1);
       tmem_ld_wait();
-      if (rows_b(info) == 0) {  // no second tile: what its columns held before could be beyond what a masked logit may be (infinite)
-#pragma unroll
-        for (int r = 0; r < 16; ++r) s1[r] = 0u;
-      }
-      if (!more) {  // what ran out since the last round's barrier: its V rows, its output
-        if (__syncthreads_or(dead)) give_up(i - 1, 0);
-        break;
-      }
+      if (!more) break;
     }
     if (info & kRoundStarts) {
 #pragma unroll
@@ -1347,12 +1327,13 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
 #pragma unroll
       for (int r = 0; r < kR; ++r) xv[r] = 0ull;
     } else {
-      // a row past the tile's tokens: finite dot product + (-inf)
-      float mk[2] = {tid < rows_a(info) ? 0.f : -INFINITY, tid < rows_b(info) ? 0.f : -INFINITY};
+      // a row past the tile's tokens: product with a scale of 0, + (-inf)
+      const bool in_a = tid < rows_a(info), in_b = tid < rows_b(info);
+      float mk[2] = {in_a ? 0.f : -INFINITY, in_b ? 0.f : -INFINITY};
       if (info & kRoundAdd) {  // additive mask that is not a plain 0 / -inf range (rare)
         const __nv_bfloat16* mrow = mask + (int64_t)mt.b * a.mk_b + tid;
-        if (mk[0] == 0.f) mk[0] = __bfloat162float(mrow[mt.pos[0]]);
-        if (mk[1] == 0.f) mk[1] = __bfloat162float(mrow[mt.pos[1]]);
+        if (in_a) mk[0] = __bfloat162float(mrow[mt.pos[0]]);
+        if (in_b) mk[1] = __bfloat162float(mrow[mt.pos[1]]);
       }
       if constexpr (!kRound) {
         const f32x2 ks = pack2(cks[0], cks[1]), ml = pack2(mk[0] * kLog2e, mk[1] * kLog2e);
@@ -1367,12 +1348,13 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
 #pragma unroll
         for (int r = 0; r < kR; ++r) {
           const float qr = sm.qsr[r];
-          xv[r] = pack2(kLog2e * rounded_logit((float)((int)s0[r] * 254 + (int)s0[8 + r]) * qr, sqrt_d, inv_sqrt_d, cks[0], quant, mk[0]),
-                        kLog2e * rounded_logit((float)((int)s1[r] * 254 + (int)s1[8 + r]) * qr, sqrt_d, inv_sqrt_d, cks[1], quant, mk[1]));
+          const float x0 = rounded_logit((float)((int)s0[r] * 254 + (int)s0[8 + r]) * qr, sqrt_d, inv_sqrt_d, cks[0], quant, mk[0]);
+          const float x1 = rounded_logit((float)((int)s1[r] * 254 + (int)s1[8 + r]) * qr, sqrt_d, inv_sqrt_d, cks[1], quant, mk[1]);
+          xv[r] = pack2(in_a ? kLog2e * x0 : -INFINITY, in_b ? kLog2e * x1 : -INFINITY);
         }
       }
     }
-    const int info_next = i >= -1 ? info_of(i + 1) : 0;
+    info_next = i >= -1 ? info_of(i + 1) : 0;
     if (info_next & kRoundValid) issue_k(i + 1, info_next);
     else cp_async_commit();  // (an empty group: behind it the V rows of this round are never the youngest group, see below)
     publish(i + 2);
@@ -1453,14 +1435,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
     cp_async_wait<0>();  // the query rows and the new token of round i+1 (without the copy engine also its K rows and V of this one)
     fence_async_smem();
     tc_fence_before();
-    if (__syncthreads_or(dead)) {
-      give_up(i, info_next);
-      if (listed && items > n_ctas && warp == kWalkerWarp && lane == 0 && pmore) {  // the ticket comes round to zero all the same
-        if (pt + 2 < pt_end) ticket = atomicInc(x.ticket, (unsigned)items - 1u);
-        for (int z = 0; z < items && n_ctas + (int)ticket < items; ++z) ticket = atomicInc(x.ticket, (unsigned)items - 1u);
-      }
-      break;
-    }
+    if (__syncthreads_or(dead)) break;
     if (i < -1) continue;
     if (i == -1 && (info_next & kRoundValid)) issue_v(0, info_next);  // behind the first query and K rows
 
@@ -1511,7 +1486,28 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
   exchange_done();
   cp_async_wait<0>();
   tc_fence_before();
-  __syncthreads();
+  // A wait ran out, in front of a round's barrier or behind that of the last one (its V rows, its output): reported; the requests of the
+  // copy engine that may still be in flight get their (bounded) time, the ticket comes round to zero all the same.
+  if (__syncthreads_or(dead)) {
+    if (tid == 0) {
+      atomicExch(status, 1);
+      if constexpr (kTma) {
+        auto landed = [&](uint64_t (&bar)[2], int round, int bits) {
+          if (!(bits & kRoundValid)) return;
+          mbar_wait(smem_u32(&bar[0]), (uint32_t)round & 1u);
+          if (rows_b(bits) > 0) mbar_wait(smem_u32(&bar[1]), bits & kRoundParB ? 1u : 0u);
+        };
+        const int round = (info & kRoundValid) ? i : i - 1;  // the last one whose V rows were requested
+        landed(sm.bar_k, i + 1, info_next);
+        landed(sm.bar_v, round, round >= 0 ? sm.meta[round & 3].info : 0);
+      }
+    }
+    if (listed && items > n_ctas && warp == kWalkerWarp && lane == 0 && pmore) {
+      if (pt + 2 < pt_end) ticket = atomicInc(x.ticket, (unsigned)items - 1u);
+      for (int z = 0; z < items && n_ctas + (int)ticket < items; ++z) ticket = atomicInc(x.ticket, (unsigned)items - 1u);
+    }
+    __syncthreads();
+  }
   if (warp == 1) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)kTmemCols) : "memory");
   }
