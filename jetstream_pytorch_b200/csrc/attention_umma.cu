@@ -15,11 +15,11 @@
 //     two partial dot products of a token arrive in the same TMEM lane and
 //     S = s (S_h + S_l / 254) is exact to 2^-16 of the row's amax;
 //   * a probability p in [0, 1] (relative to the maximum of its round), times the
-//     token's V scale relative to the largest V scale of the round, becomes a
+//     token's V scale relative to the largest V scale c of its tile, becomes a
 //     16-bit fixed-point number whose two bytes are the unsigned levels of the
-//     token's row of Pl; O = (O_0 + 2^8 O_1) c / (2^16 - 1): an error of 2^-17 of the
-//     round's largest term per token, far below the bf16 rounding of the result.
-// Every int32 sum is exact (|sum| <= 256 * 128 * 65535), so the only roundings
+//     token's row of Pl; O = (O_0 + 2^8 O_1) c / (2^16 - 1), a sum of its own for each tile: an error of
+//     2^-17 c per token and unit of its V code, far below the bf16 rounding of the result.
+// Every int32 sum is exact (|sum| <= 128 * 128 * 65535), so the only roundings
 // are the two splits above and the fp32 online-softmax arithmetic.
 //
 // A tile is 128 consecutive valid tokens of one (sequence, KV head) segment, a
@@ -81,7 +81,7 @@ namespace jpt {
 namespace {
 
 constexpr int kTileU = 128;     // tokens per tile = TMEM lanes = threads per CTA
-constexpr int kTmemCols = 64;   // S^T of the two tiles of a round: columns 0..15 and 16..31, O^T: columns 32..47
+constexpr int kTmemCols = 64;   // S^T of the two tiles of a round: columns 0..15 and 16..31, their O^T: columns 32..47 and 48..63
 constexpr int kColO = 32;
 constexpr int kCtasPerSm = 3;
 #ifndef JPT_PIECE_COST_U
@@ -123,7 +123,7 @@ struct __align__(1024) SmemU {
   unsigned long long ntw[2][8];          // ... the ranks' amax words (K, V) as they were when the round was prepared
                                          //     (one GPU: floats, the K and V maxima of the warps)
   int ntpos;                             // ... and where the token is written
-  alignas(16) float xch[4][12];          // per warp: row maxima of the round [8], largest V scale [1]
+  alignas(16) float xch[4][12];          // per warp: row maxima of the round [8], largest V scale of each tile [2]
   float red[4][8];                       // per warp: denominators at the end of a piece
   alignas(16) float qsc[8];              // s_r * sm_scale * log2(e) / 254
   float qsr[8];                          // s_r / 254 (the chain of rounded logits starts from the plain dot product)
@@ -1258,7 +1258,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
   // Iterations -2 and -1 only fill the pipeline: the code of a round exists once.  The first ones, which all CTAs of an SM work on
   // at the same time and behind a burst of row requests, do not fetch it twice.
   if (listed && warp == kWalkerWarp) open_item(cta);
-  float alpha[8], beta[8], cmax = 0.f;
+  float alpha[8], beta[8], cmax[2] = {0.f, 0.f};  // (cmax: the largest V scale of each tile of the round)
 #pragma unroll
   for (int r = 0; r < 8; ++r) m_run[r] = l_run[r] = o[r] = alpha[r] = beta[r] = 0.f;
   int info = 0;   // of the round at hand; what is needed less often is read from its record
@@ -1278,15 +1278,18 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
       if (filled && !mbar_wait(bar_s, par)) dead = true;
       if (pending && !mbar_wait(bar_o, par ^ 1u)) dead = true;
       tc_fence_after();
-      uint32_t o01[16];
-      tmem_ld16(tmem_lane + kColO, o01);  // (in iteration 0 there is none yet: not looked at)
+      uint32_t oa[16], ob[16];
+      tmem_ld16(tmem_lane + kColO, oa);  // (in iteration 0 there is none yet: not looked at)
+      tmem_ld16(tmem_lane + kColO + 16, ob);
       tmem_ld_wait();
       if (pending) {
-        const float oscale = cmax * (1.f / 65535.f);
+        const float ca = cmax[0] * (1.f / 65535.f), cb = cmax[1] * (1.f / 65535.f);  // (0 for a tile that is not there: its columns hold an earlier sum)
 #pragma unroll
-        for (int r = 0; r < kR; r += 2) {  // the two levels combine exactly in int32 (|O_0 + 256 O_1| <= 256 * 128 * 65535 < 2^31)
-          const f32x2 f = pack2((float)((int)o01[r] + ((int)o01[8 + r] << 8)), (float)((int)o01[r + 1] + ((int)o01[9 + r] << 8)));
-          unpack2(fma2(pack2(o[r], o[r + 1]), pack2(alpha[r], alpha[r + 1]), mul2(f, mul2(pack2(oscale, oscale), pack2(beta[r], beta[r + 1])))), o[r], o[r + 1]);
+        for (int r = 0; r < kR; r += 2) {  // the two levels combine exactly in int32 (|O_0 + 256 O_1| <= 128 * 128 * 65535 < 2^31)
+          const f32x2 fa = pack2((float)((int)oa[r] + ((int)oa[8 + r] << 8)), (float)((int)oa[r + 1] + ((int)oa[9 + r] << 8)));
+          const f32x2 fb = pack2((float)((int)ob[r] + ((int)ob[8 + r] << 8)), (float)((int)ob[r + 1] + ((int)ob[9 + r] << 8)));
+          const f32x2 f = fma2(fb, pack2(cb, cb), mul2(fa, pack2(ca, ca)));
+          unpack2(fma2(pack2(o[r], o[r + 1]), pack2(alpha[r], alpha[r + 1]), mul2(f, pack2(beta[r], beta[r + 1]))), o[r], o[r + 1]);
         }
       }
       if (ended) flush(sm.meta[(i - 1) & 3]);
@@ -1362,27 +1365,31 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
       if (peers && i == -1) post_amax();
     }
     if (i >= -1) {  // (once without a round, while the first rows travel: the first round then finds its instructions at hand)
-      // maxima per row (and the largest V scale) across the 256 tokens
+      // maxima per row across the 256 tokens, and the largest V scale of each tile
       {
-        float wm[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        float wm[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int r = 0; r < kR; ++r) {
           float lo, hi;
           unpack2(xv[r], lo, hi);
           wm[r] = warp_max(fmaxf(lo, hi));
         }
-        wm[8] = warp_max(fmaxf(cvs[0], cvs[1]));
+        const float ca = warp_max(cvs[0]), cb = warp_max(cvs[1]);
         if (lane == 0) {
           *reinterpret_cast<float4*>(&sm.xch[warp][0]) = make_float4(wm[0], wm[1], wm[2], wm[3]);
           if (kR > 4) *reinterpret_cast<float4*>(&sm.xch[warp][4]) = make_float4(wm[4], wm[5], wm[6], wm[7]);
-          sm.xch[warp][8] = wm[8];
+          *reinterpret_cast<float2*>(&sm.xch[warp][8]) = make_float2(ca, cb);
         }
       }
       tc_fence_before();
       __syncthreads();
 
       {
-        cmax = fmaxf(fmaxf(sm.xch[0][8], sm.xch[1][8]), fmaxf(sm.xch[2][8], sm.xch[3][8]));
+        float2 c[4];
+#pragma unroll
+        for (int w = 0; w < 4; ++w) c[w] = *reinterpret_cast<const float2*>(&sm.xch[w][8]);
+        cmax[0] = fmaxf(fmaxf(c[0].x, c[1].x), fmaxf(c[2].x, c[3].x));
+        cmax[1] = fmaxf(fmaxf(c[0].y, c[1].y), fmaxf(c[2].y, c[3].y));
         float tm[8];
 #pragma unroll
         for (int g = 0; g < (kR > 4 ? 2 : 1); ++g) {
@@ -1395,8 +1402,8 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
           tm[4 * g + 3] = fmaxf(fmaxf(t[0].w, t[1].w), fmaxf(t[2].w, t[3].w));
         }
         // p <= 1 and the product is held at 2^16 - 1 (the fast division may land one ulp above)
-        const float rc = cmax > 0.f ? __fdividef(65535.f, cmax) : 0.f;
-        const float ps0 = fminf(cvs[0] * rc, 65535.f), ps1 = fminf(cvs[1] * rc, 65535.f);
+        const float ps0 = cmax[0] > 0.f ? fminf(cvs[0] * __fdividef(65535.f, cmax[0]), 65535.f) : 0.f;
+        const float ps1 = cmax[1] > 0.f ? fminf(cvs[1] * __fdividef(65535.f, cmax[1]), 65535.f) : 0.f;
         softmax_rows<kR>(m_run, l_run, alpha, beta, tm, xv, ps0, ps1, p_addr);
       }
       if (info & kRoundEnds) {
@@ -1454,7 +1461,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
         for (int ks = 0; ks < 4; ++ks) umma_i8(tmem + kColO, va + (uint64_t)(256 * ks), pa + (uint64_t)(32 * ks), kIdescO, ks > 0);
         if (rows_b(info) > 0) {
 #pragma unroll
-          for (int ks = 0; ks < 4; ++ks) umma_i8(tmem + kColO, vb + (uint64_t)(256 * ks), pc + (uint64_t)(32 * ks), kIdescO, 1u);
+          for (int ks = 0; ks < 4; ++ks) umma_i8(tmem + kColO + 16, vb + (uint64_t)(256 * ks), pc + (uint64_t)(32 * ks), kIdescO, ks > 0);
         }
         umma_commit(bar_o);
       }
