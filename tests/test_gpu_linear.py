@@ -187,3 +187,43 @@ def test_levels_from_the_producers_equal_the_layer_s_own_split():
     err = (got.float() - ol.w8a16_linear(xin, wq, sc).float()).abs().double()
     assert (err <= ol.w8a16_tolerance(xin, wq, sc)).all()
   ulp_close(hc, ol.silu_mul(ac, bc), 0.999)
+
+
+@pytest.mark.parametrize("kept_levels", [False, True])
+@pytest.mark.parametrize("by", ["torch", "insert"])
+@pytest.mark.parametrize("m,k,n", [(7, 4096, 6144), (96, 1024, 1280), (300, 1024, 1280)])
+def test_weights_written_by_the_kernel_in_front(m, k, n, by, kept_levels):
+  """Two sets of weights by turns, each written on the stream directly in front of the call and used by it: by a torch kernel, or by this
+  package's copy kernel, which lets the next launch start before it writes.  Kept levels: that kernel is directly in front of the GEMM."""
+  from jetstream_pytorch_b200 import _lib, layers
+
+  if kept_levels and m > layers.ActivationLevels.MAX_ROWS:
+    pytest.skip("levels are kept for up to 128 rows")
+  g = torch.Generator(device=DEV).manual_seed(m)
+  sets = [torch.randint(-127, 128, (n, k), generator=g, device=DEV, dtype=torch.int8) for _ in range(2)]
+  x = torch.randn(m, k, generator=g, device=DEV, dtype=torch.bfloat16)
+  lin = layer_for(sets[0].cpu(), torch.rand(n, generator=torch.Generator().manual_seed(1)) * 0.01)
+  levels = layers.ActivationLevels.of(x) if kept_levels else None
+  want = []
+  for w in sets:
+    lin.weight.copy_(w)
+    torch.cuda.synchronize()
+    want.append(lin(x, levels=levels))
+    torch.cuda.synchronize()
+  assert not torch.equal(*want)
+  rows = lambda t: t.reshape(1, 1, -1, 128)
+  spare = torch.empty_like(lin.weight)
+
+  def write(w):
+    if by == "torch":
+      lin.weight.copy_(w)
+    else:
+      assert _lib.native.insert_dense([(rows(w), rows(w))], [(rows(spare), rows(lin.weight))], None, 0, 0, False, False)
+
+  got = []
+  for _ in range(60):
+    for w in sets:
+      write(w)
+      got.append(lin(x, levels=levels))
+  for i, y in enumerate(got):
+    assert torch.equal(y, want[i % 2]), i
