@@ -20,7 +20,7 @@ def _layer(n, k, g):
 
 
 # one row into a second block, row counts that are no multiple of eight, a channel tile with one channel, the shortest K
-@pytest.mark.parametrize("m,k,n", [(129, 128, 256), (130, 384, 257), (257, 640, 100), (1000, 256, 520), (200, 4096, 1280)])
+@pytest.mark.parametrize("m,k,n", [(129, 128, 256), (130, 384, 257), (257, 640, 100), (1000, 256, 520), (200, 4096, 1280), (1000, 128, 5121)])  # (the last: 168 tiles, more than one of some CTAs)
 def test_many_rows_match_the_oracle(m, k, n):
   g = torch.Generator().manual_seed(m + n)
   lin, w, s = _layer(n, k, g)
