@@ -87,14 +87,20 @@ struct PrefillGeom {
 // Row tile t (0: a, 1: b) of item `item` of a KV head: token block index / rep, grouped query head index % rep.  Under a causal mask a
 // tile has as many K/V tiles as blocks up to its own.
 // Folded: the longest with the shortest, the second longest with the second shortest, ..., so that every item has about
-// as much work; for grids of one wave, whose time is that of the longest item (1024 tokens, 32 / 8 heads: 42.6 -> 41.0 us
-// with the mask classes; a step of one tile alone takes nearly as long as one of two).  Else neighbours, the longest
+// as much work; for grids of one wave, whose time is that of the longest item (1024 tokens, 32 / 8 heads: 37.5 -> 35.1 us;
+// a step of one tile alone takes nearly as long as one of two, so two blocks of tokens gain nothing).  Else neighbours, the longest
 // items first, which fill up the end of several waves: items of one length would take whole waves.
+template <bool kFold>
 __device__ __forceinline__ int row_tile(const PrefillGeom& g, int rep, int item, int t, bool* have) {
   const int tiles = g.n_rows_t * rep;
-  const int idx = g.fold ? (t == 0 ? tiles - 1 - item : item) : 2 * (g.pairs - 1 - item) + t;
-  *have = g.fold ? t == 0 || item < tiles - 1 - item : idx < tiles;
-  return idx;
+  if constexpr (kFold) {
+    *have = t == 0 || item < tiles - 1 - item;
+    return t == 0 ? tiles - 1 - item : item;
+  } else {
+    const int idx = 2 * (g.pairs - 1 - item) + t;
+    *have = idx < tiles;
+    return idx;
+  }
 }
 
 __device__ __forceinline__ uint32_t smem_u32p(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -273,8 +279,8 @@ __device__ __forceinline__ bool group_all(int group, bool pred) {
 // ---------------------------------------------------------------- mask classes
 // One CTA per [128 rows x 128 keys] tile of the mask: all zero, all -inf, or mixed.  Reads the mask once (the bound).
 __global__ void __launch_bounds__(256) mask_class_kernel(AttnArgs a, uint8_t* cls, int rows_per_head, int cls_heads, int vec) {
-  grid_dependency_trigger();
   grid_dependency_wait();
+  grid_dependency_trigger();
   const int j = blockIdx.x, tb = blockIdx.y, r = blockIdx.z % cls_heads, b = blockIdx.z / cls_heads;
   const int t0 = tb * kRowsP, s0 = j * kKeysP;
   const int nr = min(kRowsP, rows_per_head - t0), nc = min(kKeysP, a.S - s0);
@@ -412,7 +418,8 @@ __device__ __noinline__ void plain_rows(const AttnArgs& a, const PrefillGeom& g,
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = warp >> 3, half = (warp >> 2) & 1;
   const int rep = a.Hq / a.Hkv, heads = a.B * a.Hkv, bh = (int)blockIdx.x % heads, b = bh / a.Hkv, hkv = bh % a.Hkv;
   bool have;
-  const int idx = row_tile(g, rep, (int)blockIdx.x / heads, t, &have), hq = hkv * rep + idx % rep;
+  const int item = (int)blockIdx.x / heads;
+  const int idx = g.fold ? row_tile<true>(g, rep, item, t, &have) : row_tile<false>(g, rep, item, t, &have), hq = hkv * rep + idx % rep;
   const int token = min(idx / rep * kRowsP + (warp & 3) * 32 + lane, a.Tq - 1);
   // (all tiles of the item are done: the rings are free.  The query rows read once a key from global memory, a line per lane,
   // were most of the time.)
@@ -498,8 +505,9 @@ __device__ __noinline__ void plain_rows(const AttnArgs& a, const PrefillGeom& g,
 }
 
 // ---------------------------------------------------------------- the kernel
-// kRound: dense_attention's logit chain with a bf16 rounding after every step; kScale: per-token K and V scales.
-template <bool kRound, bool kScale>
+// kRound: dense_attention's logit chain with a bf16 rounding after every step; kScale: per-token K and V scales; kFold: see row_tile (in
+// the geometry alone the choice cost short prompts 3 to 5 %: the main path's registers are all in use).
+template <bool kRound, bool kScale, bool kFold>
 __global__ void __launch_bounds__(kThreadsP, 1)
     prefill_attention_kernel(const __grid_constant__ PrefillMaps maps, const __grid_constant__ AttnArgs a,
                              const __grid_constant__ PrefillGeom g, int* status) {
@@ -518,7 +526,7 @@ __global__ void __launch_bounds__(kThreadsP, 1)
   bool have[2];
 #pragma unroll
   for (int t = 0; t < 2; ++t) {
-    const int idx = row_tile(g, rep, (int)blockIdx.x / heads, t, &have[t]);
+    const int idx = row_tile<kFold>(g, rep, (int)blockIdx.x / heads, t, &have[t]);
     tb[t] = idx / rep;
     hq[t] = hkv * rep + idx % rep;
   }
@@ -1020,10 +1028,14 @@ int launch_attention_prefill(const jpt_attn_params& p, const AttnArgs& a, int64_
         auto set = [&e](auto kernel) {
           if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemP));
         };
-        set(prefill_attention_kernel<true, true>);
-        set(prefill_attention_kernel<true, false>);
-        set(prefill_attention_kernel<false, true>);
-        set(prefill_attention_kernel<false, false>);
+        set(prefill_attention_kernel<true, true, false>);
+        set(prefill_attention_kernel<true, true, true>);
+        set(prefill_attention_kernel<true, false, false>);
+        set(prefill_attention_kernel<true, false, true>);
+        set(prefill_attention_kernel<false, true, false>);
+        set(prefill_attention_kernel<false, true, true>);
+        set(prefill_attention_kernel<false, false, false>);
+        set(prefill_attention_kernel<false, false, true>);
         return e;
       }))
     return rc;
@@ -1040,7 +1052,8 @@ int launch_attention_prefill(const jpt_attn_params& p, const AttnArgs& a, int64_
   g.n_rows_t = (p.Tq + kRowsP - 1) / kRowsP;
   g.n_k = t.n_k;
   g.pairs = (g.n_rows_t * (p.Hq / p.Hkv) + 1) / 2;
-  g.fold = g.pairs * p.B * p.Hkv <= sm_count();
+  // (an odd number of blocks without grouped heads: the longest tile is alone in its item either way; 600 tokens, 32 heads 35.5 us, 34.8)
+  g.fold = g.pairs * p.B * p.Hkv <= sm_count() && g.n_rows_t > 2 && (p.Hq > p.Hkv || g.n_rows_t % 2 == 0);
   g.q_b = q_b, g.q_h = q_h, g.q_t = q_t;
   g.mask_vec = p.mask_mode == JPT_MASK_ADD && aligned(p.mask, 16) && p.mk_b % 8 == 0 && p.mk_r % 8 == 0;
   g.mask_pairs = p.mask_mode == JPT_MASK_ADD && aligned(p.mask, 4) && p.mk_b % 2 == 0 && p.mk_r % 2 == 0 && p.Tq * p.mk_r % 2 == 0;
@@ -1048,19 +1061,29 @@ int launch_attention_prefill(const jpt_attn_params& p, const AttnArgs& a, int64_
     uint8_t* cls = reinterpret_cast<uint8_t*>(ws + kWorkspaceCounterBytes);
     g.cls = cls;
     g.cls_rows = t.rows, g.cls_heads = t.heads, g.cls_batch = t.batch;
-    launch_after_previous(mask_class_kernel, dim3(t.n_k, t.rows, t.heads * t.batch), dim3(256), 0, st, a, cls, (int)(p.mk_r ? p.Tq : 1),
-                          (int)t.heads, (int)g.mask_vec);
+    const dim3 tiles(t.n_k, t.rows, t.heads * t.batch), threads(256);
+    const int mask_rows = p.mk_r ? p.Tq : 1;
+    // Read 16 bytes at a time the classes take a few microseconds, and the launch starts under the one in front; its CTAs crowd on
+    // the SMs that that one leaves free, and this much shared memory keeps them to four each (1024 tokens, 32 / 8 heads 35.2 us started behind
+    // it, 34.8 under it, 34.0 kept apart).  Element by element they take several times that, and few SMs cost more than the start
+    // gains (700 tokens: 32 / 8 heads 36.4 us under it, 35.1 behind it; 64 / 8 48.5 and 41.7).
+    if (g.mask_vec)
+      launch_after_previous(mask_class_kernel, tiles, threads, 48 * 1024, st, a, cls, mask_rows, (int)t.heads, 1);
+    else
+      mask_class_kernel<<<tiles, threads, 0, st>>>(a, cls, mask_rows, t.heads, 0);
     if (int rc = check_launch("mask_class_kernel")) return rc;
   }
   const dim3 grid(g.pairs * p.B * p.Hkv), block(kThreadsP);
   const size_t smem = sizeof(SmemP);
   const bool scale = p.k_scale != nullptr;
+  auto launch = [&](auto kernel) { launch_after_previous(kernel, grid, block, smem, st, maps, a, g, status); };
+  auto pick = [&](auto plain, auto folded) { g.fold ? launch(folded) : launch(plain); };
   if (a.round_logits) {
-    if (scale) launch_after_previous(prefill_attention_kernel<true, true>, grid, block, smem, st, maps, a, g, status);
-    else launch_after_previous(prefill_attention_kernel<true, false>, grid, block, smem, st, maps, a, g, status);
+    if (scale) pick(prefill_attention_kernel<true, true, false>, prefill_attention_kernel<true, true, true>);
+    else pick(prefill_attention_kernel<true, false, false>, prefill_attention_kernel<true, false, true>);
   } else {
-    if (scale) launch_after_previous(prefill_attention_kernel<false, true>, grid, block, smem, st, maps, a, g, status);
-    else launch_after_previous(prefill_attention_kernel<false, false>, grid, block, smem, st, maps, a, g, status);
+    if (scale) pick(prefill_attention_kernel<false, true, false>, prefill_attention_kernel<false, true, true>);
+    else pick(prefill_attention_kernel<false, false, false>, prefill_attention_kernel<false, false, true>);
   }
   return check_launch("prefill_attention_kernel");
 }

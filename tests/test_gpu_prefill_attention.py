@@ -65,6 +65,8 @@ def _mask(kind, rep, t, s, g):
     (2, 8, 2, 70, 600, "broadcast", True),    # one mask row for all
     (1, 40, 1, 1, 512, "none", False),        # many grouped heads, one token
     (10, 10, 10, 650, 650, "causal", True),   # more items than SMs, an odd number of row tiles of a head: neighbours share an item
+    (1, 4, 4, 500, 500, "causal", True),      # four blocks of tokens of a head on its own: longest and shortest share an item
+    (1, 3, 1, 300, 300, "causal", True),      # nine row tiles: the middle one is alone
 ])
 @pytest.mark.parametrize("scales", ["none", "ones", "random", "random_f32"])
 def test_dense_attention_matches_the_reference(b, hq, hkv, t, s, kind, transposed, scales):
