@@ -36,6 +36,7 @@ def _lengths(kind, b, s, g):
     ("edges", 26, 64, 8, 512, False),
     ("edges", 130, 8, 2, 512, False),     # a second group of sequences
     ("spread", 257, 4, 1, 256, False),    # more sequences than are sorted
+    ("one long", 3, 8, 1, 16640, False),  # more tiles than are sorted
     ("spread", 33, 32, 32, 640, True),
     ("edges", 13, 16, 8, 520, True),
 ])
@@ -69,3 +70,63 @@ def test_every_token_of_every_segment(kind, b, hq, hkv, s, ring):
     assert (m.reshape(b, hq)[empty] == -math.inf).all() and not l.reshape(b, hq)[empty].any()
     assert torch.allclose(l.reshape(b, hq), den.reshape(b, hq), rtol=1e-3, atol=1e-6)
     assert torch.allclose(m.reshape(b, hq)[~empty], top.reshape(b, hq)[~empty], rtol=1e-3, atol=1e-3)
+
+
+def _copied_in_front(dst, src):
+  """dst = src for int32 [B], by this package's copy kernel: it lets the next launch start before it writes."""
+  from jetstream_pytorch_b200 import _lib
+
+  rows = lambda t: t.view(torch.bfloat16).reshape(1, 1, 1, -1)
+  spare = torch.empty_like(dst)
+  assert _lib.native.insert_dense([(rows(src), rows(src))], [(rows(spare), rows(dst))], None, 0, 0, False, False)
+
+
+@pytest.mark.parametrize("form", ["dense", "ring", "mask", "paged"])
+@pytest.mark.parametrize("b,hq,hkv", [(40, 32, 8), (5, 8, 2), (150, 8, 1)])
+def test_lengths_written_by_the_kernel_in_front(form, b, hq, hkv):
+  """The list is made from the lengths as they are under the kernel in front and made again when that kernel changed them: other numbers of
+  tiles, the same again, none.  Each call's rows equal those of a call whose lengths stood long before, bit for bit."""
+  from jetstream_pytorch_b200 import attention_kernel as ak
+
+  s, d, page = 1024, 128, 64
+  g = torch.Generator(device=DEV).manual_seed(b)
+  q = torch.randn(b, hq, 1, d, generator=g, device=DEV, dtype=torch.bfloat16)
+  ks, vs = (torch.rand(b, 1, s, 1, generator=g, device=DEV).mul_(0.01).add_(0.01).to(torch.bfloat16) for _ in range(2))
+  if form == "paged":
+    k, v = (torch.randint(-127, 128, (hkv, b * s // page, page, d), generator=g, device=DEV, dtype=torch.int8) for _ in range(2))
+    ks, vs = ks.reshape(1, -1, page, 1), vs.reshape(1, -1, page, 1)
+    table = torch.randperm(b * s // page, generator=g, device=DEV).to(torch.int32).reshape(b, -1)
+  else:
+    k, v = (torch.randint(-127, 128, (b, hkv, s, d), generator=g, device=DEV, dtype=torch.int8) for _ in range(2))
+  start = torch.full((b,), s // 3, dtype=torch.int32, device=DEV)
+  mask = torch.empty(b, 1, 1, s, dtype=torch.bfloat16, device=DEV)
+  at = torch.arange(s, device=DEV)
+
+  def call(end):
+    if form == "paged":
+      return ak.call_paged_attention(None, q.squeeze(2), k, v, end, table, k_scaler=ks, v_scaler=vs)
+    if form == "mask":
+      return ak.dense_attention(q, k, v, ks, vs, mask)
+    return ak.ragged_mha(q, k, v, 0, start, end, None, None, ks, vs, ring=form == "ring")[0]
+
+  lens = [torch.randint(1, s + 1, (b,), generator=g, device=DEV, dtype=torch.int32) for _ in range(3)]
+  lens += [lens[2].flip(0), torch.zeros_like(lens[0]) + (1 if form == "mask" else 0), torch.full_like(lens[0], s - 1)]
+  masks = [torch.zeros_like(mask).masked_fill_((at >= n[:, None])[:, None, None, :], -math.inf) for n in lens]
+  want = []
+  for n, m in zip(lens, masks):
+    mask.copy_(m)
+    torch.cuda.synchronize()
+    want.append(call(n))
+    torch.cuda.synchronize()
+  end = torch.empty_like(lens[0])
+  got = []
+  for turn in range(20):
+    for n, m in zip(lens, masks):
+      if form == "mask":
+        mask.copy_(m)
+      else:
+        _copied_in_front(end, n)
+      got.append(call(end))
+  for i, o in enumerate(got):
+    assert torch.equal(o, want[i % len(lens)]), i
+  assert ak.kernel_status() == 0

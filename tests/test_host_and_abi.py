@@ -128,3 +128,12 @@ def test_cuda_only_entry_points_reject_cpu_tensors():
 
   with pytest.raises(ValueError):
     quantize.quantize_tensor(torch.zeros(1, 2, 3, 16, dtype=torch.bfloat16), (-3, -1))
+
+
+def test_zero_refuses_what_it_does_not_take():
+  from jetstream_pytorch_b200 import _lib
+
+  zero = _lib.lib().jpt_zero
+  assert zero(None, 0, None) == 0 and zero(1 << 20, 0, None) == 0  # nothing to do, nothing launched
+  for p, n in ((None, 16), (8, 16), (1 << 20, 8), (1 << 20, 17)):
+    assert zero(p, n, None) < 0, (p, n)
