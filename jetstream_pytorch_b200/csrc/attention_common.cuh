@@ -118,26 +118,21 @@ __device__ __forceinline__ float load_scale(const void* base, int64_t idx, int i
                 : __bfloat162float(static_cast<const __nv_bfloat16*>(base)[idx]);
 }
 
-// Every workspace starts with this many bytes of per-segment arrival counters
-// that must stay zero between launches; no kernel puts anything else there.
-// header: 192 KiB of counters, then the one-GPU exchange area of the fused decode step, then one status
-// word in the last 256 bytes.  Everything whose meaning outlives a launch lives here, at offsets that do
-// not depend on the shape, because one workspace serves calls of any shape (whose partials would
-// otherwise land on another shape's state).
+// Every workspace starts with this header, which must stay zero between launches (but for the status word): 192 KiB of
+// per-segment arrival counters, then the ticket of the work list, one status word in the last 256 bytes.  Everything
+// whose meaning outlives a launch lives here, at offsets that do not depend on the shape, because one workspace serves
+// calls of any shape (whose partials would otherwise land on another shape's state).
 constexpr size_t kWorkspaceCounterBytes = 256 * 1024;
 constexpr size_t kWorkspaceStatusOffset = kWorkspaceCounterBytes - 256;
-constexpr size_t kWorkspaceExchangeOffset = 192 * 1024;
-constexpr size_t kWorkspaceTicketOffset = kWorkspaceExchangeOffset + 32;  // in the exchange state's 64 bytes, which use the first 12
-constexpr size_t kWorkspaceExchangeBytes = kWorkspaceStatusOffset - kWorkspaceExchangeOffset;
-constexpr size_t kWorkspaceMaxSegments = kWorkspaceExchangeOffset / sizeof(unsigned);  // (sequence, head) pairs
+constexpr size_t kWorkspaceTicketOffset = 192 * 1024;
+constexpr size_t kWorkspaceMaxSegments = kWorkspaceTicketOffset / sizeof(unsigned);  // (sequence, head) pairs
 
 // The new token of a decode step, handed to the attention launch itself
 // (jpt_decode_update_attend): quantised with the decode quantiser, written to
 // the cache row and / or the stash outputs, and attended to together with the
 // existing tokens.  The per-token amax over all heads travels through exchange
 // slots: one 64-bit word (launch number << 32 | amax bits) per (K|V, slot) and
-// writer rank, in the buffers of a jpt_peer_exchange or (one GPU) in the
-// workspace.
+// writer rank, in the buffers of a jpt_peer_exchange.  Without one (px_world 0) the CTA that needs the amax takes it itself.
 struct NewTokenArgs {
   const void* x[2];        // xk, xv [B,Hkv,1,D]
   int8_t* quant[2];        // [B,Hkv,1,D] out, may be null

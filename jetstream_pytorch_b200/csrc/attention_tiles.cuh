@@ -364,13 +364,13 @@ inline int configure_once_per_device(std::atomic<bool> (&done)[kMaxDevices], con
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 struct ScratchLayout {
-  size_t counters, seqinfo, exchange, part_m, part_l, part_t, part_o, total;
+  size_t counters, seqinfo, part_m, part_l, part_t, part_o, total;
   int num_ctas;
 };
 
 // Exchange area of one rank for the per-token amax of a decode step: 64 bytes of
 // state {launches done, CTAs done, gave up}, then slots[parity][writer rank][2 B]
-// of 64-bit words.  The same layout serves jpt_peer_exchange buffers.
+// of 64-bit words (the buffers of a jpt_peer_exchange).
 constexpr size_t kExchangeStateBytes = 64;
 inline size_t exchange_bytes(int B, int world) {
   return kExchangeStateBytes + (size_t)2 * world * 2 * B * sizeof(unsigned long long);
@@ -385,7 +385,6 @@ inline ScratchLayout scratch_layout(const jpt_attn_params& p, int num_ctas) {
   off = kWorkspaceCounterBytes;
   s.seqinfo = off;
   off = align_up(off + sizeof(int32_t) * 4 * p.B, 256);
-  s.exchange = kWorkspaceExchangeOffset;  // one-GPU exchange slots of the fused update, inside the header
   s.part_m = off;
   off = align_up(off + sizeof(float) * s.num_ctas * 2 * kMaxRows, 256);
   s.part_l = off;

@@ -101,7 +101,7 @@ struct RoundRec {
   int pos[2];               // position of each tile's first row (paged: token index)
   int parts;                // pieces of the segment; their partial results (unless there is just one):
   int slot, first, stride;  // this piece's slot, and PartSlots of the segment
-  int pad[3];
+  int pad[3];               // (three 16-byte stores)
 };
 constexpr int kRoundValid = 1;                   // without it the CTA is done
 constexpr int kRoundStarts = 2, kRoundEnds = 4;  // first / last round of a piece
@@ -1686,12 +1686,6 @@ int launch_attention_umma(const jpt_attn_params& p, const AttnArgs& a, cudaStrea
   memset(&nt, 0, sizeof(nt));
   if (nt_in) {
     nt = *nt_in;
-    if (nt.px_state == nullptr) {  // one GPU: the exchange slots live in the workspace
-      nt.px_state = reinterpret_cast<unsigned*>(ws + lay.exchange);
-      nt.px_slots[0] = reinterpret_cast<unsigned long long*>(ws + lay.exchange + kExchangeStateBytes);
-      nt.px_rank = 0;
-      nt.px_world = 1;
-    }
     if (nt.px_wait_cycles <= 0) nt.px_wait_cycles = kWaitCycles;
     nt.enabled = 1;
   }

@@ -224,3 +224,21 @@ def test_fused_step_token_in_the_only_or_last_round(hkv, lazy):
     assert attention_close(o, eo), describe(o, eo)
     assert torch.equal(c.cache_v.cpu(), cv if lazy else e[1])
   assert ak.kernel_status() == 0
+
+
+def test_fused_step_of_many_sequences():
+  """More sequences than a GPU has rows of anything: equal shares, no exchange."""
+  from jetstream_pytorch_b200 import attention_kernel as ak
+  from jetstream_pytorch_b200.cache_manager import Int8KVCacheGenerate
+
+  b, hq, hkv, s, d = 2100, 4, 1, 16, 128
+  ck, cv, ks, vs, q, xk, xv, start, end, input_pos = _case(409, b, hq, hkv, s, d, False)
+  env = make_env(batch_size=b, cache_sequence_length=s, ring_buffer=False)
+  dev = lambda x: x.to(DEV)
+  c = Int8KVCacheGenerate(dev(ck).clone(), dev(cv).clone(), dev(ks).clone(), dev(vs).clone(), dev(input_pos), env=env)
+  r, (o, m, l) = c.update_and_attend(dev(q), dev(xk), dev(xv), 0, dev(start), dev(end))
+  e = oc.int8_update(ck, cv, ks, vs, xk, xv, input_pos, ring_buffer=False, lazy=False)
+  assert torch.equal(r[0].cpu(), e[0]) and torch.equal(r[5].cpu(), e[5])
+  eo, (em, el) = oa.ragged_mha(q, e[0], e[1], 0, start, end + 1, e[4], e[5], bk=16)
+  assert attention_close(o, eo), describe(o, eo)
+  assert torch.allclose(l.cpu(), el, atol=1e-3, rtol=1e-3) and ak.kernel_status() == 0
