@@ -10,10 +10,11 @@
 //
 // "Levels" make the small operands 8-bit without losing the precision of the
 // bf16 / fp32 values they stand for:
-//   * a query row q (bf16) is split as q = s (h + l / 254) with s = amax|q| / 127 (values of the row's amax are exact)
-//     and h, l signed bytes; rows 0..7 of Ql hold h, rows 8..15 hold l, so the
-//     two partial dot products of a token arrive in the same TMEM lane and
-//     S = s (S_h + S_l / 254) is exact to 2^-16 of the row's amax;
+//   * a query row q (bf16) is split as q = u (256 h + l) with u a power of two and h, l
+//     signed bytes: exact but for values below 1/127 of the row's largest, which are rounded to
+//     u (2^-14 of it at most); rows 0..7 of Ql hold h, rows 8..15 hold l, so the two partial
+//     dot products of a token arrive in the same TMEM lane and S = u (256 S_h + S_l).  (The
+//     chain of rounded logits keeps q = s (h + l / 254), s = amax|q| / 127.)
 //   * a probability p in [0, 1] (relative to the maximum of its round), times the
 //     token's V scale relative to the largest V scale c of its tile, becomes a
 //     16-bit fixed-point number whose two bytes are the unsigned levels of the
@@ -47,7 +48,7 @@
 // round ahead (the scales' addresses waited 4000 cycles a round for them), a piece's rows leave
 // with the next round's logits, and segments are not cut where they need not be.
 // B200, 96 sequences of 8 KV heads, a step of two layers with these changes and the row's L2 policy: 1 .. 2047 tokens with the
-// new token 129.7 -> 108.2 us; paged, 512 .. 2047 tokens, 131.3 -> 106.3.
+// new token 130.2 -> 107.2 us; paged, 512 .. 2047 tokens, 131.8 -> 108.2.
 //
 // Fused decode update (jpt_decode_update_attend): the launch also takes the
 // step's new K/V token, which becomes the last token of its segment: the
@@ -125,7 +126,7 @@ struct __align__(1024) SmemU {
   int ntpos;                             // ... and where the token is written
   alignas(16) float xch[4][12];          // per warp: row maxima of the round [8], largest V scale of each tile [2]
   float red[4][8];                       // per warp: denominators at the end of a piece
-  alignas(16) float qsc[8];              // s_r * sm_scale * log2(e) / 254
+  alignas(16) float qsc[8];              // u_r * sm_scale * log2(e)
   float qsr[8];                          // s_r / 254 (the chain of rounded logits starts from the plain dot product)
   float ntx[4];                          // new token: K amax, V amax
   uint64_t bar[2];                       // MMA completion: S^T, O^T
@@ -200,7 +201,7 @@ __device__ __forceinline__ void store_levels(uint32_t addr, const uint32_t (&y)[
 }
 // The thread's two tokens: new running maxima, rescale factors, probabilities and denominator shares of its kR rows, and the levels.
 // The probabilities are relative to the round's own maximum, so that every round has all 16 bits (relative to the running maximum, long
-// pieces had 4.0e-5 of their rows' norm, not 3.9e-5, from fixed point): the sums so far are scaled by `alpha`, the round's by `beta`.
+// pieces had 4.1e-5 of their rows' norm, not 4.0e-5): the sums so far are scaled by `alpha`, the round's by `beta`.
 // Adding 2^23 rounds a probability's product to its fixed-point number and leaves that in the low bits of the float.
 // m_run starts at kNoMax (finite), so exp2(old - new) and exp2(-inf - new) need no special case.
 template <int kR>
@@ -1148,21 +1149,38 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
       for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(f[e]));
 #pragma unroll
       for (int sh = 1; sh <= 8; sh <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, sh));
-      const float inv = amax > 0.f ? 127.f / amax : 0.f;
       uint32_t hi[2] = {0u, 0u}, lo[2] = {0u, 0u};
+      float unit;  // of the dot products
+      if constexpr (kRound) {
+        const float inv = amax > 0.f ? 127.f / amax : 0.f;
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const float t = f[e] * inv;
-        const float h = rintf(t);
-        const float l = rintf((t - h) * 254.f);
-        hi[e >> 2] |= ((uint32_t)(int)h & 0xffu) << (8 * (e & 3));
-        lo[e >> 2] |= ((uint32_t)(int)l & 0xffu) << (8 * (e & 3));
+        for (int e = 0; e < 8; ++e) {
+          const float t = f[e] * inv;
+          const float h = rintf(t);
+          const float l = rintf((t - h) * 254.f);
+          hi[e >> 2] |= ((uint32_t)(int)h & 0xffu) << (8 * (e & 3));
+          lo[e >> 2] |= ((uint32_t)(int)l & 0xffu) << (8 * (e & 3));
+        }
+        unit = amax * (1.f / 127.f) * (1.f / 254.f);
+      } else {
+        // 2^(E - 14) for an amax in [2^E, 2^(E + 1)), twice that for the amax of mantissa 255 (its 32640 units would be an h of 128); normal
+        // numbers.  An infinite amax leaves levels of zero and an infinite unit: no logit of the row is a number.
+        const int e2 = max((int)((__float_as_uint(amax) + 0x10000u) >> 23), 27);
+        const bool finite = amax < INFINITY;
+        unit = finite ? __uint_as_float((uint32_t)(e2 - 14) << 23) : INFINITY;
+        const float inv = finite ? __uint_as_float((uint32_t)(268 - e2) << 23) : 0.f;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const int t = __float2int_rn(f[e] * inv);  // (|t| < 32640)
+          hi[e >> 2] |= ((uint32_t)((t + 128) >> 8) & 0xffu) << (8 * (e & 3));
+          lo[e >> 2] |= ((uint32_t)t & 0xffu) << (8 * (e & 3));  // (t - 256 h is -128 .. 127)
+        }
       }
       *reinterpret_cast<uint2*>(&sm.qlev[swz(row, 8 * ch)]) = make_uint2(hi[0], hi[1]);
       *reinterpret_cast<uint2*>(&sm.qlev[swz(8 + row, 8 * ch)]) = make_uint2(lo[0], lo[1]);
       if (ch == 0) {
-        sm.qsc[row] = amax * (1.f / 127.f) * unit2 * (1.f / 254.f);
-        if constexpr (kRound) sm.qsr[row] = amax * (1.f / 127.f) * (1.f / 254.f);
+        if constexpr (kRound) sm.qsr[row] = unit;
+        else sm.qsc[row] = unit * unit2;
       }
       fence_async_smem();
       tc_fence_before();
@@ -1343,7 +1361,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
 #pragma unroll
         for (int r = 0; r < kR; ++r) {
           const float qc = sm.qsc[r];
-          xv[r] = fma2(pack2((float)((int)s0[r] * 254 + (int)s0[8 + r]), (float)((int)s1[r] * 254 + (int)s1[8 + r])), mul2(pack2(qc, qc), ks), ml);
+          xv[r] = fma2(pack2((float)((int)s0[r] * 256 + (int)s0[8 + r]), (float)((int)s1[r] * 256 + (int)s1[8 + r])), mul2(pack2(qc, qc), ks), ml);
         }
       } else {
         // dense_attention on bf16 tensors: the reference rounds the logit to bf16 after every step

@@ -38,3 +38,26 @@ def test_each_tile_is_rounded_against_its_own_largest_value_scale(even, odd):
   deviation = ((largest**2).sum(1) * codes.double().pow(2).mean() / 12).sqrt() / 65535 / (lens + 1)
   measured = (err / deviation[:, None]).pow(2).mean().sqrt()
   assert measured < 1.2, float(measured)
+
+
+@pytest.mark.parametrize("hq", [1, 4, 8])
+def test_dot_products_of_queries_within_a_factor_of_127_are_exact(hq):
+  """The unrounded logits of one-token sequences, read from the row maximum: the integer sums are exact, what is left is the conversion and six
+  float32 products (2^-24 each).  Rows whose largest value has the mantissa 255, 254 or 128, and scales over the range of bf16."""
+  from jetstream_pytorch_b200 import _lib
+  from jetstream_pytorch_b200 import attention_kernel as ak
+
+  g = torch.Generator().manual_seed(hq)
+  b, d = 96, 128
+  q = torch.randn(b, hq, 1, d, generator=g).to(torch.bfloat16)
+  q[0::4, :, :, 7], q[1::4, :, :, 7], q[2::4, :, :, 7] = 255 / 64, -254 / 64, 4.0  # (with mantissas 255, 254, 128: the largest of nearly all rows)
+  q = torch.where(q.abs() * 127 < q.abs().amax(-1, keepdim=True), torch.zeros_like(q), q)
+  q = (q.double() * 2.0 ** torch.linspace(-90, 60, b).round()[:, None, None, None]).to(torch.bfloat16)
+  k = torch.randint(-127, 128, (b, 1, 1, d), generator=g, dtype=torch.int8)
+  ks = (torch.rand(b, 1, 1, 1, generator=g) + 0.5).to(torch.bfloat16)
+  _, m, _ = ak._flash_decode(q.to(DEV), k.to(DEV), k.to(DEV), k_scale=ks.to(DEV), v_scale=ks.to(DEV), scale_strides=(1, 1),
+                             mask_mode=_lib.MASK_LENGTH, end=torch.ones(b, dtype=torch.int32), sm_scale=d**-0.5, kv_strides=(d, d, d),
+                             n_kv_heads=1, seq=1)
+  want = (q.double() * k.double()).sum(-1).reshape(b, hq) * ks.double().reshape(b, 1) * d**-0.5
+  err = (m.reshape(b, hq).double().cpu() - want).abs()
+  assert (err <= 7 * 2.0**-24 * want.abs()).all(), float((err / want.abs()).max())
