@@ -122,8 +122,9 @@ __device__ __forceinline__ uint64_t desc_k_major_128b(uint32_t addr) {
 }
 // The box: a number of 128-byte steps of K from step `z` on, each a swizzled tile of rows from `y` on.  (A CTA of a pair: the bytes
 // land in this CTA, the barrier `bar`, a shared::cluster address, may be the other one's.)
-// `policy`: how long its lines stay in L2.  Weights of more than half of L2 leave first: the next call finds none of them there in any case, and
-// the activation levels that all CTAs read stay (block 8192 / 28672 with 96 rows: 191.2 -> 185.3 us).  Smaller ones stay for the next call.
+// `policy`: how long its lines stay in L2.  Weights of more than half of L2 leave first: even a program that calls one layer over and over
+// finds little of them there, and the activation levels that all CTAs read stay (hint on and off in turn: block 8192 / 28672 with 96
+// rows 169.2 -> 164.8 us, 5120 / 13824 with 1 row 58.3 -> 55.8).  Smaller ones keep the usual policy.
 __device__ __forceinline__ uint64_t l2_policy(bool once) {
   uint64_t first, normal;
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(first));
